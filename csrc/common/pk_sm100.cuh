@@ -70,6 +70,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// The same for a warp whose wait is usually over when it begins: one poll by all lanes, then lane 0.
+__device__ __forceinline__ bool mbar_wait_uniform(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status, uint32_t code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp(bar, parity, abort_flag, status, code);
+}
+
 // Generic-proxy writes to shared memory become visible to the async proxy (TMA, tcgen05).
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -29,6 +29,8 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     src/components/gguf/quantized_ops.py:9-76)."""
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
+    if M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name):
+        return _umma_linear(x.contiguous(), w_raw, type_name, N, gamma, eps, epi)
     if M >= TENSOR_CORE_MIN_ROWS and K % 64 == 0 and (epi != 1 or (N // 2) % 128 == 0):
         from . import gemm_bf16, rmsnorm, EPI_BF16, EPI_SWIGLU, EPI_F32
         w = _dequant_scratch(w_raw, type_name, N, K)
@@ -44,6 +46,103 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
                                            c_int(_sm_count()), _stream())
         _check(st, "pk_gguf_linear")
     return y
+
+
+# Block types whose integer part fits fp16: decoded inside the tensor-core kernel (`csrc/kernels/quant_umma.cu`)
+UMMA_TYPES = frozenset({"iq2_xxs", "q4_k", "q5_k"})
+UMMA_MAX_ROWS = 129
+# Up to 64 routes the kernels with one block set per route leave no SM idle: 8 routes of the MiniMax-M2 shape take 50 + 32 us there and
+# 47 + 28 and two stagings of 3.5 us here; 184 routes 1233 + 628 and 390 + 207 us.
+UMMA_MIN_ROUTES = 64
+UMMA_MAX_GROUPS = 512
+_status: dict = {}
+
+
+def _umma_takes(w_raw: torch.Tensor, type_name: str, groups: int = 1) -> bool:
+    # whole words: the kernel copies IQ2 blocks by four bytes
+    return type_name in UMMA_TYPES and w_raw.data_ptr() % 16 == 0 and w_raw.numel() % (4 * groups) == 0 and w_raw.numel() // groups < 1 << 32
+
+
+def _umma_status(dev) -> torch.Tensor:
+    """Error word of the bounded waits."""
+    if dev.index not in _status:
+        _status[dev.index] = torch.zeros(1, device=dev, dtype=torch.int32)
+    return _status[dev.index]
+
+
+class _Staged:
+    """Token rows for the tensor-core kernel and the work space of one product, in one allocation."""
+
+    def __init__(self, x: torch.Tensor, type_name: str, rows: int, terms: int, *, index=None, gamma=None, eps: float = 0.0, counters: int = 0,
+                 ws_floats: int = 0):
+        K = x.shape[1]
+        pitch = _lib.kernels().pk_quant_stage_pitch(c_int(DEVICE_TYPE[type_name]), c_int(K))
+        sizes = (rows * terms * pitch * 2, rows * 4, counters * 4, ws_floats * 4)
+        offs, at = [], 0
+        for n in sizes:
+            offs.append(at)
+            at += -(-n // 256) * 256
+        self.buf = torch.empty(at, device=x.device, dtype=torch.uint8)
+        self.rows, self.terms = rows, terms
+        p = self.buf.data_ptr()
+        self.data, self.scale, self.counters, self.ws = (c_void_p(p + o) for o in offs)
+        _check(_lib.kernels().pk_quant_stage_rows(_ptr(x), c_int(int(x.dtype == torch.float32)), c_int(x.stride(0)), c_int(K), _ptr(index), c_int(rows),
+                                                 _ptr(gamma), c_float(eps), c_int(0), c_void_p(0), c_void_p(0), c_void_p(0), c_int(DEVICE_TYPE[type_name]), c_int(terms), self.data, self.scale,
+                                                 self.counters, c_int(counters), _stream()), "pk_quant_stage_rows")
+
+
+def _umma(st: _Staged, w_raw: torch.Tensor, type_name: str, N: int, K: int, seg, groups: int, epi: int, out: torch.Tensor, limit: float, columns: int,
+          splits: int) -> None:
+    _check(_lib.kernels().pk_quant_rows(_ptr(w_raw), c_int(DEVICE_TYPE[type_name]), c_int(N), c_int(K), _ptr(seg), c_int(groups), c_int(st.rows), st.data,
+                                       st.scale, c_int(st.terms), c_int(epi), _ptr(out), c_int(out.stride(0)), c_void_p(0), c_float(limit), c_int(columns),
+                                       c_int(splits), st.ws, st.counters, _ptr(_umma_status(out.device)), c_void_p(0), c_int(0), c_int(_sm_count()), _stream()), "pk_quant_rows")
+
+
+def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, gamma, eps: float, epi: int) -> torch.Tensor:
+    M, K = x.shape
+    columns = 16 if M <= 16 else 32 if M <= 32 else 64
+    tiles = (-(-(N // 2) // 64) if epi == 1 else -(-N // 128)) * -(-M // columns)
+    # parts of K until every resident CTA has work; two 256-weight blocks at least in a part
+    splits = max(1, min(K // 512, _sm_count() * (1 if columns == 64 else 2) // tiles))
+    st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
+    y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
+    _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits)
+    return y
+
+
+def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, inter: int, routes: "Routes", limit: float,
+                  expert_offset: int, local: int, terms: int) -> torch.Tensor:
+    """fp32 [R, H]: every route's expert output, without its weight. `terms`: fp16 terms that a hidden value is multiplied as."""
+    seg, tok, _ = routes
+    H, R, dev = x.shape[1], tok.numel(), x.device
+    seg = seg[expert_offset:]
+
+    def columns(t: int) -> int:      # of an expert's tile: what most experts with routes need
+        n = t * R / local
+        return 16 if n <= 10 else 32 if n <= 24 else 64
+
+    h = torch.empty(R, inter, device=dev, dtype=torch.float32)
+    y = torch.empty(R, H, device=dev, dtype=torch.float32)
+    st = _Staged(x, type13, R, 1, index=tok)
+    _umma(st, w13_raw, type13, 2 * inter, H, seg, local, 3, h, limit, columns(1), 1)
+    st2 = _Staged(h, type2, R, terms)
+    _umma(st2, w2_raw, type2, H, inter, seg, local, 2, y, 0.0, columns(terms), 1)
+    return y
+
+
+def _umma_experts_take(w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, H: int, inter: int, local: int) -> bool:
+    return (_umma_takes(w13_raw, type13, local) and _umma_takes(w2_raw, type2, local) and H % 256 == 0 and inter % 256 == 0 and max(H, inter) * 4 <= 200 * 1024
+            and local <= UMMA_MAX_GROUPS)
+
+
+def _reduce_routes(y: torch.Tensor, routes: "Routes", shape, expert_offset: int, local: int, out: torch.Tensor) -> torch.Tensor:
+    """out[t] += sum over the token's local routes, in route order, of weight * y[route]."""
+    seg, tok, rw = routes
+    T, H = shape
+    pos = torch.empty(tok.numel(), device=y.device, dtype=torch.int32)
+    _check(_lib.kernels().pk_moe_reduce_routes(_ptr(y), _ptr(rw), _ptr(routes.src), _ptr(seg), c_int(T), c_int(routes.topk), c_int(H),
+                                               c_int(expert_offset), c_int(local), _ptr(pos), _ptr(out), _stream()), "pk_moe_reduce_routes")
+    return out
 
 
 TENSOR_CORE_MIN_ROWS = 32
@@ -111,6 +210,10 @@ def gguf_moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tenso
     local = E if local_experts is None else local_experts
     if out is None:
         out = torch.zeros(T, H, device=x.device, dtype=torch.float32)
+    if routes is not None and R > UMMA_MIN_ROUTES and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
+        # hidden values in two fp16 terms: as good as the fp32 values of the kernels that decode in registers
+        y = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, limit, expert_offset, local, 2)
+        return _reduce_routes(y, routes, x.shape, expert_offset, local, out)
     hbuf = torch.empty(R, inter, device=x.device, dtype=torch.float32)
     if routes is not None:
         ybuf = torch.empty(R, H, device=x.device, dtype=torch.float32)
@@ -150,41 +253,43 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     dev = x.device
     if out is None:
         out = torch.zeros(T, H, device=dev, dtype=torch.float32)
-    key = (dev.index, local, H, inter)
-    sc = _GROUPED_SCRATCH.get(key)
-    if sc is None:
-        sc = (torch.empty(local * 2 * inter, H, device=dev, dtype=torch.bfloat16), torch.empty(local * H, inter, device=dev, dtype=torch.bfloat16))
-        _GROUPED_SCRATCH.clear()          # one shape at a time: the scratch is as large as the layer's experts in bf16
-        _GROUPED_SCRATCH[key] = sc
-    w13, w2 = sc
     K = _lib.kernels()
-    _check(K.pk_gguf_dequant_rows(_ptr(w13_raw), c_int(DEVICE_TYPE[type13]), c_void_p(0), c_int(local * 2 * inter), c_int(H), c_int(0),
-                                  c_int(local * 2 * inter), _ptr(w13), _stream()), "pk_gguf_dequant_rows(w13)")
-    _check(K.pk_gguf_dequant_rows(_ptr(w2_raw), c_int(DEVICE_TYPE[type2]), c_void_p(0), c_int(local * H), c_int(inter), c_int(0), c_int(local * H),
-                                  _ptr(w2), _stream()), "pk_gguf_dequant_rows(w2)")
-    xg = x.index_select(0, tok.long())                                   # [R, H] rows in expert order
-    hbuf = torch.empty(R, inter, device=dev, dtype=torch.bfloat16)
-    ybuf = torch.empty(R, H, device=dev, dtype=torch.float32)
-    status = torch.zeros(1, device=dev, dtype=torch.int32)
-    segl = seg[expert_offset:]
-    _check(K.pk_gemm_bf16_grouped(_ptr(xg), c_int(H), _ptr(w13), _ptr(segl), c_int(local), c_int(R), c_int(2 * inter), c_int(H), c_int(EPI_SWIGLU),
-                                  _ptr(hbuf), c_int(inter), _ptr(status), c_int(_sm_count()), _stream()), "pk_gemm_bf16_grouped(w13)")
-    _check(K.pk_gemm_bf16_grouped(_ptr(hbuf), c_int(inter), _ptr(w2), _ptr(segl), c_int(local), c_int(R), c_int(H), c_int(inter), c_int(EPI_F32),
-                                  _ptr(ybuf), c_int(H), _ptr(status), c_int(_sm_count()), _stream()), "pk_gemm_bf16_grouped(w2)")
-    pos = torch.empty(R, device=dev, dtype=torch.int32)
+    if R <= UMMA_MAX_ROUTES_PER_EXPERT * local and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
+        ybuf = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, 0.0, expert_offset, local, 1)
+    else:
+        key = (dev.index, local, H, inter)
+        sc = _GROUPED_SCRATCH.get(key)
+        if sc is None:
+            sc = (torch.empty(local * 2 * inter, H, device=dev, dtype=torch.bfloat16), torch.empty(local * H, inter, device=dev, dtype=torch.bfloat16))
+            _GROUPED_SCRATCH.clear()          # one shape at a time: the scratch is as large as the layer's experts in bf16
+            _GROUPED_SCRATCH[key] = sc
+        w13, w2 = sc
+        _check(K.pk_gguf_dequant_rows(_ptr(w13_raw), c_int(DEVICE_TYPE[type13]), c_void_p(0), c_int(local * 2 * inter), c_int(H), c_int(0),
+                                      c_int(local * 2 * inter), _ptr(w13), _stream()), "pk_gguf_dequant_rows(w13)")
+        _check(K.pk_gguf_dequant_rows(_ptr(w2_raw), c_int(DEVICE_TYPE[type2]), c_void_p(0), c_int(local * H), c_int(inter), c_int(0), c_int(local * H),
+                                      _ptr(w2), _stream()), "pk_gguf_dequant_rows(w2)")
+        xg = x.index_select(0, tok.long())                                   # [R, H] rows in expert order
+        hbuf = torch.empty(R, inter, device=dev, dtype=torch.bfloat16)
+        ybuf = torch.empty(R, H, device=dev, dtype=torch.float32)
+        status = torch.zeros(1, device=dev, dtype=torch.int32)
+        segl = seg[expert_offset:]
+        _check(K.pk_gemm_bf16_grouped(_ptr(xg), c_int(H), _ptr(w13), _ptr(segl), c_int(local), c_int(R), c_int(2 * inter), c_int(H), c_int(EPI_SWIGLU),
+                                      _ptr(hbuf), c_int(inter), _ptr(status), c_int(_sm_count()), _stream()), "pk_gemm_bf16_grouped(w13)")
+        _check(K.pk_gemm_bf16_grouped(_ptr(hbuf), c_int(inter), _ptr(w2), _ptr(segl), c_int(local), c_int(R), c_int(H), c_int(inter), c_int(EPI_F32),
+                                      _ptr(ybuf), c_int(H), _ptr(status), c_int(_sm_count()), _stream()), "pk_gemm_bf16_grouped(w2)")
     routes.combined = False
     if peer is not None and T * H <= peer.capacity:
+        pos = torch.empty(R, device=dev, dtype=torch.int32)
         # several ranks: the per-token reduce is the producer of the combine kernel, which stores this rank's sums into every
         # rank's arena, signals, waits (bounded) and adds the ranks' slots: `out` is the sum over all ranks' experts
         _check(K.pk_invert_routes(_ptr(routes.src), c_int(R), _ptr(pos), _stream()), "pk_invert_routes")
         peer.moe_combine(ybuf, rw, pos, seg, expert_offset, local, T, routes.topk, out)
         routes.combined = True
         return out
-    _check(K.pk_moe_reduce_routes(_ptr(ybuf), _ptr(rw), _ptr(routes.src), _ptr(seg), c_int(T), c_int(routes.topk), c_int(H), c_int(expert_offset),
-                                  c_int(local), _ptr(pos), _ptr(out), _stream()), "pk_moe_reduce_routes")
-    return out
+    return _reduce_routes(ybuf, routes, x.shape, expert_offset, local, out)
 
 
+UMMA_MAX_ROUTES_PER_EXPERT = 256      # above this a decode per 64 routes costs more than one decode to a bf16 scratch
 GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local expert costs more than the route kernels' per-route decode
 
 

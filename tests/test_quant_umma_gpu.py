@@ -1,0 +1,94 @@
+"""Raw GGUF blocks through the tensor cores (`csrc/kernels/quant_umma.cu`) against the dequantised weights in 64 bits: edges of the
+row and column tiles, one and many blocks, parts of K, ragged and empty groups."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _raw(name, rows, K, seed):
+    from pocketllm_b200.formats import gguf_quants as gq
+    w = (np.random.default_rng(seed).standard_normal((rows, K)) * 0.02).astype(np.float32)
+    blocks = gq.quantize(w, name)
+    return torch.from_numpy(blocks).cuda().view(-1), torch.from_numpy(gq.dequantize(blocks, name).reshape(rows, K)).cuda().double()
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+# products are exact and sums fp32 (a few hundred terms to a block, a few blocks): 2^-24 * sqrt(K) / 2 at most, 1e-6 at K = 3072
+TOL = 1e-6
+
+
+@pytest.mark.parametrize("name", ["iq2_xxs", "q4_k", "q5_k"])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (1, 300, 3072), (5, 64, 768), (16, 129, 1536), (17, 256, 512), (33, 130, 1280), (64, 2, 2304), (65, 384, 1024), (128, 200, 256)])
+def test_linear(name, M, N, K):
+    from pocketllm_b200.ops import gguf_ops as go
+    raw, w = _raw(name, N, K, M + N)
+    g = torch.Generator("cuda").manual_seed(K)
+    x = torch.randn(M, K, device="cuda", generator=g) * torch.logspace(-4, 4, M, device="cuda")[:, None]
+    x = x.to(torch.bfloat16)
+    assert _rel(go.gguf_linear(x, raw, name, N, epi=2), x.double() @ w.T) < TOL
+    gamma = 1 + 0.1 * torch.randn(K, device="cuda", generator=g)
+    n = (x.float() * torch.rsqrt((x.float() ** 2).mean(-1, keepdim=True) + 1e-6) * gamma).to(torch.bfloat16).double()
+    # a norm that rounds to the other side of a bf16 tie: a part of the values by 2^-8 at most
+    assert _rel(go.gguf_linear(x, raw, name, N, gamma=gamma, epi=2), n @ w.T) < 2e-4
+    assert _rel(go.gguf_linear(x, raw, name, N), x.double() @ w.T) < 2 ** -8
+    if N % 2 == 0:
+        z = x[:, :].double() / x.double().norm(dim=1, keepdim=True) * 30
+        xs = z.to(torch.bfloat16)
+        a, b = (xs.double() @ w.T).chunk(2, -1)
+        assert _rel(go.gguf_linear(xs, raw, name, N, epi=1), torch.nn.functional.silu(a) * b) < 2 ** -8
+
+
+def test_linear_rows_of_zeros_and_infinities():
+    from pocketllm_b200.ops import gguf_ops as go
+    raw, w = _raw("q5_k", 256, 512, 0)
+    x = torch.randn(4, 512, device="cuda").to(torch.bfloat16)
+    x[1] = 0
+    x[2, 7] = float("inf")
+    x[3] *= 2.0 ** 100
+    y = go.gguf_linear(x, raw, "q5_k", 256, epi=2)
+    assert (y[1] == 0).all() and not torch.isfinite(y[2]).any()
+    assert _rel(y[0], x[0].double() @ w.T) < TOL and _rel(y[3], x[3].double() @ w.T) < TOL
+
+
+@pytest.mark.parametrize("t13,t2", [("iq2_xxs", "iq2_xxs"), ("q4_k", "iq2_xxs"), ("iq2_xxs", "q5_k")])
+@pytest.mark.parametrize("T,E,topk,limit", [(17, 40, 4, 0.0), (33, 40, 3, 0.0), (90, 8, 2, 0.5), (300, 5, 2, 0.0)])
+def test_experts(t13, t2, T, E, topk, limit):
+    from pocketllm_b200.ops import gguf_ops as go
+    H, I = 512, 256 + 512 * (T % 2)
+    raw13, w13 = _raw(t13, E * 2 * I, H, 1)
+    raw2, w2 = _raw(t2, E * H, I, 2)
+    w13, w2 = w13.view(E, 2 * I, H), w2.view(E, H, I)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+    # the last expert gets nothing, the first one more than the others
+    ids = torch.stack([torch.randperm(E - 1, generator=g)[:topk] for _ in range(T)]).int()
+    ids[::2, 0] = torch.where((ids[::2, 1:] == 0).any(-1), ids[::2, 0], torch.zeros_like(ids[::2, 0]))
+    weight = torch.rand(T, topk, generator=g)
+    ids, weight = ids.cuda(), weight.cuda()
+    routes = go.group_routes(ids, weight, E)
+
+    def exact(lo, hi):
+        y = torch.zeros(T, H, device="cuda", dtype=torch.float64)
+        for e in range(lo, hi):
+            t, j = (ids == e).nonzero(as_tuple=True)
+            a, b = (x[t].double() @ w13[e].T).chunk(2, -1)
+            if limit:
+                a, b = a.clamp(max=limit), b.clamp(-limit, limit)
+            y.index_add_(0, t, weight[t, j, None].double() * ((torch.nn.functional.silu(a) * b) @ w2[e].T))
+        return y
+
+    run = lambda **k: go.gguf_moe_forward(x, k.pop("a", raw13), k.pop("b", raw2), t13, t2, E, I, *routes, limit=limit, routes=routes, **k)
+    # fp32 sums and the exponential of a SiLU; hidden values in two fp16 terms (2^-22)
+    want = exact(0, E)
+    assert _rel(run(), want) < 2e-6
+    half = E // 2
+    n13, n2 = raw13.numel() // E * half, raw2.numel() // E * half
+    assert _rel(run(a=raw13[:n13], b=raw2[:n2], local_experts=half), exact(0, half)) < 2e-6
+    assert _rel(run(a=raw13[n13:].clone(), b=raw2[n2:].clone(), expert_offset=half, local_experts=E - half), exact(half, E)) < 2e-6
+    if not limit:       # hidden values in one fp16 term
+        assert _rel(go.gguf_moe_forward_grouped(x, raw13, raw2, t13, t2, E, I, routes), want) < 5e-4
