@@ -526,6 +526,68 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
   }
 }
 
+// The same for many tokens: a block has 16 tokens x 64 experts, four groups of 128 threads take a quarter of the K steps each and
+// add up in their order; a thread has 2 x 4 sums, four values of K at a time (shared-memory reads and multiply-adds then take about
+// as long). 256 tokens of 3072 by 256 experts: 76 -> 60 us, 1500 tokens: 365 -> 174 us (the form above reads the router's rows once
+// per 8 tokens).
+constexpr int kRt = 16, kRe = 64, kRk = 32;
+__global__ void __launch_bounds__(512) router_logits_tile_kernel(const bf16* __restrict__ x, const float* __restrict__ rw, int H, int E, int T, float* logits) {
+  __shared__ __align__(16) float ws[4][kRe][kRk + 4];
+  __shared__ __align__(16) float xs[4][kRt][kRk + 4];
+  const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, tx = t & 15, ty = t >> 4;      // experts tx + 16 j, tokens 2 ty ..
+  const int t0 = blockIdx.y * kRt, e0 = blockIdx.x * kRe;
+  float acc[2][4] = {};
+  const int steps = (H + kRk - 1) / kRk;
+  float wn[16], xn[4];      // the next step's share of the tiles, on its way while this one is multiplied
+  auto fetch = [&](int s) {
+    const int k = s * kRk + (t & 31);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int r = e0 + (t >> 5) + 4 * i;
+      wn[i] = s < steps && r < E && k < H ? __ldg(rw + (size_t)r * H + k) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = t0 + (t >> 5) + 4 * i;
+      xn[i] = s < steps && r < T && k < H ? __bfloat162float(x[(size_t)r * H + k]) : 0.f;
+    }
+  };
+  fetch(grp);
+  for (int s = grp; s - grp < steps; s += 4) {      // every group takes part in the barriers
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) ws[grp][(t >> 5) + 4 * i][t & 31] = wn[i];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xs[grp][(t >> 5) + 4 * i][t & 31] = xn[i];
+    fetch(s + 4);
+    __syncthreads();
+    if (s < steps) {
+#pragma unroll
+      for (int k = 0; k < kRk; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&xs[grp][ty * 2][k]), b = *reinterpret_cast<const float4*>(&xs[grp][ty * 2 + 1][k]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 w = *reinterpret_cast<const float4*>(&ws[grp][tx + 16 * j][k]);
+          acc[0][j] = fmaf(w.w, a.w, fmaf(w.z, a.z, fmaf(w.y, a.y, fmaf(w.x, a.x, acc[0][j]))));
+          acc[1][j] = fmaf(w.w, b.w, fmaf(w.z, b.z, fmaf(w.y, b.y, fmaf(w.x, b.x, acc[1][j]))));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  float* sums = &ws[0][0][0];      // [4][kRt][kRe]
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sums[(grp * kRt + ty * 2 + i) * kRe + tx + 16 * j] = acc[i][j];
+  __syncthreads();
+  for (int o = threadIdx.x; o < kRt * kRe; o += 512) {
+    const int r = o / kRe, e = o - r * kRe;
+    if (t0 + r < T && e0 + e < E)
+      logits[(size_t)(t0 + r) * E + e0 + e] = (sums[o] + sums[kRt * kRe + o]) + (sums[2 * kRt * kRe + o] + sums[3 * kRt * kRe + o]);
+  }
+}
+
 // One block per token: scores from the logits, top-k with lowest-id tie break.
 // score_func 0 softmax, 1 sigmoid, 2 sqrt(softplus); selection on score + bias.
 __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, const float* bias, int E,
@@ -588,47 +650,74 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, c
   }
 }
 
-// Group routes by expert (single block; T * topk routes): counts, exclusive scan, fill in
-// token order so that the layout is deterministic.
-__global__ void __launch_bounds__(256) group_routes_kernel(const int* ids, const float* weights, int T, int topk, int E,
-                                                           int* seg_start, int* route_token, float* route_weight,
-                                                           int* route_src) {
-  extern __shared__ int cnt[];  // [E + 1]
-  const int tid = threadIdx.x, R = T * topk;
-  for (int e = tid; e <= E; e += 256) cnt[e] = 0;
+// Group routes by expert, those of an expert in increasing route index (one block). Every warp counts a contiguous share of the
+// routes in counters of its own, the counts become offsets (warp by warp within an expert, expert by expert), and the warps walk
+// their shares again: 32 routes at a time, a route's place among them from a match of the expert ids. The first form scanned all
+// routes once per expert: 122 us for 2048 routes and 720 us for 12000 over 256 experts, against 9 and 26 us.
+__global__ void __launch_bounds__(1024) group_routes_kernel(const int* ids, const float* weights, int T, int topk, int E,
+                                                            int* seg_start, int* route_token, float* route_weight,
+                                                            int* route_src) {
+  extern __shared__ int cnt[];  // [warps][E]
+  __shared__ int part[33];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5, R = T * topk;
+  const int share = ((R + warps - 1) / warps + 31) & ~31, r0 = min(warp * share, R), r1 = min(r0 + share, R);
+  for (int e = tid; e < warps * E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int r = tid; r < R; r += 256) {
+  int* mine = cnt + warp * E;
+  for (int r = r0 + lane; r < r1; r += 32) {
+    const int e = ids[r];
+    if ((unsigned)e < (unsigned)E) atomicAdd(&mine[e], 1);
 #if PK_DEBUG_BUILD
-    if (ids[r] < 0 || ids[r] >= E) {
-      PK_DEBUG_RECORD(102, ids[r], E);
-      continue;
-    }
+    else PK_DEBUG_RECORD(102, e, E);
 #endif
-    atomicAdd(&cnt[ids[r]], 1);
   }
   __syncthreads();
-  if (tid == 0) {
-    int run = 0;
-    for (int e = 0; e < E; ++e) {
-      const int c = cnt[e];
-      cnt[e] = run;
-      seg_start[e] = run;
-      run += c;
-    }
-    cnt[E] = run;
-    seg_start[E] = run;
-  }
-  __syncthreads();
-  // deterministic fill: expert e's routes in increasing route index
-  for (int e = tid; e < E; e += 256) {
-    int pos = cnt[e];
-    for (int r = 0; r < R; ++r)
-      if (ids[r] == e) {
-        route_token[pos] = r / topk;
-        route_weight[pos] = weights[r];
-        if (route_src) route_src[pos] = r;
-        ++pos;
+  // counts of a block of experts -> offsets; `run` routes before the block
+  int run = 0;
+  for (int e0 = 0; e0 < E; e0 += blockDim.x) {
+    const int e = e0 + tid;
+    int n = 0;
+    if (e < E)
+      for (int w = 0; w < warps; ++w) {
+        const int c = cnt[w * E + e];
+        cnt[w * E + e] = n;
+        n += c;
       }
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) part[warp] = inc;
+    __syncthreads();
+    int before = run;
+    for (int w = 0; w < warp; ++w) before += part[w];
+    int total = 0;
+    for (int w = 0; w < warps; ++w) total += part[w];
+    if (e < E) {
+      const int start = before + inc - n;
+      seg_start[e] = start;
+      for (int w = 0; w < warps; ++w) cnt[w * E + e] += start;
+    }
+    run += total;
+    __syncthreads();
+  }
+  if (tid == 0) seg_start[E] = run;
+  for (int base = r0; base < r1; base += 32) {
+    const int r = base + lane, e = r < r1 ? ids[r] : -1;
+    const bool ok = (unsigned)e < (unsigned)E;
+    const unsigned same = __match_any_sync(0xffffffffu, ok ? e : -1);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    const int pos = ok ? mine[e] + rank : 0;
+    __syncwarp();
+    if (ok) {
+      if (rank == 0) mine[e] += __popc(same);
+      route_token[pos] = r / topk;
+      route_weight[pos] = weights[r];
+      if (route_src) route_src[pos] = r;
+    }
+    __syncwarp();
   }
 }
 
@@ -735,6 +824,9 @@ static float* router_scratch(size_t floats) {
   return buf[dev];
 }
 
+// From 128 tokens the tiles of 16 tokens fill the SMs; with fewer the form of one warp per expert has more blocks.
+static constexpr int kRouterTileMin = 128;
+
 PK_API int pk_router_topk(const void* x, const float* router_w, const float* bias, int T, int H, int E, int topk,
                           int score_func, int norm_topk, float route_scale, int* ids, float* weights,
                           cudaStream_t stream) {
@@ -754,7 +846,10 @@ PK_API int pk_router_topk(const void* x, const float* router_w, const float* bia
   }
   float* logits = router_scratch((size_t)T * E);
   if (logits == nullptr) return PK_ERR_CUDA;
-  router_logits_kernel<<<dim3((E + 7) / 8, (T + 7) / 8), 256, smem_x, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);
+  if (T >= kRouterTileMin)
+    router_logits_tile_kernel<<<dim3((E + kRe - 1) / kRe, (T + kRt - 1) / kRt), 512, 0, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);
+  else
+    router_logits_kernel<<<dim3((E + 7) / 8, (T + 7) / 8), 256, smem_x, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);
   PK_CHECK_LAUNCH();
   router_topk_kernel<<<T, 256, (size_t)2 * E * sizeof(float), stream>>>(logits, bias, E, topk, score_func, norm_topk, route_scale, ids,
                                                                         weights);
@@ -765,8 +860,21 @@ PK_API int pk_router_topk(const void* x, const float* router_w, const float* bia
 PK_API int pk_group_routes(const int* ids, const float* weights, int T, int topk, int E, int* seg_start, int* route_token,
                            float* route_weight, int* route_src, cudaStream_t stream) {
   if (E + 1 > 12000) return PK_ERR_UNSUPPORTED;
-  group_routes_kernel<<<1, 256, (size_t)(E + 1) * sizeof(int), stream>>>(ids, weights, T, topk, E, seg_start, route_token,
-                                                                         route_weight, route_src);
+  const int R = T * topk;
+  int warps = min(32, max(1, (R + 31) / 32));
+  while (warps > 4 && (size_t)warps * E * sizeof(int) > 192 * 1024) warps >>= 1;
+  const size_t smem = (size_t)warps * E * sizeof(int);
+  if (smem > 48 * 1024) {
+    static PkDeviceOnce once;
+    if (PkDeviceOnceGuard once_guard{once}; once_guard.needed()) {
+      if (cudaFuncSetAttribute(group_routes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024) != cudaSuccess) {
+        pk_set_last_cuda_error((int)cudaGetLastError());
+        return PK_ERR_CUDA;
+      }
+      once_guard.done();
+    }
+  }
+  group_routes_kernel<<<1, warps * 32, smem, stream>>>(ids, weights, T, topk, E, seg_start, route_token, route_weight, route_src);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

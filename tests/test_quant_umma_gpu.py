@@ -92,3 +92,31 @@ def test_experts(t13, t2, T, E, topk, limit):
     assert _rel(run(a=raw13[n13:].clone(), b=raw2[n2:].clone(), expert_offset=half, local_experts=E - half), exact(half, E)) < 2e-6
     if not limit:       # hidden values in one fp16 term
         assert _rel(go.gguf_moe_forward_grouped(x, raw13, raw2, t13, t2, E, I, routes), want) < 5e-4
+
+
+@pytest.mark.parametrize("T,topk,E", [(1, 8, 256), (3, 2, 5), (700, 8, 256), (129, 6, 2000), (40, 1, 11000)])
+def test_grouped_routes(T, topk, E):
+    from pocketllm_b200.ops import gguf_ops as go
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, E, (T, topk), generator=g, dtype=torch.int32)
+    ids[::3] = ids[0, 0]
+    weight = torch.rand(T, topk, generator=g)
+    routes = go.group_routes(ids.cuda(), weight.cuda(), E)
+    order = torch.sort(ids.view(-1), stable=True).indices
+    seg, tok, w = (t.cpu() for t in routes)
+    assert torch.equal(seg[1:].long(), torch.bincount(ids.view(-1), minlength=E).cumsum(0)) and int(seg[0]) == 0
+    assert torch.equal(routes.src.cpu().long(), order) and torch.equal(tok.long(), order // topk) and torch.equal(w, weight.view(-1)[order])
+
+
+@pytest.mark.parametrize("T,E,H", [(127, 64, 256), (128, 60, 96), (130, 65, 3072), (300, 256, 1000)])
+def test_router_of_many_tokens(T, E, H):
+    from pocketllm_b200.ops import gguf_ops as go
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(E, H, device="cuda", generator=g) * H ** -0.5
+    ids, weight = go.router_topk(x, w, 4, score_func="sigmoid", norm_topk=False)
+    p = torch.sigmoid(x.double() @ w.double().T)
+    top = p.topk(5, -1).values
+    clear = ((top[:, :-1] - top[:, 1:]) > 1e-5).all(-1)          # a choice that fp32 sums decide as well
+    assert clear.float().mean() > 0.9 and torch.equal(ids[clear].long(), p.topk(4, -1).indices[clear])
+    assert (weight.double() - p.gather(1, ids.long())).abs().max() < 2e-6
