@@ -92,6 +92,13 @@ int pk_gqa_prefill_umma(const void* q, const void* kcache, const void* vcache, c
                         float scale, const void* gate_proj, int ld, void* out, uint32_t* status, cudaStream_t stream);
 int pk_gemm_bf16_grouped(const void* A, int lda, const void* W, const int* seg, int n_groups, int R, int N, int K, int epi, void* C, int ldc,
                          uint32_t* status, int sm_count, cudaStream_t stream);
+int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const int* index, int rows, const float* gamma, float eps, int plus_one,
+                        const float* add, void* sum, void* norm, int type, int terms, void* staged, float* row_scale, uint32_t* counters, int n_counters,
+                        cudaStream_t stream);
+int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, int n_groups, int rows, const void* staged, const float* row_scale,
+                  int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int splits, float* ws, uint32_t* counters,
+                  uint32_t* status, const float* w_scale, int w_ld, int sm_count, cudaStream_t stream);
+int pk_linear_narrow(const void* x, int ldx, const void* w, int M, int N, int K, void* y, int ldy, cudaStream_t stream);
 int pk_scatter_rows(const void* src, const int* slots, int n, int row_bytes, void* pool, cudaStream_t stream);
 int pk_topk_select(const float* score, const int* lengths, int M, int n, int ld, int k, int* out, cudaStream_t stream);
 int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int K, int epi, void* C, const void* resid, int ldc,

@@ -20,6 +20,10 @@ namespace {
 
 constexpr int kHeadDim = 128;
 constexpr int kSmallRows = 8;
+// Rows that are multiplied with the weights as the M side (quant_umma.cu): every weight byte is read once and the product costs the
+// same for 3 rows as for 16. Measured at the 27B widths, mean of the 16 products of four layers: 5 rows 97 -> 38 us (one multiply-add
+// per weight and row), 13 rows 65 -> 46 us (128-row tiles of the FP8 GEMM); at 64 rows the FP8 GEMM's tiles are half full.
+constexpr int kQuantRows = 64, kQuantType = 20, kQuantItems = 640;
 constexpr int kArgmaxBlocks = 64;
 constexpr int kCandStride = 32;   // sampler candidates per rank in the exchange arrays; entry 31 of the index row is the rank's status word
 
@@ -293,6 +297,15 @@ void QwenEngine::alloc_buffers() {
   out_cap_ = 1 << 16;
   out_tokens_dev_ = (int*)dalloc(out_cap_ * sizeof(int));
   out_counter_dev_ = (int*)dalloc(sizeof(int));
+  if (opt_.tp_world == 1) {
+    int kmax = hidden_;
+    for (int k : {inter_l_, vd_l_, hq_l_ * kHeadDim}) kmax = std::max(kmax, k);
+    quant_rows_ = dalloc((size_t)kQuantRows * kmax * 2);
+    quant_scale_ = (float*)dalloc(kQuantRows * sizeof(float));
+    quant_ws_ = (float*)dalloc((size_t)kQuantItems * kQuantRows * 128 * sizeof(float));
+    quant_counters_ = (uint32_t*)dalloc(kQuantItems * sizeof(uint32_t));
+    cuda_check(cudaMemset(quant_counters_, 0, kQuantItems * sizeof(uint32_t)), "memset");
+  }
   gemm_status_ = (uint32_t*)dalloc(sizeof(uint32_t));
   cuda_check(cudaMemset(gemm_status_, 0, sizeof(uint32_t)), "memset");
   if (opt_.mtp) {
@@ -903,6 +916,46 @@ PkPush QwenEngine::make_push(int site, bool big, int rows_per_rank) const {
 }
 
 // ---------------------------------------------------------------------------------------
+// few rows on the tensor cores
+
+bool QwenEngine::quant_takes(const Fp8Linear& w, int M) const {
+  // Loops that compare the picks of passes over different numbers of rows keep one order of addition: engines whose single rows take
+  // one launch per projection (also for the predictor or an external drafter's taps), and POCKET_MATVEC_RING=0.
+  const char* ring = getenv("POCKET_MATVEC_RING");
+  const char* persistent = getenv("POCKET_DECODE_PERSISTENT");
+  const bool one_order = opt_.mtp || !tap_layers_.empty() || (persistent ? atoi(persistent) : opt_.persistent_decode) == 0 || (ring != nullptr && atoi(ring) == 0);
+  return quant_rows_ != nullptr && !one_order && !nccl_mode_ && w.w != nullptr && w.scale != nullptr && M <= kQuantRows && (w.K & 127) == 0;
+}
+
+// fp16 rows of x for the products that follow; gamma: RMSNorm (1 + gamma) with a bf16 result; add: fp32 rows added first, the bf16
+// sum kept in `sum` (row stride ldx); norm: the normed rows are kept there.
+void QwenEngine::quant_stage(const void* x, int ldx, int K, int M, const float* gamma, const float* add, void* sum, void* norm) {
+  check(pk_quant_stage_rows(x, 0, ldx, K, nullptr, M, gamma, (float)cfg_.rms_norm_eps, 1, add, sum, norm, kQuantType, 1, quant_rows_, quant_scale_, nullptr, 0,
+                            stream_),
+        "quant_stage_rows");
+}
+
+void QwenEngine::quant_product(const Fp8Linear& w, int M, int epi, void* out, int ldo, const void* resid) {
+  const int columns = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+  const int tiles = epi == 1 ? (w.N / 2 + 63) / 64 : (w.N + 127) / 128;
+  // Parts of K: the fewest with which the last round of CTAs is about as full as it gets, four 128-wide blocks in a part at least.
+  // 40 tiles of a 5120-row projection leave most SMs idle without.
+  int splits = 1;
+  double best = 0;
+  for (int s = 1; s <= w.K / 512 && tiles * s <= kQuantItems; ++s) {
+    const int items = tiles * s;
+    const double full = (double)items / ((items + sm_count_ - 1) / sm_count_ * sm_count_) - 0.01 * s;
+    if (full > best) {
+      best = full;
+      splits = s;
+    }
+  }
+  check(pk_quant_rows(w.w, kQuantType, w.N, w.K, nullptr, 1, M, quant_rows_, quant_scale_, 1, epi, out, ldo, resid, 0.f, columns, splits, quant_ws_,
+                      quant_counters_, gemm_status_, w.scale, w.K / 128, sm_count_, stream_),
+        "quant_rows");
+}
+
+// ---------------------------------------------------------------------------------------
 // forward, weight-streaming path (1..8 rows)
 
 void QwenEngine::run_small(int M, bool all_logits, bool mtp) {
@@ -922,6 +975,7 @@ void QwenEngine::run_small(int M, bool all_logits, bool mtp) {
     check(pk_embedding(tokens_dev_, M, embed_, hidden_, 0, (int)cfg_.vocab_size, hidden_buf_[cur_], nullptr, stream_), "embedding");
   }
   int pending = -1;  // site whose partial sums still wait to be added to the residual stream
+  const bool few = M >= 3 && !mtp;     // one and two rows stream through the rings of matvec.cu
 
   auto consume = [&](const Fp8Linear* w, const void* wb, int nb, const float* gamma, int epi, void* y, int ldy,
                      const PkPush* push) {
@@ -929,6 +983,16 @@ void QwenEngine::run_small(int M, bool all_logits, bool mtp) {
     const float* parts = pending >= 0 ? slot_parts(pending) : nullptr;
     PkWait wt = make_wait(pending >= 0 ? pending : 0);
     void* hout = pending >= 0 ? hidden_buf_[cur_ ^ 1] : nullptr;
+    if (w != nullptr && few && quant_takes(*w, M)) {
+      quant_stage(hidden_buf_[cur_], hidden_, hidden_, M, gamma, parts, hout, nb > 0 ? xn_ : nullptr);
+      if (pending >= 0) cur_ ^= 1;
+      pending = -1;
+      quant_product(*w, M, epi, y, ldy, nullptr);
+      if (nb > 0)
+        check(pk_linear_narrow(xn_, hidden_, wb, M, nb, hidden_, (char*)y + (size_t)w->N * 2, ldy, stream_),
+              "linear_narrow");
+      return;
+    }
     check(pk_matvec(w ? w->w : nullptr, w ? w->scale : nullptr, wb, w ? w->N : 0, nb, hidden_, M, hidden_buf_[cur_], parts,
                     kernel_world(), hout, gamma, 1, eps, pending >= 0 && !nccl_mode_ ? &wt : nullptr, epi, y, ldy, push, sm_count_, stream_),
           "matvec(consume)");
@@ -938,6 +1002,12 @@ void QwenEngine::run_small(int M, bool all_logits, bool mtp) {
     pending = -1;
   };
   auto produce = [&](const Fp8Linear& w, const void* x, int site) {
+    if (few && quant_takes(w, M)) {
+      quant_stage(x, w.K, w.K, M, nullptr, nullptr, nullptr, nullptr);
+      quant_product(w, M, 2, slot_parts(site), hidden_, nullptr);
+      pending = site;
+      return;
+    }
     PkPush ps = make_push(site);
     check(pk_matvec(w.w, w.scale, nullptr, w.N, 0, w.K, M, x, nullptr, 0, nullptr, nullptr, 0, eps, nullptr, 3,
                     nullptr, hidden_, &ps, sm_count_, stream_),
@@ -1055,7 +1125,7 @@ void QwenEngine::sample_rows(int M, const float* logits, int* out) {
 // ---------------------------------------------------------------------------------------
 // forward, tensor-core path (more than 8 rows, one rank)
 
-void QwenEngine::run_chunk(int M, bool mtp) {
+void QwenEngine::run_chunk(int M, bool mtp, bool more) {
   if (!peers_set_) throw std::runtime_error("peer arenas not registered");
   const float eps = (float)cfg_.rms_norm_eps;
   const int W = opt_.tp_world;
@@ -1077,6 +1147,7 @@ void QwenEngine::run_chunk(int M, bool mtp) {
   // tcgen05 kind::f8f6f4 on them and on the stored weight codes. Shapes the kernel does not take fall through.
   // true while act_q_ / act_scale_ hold the quantised rows of xn_ (written by the norm kernel itself)
   bool xn_quantised = false;
+  bool xn_staged = false;      // the same of the fp16 rows behind quant_product
   auto gemm_native = [&](const void* A, int lda, const Fp8Linear& w, int epi, void* C, const void* resid, int ldc, const PkPush* ps) -> bool {
     if (act_q_ == nullptr || w.w == nullptr || w.scale == nullptr || (w.K & 127) != 0 || (lda & 3) != 0 || M > act_rows_) return false;   // bf16-only linears have no codes
     if (epi == 1 && ((w.N >> 1) & 127) != 0) return false;
@@ -1090,6 +1161,12 @@ void QwenEngine::run_chunk(int M, bool mtp) {
     return true;
   };
   auto gemm = [&](const void* A, int lda, const Fp8Linear& w, int epi, void* C, const void* resid, int ldc) {
+    if ((gemm_mode_ == 2 || gemm_mode_ == 3) && (lda & 3) == 0 && quant_takes(w, M)) {
+      if (A != xn_ || !xn_staged) quant_stage(A, lda, w.K, M, nullptr, nullptr, nullptr, nullptr);
+      xn_staged = false;
+      quant_product(w, M, epi == 2 ? 4 : epi, C, ldc, resid);
+      return;
+    }
     if (gemm_native(A, lda, w, epi, C, resid, ldc, nullptr)) return;
     if (w.wb != nullptr) {
       // persistent 128x256 kernel; shapes it does not take (SwiGLU halves not a multiple of 128) go to the 128x128 one
@@ -1143,6 +1220,9 @@ void QwenEngine::run_chunk(int M, bool mtp) {
       if (y != nullptr && y != xn_)
         cuda_check(cudaMemcpyAsync(y, xn_, (size_t)M * hidden_ * 2, cudaMemcpyDeviceToDevice, stream_), "copy normalised rows");
       pending = -1;
+    } else if (y == xn_ && (gemm_mode_ == 2 || gemm_mode_ == 3) && (hidden_ & 127) == 0 && quant_takes(layers_[0].gate_up, M)) {
+      quant_stage(hid, hidden_, hidden_, M, gamma, nullptr, nullptr, y);
+      xn_staged = true;
     } else if (y == xn_ && act_q_ != nullptr && (gemm_mode_ == 2 || gemm_mode_ == 3) && (hidden_ & 127) == 0 && M <= act_rows_) {
       // the rows feed a native FP8 GEMM next: the norm kernel quantises them on the way out
       check(pk_rmsnorm_quant(hid, M, hidden_, gamma, 1, eps, y, gemm_mode_ == 3 ? 1 : 2, act_q_, act_rows_, act_scale_, act_rows_, stream_),
@@ -1178,9 +1258,8 @@ void QwenEngine::run_chunk(int M, bool mtp) {
       gemm_out(attn_out_, hq_l_ * kHeadDim, L.o_proj, 2 * i);
     } else {
       gemm(xn_, hidden_, L.in_proj, 0, proj_, nullptr, ld_proj_);
-      check(pk_gemm_umma(xn_, hidden_, L.in_proj_ab, nullptr, 1, M, 2 * vh_l_, hidden_, 0,
-                         (char*)proj_ + (size_t)L.in_proj.N * 2, nullptr, ld_proj_, gemm_status_, nullptr, stream_),
-            "gemm_umma(ab)");
+      check(pk_linear_narrow(xn_, hidden_, L.in_proj_ab, M, 2 * vh_l_, hidden_, (char*)proj_ + (size_t)L.in_proj.N * 2, ld_proj_, stream_),
+            "linear_narrow(ab)");
       if (M >= 32) {
         check(pk_deltanet_chunked(proj_, ld_proj_, M, kh_l_, vh_l_, kHeadDim, kHeadDim, L.conv_w, L.conv_state, L.A_log,
                                   L.dt_bias, L.lin_norm, eps, L.lin_state, attn_out_, lin_ws_, stream_),
@@ -1230,6 +1309,7 @@ void QwenEngine::run_chunk(int M, bool mtp) {
     sample_rows(1, logits_, next_tok_dev_);
     return;
   }
+  if (more && !mtp) return;      // the prompt goes on: nobody reads this chunk's logits
   const char* last = (const char*)hid + (size_t)(M - 1) * hidden_ * 2;
   if (mtp) {
     check(pk_rmsnorm(last, nullptr, 0, 1, hidden_, nullptr, mtp_norm_, 1, eps, mtp_out_, nullptr, stream_), "mtp norm");
@@ -1273,7 +1353,7 @@ int QwenEngine::prefill(const int* tokens_host, int n) {
     cuda_check(cudaMemcpyAsync(tokens_dev_, pinned_tok_ + (done - stage_base), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, stream_), "h2d tokens");
     check(pk_iota_int(pos_dev_, M, nullptr, pos_, stream_), "iota");
     if (M <= kSmallRows) run_small(M, false);
-    else run_chunk(M);
+    else run_chunk(M, false, done + M < n);
     if (opt_.mtp) {
       // prime the predictor: row i pairs the target's hidden of position i with the token of position i + 1; the
       // very last row takes the token the target has just produced

@@ -262,7 +262,7 @@ class QwenEngine {
   // `mtp` runs the predictor stack (input = [norm(embed(mtp_tok_dev_)) | norm(mtp_in_)] through fc, one layer,
   // mtp.norm, logits of the last row) instead of the target.
   void run_small(int M, bool all_logits, bool mtp = false);    // M <= 8 rows: weight-streaming path
-  void run_chunk(int M, bool mtp = false);                     // M > 8 rows: tensor-core path
+  void run_chunk(int M, bool mtp = false, bool more = false);  // M > 8 rows: tensor-core path; more: another chunk of the prompt follows
   void sample_rows(int M, const float* logits, int* out);
   void mtp_forward(int M, const void* hidden_rows, int position);   // tokens already in mtp_tok_dev_
   int mtp_row(int token, const void* hidden_row, int position);     // one row; returns the predicted token
@@ -314,6 +314,14 @@ class QwenEngine {
   void* act_q_ = nullptr;        // [2][rows_cap_ up to 128][K max] E4M3 terms of the GEMM input being multiplied
   float* act_scale_ = nullptr;   // [K max / 128][that row count]
   int act_rows_ = 0;
+  // products of 3 to kQuantRows rows (one rank): staged fp16 rows, their factors, partial sums of parts of K with one counter a tile
+  void* quant_rows_ = nullptr;
+  float* quant_scale_ = nullptr;
+  float* quant_ws_ = nullptr;
+  uint32_t* quant_counters_ = nullptr;
+  bool quant_takes(const Fp8Linear& w, int M) const;
+  void quant_stage(const void* x, int ldx, int K, int M, const float* gamma, const float* add, void* sum, void* norm);
+  void quant_product(const Fp8Linear& w, int M, int epi, void* out, int ldo, const void* resid);
   size_t kv_bytes_ = 0;
   std::vector<void*> allocs_;
 

@@ -94,6 +94,57 @@ def test_experts(t13, t2, T, E, topk, limit):
         assert _rel(go.gguf_moe_forward_grouped(x, raw13, raw2, t13, t2, E, I, routes), want) < 5e-4
 
 
+def _e4m3(x, w, scale, epi, resid, columns, splits):
+    from ctypes import c_float, c_int, c_void_p
+    from pocketllm_b200 import ops
+    M, K = x.shape
+    N = w.shape[0]
+    lib, null = ops._lib.kernels(), c_void_p(0)
+    staged, factor = torch.empty(M, K, device="cuda", dtype=torch.float16), torch.empty(M, device="cuda")
+    cols = N // 2 if epi == 1 else N
+    y = torch.full((M, cols), float("nan"), device="cuda", dtype=torch.float32 if epi == 2 else torch.bfloat16)
+    tiles = -(-N // 128) if epi != 1 else -(-(N // 2) // 64)
+    ws, counters = torch.empty(tiles * splits * columns * 128, device="cuda"), torch.zeros(tiles, device="cuda", dtype=torch.int32)
+    status = torch.zeros(1, device="cuda", dtype=torch.int32)
+    ops._check(lib.pk_quant_stage_rows(ops._ptr(x), c_int(0), c_int(K), c_int(K), null, c_int(M), null, c_float(0), c_int(0), null, null, null, c_int(20), c_int(1),
+                                       ops._ptr(staged), ops._ptr(factor), null, c_int(0), ops._stream()), "stage")
+    for _ in range(2):      # the counters are zero again after a launch
+        ops._check(lib.pk_quant_rows(ops._ptr(w), c_int(20), c_int(N), c_int(K), null, c_int(1), c_int(M), ops._ptr(staged), ops._ptr(factor), c_int(1), c_int(epi),
+                                     ops._ptr(y), c_int(cols), ops._ptr(resid), c_float(0), c_int(columns), c_int(splits), ops._ptr(ws), ops._ptr(counters),
+                                     ops._ptr(status), ops._ptr(scale), c_int(K // 128), c_int(ops._sm_count()), ops._stream()), "rows")
+    assert int(status) == 0
+    return y
+
+
+@pytest.mark.parametrize("M,N,K,splits", [(3, 128, 128, 1), (16, 130, 640, 5), (17, 384, 1280, 3), (33, 40, 512, 2), (64, 512, 2176, 4), (5, 38400, 256, 1)])
+def test_e4m3_blocks(M, N, K, splits):
+    g = torch.Generator("cuda").manual_seed(M)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
+    scale = torch.rand(-(-N // 128), K // 128, device="cuda", generator=g) * 1e-3 + 1e-4
+    wd = w.double() * scale.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+    x = (torch.randn(M, K, device="cuda", generator=g) * torch.logspace(-2, 2, M, device="cuda")[:, None]).to(torch.bfloat16)
+    resid = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
+    columns = 16 if M <= 16 else 32 if M <= 32 else 64
+    want = x.double() @ wd.T
+    assert _rel(_e4m3(x, w, scale, 2, None, columns, splits), want) < TOL
+    assert _rel(_e4m3(x, w, scale, 0, None, columns, splits), want) < 2 ** -8
+    assert _rel(_e4m3(x, w, scale, 4, resid, columns, splits), want + resid.double()) < 2 ** -8
+    a, b = want.chunk(2, -1)
+    assert _rel(_e4m3(x, w, scale, 1, None, columns, splits), torch.nn.functional.silu(a) * b) < 2 ** -8
+
+
+@pytest.mark.parametrize("M", [1, 15, 17, 100])
+@pytest.mark.parametrize("N,K", [(1, 64), (64, 576), (65, 5120), (128, 192)])
+def test_narrow_linear(M, N, K):
+    from ctypes import c_int
+    from pocketllm_b200 import ops
+    g = torch.Generator("cuda").manual_seed(M + N)
+    x, w = (torch.randn(r, K, device="cuda", generator=g).to(torch.bfloat16) for r in (M, N))
+    y = torch.full((M, N + 3), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops._check(ops._lib.kernels().pk_linear_narrow(ops._ptr(x), c_int(K), ops._ptr(w), c_int(M), c_int(N), c_int(K), ops._ptr(y), c_int(N + 3), ops._stream()), "narrow")
+    assert _rel(y[:, :N], x.double() @ w.double().T) < 2 ** -8 and torch.isnan(y[:, N:]).all()
+
+
 @pytest.mark.parametrize("T,topk,E", [(1, 8, 256), (3, 2, 5), (700, 8, 256), (129, 6, 2000), (40, 1, 11000)])
 def test_grouped_routes(T, topk, E):
     from pocketllm_b200.ops import gguf_ops as go
