@@ -269,29 +269,37 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(0, 0, BM, BN);   // E4M3 x E4M3, fp32 accumulate
-      uint32_t it = 0;
-      WorkIter work(p, num_kb);
-      Seg sg;
-      bool ok = true;
-      while (ok && !sm.abort_flag && work.next(sg)) {
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          const int buf = it & 1;
-          // the fold of the k block that used this accumulator two blocks ago must have read it (passes at once at first)
-          if (!mbar_wait(&sm.acc_empty[buf], ((it >> 1) & 1) ^ 1, &sm.abort_flag, p.status, 32)) { ok = false; break; }
-          if (!mbar_wait(&sm.full[s], (it / kStages) & 1, &sm.abort_flag, p.status, 33)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t tmem_acc = tmem_base + (uint32_t)buf * BN;
-          const uint32_t a_addr = smem_u32(sm.a[s]), b_addr = smem_u32(sm.b[s]);
+    // The whole warp walks the loop and one lane issues: addresses and descriptors are then uniform, which is what the
+    // instructions take.
+    constexpr uint32_t idesc = umma_idesc(0, 0, BM, BN);   // E4M3 x E4M3, fp32 accumulate
+    const uint64_t da0 = smem_desc_k_sw128(smem_u32(sm.a[0])), db0 = smem_desc_k_sw128(smem_u32(sm.b[0]));
+    const bool leader = elect_one();
+    uint32_t it = 0, s = 0, ph = 0;
+    WorkIter work(p, num_kb);
+    Seg sg;
+    bool ok = true;
+    while (ok && work.next(sg)) {
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
+        const int buf = it & 1;
+        // the fold of the k block that used this accumulator two blocks ago must have read it (passes at once at first)
+        if (!mbar_wait_uniform(&sm.acc_empty[buf], ((it >> 1) & 1) ^ 1, &sm.abort_flag, p.status, 32)) { ok = false; break; }
+        if (!mbar_wait_uniform(&sm.full[s], ph, &sm.abort_flag, p.status, 33)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t tmem_acc = tmem_base + (uint32_t)buf * BN;
+        const uint64_t da = da0 + s * (uint32_t)(TERMS * kABytes >> 4), db = db0 + s * (uint32_t)(kBBytes >> 4);
+        if (leader) {
 #pragma unroll
           for (int t = 0; t < TERMS; ++t)
 #pragma unroll
             for (int k = 0; k < BK / 32; ++k)
-              umma_f8f6f4(tmem_acc, smem_desc_k_sw128(a_addr + t * kABytes + k * 32), smem_desc_k_sw128(b_addr + k * 32), idesc, (t > 0 || k > 0) ? 1u : 0u);
+              umma_f8f6f4(tmem_acc, da + (t * kABytes + k * 32 >> 4), db + (k * 32 >> 4), idesc, (t > 0 || k > 0) ? 1u : 0u);
           umma_commit(&sm.empty[s]);
           umma_commit(&sm.acc_full[buf]);
+        }
+        __syncwarp();
+        if (++s == (uint32_t)kStages) {
+          s = 0;
+          ph ^= 1u;
         }
       }
     }
