@@ -335,6 +335,69 @@ __global__ void __launch_bounds__(256) full_qk_norm_rope_append_kernel(const Ful
   }
 }
 
+// The same for rows of whole 16-byte pieces whose rotated halves are whole pieces as well: the row is loaded once, eight elements a
+// thread, and kept in shared memory, where an element finds its partner. One row of 48 heads 15 -> 4.8 us, 256 rows 14 -> 9 us; with 1500 rows the form above has
+// enough blocks to hide its loads and fewer threads without an element (30 against 37 us).
+constexpr int kFullQkThreads = 512, kFullQkVecRows = 512;
+__global__ void __launch_bounds__(kFullQkThreads) full_qk_norm_rope_append_vec_kernel(const FullQkParams p) {
+  extern __shared__ __align__(16) float xs[];      // [heads * D]
+  __shared__ float red[40];
+  const int t = blockIdx.x, is_k = blockIdx.y, tid = threadIdx.x;
+  const int H = is_k ? p.Hkv : p.Hq, n = H * kD;
+  const bf16* x = is_k ? p.k + (size_t)t * p.ldk : p.q + (size_t)t * p.ldq;
+  const float* gamma = is_k ? p.k_gamma : p.q_gamma;
+  const int pos = p.pos[t], half = p.rope_dim >> 1;
+  float ss = 0.f;
+#pragma unroll 2
+  for (int i = tid * 8; i < n; i += kFullQkThreads * 8) {
+    const uint4 u = *reinterpret_cast<const uint4*>(x + i);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[2 * j] = __uint_as_float(w[j] << 16);
+      v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+    }
+    *reinterpret_cast<float4*>(xs + i) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(xs + i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+  }
+  ss = block_sum(ss, red);
+  const float rs = rsqrtf(ss / (float)n + p.eps);
+  const bool in_cache = pos >= 0 && pos < p.ctx_cap;
+  if (!in_cache && threadIdx.x == 0) PK_DEBUG_RECORD(101, pos, p.ctx_cap);
+  for (int i = tid * 8; i < n; i += kFullQkThreads * 8) {
+    const int head = i >> 7, d = i & (kD - 1);
+    float y[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) y[e] = xs[i + e] * rs * gamma[i + e];
+    if (d < p.rope_dim) {
+      const int j = d < half ? d : d - half, o = d < half ? i + half : i - half;
+      const float* cs = p.cos_t + (size_t)pos * half + j;
+      const float* sn = p.sin_t + (size_t)pos * half + j;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float yo = xs[o + e] * rs * gamma[o + e];
+        y[e] = d < half ? y[e] * cs[e] - yo * sn[e] : y[e] * cs[e] + yo * sn[e];
+      }
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __nv_bfloat162 pr = __floats2bfloat162_rn(y[2 * e], y[2 * e + 1]);
+      w[e] = *reinterpret_cast<const uint32_t*>(&pr);
+    }
+    if (!is_k) {
+      *reinterpret_cast<uint4*>(p.q_out + ((size_t)t * p.Hq + head) * kD + d) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else if (in_cache) {
+      const size_t ci = ((size_t)head * p.ctx_cap + pos) * kD + d;
+      *reinterpret_cast<uint4*>(p.kcache + ci) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(p.vcache + ci) = *reinterpret_cast<const uint4*>(p.v + (size_t)t * p.ldv + i);
+    }
+  }
+}
+
 }  // namespace
 
 PK_API int pk_full_qk_norm_rope_append(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, int T, int Hq, int Hkv,
@@ -345,7 +408,12 @@ PK_API int pk_full_qk_norm_rope_append(const void* q, int ldq, const void* k, in
   if (T < 1 || rope_dim < 0 || rope_dim > kD || (rope_dim & 1)) return PK_ERR_BAD_ARG;
   FullQkParams p{(const pk::bf16*)q, (const pk::bf16*)k, (const pk::bf16*)v, ldq, ldk, ldv, Hq, Hkv, pos, q_gamma, k_gamma, eps, rope_dim, cos_t, sin_t,
                  (pk::bf16*)q_out, (pk::bf16*)kcache, (pk::bf16*)vcache, ctx_cap};
-  full_qk_norm_rope_append_kernel<<<dim3(T, 2), 256, 0, stream>>>(p);
+  const uintptr_t at = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)q_out | (uintptr_t)kcache | (uintptr_t)vcache;
+  const size_t smem = (size_t)(Hq > Hkv ? Hq : Hkv) * kD * sizeof(float);
+  if ((at & 15) == 0 && ((ldq | ldk | ldv) & 7) == 0 && (rope_dim & 15) == 0 && smem <= 48 * 1024 && T <= kFullQkVecRows)
+    full_qk_norm_rope_append_vec_kernel<<<dim3(T, 2), kFullQkThreads, smem, stream>>>(p);
+  else
+    full_qk_norm_rope_append_kernel<<<dim3(T, 2), 256, 0, stream>>>(p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

@@ -391,8 +391,8 @@ class MiniMaxM2Model:
             # prefill chunks (consecutive positions) through the tcgen05 flash kernel, decode steps through the split kernel
             o = ops.gqa_prefill(q, L["kc"], L["vc"], pos) if T >= 16 else ops.gqa_decode(q, L["kc"], L["vc"], pos, nsplit=1 if T > 8 else 8)
             att = go.gguf_linear(o, L["o"], self.types[b + "attn_output.weight"], c.dim, epi=2)
-            h = (h + att).to(torch.bfloat16)                     # bf16 + fp32 promotes to fp32: the sum is rounded once
-            xn = ops.rmsnorm(h, L["ffn_norm"], mode=2, eps=c.norm_eps)
+            before, h = h, torch.empty_like(h)                   # h <- bf16(h + att), one rounding, on the way into the norm
+            xn = ops.rmsnorm(before, L["ffn_norm"], mode=2, eps=c.norm_eps, parts=att.unsqueeze(0), hidden_out=h)
             ids, wt = go.router_topk(xn, L["router"], c.n_experts_used, bias=L["bias"], score_func="sigmoid", norm_topk=True)
             if self.balanced_routes:
                 # benchmark aid for random weights (whose hidden states collapse and send every token to the same few
@@ -409,7 +409,7 @@ class MiniMaxM2Model:
                                        self.types[b + "ffn_down_exps.weight"], c.expert_inter)
                 if self.world > 1:
                     self._combine(y)
-                h = (h + y).to(torch.bfloat16)
+                h = ops.residual_add(h, y)
                 continue
             routes = go.group_routes(ids, wt, c.n_experts)
             # many routes per expert (prefill): grouped tensor-core GEMMs; else the per-route streaming kernels
@@ -417,7 +417,7 @@ class MiniMaxM2Model:
                                c.n_experts, c.expert_inter, routes, expert_offset=self.e_start, local_experts=self.e_local, peer=self._peer())
             if self.world > 1 and not routes.combined:
                 self._combine(y)
-            h = (h + y).to(torch.bfloat16)
+            h = ops.residual_add(h, y)
         return go.gguf_linear(h[-1:], self.head, self.types["output.weight"], c.vocab_size, gamma=self.final_norm, eps=c.norm_eps, epi=2)[0]
 
     def forward_logits(self, tokens: Sequence[int]) -> torch.Tensor:

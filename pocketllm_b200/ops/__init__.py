@@ -247,6 +247,15 @@ def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, *, mode: int = 1, eps: float =
     return y
 
 
+def residual_add(x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+    """bf16(x + y) for bf16 x and fp32 y [M, K]: one launch and one rounding (the sum in fp32 and its conversion are two)."""
+    out = torch.empty_like(x)
+    st = _lib.kernels().pk_rmsnorm(_ptr(x), _ptr(y), c_int(1), c_int(x.shape[0]), c_int(x.shape[1]), _ptr(out), c_void_p(0), c_int(1), c_float(0.0),
+                                   c_void_p(0), c_void_p(0), _stream())
+    _check(st, "pk_rmsnorm")
+    return out
+
+
 def rmsnorm_quant(x: torch.Tensor, gamma: torch.Tensor, *, mode: int = 1, eps: float = 1e-6, terms: int = 2):
     """RMSNorm of contiguous bf16 x [M, K] that also quantises its output rows for `gemm_fp8` in the same kernel:
     returns (y bf16 [M, K], codes uint8 [terms, m_pad, K], scales fp32 [K / 128, m_pad]), the codes and scales exactly
