@@ -504,10 +504,9 @@ class QwenEngine:
         return self._L.pk_qwen_mtp_next_token(self._h)
 
     def mtp_logits(self) -> torch.Tensor:
-        n = self._L.pk_qwen_vocab_local(self._h)
-        buf = (ctypes.c_float * n)()
-        self._ck(self._L.pk_qwen_copy_mtp_logits(self._h, buf))
-        return torch.tensor(list(buf), dtype=torch.float32)
+        out = torch.empty(self._L.pk_qwen_vocab_local(self._h), dtype=torch.float32)
+        self._ck(self._L.pk_qwen_copy_mtp_logits(self._h, ctypes.c_void_p(out.data_ptr())))
+        return out
 
     def set_draft_replay(self, tokens: Sequence[int]) -> None:
         """Test hook: take drafts from a known continuation (the tokens after the first generated one); empty clears."""
@@ -568,10 +567,10 @@ class QwenEngine:
         return [first] + self.decode(max_new_tokens - 1)
 
     def logits(self, row: int = 0) -> torch.Tensor:
-        n = self._L.pk_qwen_vocab_local(self._h)
-        buf = (ctypes.c_float * n)()
-        self._ck(self._L.pk_qwen_copy_logits(self._h, buf, row))
-        return torch.tensor(list(buf), dtype=torch.float32)
+        # straight into the tensor's memory: by way of a Python list 16384 values took 1.35 ms (a decode step takes 0.45)
+        out = torch.empty(self._L.pk_qwen_vocab_local(self._h), dtype=torch.float32)
+        self._ck(self._L.pk_qwen_copy_logits(self._h, ctypes.c_void_p(out.data_ptr()), row))
+        return out
 
     @property
     def weight_bytes(self) -> int:
