@@ -98,6 +98,9 @@ int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const int* ind
 int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, int n_groups, int rows, const void* staged, const float* row_scale,
                   int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int splits, float* ws, uint32_t* counters,
                   uint32_t* status, const float* w_scale, int w_ld, int sm_count, cudaStream_t stream);
+int pk_rows_fp8(const void* W, const float* w_scale, int w_ld, int M, int N, int K, const void* staged, const float* row_scale, int epi, void* y, int ldy,
+                const void* resid, int sm_count, cudaStream_t stream);
+int pk_linear_rows(const void* x, int ldx, const void* w, int M, int N, int K, int epi, void* y, int ldy, int sm_count, cudaStream_t stream);
 int pk_linear_narrow(const void* x, int ldx, const void* w, int M, int N, int K, void* y, int ldy, cudaStream_t stream);
 int pk_scatter_rows(const void* src, const int* slots, int n, int row_bytes, void* pool, cudaStream_t stream);
 int pk_topk_select(const float* score, const int* lengths, int M, int n, int ld, int k, int* out, cudaStream_t stream);

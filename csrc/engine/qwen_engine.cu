@@ -20,9 +20,10 @@ namespace {
 
 constexpr int kHeadDim = 128;
 constexpr int kSmallRows = 8;
-// Rows that are multiplied with the weights as the M side (quant_umma.cu): every weight byte is read once and the product costs the
-// same for 3 rows as for 16. Measured at the 27B widths, mean of the 16 products of four layers: 5 rows 97 -> 38 us (one multiply-add
-// per weight and row), 13 rows 65 -> 46 us (128-row tiles of the FP8 GEMM); at 64 rows the FP8 GEMM's tiles are half full.
+// Rows that are multiplied with the weights as the M side: every weight byte is read once and the product costs about the same for 3
+// rows as for 16 (rows_fp8.cu), with tensor memory in between up to 64 (quant_umma.cu). Measured at the 27B widths, mean of the 16
+// products of four layers: 5 rows 97 -> 26 us (before: one multiply-add per weight and row), 13 rows 65 -> 35 us (before: 128-row tiles
+// of the FP8 GEMM, which are half full from 64 rows on).
 constexpr int kQuantRows = 64, kQuantType = 20, kQuantItems = 640;
 constexpr int kArgmaxBlocks = 64;
 constexpr int kCandStride = 32;   // sampler candidates per rank in the exchange arrays; entry 31 of the index row is the rank's status word
@@ -936,9 +937,13 @@ void QwenEngine::quant_stage(const void* x, int ldx, int K, int M, const float* 
 }
 
 void QwenEngine::quant_product(const Fp8Linear& w, int M, int epi, void* out, int ldo, const void* resid) {
+  if (M <= 16) {
+    check(pk_rows_fp8(w.w, w.scale, w.K / 128, M, w.N, w.K, quant_rows_, quant_scale_, epi, out, ldo, resid, sm_count_, stream_), "rows_fp8");
+    return;
+  }
   const int columns = M <= 16 ? 16 : M <= 32 ? 32 : 64;
   const int tiles = epi == 1 ? (w.N / 2 + 63) / 64 : (w.N + 127) / 128;
-  // Parts of K: the fewest with which the last round of CTAs is about as full as it gets, four 128-wide blocks in a part at least.
+  // More than 16 rows. Parts of K: the fewest with which the last round of CTAs is about as full as it gets, four 128-wide blocks in a part at least.
   // 40 tiles of a 5120-row projection leave most SMs idle without.
   int splits = 1;
   double best = 0;
@@ -1063,7 +1068,14 @@ void QwenEngine::run_small(int M, bool all_logits, bool mtp) {
     return;
   }
   // final norm + lm_head on every row (speculative verify) or on the last row only
-  if (all_logits || M == 1) {
+  if (all_logits && few && quant_takes(layers_[0].gate_up, M)) {
+    // the rows once through the norm, then 16 vocabulary rows a warp against all of them
+    check(pk_rmsnorm(hidden_buf_[cur_], slot_parts(pending), kernel_world(), M, hidden_, hidden_buf_[cur_], final_norm_, 1, eps, xn_, nullptr, stream_),
+          "final norm");
+    pending = -1;
+    check(pk_linear_rows(xn_, hidden_, lm_head_, M, vocab_l_, hidden_, 2, logits_, vocab_l_, sm_count_, stream_), "lm_head");
+    sample_rows(M, logits_, next_tok_dev_);
+  } else if (all_logits || M == 1) {
     consume(nullptr, lm_head_, vocab_l_, final_norm_, 2, logits_, vocab_l_, nullptr);
     sample_rows(M, logits_, next_tok_dev_);
   } else {

@@ -23,7 +23,7 @@ TOL = 1e-6
 
 
 @pytest.mark.parametrize("name", ["iq2_xxs", "q4_k", "q5_k"])
-@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (1, 300, 3072), (5, 64, 768), (16, 129, 1536), (17, 256, 512), (33, 130, 1280), (64, 2, 2304), (65, 384, 1024), (128, 200, 256)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (1, 300, 3072), (5, 64, 768), (16, 129, 1536), (17, 256, 512), (33, 130, 1280), (64, 2, 2304), (65, 384, 1024), (128, 200, 256), (256, 130, 512)])
 def test_linear(name, M, N, K):
     from pocketllm_b200.ops import gguf_ops as go
     raw, w = _raw(name, N, K, M + N)
@@ -56,7 +56,7 @@ def test_linear_rows_of_zeros_and_infinities():
 
 
 @pytest.mark.parametrize("t13,t2", [("iq2_xxs", "iq2_xxs"), ("q4_k", "iq2_xxs"), ("iq2_xxs", "q5_k")])
-@pytest.mark.parametrize("T,E,topk,limit", [(17, 40, 4, 0.0), (33, 40, 3, 0.0), (90, 8, 2, 0.5), (300, 5, 2, 0.0)])
+@pytest.mark.parametrize("T,E,topk,limit", [(1, 16, 4, 0.0), (9, 40, 3, 0.0), (17, 40, 4, 0.0), (33, 40, 3, 0.0), (90, 8, 2, 0.5), (300, 5, 2, 0.0)])
 def test_experts(t13, t2, T, E, topk, limit):
     from pocketllm_b200.ops import gguf_ops as go
     H, I = 512, 256 + 512 * (T % 2)
@@ -104,10 +104,14 @@ def _e4m3(x, w, scale, epi, resid, columns, splits):
     cols = N // 2 if epi == 1 else N
     y = torch.full((M, cols), float("nan"), device="cuda", dtype=torch.float32 if epi == 2 else torch.bfloat16)
     tiles = -(-N // 128) if epi != 1 else -(-(N // 2) // 64)
-    ws, counters = torch.empty(tiles * splits * columns * 128, device="cuda"), torch.zeros(tiles, device="cuda", dtype=torch.int32)
+    ws, counters = torch.empty(max(1, tiles * splits * columns * 128), device="cuda"), torch.zeros(tiles, device="cuda", dtype=torch.int32)
     status = torch.zeros(1, device="cuda", dtype=torch.int32)
     ops._check(lib.pk_quant_stage_rows(ops._ptr(x), c_int(0), c_int(K), c_int(K), null, c_int(M), null, c_float(0), c_int(0), null, null, null, c_int(20), c_int(1),
                                        ops._ptr(staged), ops._ptr(factor), null, c_int(0), ops._stream()), "stage")
+    if splits == 0:         # the kernel of up to 16 rows
+        ops._check(lib.pk_rows_fp8(ops._ptr(w), ops._ptr(scale), c_int(K // 128), c_int(M), c_int(N), c_int(K), ops._ptr(staged), ops._ptr(factor), c_int(epi),
+                                   ops._ptr(y), c_int(cols), ops._ptr(resid), c_int(ops._sm_count()), ops._stream()), "rows")
+        return y
     for _ in range(2):      # the counters are zero again after a launch
         ops._check(lib.pk_quant_rows(ops._ptr(w), c_int(20), c_int(N), c_int(K), null, c_int(1), c_int(M), ops._ptr(staged), ops._ptr(factor), c_int(1), c_int(epi),
                                      ops._ptr(y), c_int(cols), ops._ptr(resid), c_float(0), c_int(columns), c_int(splits), ops._ptr(ws), ops._ptr(counters),
@@ -116,7 +120,8 @@ def _e4m3(x, w, scale, epi, resid, columns, splits):
     return y
 
 
-@pytest.mark.parametrize("M,N,K,splits", [(3, 128, 128, 1), (16, 130, 640, 5), (17, 384, 1280, 3), (33, 40, 512, 2), (64, 512, 2176, 4), (5, 38400, 256, 1)])
+@pytest.mark.parametrize("M,N,K,splits", [(3, 128, 128, 1), (16, 130, 640, 5), (17, 384, 1280, 3), (33, 40, 512, 2), (64, 512, 2176, 4), (5, 38400, 256, 1),
+                                          (1, 16, 128, 0), (8, 130, 640, 0), (9, 40, 1280, 0), (16, 4112, 5120, 0), (5, 66, 17408, 0)])
 def test_e4m3_blocks(M, N, K, splits):
     g = torch.Generator("cuda").manual_seed(M)
     w = (torch.randn(N, K, device="cuda", generator=g) * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
@@ -171,3 +176,22 @@ def test_router_of_many_tokens(T, E, H):
     clear = ((top[:, :-1] - top[:, 1:]) > 1e-5).all(-1)          # a choice that fp32 sums decide as well
     assert clear.float().mean() > 0.9 and torch.equal(ids[clear].long(), p.topk(4, -1).indices[clear])
     assert (weight.double() - p.gather(1, ids.long())).abs().max() < 2e-6
+
+
+@pytest.mark.parametrize("M", [1, 3, 8])
+@pytest.mark.parametrize("N,K,split", [(8, 64, 0), (40, 128, 16), (130, 960, 0), (66, 4096, 32), (4112, 192, 0)])
+def test_bf16_rows(M, N, K, split):
+    """Rows of whole steps of 64: fewer steps than the ring holds and more, K cut over warps, ragged groups, two inputs."""
+    from pocketllm_b200.ops import mixer_ops as mo
+    g = torch.Generator("cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    x, x2, w, st = r(M, K), r(M, K), r(N, K) * K ** -0.5, torch.zeros(1, device="cuda", dtype=torch.int32)
+    want = x.double() @ w.double().T
+    y = lambda n, dt: torch.full((M, n), float("nan"), device="cuda", dtype=dt)
+    assert _rel(mo.linear(x, w, y(N, torch.float32), st), want) < TOL
+    assert _rel(mo.linear(x, w, y(N, torch.bfloat16), st), want) < 2 ** -8
+    a, b = want.chunk(2, -1)
+    assert _rel(mo.linear(x, w, y(N // 2, torch.bfloat16), st, swiglu=True), torch.nn.functional.silu(a) * b) < 2 ** -8
+    if split:
+        want[:, split:] = x2.double() @ w[split:].double().T
+        assert _rel(mo.linear2(x, x2, split, w, y(N, torch.float32), st), want) < TOL
