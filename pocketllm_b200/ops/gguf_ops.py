@@ -29,8 +29,8 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     src/components/gguf/quantized_ops.py:9-76)."""
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
-    if M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name):
-        return _umma_linear(x.contiguous(), w_raw, type_name, N, gamma, eps, epi)
+    if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name):
+        return _umma_linear(_aligned(x), w_raw, type_name, N, _aligned(gamma), eps, epi)
     if M >= TENSOR_CORE_MIN_ROWS and K % 64 == 0 and (epi != 1 or (N // 2) % 128 == 0):
         from . import gemm_bf16, rmsnorm, EPI_BF16, EPI_SWIGLU, EPI_F32
         w = _dequant_scratch(w_raw, type_name, N, K)
@@ -50,10 +50,10 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
 
 # Block types whose integer part fits fp16: decoded inside the tensor-core kernel (`csrc/kernels/quant_umma.cu`)
 UMMA_TYPES = frozenset({"iq2_xxs", "q4_k", "q5_k"})
-UMMA_MAX_ROWS = 129
-# Up to 64 routes the kernels with one block set per route leave no SM idle: 8 routes of the MiniMax-M2 shape take 50 + 32 us there and
-# 47 + 28 and two stagings of 3.5 us here; 184 routes 1233 + 628 and 390 + 207 us.
-UMMA_MIN_ROUTES = 64
+# Q5_K rows of 8192 x 3072 / 3072 x 6144, us, against decoding per eight rows or (from 32 rows) to a bf16 scratch: 1 row 22 / 21 against
+# 25 / 23, 8 rows 22 / 21 against 93 / 86, 64 rows 27 / 27 against 59 / 65, 256 rows 60 / 54 against 63 / 69.
+UMMA_MAX_ROWS = 257
+UMMA_SPLIT_ROUTES = 64
 UMMA_MAX_GROUPS = 512
 _status: dict = {}
 
@@ -68,6 +68,14 @@ def _umma_status(dev) -> torch.Tensor:
     if dev.index not in _status:
         _status[dev.index] = torch.zeros(1, device=dev, dtype=torch.int32)
     return _status[dev.index]
+
+
+def _aligned(t: torch.Tensor | None) -> torch.Tensor | None:
+    """`t` itself, or a copy that begins on 16 bytes and has its rows one after the other."""
+    if t is None:
+        return None
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 class _Staged:
@@ -87,23 +95,40 @@ class _Staged:
         p = self.buf.data_ptr()
         self.data, self.scale, self.counters, self.ws = (c_void_p(p + o) for o in offs)
         _check(_lib.kernels().pk_quant_stage_rows(_ptr(x), c_int(int(x.dtype == torch.float32)), c_int(x.stride(0)), c_int(K), _ptr(index), c_int(rows),
-                                                 _ptr(gamma), c_float(eps), c_int(0), c_void_p(0), c_void_p(0), c_void_p(0), c_int(DEVICE_TYPE[type_name]), c_int(terms), self.data, self.scale,
-                                                 self.counters, c_int(counters), _stream()), "pk_quant_stage_rows")
+                                                 _ptr(gamma), c_float(eps), c_int(0), c_void_p(0), c_void_p(0), c_void_p(0),
+                                                 c_int(DEVICE_TYPE[type_name]), c_int(terms), self.data, self.scale, self.counters, c_int(counters),
+                                                 _stream()), "pk_quant_stage_rows")
 
 
 def _umma(st: _Staged, w_raw: torch.Tensor, type_name: str, N: int, K: int, seg, groups: int, epi: int, out: torch.Tensor, limit: float, columns: int,
           splits: int) -> None:
     _check(_lib.kernels().pk_quant_rows(_ptr(w_raw), c_int(DEVICE_TYPE[type_name]), c_int(N), c_int(K), _ptr(seg), c_int(groups), c_int(st.rows), st.data,
                                        st.scale, c_int(st.terms), c_int(epi), _ptr(out), c_int(out.stride(0)), c_void_p(0), c_float(limit), c_int(columns),
-                                       c_int(splits), st.ws, st.counters, _ptr(_umma_status(out.device)), c_void_p(0), c_int(0), c_int(_sm_count()), _stream()), "pk_quant_rows")
+                                       c_int(splits), st.ws, st.counters, _ptr(_umma_status(out.device)), c_void_p(0), c_int(0),
+                                       c_int(_sm_count()), _stream()), "pk_quant_rows")
+
+
+def _umma_splits(tiles: int, K: int, slots: int) -> int:
+    """Parts of K for `tiles` tiles on `slots` CTAs: the fewest with which the last round of CTAs is about as full as it gets, two
+    256-weight blocks in a part at least."""
+    best, most = 1, 0.0
+    for s in range(1, min(K // 512, 4 * slots // tiles) + 1):
+        items = tiles * s
+        full = items / (-(-items // slots) * slots) - 0.01 * s
+        if full > most:
+            best, most = s, full
+    return best
+
+
+def _umma_slots(type_name: str, columns: int) -> int:
+    return _sm_count() * (2 if type_name == "iq2_xxs" and columns < 64 else 1)      # resident CTAs of the kernel
 
 
 def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, gamma, eps: float, epi: int) -> torch.Tensor:
     M, K = x.shape
     columns = 16 if M <= 16 else 32 if M <= 32 else 64
     tiles = (-(-(N // 2) // 64) if epi == 1 else -(-N // 128)) * -(-M // columns)
-    # parts of K until every resident CTA has work; two 256-weight blocks at least in a part
-    splits = max(1, min(K // 512, _sm_count() * (1 if columns == 64 else 2) // tiles))
+    splits = _umma_splits(tiles, K, _umma_slots(type_name, columns))
     st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
     y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
     _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits)
@@ -111,22 +136,29 @@ def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, g
 
 
 def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, inter: int, routes: "Routes", limit: float,
-                  expert_offset: int, local: int, terms: int) -> torch.Tensor:
+                  E: int, expert_offset: int, local: int, terms: int) -> torch.Tensor:
     """fp32 [R, H]: every route's expert output, without its weight. `terms`: fp16 terms that a hidden value is multiplied as."""
     seg, tok, _ = routes
     H, R, dev = x.shape[1], tok.numel(), x.device
     seg = seg[expert_offset:]
 
     def columns(t: int) -> int:      # of an expert's tile: what most experts with routes need
-        n = t * R / local
+        n = t * R / E      # a rank's experts see their share of the routes: the same tiles however the experts are split
         return 16 if n <= 10 else 32 if n <= 24 else 64
+
+    def product(x, w_raw, type_name, N, K, t, epi, out, limit, index):
+        c, row_tiles = columns(t), -(-(N // 2) // 64) if epi == 3 else -(-N // 128)
+        splits = 1
+        if R <= UMMA_SPLIT_ROUTES:       # every route may be an expert of its own; beyond, the tiles fill the SMs
+            splits = _umma_splits(max(1, min(R, local)) * row_tiles, K, _umma_slots(type_name, c))
+        tiles = (min(R, local) + R * t // c) * row_tiles if splits > 1 else 0
+        st = _Staged(x, type_name, R, t, index=index, counters=tiles, ws_floats=tiles * splits * c * 128)
+        _umma(st, w_raw, type_name, N, K, seg, local, epi, out, limit, c, splits)
 
     h = torch.empty(R, inter, device=dev, dtype=torch.float32)
     y = torch.empty(R, H, device=dev, dtype=torch.float32)
-    st = _Staged(x, type13, R, 1, index=tok)
-    _umma(st, w13_raw, type13, 2 * inter, H, seg, local, 3, h, limit, columns(1), 1)
-    st2 = _Staged(h, type2, R, terms)
-    _umma(st2, w2_raw, type2, H, inter, seg, local, 2, y, 0.0, columns(terms), 1)
+    product(_aligned(x), w13_raw, type13, 2 * inter, H, 1, 3, h, limit, tok)
+    product(h, w2_raw, type2, H, inter, terms, 2, y, 0.0, None)
     return y
 
 
@@ -210,9 +242,9 @@ def gguf_moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tenso
     local = E if local_experts is None else local_experts
     if out is None:
         out = torch.zeros(T, H, device=x.device, dtype=torch.float32)
-    if routes is not None and R > UMMA_MIN_ROUTES and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
+    if routes is not None and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
         # hidden values in two fp16 terms: as good as the fp32 values of the kernels that decode in registers
-        y = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, limit, expert_offset, local, 2)
+        y = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, limit, E, expert_offset, local, 2)
         return _reduce_routes(y, routes, x.shape, expert_offset, local, out)
     hbuf = torch.empty(R, inter, device=x.device, dtype=torch.float32)
     if routes is not None:
@@ -254,8 +286,8 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     if out is None:
         out = torch.zeros(T, H, device=dev, dtype=torch.float32)
     K = _lib.kernels()
-    if R <= UMMA_MAX_ROUTES_PER_EXPERT * local and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
-        ybuf = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, 0.0, expert_offset, local, 1)
+    if R <= UMMA_MAX_ROUTES_PER_EXPERT * E and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
+        ybuf = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, 0.0, E, expert_offset, local, 1)
     else:
         key = (dev.index, local, H, inter)
         sc = _GROUPED_SCRATCH.get(key)
@@ -289,7 +321,8 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     return _reduce_routes(ybuf, routes, x.shape, expert_offset, local, out)
 
 
-UMMA_MAX_ROUTES_PER_EXPERT = 256      # above this a decode per 64 routes costs more than one decode to a bf16 scratch
+UMMA_MAX_ROUTES_PER_EXPERT = 192      # above this a decode per 64 routes costs more than one decode to a bf16 scratch: 128 routes 4.2 against
+#                                        5.4 ms, 192 6.0 against 5.9, 256 7.7 against 6.5 (256 experts of the MiniMax-M2 shape)
 GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local expert costs more than the route kernels' per-route decode
 
 
