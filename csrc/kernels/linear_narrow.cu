@@ -1,8 +1,9 @@
 // Products with a few dozen weight rows: y[M, N] = x[M, K] W[N, K]^T, all bf16 with fp32 sums (the gates of a DeltaNet layer: 64 rows
-// of 5120). A tile GEMM has one tile for all of W and walks K alone: 35 us for 13 rows as for 512, 17 here. The K range of 16 token
-// rows and 64 weight rows is cut into eight warps' shares, added in their order.
+// of 5120). A tile GEMM has one tile for all of W and walks K alone: 35 us for 13 rows as for 512, 12 here (18 with
+// eight warps of 64 rows, each lane 32 bytes in a row). The K range of 16 token
+// rows and 32 weight rows is cut into sixteen warps' shares, added in their order.
 //
-// A lane loads 16 consecutive values of its row for four m16n8k16 products: which of the 64 values of a step a product takes is
+// A lane loads two times eight consecutive values of its row for four m16n8k16 products: which of the 64 values of a step a product takes is
 // the same for both operands, so no value has to change lanes. The work is a few hundred products per warp and waits for its loads:
 // the tensor-memory path's set-up would cost more than the whole.
 #include "../common/pk_common.cuh"
@@ -11,7 +12,7 @@ namespace {
 
 using namespace pk;
 
-constexpr int kWarps = 8, kTok = 16, kRows = 64;
+constexpr int kWarps = 16, kTok = 16, kRows = 32;
 
 struct NarrowParams {
   const bf16* x;
@@ -33,18 +34,18 @@ __global__ void __launch_bounds__(32 * kWarps) linear_narrow_kernel(const Narrow
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int m0 = blockIdx.x * kTok, n0 = blockIdx.y * kRows;
   float acc[kRows / 8][4] = {};
-  const bf16* xa = p.x + (size_t)min(m0 + g, p.M - 1) * p.ldx + t * 16;
-  const bf16* xb = p.x + (size_t)min(m0 + g + 8, p.M - 1) * p.ldx + t * 16;
+  const bf16* xa = p.x + (size_t)min(m0 + g, p.M - 1) * p.ldx + t * 8;
+  const bf16* xb = p.x + (size_t)min(m0 + g + 8, p.M - 1) * p.ldx + t * 8;
   const bf16* wr[kRows / 8];
 #pragma unroll
-  for (int j = 0; j < kRows / 8; ++j) wr[j] = p.w + (size_t)min(n0 + j * 8 + g, p.N - 1) * p.K + t * 16;
+  for (int j = 0; j < kRows / 8; ++j) wr[j] = p.w + (size_t)min(n0 + j * 8 + g, p.N - 1) * p.K + t * 8;
 #pragma unroll 2
   for (int k = warp * 64; k < p.K; k += 64 * kWarps) {
-    const uint4 a0 = __ldg(reinterpret_cast<const uint4*>(xa + k)), a1 = __ldg(reinterpret_cast<const uint4*>(xa + k + 8));
-    const uint4 b0 = __ldg(reinterpret_cast<const uint4*>(xb + k)), b1 = __ldg(reinterpret_cast<const uint4*>(xb + k + 8));
+    const uint4 a0 = __ldg(reinterpret_cast<const uint4*>(xa + k)), a1 = __ldg(reinterpret_cast<const uint4*>(xa + k + 32));
+    const uint4 b0 = __ldg(reinterpret_cast<const uint4*>(xb + k)), b1 = __ldg(reinterpret_cast<const uint4*>(xb + k + 32));
 #pragma unroll
     for (int j = 0; j < kRows / 8; ++j) {
-      const uint4 w0 = __ldg(reinterpret_cast<const uint4*>(wr[j] + k)), w1 = __ldg(reinterpret_cast<const uint4*>(wr[j] + k + 8));
+      const uint4 w0 = __ldg(reinterpret_cast<const uint4*>(wr[j] + k)), w1 = __ldg(reinterpret_cast<const uint4*>(wr[j] + k + 32));
       mma16816(acc[j], a0.x, b0.x, a0.y, b0.y, w0.x, w0.y);
       mma16816(acc[j], a0.z, b0.z, a0.w, b0.w, w0.z, w0.w);
       mma16816(acc[j], a1.x, b1.x, a1.y, b1.y, w1.x, w1.y);
