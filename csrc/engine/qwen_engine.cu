@@ -941,7 +941,7 @@ void QwenEngine::quant_product(const Fp8Linear& w, int M, int epi, void* out, in
     check(pk_rows_fp8(w.w, w.scale, w.K / 128, M, w.N, w.K, quant_rows_, quant_scale_, epi, out, ldo, resid, sm_count_, stream_), "rows_fp8");
     return;
   }
-  const int columns = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+  const int columns = M <= 32 ? 32 : 64;
   const int tiles = epi == 1 ? (w.N / 2 + 63) / 64 : (w.N + 127) / 128;
   // More than 16 rows. Parts of K: the fewest with which the last round of CTAs is about as full as it gets, four 128-wide blocks in a part at least.
   // 40 tiles of a 5120-row projection leave most SMs idle without.

@@ -11,7 +11,8 @@
 //
 // Measured per layer of the MiniMax-M2 shape (256 experts of 3 x 1536 x 3072 in IQ2_XXS, top 8), experts alone: 23 tokens 1860 -> 650 us
 // (kernels that decode in registers), 256 tokens 4590 -> 1215 us (decode to a bf16 scratch, bf16 GEMM), 1500 tokens 4750 -> 1470 us. Bound by
-// the decode's instructions: 0.14 ms of weights at the copy rate. E4M3, 13 rows of 34816 x 5120: 60 us, 3.0 TB/s.
+// the decode's instructions: 0.14 ms of weights at the copy rate. One token's 8 routes: 50 + 32 -> 39 + 26 us with K in parts. E4M3, 40
+// rows of 34816 x 5120: 71 us, 2.5 TB/s.
 //
 //   warps 0-3 (0-7 for 64 columns)  fold: TMEM -> fp32 registers with the block factors, epilogue
 //   next warp                       MMA issuer
@@ -667,15 +668,15 @@ struct StageParams {
   int n_counters;
 };
 
-__global__ void __launch_bounds__(256) quant_stage_rows_kernel(const StageParams p) {
+__global__ void __launch_bounds__(1024) quant_stage_rows_kernel(const StageParams p) {
   extern __shared__ __align__(16) float xs[];      // [K]
   __shared__ float red[40];
-  const int r = blockIdx.x, tid = threadIdx.x;
+  const int r = blockIdx.x, tid = threadIdx.x, stride = blockDim.x * 4;
   if (r == 0)
-    for (int i = tid; i < p.n_counters; i += 256) p.counters[i] = 0u;
+    for (int i = tid; i < p.n_counters; i += blockDim.x) p.counters[i] = 0u;
   const long long src = p.index ? p.index[r] : r;
   float ss = 0.f, mx = 0.f;
-  for (int k = tid * 4; k < p.K; k += 1024) {
+  for (int k = tid * 4; k < p.K; k += stride) {
     float4 v;
     if (p.x_f32) {
       v = *reinterpret_cast<const float4*>((const float*)p.x + src * p.ldx + k);
@@ -697,7 +698,7 @@ __global__ void __launch_bounds__(256) quant_stage_rows_kernel(const StageParams
   if (p.gamma != nullptr) {
     const float rs = rsqrtf(block_sum(ss, red) / (float)p.K + p.eps);
     mx = 0.f;
-    for (int k = tid * 4; k < p.K; k += 1024) {
+    for (int k = tid * 4; k < p.K; k += stride) {
       float4 v = *reinterpret_cast<const float4*>(xs + k);
       float4 g = *reinterpret_cast<const float4*>(p.gamma + k);
       if (p.plus_one) g = make_float4(1.f + g.x, 1.f + g.y, 1.f + g.z, 1.f + g.w);
@@ -721,7 +722,7 @@ __global__ void __launch_bounds__(256) quant_stage_rows_kernel(const StageParams
   if (tid == 0) p.row_scale[r] = down;
   const int pitch = p.mins ? (p.K >> 8) * 320 : p.K;
   __half* out = p.out + (size_t)r * p.terms * pitch;
-  for (int k = tid * 4; k < p.K; k += 1024) {      // K is a multiple of 128: whole warps
+  for (int k = tid * 4; k < p.K; k += stride) {      // K is a multiple of 128: whole warps
     const float4 v = *reinterpret_cast<const float4*>(xs + k);
     const float a[4] = {v.x * up, (p.natural ? v.y : v.z) * up, (p.natural ? v.z : v.y) * up, v.w * up};
     const int at = p.mins ? (k >> 8) * 320 + (k & 255) : k;
@@ -839,7 +840,9 @@ PK_API int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const i
     }
   }
   const StageParams p{x, x_f32, ldx, K, index, gamma, eps, plus_one, add, (pk::bf16*)sum, (pk::bf16*)norm, terms, has_mins(type) ? 1 : 0, type == T_E4M3 ? 1 : 0, (__half*)staged, row_scale, counters, n_counters};
-  quant_stage_rows_kernel<<<rows, 256, smem, stream>>>(p);
+  // a block per row: with few rows a thread per four elements (13 rows of 5120 to 17408: mean 6.2 -> 4.6 us, one of 3072: 3.8 -> 2.9), with many the blocks hide one another
+  const int threads = rows <= 148 ? min(1024, (K / 4 + 31) / 32 * 32) : 256;
+  quant_stage_rows_kernel<<<rows, threads, smem, stream>>>(p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -847,14 +850,15 @@ PK_API int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const i
 // out[t, n] = row_scale[t] * staged[t] . W[g(t), n]: W [n_groups * N] raw rows of `type`; token rows seg[g] .. seg[g + 1] belong to
 // group g (seg null: all `rows` to the one group). epi 0 bf16, 1 SwiGLU bf16, 2 fp32, 3 SwiGLU fp32 (N / 2 gate rows, then as
 // many up rows), 4 bf16 with `resid` added. `columns` 16, 32 or 64 of a tile. splits > 1 needs ws (tiles * splits * columns * 128 floats) and one zeroed
-// counter per tile. E4M3 (type 20): W [N, K] codes, w_scale [ceil(N / 128), w_ld] factors of its 128 x 128 blocks.
+// counter per tile. E4M3 (type 20): W [N, K] codes, w_scale [ceil(N / 128), w_ld] factors of its 128 x 128 blocks;
+// 32 or 64 columns (up to 16 rows are rows_fp8.cu's).
 PK_API int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, int n_groups, int rows, const void* staged, const float* row_scale,
                          int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int splits, float* ws, uint32_t* counters, uint32_t* status,
                          const float* w_scale, int w_ld, int sm_count, cudaStream_t stream) {
   if (W == nullptr || staged == nullptr || row_scale == nullptr || out == nullptr || rows < 1 || N < 1 || n_groups < 1 || n_groups > kMaxGroups ||
       (seg == nullptr && n_groups != 1) || terms < 1 || terms > 2 || epi < 0 || epi > 4 || (epi == OUT_RESID && resid == nullptr) || ((epi & 1) && (N & 1)) || splits < 1 ||
       (splits > 1 && (ws == nullptr || counters == nullptr)) || (columns != 16 && columns != 32 && columns != 64) || pk_quant_stage_pitch(type, K) == 0 ||
-      splits > K / type_k(type) || (type == T_E4M3 && (w_scale == nullptr || terms != 1 || n_groups != 1)) || ((uintptr_t)W & 15) != 0 || ((uintptr_t)staged & 15) != 0)
+      splits > K / type_k(type) || (type == T_E4M3 && (w_scale == nullptr || terms != 1 || n_groups != 1 || columns == 16)) || ((uintptr_t)W & 15) != 0 || ((uintptr_t)staged & 15) != 0)
     return PK_ERR_BAD_ARG;
   const int nblk = K / type_k(type);
   const long long group_bytes = (long long)nblk * type_bytes(type) * N;      // IQ2 blocks are copied by four bytes
@@ -865,7 +869,6 @@ PK_API int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, 
   if (type == T_IQ2_XXS) return launch_shape<T_IQ2_XXS>(columns, terms, staged, rows, p, sms, stream);
   if (type == T_Q4_K) return launch_shape<T_Q4_K>(columns, terms, staged, rows, p, sms, stream);
   if (type == T_Q5_K) return launch_shape<T_Q5_K>(columns, terms, staged, rows, p, sms, stream);
-  if (columns == 16) return launch<T_E4M3, 16, 1>(staged, rows, p, sms, stream);
   if (columns == 32) return launch<T_E4M3, 32, 1>(staged, rows, p, sms, stream);
   return launch<T_E4M3, 64, 1>(staged, rows, p, sms, stream);
 }
