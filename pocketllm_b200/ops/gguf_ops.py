@@ -23,10 +23,10 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
                 eps: float = 1e-6, epi: int = 0) -> torch.Tensor:
     """y = rmsnorm?(x) @ dequant(W)^T for any number of rows.
 
-    Up to `TENSOR_CORE_MIN_ROWS - 1` rows stream the quantised blocks and decode them in registers (groups of up to 8
-    rows per launch). From there on the weight is decoded once into a bf16 scratch and the product runs on the
-    tcgen05 GEMM: one decode instead of one per 8 rows (the reference switches to its prefill kernels for rows > 1,
-    src/components/gguf/quantized_ops.py:9-76)."""
+    Up to `UMMA_MAX_ROWS - 1` rows of the types in `UMMA_TYPES` are decoded inside a tensor-core kernel, once for all rows.
+    Of the other types, up to `TENSOR_CORE_MIN_ROWS - 1` rows decode the blocks in registers (groups of up to 8 rows per
+    launch). Above, the weight is decoded once into a bf16 scratch and the product runs on the tcgen05 GEMM (the
+    reference switches to its prefill kernels for rows > 1, src/components/gguf/quantized_ops.py:9-76)."""
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
     if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name):
@@ -270,8 +270,9 @@ _GROUPED_SCRATCH: dict = {}
 def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, E: int, inter: int,
                              routes: "Routes", *, expert_offset: int = 0, local_experts: int | None = None,
                              out: torch.Tensor | None = None, peer=None) -> torch.Tensor:
-    """Routed experts of this rank on the tensor cores, for steps with many routes (prefill): the rank's experts are decoded
-    to bf16 once per call into a scratch that is reused across layers, token rows are gathered in expert order, and two
+    """Routed experts of this rank on the tensor cores, for steps with many routes (prefill). Types in `UMMA_TYPES` are decoded
+    inside the product up to `UMMA_MAX_ROUTES_PER_EXPERT`; otherwise the rank's experts are decoded to bf16 once per call
+    into a scratch that is reused across layers, token rows are gathered in expert order, and two
     grouped tcgen05 GEMMs (gate|up with the SwiGLU epilogue, then down) run one persistent launch each over every
     (expert, row tile, column block) that has rows; the tile list comes from the route segments on the device. The
     per-token sum runs in route order (bitwise reproducible). Same result as `gguf_moe_forward` up to bf16 rounding of the
@@ -328,8 +329,8 @@ GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local exp
 
 def moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, E: int, inter: int, routes: "Routes", *,
                 limit: float = 0.0, expert_offset: int = 0, local_experts: int | None = None, peer=None) -> torch.Tensor:
-    """Routed experts of this rank, fp32 [T, H]: the grouped tensor-core path for steps with many routes per expert
-    (prefill), the per-route streaming kernels otherwise (decode, clamped SwiGLU)."""
+    """Routed experts of this rank, fp32 [T, H]: the grouped form for steps with many routes per expert (prefill),
+    otherwise (decode, clamped SwiGLU) the form that keeps hidden values in fp32."""
     seg, tok, rw = routes
     local = E if local_experts is None else local_experts
     H = x.shape[1]
