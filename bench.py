@@ -260,8 +260,8 @@ def run_minimax(args) -> dict:
         "value": round(decode_tok_s, 2), "unit": "tok/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round((pre_ms + dec_ms) / args.steps, 3), "higher_is_better": True, "scaling": "strong",
         "vs_baseline": round(decode_tok_s / 7.55, 3),
-        "dtype": "bf16 activations; weights stay GGUF blocks (IQ2_XXS experts, Q5_K attention) decoded in registers for decode and to bf16 "
-                 "tensor-core operands for prefill",
+        "dtype": "bf16 activations; weights stay GGUF blocks (IQ2_XXS experts, Q5_K attention) decoded to exact fp16 integers "
+                 "as tensor-core operands, block factors applied in fp32",
         "data": "synthetic: uniform-random token prompts, random GGUF block payloads made on the device (finite scales), balanced routes",
         "prefill_tok_s": round(prefill_tok_s, 1), "prefill_vs_baseline": round(prefill_tok_s / 106.0, 2),
         "prefill_ms": round(pre_ms / args.steps, 3), "decode_ms_per_token": round(dec_ms / args.steps / decode_len, 4),
