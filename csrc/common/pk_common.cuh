@@ -188,6 +188,10 @@ __device__ __forceinline__ uint2 ld_stream_u2(const void* p) {
   return v;
 }
 
+// Dynamic shared memory that a launch may ask for without opting in: 48 KB hold a block's static arrays (under 1 KB wherever this is
+// used) as well.
+constexpr size_t kPlainSmem = 47 * 1024;
+
 }  // namespace pk
 
 // Per-device one-time set-up of a kernel (cudaFuncSetAttribute applies to the current device only, so a process that

@@ -410,7 +410,7 @@ PK_API int pk_full_qk_norm_rope_append(const void* q, int ldq, const void* k, in
                  (pk::bf16*)q_out, (pk::bf16*)kcache, (pk::bf16*)vcache, ctx_cap};
   const uintptr_t at = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)q_out | (uintptr_t)kcache | (uintptr_t)vcache;
   const size_t smem = (size_t)(Hq > Hkv ? Hq : Hkv) * kD * sizeof(float);
-  if ((at & 15) == 0 && ((ldq | ldk | ldv) & 7) == 0 && (rope_dim & 15) == 0 && smem <= 48 * 1024 && T <= kFullQkVecRows)
+  if ((at & 15) == 0 && ((ldq | ldk | ldv) & 7) == 0 && (rope_dim & 15) == 0 && smem <= kPlainSmem && T <= kFullQkVecRows)
     full_qk_norm_rope_append_vec_kernel<<<dim3(T, 2), kFullQkThreads, smem, stream>>>(p);
   else
     full_qk_norm_rope_append_kernel<<<dim3(T, 2), 256, 0, stream>>>(p);

@@ -874,7 +874,7 @@ PK_API int pk_group_routes(const int* ids, const float* weights, int T, int topk
   int warps = min(32, max(1, (R + 31) / 32));
   while (warps > 4 && (size_t)warps * E * sizeof(int) > 192 * 1024) warps >>= 1;
   const size_t smem = (size_t)warps * E * sizeof(int);
-  if (smem > 48 * 1024) {
+  if (smem > kPlainSmem) {
     static PkDeviceOnce once;
     if (PkDeviceOnceGuard once_guard{once}; once_guard.needed()) {
       if (cudaFuncSetAttribute(group_routes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024) != cudaSuccess) {

@@ -404,8 +404,8 @@ PK_API int pk_rmsnorm(const void* x, const float* parts, int nparts, int M, int 
   const size_t smem = (size_t)K * sizeof(float);
   if (smem > 200 * 1024) return PK_ERR_UNSUPPORTED;
   const bool vec = (K & 7) == 0 && (((uintptr_t)x | (uintptr_t)parts | (uintptr_t)hidden_out | (uintptr_t)gamma | (uintptr_t)y) & 15) == 0;
-  if (smem > 48 * 1024) {
-    // rows beyond 12288 elements only; the attribute is per device, so it is simply set on every such call
+  if (smem > kPlainSmem) {
+    // rows from 12032 elements only; the attribute is per device, so it is simply set on every such call
     if (cudaFuncSetAttribute(vec ? rmsnorm_vec_kernel : rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
       pk_set_last_cuda_error((int)cudaGetLastError());
       return PK_ERR_CUDA;
@@ -429,7 +429,7 @@ PK_API int pk_rmsnorm_quant(const void* x, int M, int K, const float* gamma, int
   NormQuantParams p{(const pk::bf16*)x, M, K, gamma, mode, eps, (pk::bf16*)y, terms, (uint8_t*)q, m_pad, scale_t, s_ld};
   const size_t smem = (size_t)K * sizeof(float);
   if (smem > 200 * 1024) return PK_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024 &&
+  if (smem > kPlainSmem &&
       cudaFuncSetAttribute(rmsnorm_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     pk_set_last_cuda_error((int)cudaGetLastError());
     return PK_ERR_CUDA;
@@ -462,7 +462,7 @@ PK_API int pk_rmsnorm_rs_ag(void* hidden, const float* parts, int world, int ran
   p.wait_ag = *wait_ag;
   const size_t smem = (size_t)K * sizeof(float);
   if (smem > 200 * 1024) return PK_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024 &&
+  if (smem > kPlainSmem &&
       cudaFuncSetAttribute(rmsnorm_rs_ag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     pk_set_last_cuda_error((int)cudaGetLastError());
     return PK_ERR_CUDA;

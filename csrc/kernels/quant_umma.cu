@@ -829,7 +829,7 @@ PK_API int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const i
     return PK_ERR_BAD_ARG;
   const size_t smem = (size_t)K * sizeof(float);
   if (smem > 200 * 1024) return PK_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024) {
+  if (smem > kPlainSmem) {
     static PkDeviceOnce once;
     if (PkDeviceOnceGuard once_guard{once}; once_guard.needed()) {
       if (cudaFuncSetAttribute(quant_stage_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) {
