@@ -66,7 +66,7 @@ struct Params {
   int splits;             // parts of K, added by the last of a tile's CTAs in their order
   float* ws;              // [tile][split][column][128]
   uint32_t* counters;     // [tile], zero between launches
-  uint32_t* status;
+  uint32_t* status;       // first wait that ran out; a launch that finds it set does no work
 };
 
 // IQ2_XXS with few columns has two CTAs per SM, which hide one another's waits; the others have more bytes per weight and one CTA with
@@ -93,6 +93,7 @@ struct __align__(1024) Smem {
   uint64_t grid[PITCH == 68 ? 256 : 1];
   uint64_t full[S::kStages], empty[S::kStages];
   uint64_t acc_full[2], acc_empty[2];
+  uint64_t drained;
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
   uint32_t last;
@@ -303,7 +304,9 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row_tiles = (p.epi & 1) ? ((p.rows >> 1) + 63) / 64 : (p.rows + BM - 1) / BM;
 
+  uint32_t failed = 0;
   if (tid == 0) {
+    if (p.status != nullptr) failed = *(const volatile uint32_t*)p.status;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&sm.full[s], S::kDecWarps + 1);
       mbar_init(&sm.empty[s], 1);
@@ -312,7 +315,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       mbar_init(&sm.acc_full[b], 1);
       mbar_init(&sm.acc_empty[b], S::kFoldWarps);
     }
-    sm.abort_flag = 0;
+    mbar_init(&sm.drained, 1);
     mbar_fence_init();
   }
   for (int g = tid; g < p.n_groups; g += S::kThreads) {
@@ -320,6 +323,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
     sm.prefix[g] = (n + NT / TERMS - 1) / (NT / TERMS);
   }
   __syncthreads();
+  if (tid == 0) sm.abort_flag = failed;      // the load had the barrier's time
   if (warp == 1) {
     // token tiles before each group, 32 groups at a time
     int run = 0;
@@ -350,6 +354,8 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
 
   if (warp < S::kFoldWarps) {
     // ---------------- fold and epilogue ----------------
+    // A wait that ran out makes NaN of this item and the CTA's later ones, and they are counted all the same: the result cannot be
+    // taken for one, and the counters are back at zero when the launch is over. (A SwiGLU limit takes NaN for the limit.)
     const int q = warp & 3, c0 = (warp >> 2) * S::kFoldCols, lr = q * 32 + lane;
     uint32_t blk = 0;
     Item w;
@@ -367,7 +373,8 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       }
       auto factor = [&](int b) { return TYPE == T_E4M3 ? __ldg(ws + b) : ld_half(row + b * BB); };
       float d = factor(w.b0), dm = MINS ? ld_half(row + w.b0 * BB + 2) : 0.f;
-      for (int b = w.b0; b < w.b1; ++b, ++blk) {
+      ok = ok && !__any_sync(0xffffffffu, sm.abort_flag);
+      for (int b = w.b0; ok && b < w.b1; ++b, ++blk) {
         const int nb = min(b + 1, p.nblk - 1);
         const float dn = factor(nb), dmn = MINS ? ld_half(row + nb * BB + 2) : 0.f;
         const int buf = blk & 1;
@@ -398,8 +405,11 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
         d = dn;
         dm = dmn;
       }
+      if (!ok) {
+#pragma unroll
+        for (int c = 0; c < S::kFoldCols; ++c) acc[c] = __uint_as_float(0x7fffffffu);
+      }
       if (p.splits > 1) {
-        // a warp that gave up takes part in the barriers all the same; the CTA leaves together (last = 2)
         float* part = p.ws + ((size_t)w.tile * p.splits + w.split) * NT * BM + lr;
 #pragma unroll
         for (int c = 0; c < S::kFoldCols; ++c) __stcg(part + (size_t)(c0 + c) * BM, acc[c]);
@@ -407,15 +417,14 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
         fold_sync<S::kFoldWarps>();
         if (tid == 0) {
           const uint32_t n = atomicAdd(p.counters + w.tile, 1u);
-          sm.last = sm.abort_flag ? 2u : n == (uint32_t)p.splits - 1u ? 1u : 0u;
-          if (sm.last == 1u) p.counters[w.tile] = 0u;
+          sm.last = n == (uint32_t)p.splits - 1u;
+          if (sm.last) p.counters[w.tile] = 0u;
           __threadfence();
         }
         fold_sync<S::kFoldWarps>();
         const uint32_t last = sm.last;
         fold_sync<S::kFoldWarps>();
-        if (last == 2u) break;
-        if (last == 0u) continue;
+        if (!last) continue;
         __threadfence();
         const float* all = p.ws + (size_t)w.tile * p.splits * NT * BM + lr;
 #pragma unroll
@@ -423,8 +432,6 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
         for (int s = 0; s < p.splits; ++s)
 #pragma unroll
           for (int c = 0; c < S::kFoldCols; ++c) acc[c] += __ldcg(all + ((size_t)s * NT + c0 + c) * BM);
-      } else if (!ok) {
-        break;
       }
       // columns of a token row next to one another
       constexpr int kRows = S::kFoldCols / TERMS;
@@ -477,7 +484,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
     const bool leader = elect_one();
     uint32_t st = 0, ph = 0, blk = 0;
     Item w;
-    bool ok = true;
+    bool ok = !__any_sync(0xffffffffu, sm.abort_flag);
     for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
       for (int b = w.b0; ok && b < w.b1; ++b, ++blk) {
         const int buf = blk & 1;
@@ -514,13 +521,19 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
         }
       }
     }
+    if (!ok) {
+      // gave up: the products in flight end before their tensor memory is freed
+      if (leader) umma_commit(&sm.drained);
+      __syncwarp();
+      for (uint32_t n = 0; n < (1u << 20) && !mbar_try_wait(&sm.drained, 0); ++n) {}
+    }
   } else if (warp == S::kFoldWarps + 1) {
     // ---------------- token tiles ----------------
     if (lane == 0) {
       tma_prefetch_desc(&tmap);
       uint32_t st = 0, ph = 1, issued = 0;
       Item w;
-      bool ok = true;
+      bool ok = !sm.abort_flag;
       for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x)
         for (int x = w.b0 * Fmt<TYPE>::cols; ok && x < w.b1 * Fmt<TYPE>::cols;) {
 #pragma unroll
@@ -600,7 +613,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
     const uint32_t grid = smem_u32(sm.grid);
     uint32_t st = 0, ph = 1, slot = 0;
     Item w;
-    bool ok = true;
+    bool ok = !__any_sync(0xffffffffu, sm.abort_flag);
     for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
       const uint32_t own = tile_row(p, w, lr);
       for (int b = w.b0; ok && b < w.b1; ++b) {

@@ -94,7 +94,7 @@ def test_experts(t13, t2, T, E, topk, limit):
         assert _rel(go.gguf_moe_forward_grouped(x, raw13, raw2, t13, t2, E, I, routes), want) < 5e-4
 
 
-def _e4m3(x, w, scale, epi, resid, columns, splits):
+def _e4m3(x, w, scale, epi, resid, columns, splits, failed=0):
     from ctypes import c_float, c_int, c_void_p
     from pocketllm_b200 import ops
     M, K = x.shape
@@ -105,7 +105,7 @@ def _e4m3(x, w, scale, epi, resid, columns, splits):
     y = torch.full((M, cols), float("nan"), device="cuda", dtype=torch.float32 if epi == 2 else torch.bfloat16)
     tiles = -(-N // 128) if epi != 1 else -(-(N // 2) // 64)
     ws, counters = torch.empty(max(1, tiles * splits * columns * 128), device="cuda"), torch.zeros(tiles, device="cuda", dtype=torch.int32)
-    status = torch.zeros(1, device="cuda", dtype=torch.int32)
+    status = torch.full((1,), failed, device="cuda", dtype=torch.int32)
     ops._check(lib.pk_quant_stage_rows(ops._ptr(x), c_int(0), c_int(K), c_int(K), null, c_int(M), null, c_float(0), c_int(0), null, null, null, c_int(20), c_int(1),
                                        ops._ptr(staged), ops._ptr(factor), null, c_int(0), ops._stream()), "stage")
     if splits == 0:         # the kernel of up to 16 rows
@@ -116,7 +116,7 @@ def _e4m3(x, w, scale, epi, resid, columns, splits):
         ops._check(lib.pk_quant_rows(ops._ptr(w), c_int(20), c_int(N), c_int(K), null, c_int(1), c_int(M), ops._ptr(staged), ops._ptr(factor), c_int(1), c_int(epi),
                                      ops._ptr(y), c_int(cols), ops._ptr(resid), c_float(0), c_int(columns), c_int(splits), ops._ptr(ws), ops._ptr(counters),
                                      ops._ptr(status), ops._ptr(scale), c_int(K // 128), c_int(ops._sm_count()), ops._stream()), "rows")
-    assert int(status) == 0
+    assert int(status) == failed and not counters.any()
     return y
 
 
@@ -136,6 +136,16 @@ def test_e4m3_blocks(M, N, K, splits):
     assert _rel(_e4m3(x, w, scale, 4, resid, columns, splits), want + resid.double()) < 2 ** -8
     a, b = want.chunk(2, -1)
     assert _rel(_e4m3(x, w, scale, 1, None, columns, splits), torch.nn.functional.silu(a) * b) < 2 ** -8
+
+
+@pytest.mark.parametrize("splits", [1, 3])
+def test_after_a_wait_that_ran_out(splits):
+    """A product that finds the error word set gives NaN in every place and leaves the counters of its parts at zero."""
+    w = torch.randn(300, 768, device="cuda").to(torch.float8_e4m3fn)
+    x, scale = torch.randn(20, 768, device="cuda").to(torch.bfloat16), torch.ones(3, 6, device="cuda")
+    assert torch.isnan(_e4m3(x, w, scale, 2, None, 32, splits, failed=31)).all()
+    assert torch.isnan(_e4m3(x, w, scale, 1, None, 32, splits, failed=31)).all()
+    assert _rel(_e4m3(x, w, scale, 2, None, 32, splits), x.double() @ w.double().T) < TOL
 
 
 @pytest.mark.parametrize("M", [1, 15, 17, 100])
