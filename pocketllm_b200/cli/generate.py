@@ -116,6 +116,8 @@ def main(argv=None) -> int:
                     lg = dsv4_rt.forward_logits([t])
                     lg = lg[0] if lg.dim() > 1 else lg
                     t = sample_token(lg.float().cpu(), SamplingParams(max_tokens=1, temperature=args.temperature, top_p=args.top_p), gen)
+                    if hasattr(dsv4_rt, "combine"):
+                        dsv4_rt.combine.check_step("cuda")
                 else:
                     t = step(t)
         dt = time.perf_counter() - t0

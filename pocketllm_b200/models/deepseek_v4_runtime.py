@@ -168,6 +168,8 @@ class DSV4Runtime:
         self.rank, self.world = rank, world
         from ..parallel.combine import ExpertCombine
         self.combine = ExpertCombine(world, group, capacity=max_rows * cfg.dim, use_peer=use_peer_allreduce)
+        if raw_experts is not None:
+            self.combine.products = torch.zeros(1, device="cuda", dtype=torch.int32)
         per = cfg.n_routed_experts // world
         e_lo, e_hi = rank * per, (rank + 1) * per
         self.max_context = max_context or cfg.max_seq_len
@@ -280,7 +282,8 @@ class DSV4Runtime:
         routes = gk.group_routes(ids, w, cfg.n_routed_experts)
         seg, tok, rw = routes
         y = gk.gguf_moe_forward(x, self.w_flat(b.w13), self.w_flat(b.w2), b.type13, b.type2, cfg.n_routed_experts, cfg.moe_inter_dim,
-                                seg, tok, rw, limit=cfg.swiglu_limit, expert_offset=b.e_lo, local_experts=b.e_hi - b.e_lo, routes=routes)
+                                seg, tok, rw, limit=cfg.swiglu_limit, expert_offset=b.e_lo, local_experts=b.e_hi - b.e_lo, routes=routes,
+                                status=self.combine.products)
         y = self.combine(y)
         hs = ops.silu_mul(b.s_w13(x), cfg.swiglu_limit)
         return y, b.s_w2(hs, f32=True)
@@ -363,7 +366,7 @@ class DSV4Runtime:
 
     def forward_rows(self, tokens: Sequence[int]) -> list[int]:
         nxt = self.forward_logits(tokens).argmax(-1).tolist()
-        # collective verdict on the peer all-reduces of this forward: raises on every rank, no token is returned
+        # collective verdict on the peer all-reduces and the expert products of this forward: raises on every rank, no token is returned
         self.combine.check_step("cuda")
         self.last_token = nxt[-1]
         return nxt

@@ -399,6 +399,7 @@ class GLMDSAModel:
                                                      slots=expert_slots, device=self.device)
         self.cache = [{"latent": [], "krope": [], "ki": []} for _ in range(c.n_layers)]
         self.max_context, self.pos = max_context, 0
+        self._word = go.StepWord(self.device)
 
     def _combine(self, y: torch.Tensor) -> torch.Tensor:
         """Sum the ranks' expert outputs (peer-memory all-reduce for small payloads, NCCL for large ones)."""
@@ -420,10 +421,10 @@ class GLMDSAModel:
         go, xb = self.go, x.to(torch.bfloat16).contiguous()
         N = self.shapes[name][0]
         if swiglu_with is not None:
-            g = go.gguf_linear(xb, self.raw[name], self.types[name], N, gamma=gamma, eps=eps, epi=2)
-            u = go.gguf_linear(xb, self.raw[swiglu_with], self.types[swiglu_with], N, gamma=gamma, eps=eps, epi=2)
+            g = go.gguf_linear(xb, self.raw[name], self.types[name], N, gamma=gamma, eps=eps, epi=2, status=self._word.status)
+            u = go.gguf_linear(xb, self.raw[swiglu_with], self.types[swiglu_with], N, gamma=gamma, eps=eps, epi=2, status=self._word.status)
             return (torch.nn.functional.silu(g) * u).to(torch.bfloat16)
-        return go.gguf_linear(xb, self.raw[name], self.types[name], N, gamma=gamma, eps=eps, epi=2)
+        return go.gguf_linear(xb, self.raw[name], self.types[name], N, gamma=gamma, eps=eps, epi=2, status=self._word.status)
 
     def moe(self, i: int, xn: torch.Tensor) -> torch.Tensor:
         c, go, b = self.cfg, self.go, f"blk.{i}."
@@ -437,14 +438,14 @@ class GLMDSAModel:
             ids_l = torch.where(mine, ids - self.e_start, torch.zeros_like(ids)).contiguous()
             wt_l = torch.where(mine, wt, torch.zeros_like(wt)).contiguous()
             y = staged_moe_forward(self.staging[i], xb, ids_l, wt_l, self.types[b + "ffn_gate_exps.weight"],
-                                   self.types[b + "ffn_down_exps.weight"], self.inter_local)
+                                   self.types[b + "ffn_down_exps.weight"], self.inter_local, status=self._word.status)
             if self.world > 1:
                 self._combine(y)
             return y
         routes = go.group_routes(ids, wt, c.n_experts)
         y = go.moe_forward(xb, self.raw[b + "w13"], self.raw[b + "ffn_down_exps.weight"], self.types[b + "ffn_gate_exps.weight"],
                            self.types[b + "ffn_down_exps.weight"], c.n_experts, self.inter_local, routes,
-                           expert_offset=self.e_start, local_experts=self.e_local)
+                           expert_offset=self.e_start, local_experts=self.e_local, status=self._word.status)
         if self.world > 1:
             self._combine(y)
         return y
@@ -527,18 +528,26 @@ class GLMDSAModel:
         self.pos += T
         return lin(h[-1:], "output.weight", gamma=w["output_norm.weight"], eps=c.norm_eps).float()[0]
 
-    def _checked(self, token: int) -> int:
-        """The step's token, or `StepFailed` on every rank when a peer all-reduce timed out (collective check)."""
+    def check_step(self, failed: int | None = None) -> None:
+        """Raises `StepFailed`, on every rank, when a peer all-reduce or a product of the step gave up waiting (collective). `failed`:
+        the error word of the products where it has been read; otherwise it is read here."""
+        if failed is None:
+            failed = self._word.read()[1]
         if self._combiner is not None:
-            self._combiner.check_step(self.device)
-        return token
+            self._combiner.check_step(self.device, failed)
+        elif failed:
+            from ..parallel.combine import StepFailed
+            raise StepFailed(f"a product gave up waiting (status {failed}): the step is discarded")
 
     def forward_logits(self, tokens: Sequence[int]) -> torch.Tensor:
         """fp32 logits after feeding `tokens` at the current position (for host-side sampling and log-probabilities)."""
         return self.forward(tokens)
 
     def prefill(self, tokens: Sequence[int]) -> int:
-        return self._checked(int(torch.argmax(self.forward(tokens))))
+        self._word.pick(self.forward(tokens))
+        token, failed = self._word.read()
+        self.check_step(failed)
+        return token
 
     def decode_one(self, token: int) -> int:
-        return self._checked(int(torch.argmax(self.forward([token]))))
+        return self.prefill([token])

@@ -326,6 +326,7 @@ class MiniMaxM2Model:
         if any("cache" in L for L in self.layers):
             self.use_graph = False     # staged experts: which experts a step needs is read on the host
         self._graph = None
+        self._word = self.go.StepWord(self.device)
 
     def _combine(self, y: torch.Tensor) -> torch.Tensor:
         """Sum the ranks' expert outputs (peer-memory all-reduce for small payloads, NCCL for large ones)."""
@@ -371,7 +372,7 @@ class MiniMaxM2Model:
         """The forward pass with the positions given as a device tensor (nothing here depends on host-side position
         arithmetic, so a single-token call can be captured into a CUDA graph)."""
         from .. import ops
-        c, go = self.cfg, self.go
+        c, go, st = self.cfg, self.go, self._word.status
         T = tokens.numel()
         h = go.gguf_dequant_rows(self.embed, self.types["token_embd.weight"], c.dim, tokens)
         for i, L in enumerate(self.layers):
@@ -379,18 +380,18 @@ class MiniMaxM2Model:
             ta = self.types[b + "attn_q.weight"]
             nq, nkv = c.n_heads * c.head_dim, c.n_kv_heads * c.head_dim
             if "qkv" in L:                                       # one projection for q, k and v (same block type): rows q | k | v
-                qkv = go.gguf_linear(h, L["qkv"], ta, nq + 2 * nkv, gamma=L["attn_norm"], eps=c.norm_eps)
+                qkv = go.gguf_linear(h, L["qkv"], ta, nq + 2 * nkv, gamma=L["attn_norm"], eps=c.norm_eps, status=st)
                 q, k, v = qkv[:, :nq], qkv[:, nq:nq + nkv], qkv[:, nq + nkv:]
             else:
-                q = go.gguf_linear(h, L["q"], ta, nq, gamma=L["attn_norm"], eps=c.norm_eps)
-                k = go.gguf_linear(h, L["k"], self.types[b + "attn_k.weight"], nkv, gamma=L["attn_norm"], eps=c.norm_eps)
-                v = go.gguf_linear(h, L["v"], self.types[b + "attn_v.weight"], nkv, gamma=L["attn_norm"], eps=c.norm_eps)
+                q = go.gguf_linear(h, L["q"], ta, nq, gamma=L["attn_norm"], eps=c.norm_eps, status=st)
+                k = go.gguf_linear(h, L["k"], self.types[b + "attn_k.weight"], nkv, gamma=L["attn_norm"], eps=c.norm_eps, status=st)
+                v = go.gguf_linear(h, L["v"], self.types[b + "attn_v.weight"], nkv, gamma=L["attn_norm"], eps=c.norm_eps, status=st)
             # whole-vector RMS with per-element gamma, rotation at `pos`, k / v appended to the caches: one kernel
             q = ops.full_qk_norm_rope_append(q, k, v, pos, L["q_norm"], L["k_norm"], self.rope_cos, self.rope_sin, L["kc"], L["vc"],
                                              n_heads=c.n_heads, n_kv_heads=c.n_kv_heads, rope_dim=c.rope_dim, eps=c.norm_eps)
             # prefill chunks (consecutive positions) through the tcgen05 flash kernel, decode steps through the split kernel
             o = ops.gqa_prefill(q, L["kc"], L["vc"], pos) if T >= 16 else ops.gqa_decode(q, L["kc"], L["vc"], pos, nsplit=1 if T > 8 else 8)
-            att = go.gguf_linear(o, L["o"], self.types[b + "attn_output.weight"], c.dim, epi=2)
+            att = go.gguf_linear(o, L["o"], self.types[b + "attn_output.weight"], c.dim, epi=2, status=st)
             before, h = h, torch.empty_like(h)                   # h <- bf16(h + att), one rounding, on the way into the norm
             xn = ops.rmsnorm(before, L["ffn_norm"], mode=2, eps=c.norm_eps, parts=att.unsqueeze(0), hidden_out=h)
             ids, wt = go.router_topk(xn, L["router"], c.n_experts_used, bias=L["bias"], score_func="sigmoid", norm_topk=True)
@@ -406,7 +407,7 @@ class MiniMaxM2Model:
                 mine = (ids >= self.e_start) & (ids < self.e_start + self.e_local)
                 y = staged_moe_forward(L["cache"], xn, torch.where(mine, ids - self.e_start, torch.zeros_like(ids)).contiguous(),
                                        torch.where(mine, wt, torch.zeros_like(wt)).contiguous(), self.types[b + "ffn_gate_exps.weight"],
-                                       self.types[b + "ffn_down_exps.weight"], c.expert_inter)
+                                       self.types[b + "ffn_down_exps.weight"], c.expert_inter, status=st)
                 if self.world > 1:
                     self._combine(y)
                 h = ops.residual_add(h, y)
@@ -414,33 +415,42 @@ class MiniMaxM2Model:
             routes = go.group_routes(ids, wt, c.n_experts)
             # many routes per expert (prefill): grouped tensor-core GEMMs; else the per-route streaming kernels
             y = go.moe_forward(xn, L["w13"], L["w2"], self.types[b + "ffn_gate_exps.weight"], self.types[b + "ffn_down_exps.weight"],
-                               c.n_experts, c.expert_inter, routes, expert_offset=self.e_start, local_experts=self.e_local, peer=self._peer())
+                               c.n_experts, c.expert_inter, routes, expert_offset=self.e_start, local_experts=self.e_local, peer=self._peer(), status=st)
             if self.world > 1 and not routes.combined:
                 self._combine(y)
             h = ops.residual_add(h, y)
-        return go.gguf_linear(h[-1:], self.head, self.types["output.weight"], c.vocab_size, gamma=self.final_norm, eps=c.norm_eps, epi=2)[0]
+        return go.gguf_linear(h[-1:], self.head, self.types["output.weight"], c.vocab_size, gamma=self.final_norm, eps=c.norm_eps, epi=2, status=st)[0]
 
     def forward_logits(self, tokens: Sequence[int]) -> torch.Tensor:
         """fp32 logits after feeding `tokens` at the current position (for host-side sampling and log-probabilities)."""
         return self.forward(torch.tensor(list(tokens), dtype=torch.int32, device=self.device))
 
     # protocol of the generic generation runtime
-    def _checked(self, token: int) -> int:
-        """The step's token, or `StepFailed` on every rank when a peer all-reduce timed out (collective check; the
-        token was read from the device just before, so the step is complete)."""
+    def check_step(self, failed: int | None = None) -> None:
+        """Raises `StepFailed`, on every rank, when a peer all-reduce or a product of the step gave up waiting (collective). `failed`:
+        the error word of the products where it has been read; otherwise it is read here."""
+        if failed is None:
+            failed = self._word.read()[1]
         if self._combiner is not None:
-            self._combiner.check_step(self.device)
+            self._combiner.check_step(self.device, failed)
+        elif failed:
+            from ..parallel.combine import StepFailed
+            raise StepFailed(f"a product gave up waiting (status {failed}): the step is discarded")
+
+    def _token(self) -> int:
+        token, failed = self._word.read()
+        self.check_step(failed)
         return token
 
     def prefill(self, tokens: Sequence[int]) -> int:
         t = torch.tensor(list(tokens), dtype=torch.int32, device=self.device)
-        return self._checked(int(torch.argmax(self.forward(t))))
+        self._word.pick(self.forward(t))
+        return self._token()
 
     @torch.no_grad()
     def _capture_decode(self) -> None:
         self._tok_buf = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._pos_buf = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self._next_buf = torch.zeros((), dtype=torch.int64, device=self.device)
         self._pos_buf.fill_(self.pos)
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream(self.device))
@@ -450,12 +460,12 @@ class MiniMaxM2Model:
         torch.cuda.synchronize(self.device)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
-            self._next_buf.copy_(torch.argmax(self._forward_at(self._tok_buf, self._pos_buf)))
+            self._word.pick(self._forward_at(self._tok_buf, self._pos_buf))
         self._graph = g
 
     def decode_one(self, token: int) -> int:
         if not self.use_graph:
-            return self._checked(int(torch.argmax(self.forward(torch.tensor([token], dtype=torch.int32, device=self.device)))))
+            return self.prefill([token])
         if self.pos + 1 > self.max_context:
             raise ValueError("context exceeds max_context")
         if self._graph is None:
@@ -464,9 +474,8 @@ class MiniMaxM2Model:
         self._pos_buf.fill_(self.pos)
         self._graph.replay()
         self.pos += 1
-        nxt = int(self._next_buf)
         try:
-            return self._checked(nxt)
+            return self._token()
         except TimeoutError:
-            self._graph = None     # the captured graph holds the peer all-reduce; recapture on the NCCL path
+            self._graph = None     # the captured graph may hold the peer all-reduce; recapture on the NCCL path
             raise

@@ -132,7 +132,7 @@ class ExpertStagingCache:
 
 
 def staged_moe_forward(cache: ExpertStagingCache, x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, type13: str, type2: str,
-                       inter: int, *, limit: float = 0.0, w13: str = "w13", w2: str = "w2") -> torch.Tensor:
+                       inter: int, *, limit: float = 0.0, w13: str = "w13", w2: str = "w2", status: torch.Tensor | None = None) -> torch.Tensor:
     """Routed experts through the staging cache: y [T, H] fp32. Steps whose distinct experts exceed the slots run in waves."""
     from ..ops import gguf_ops as go
     T, H = x.shape
@@ -144,5 +144,5 @@ def staged_moe_forward(cache: ExpertStagingCache, x: torch.Tensor, ids: torch.Te
         routes = go.group_routes(slot_ids, weights[lo:hi].contiguous(), cache.lru.n)
         seg, tok, rw = routes
         go.gguf_moe_forward(x[lo:hi].contiguous(), cache.slab[w13].view(-1), cache.slab[w2].view(-1), type13, type2, cache.lru.n, inter, seg, tok, rw,
-                            limit=limit, out=y[lo:hi], routes=routes)
+                            limit=limit, out=y[lo:hi], routes=routes, status=status)
     return y

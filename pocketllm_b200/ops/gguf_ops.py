@@ -20,8 +20,12 @@ def row_bytes(type_name: str, K: int) -> int:
 
 
 def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *, gamma: torch.Tensor | None = None,
-                eps: float = 1e-6, epi: int = 0) -> torch.Tensor:
+                eps: float = 1e-6, epi: int = 0, status: torch.Tensor | None = None) -> torch.Tensor:
     """y = rmsnorm?(x) @ dequant(W)^T for any number of rows.
+
+    `status` (int32 [1], here and in the expert functions): the first bounded wait that ran out is recorded there. A product of
+    `UMMA_TYPES` whose wait ran out gives NaN, and so does one that finds the word set; its owner reads the word once per step
+    (`StepWord`) and clears it.
 
     Up to `UMMA_MAX_ROWS - 1` rows of the types in `UMMA_TYPES` are decoded inside a tensor-core kernel, once for all rows.
     Of the other types, up to `TENSOR_CORE_MIN_ROWS - 1` rows decode the blocks in registers (groups of up to 8 rows per
@@ -30,12 +34,12 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
     if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name):
-        return _umma_linear(_aligned(x), w_raw, type_name, N, _aligned(gamma), eps, epi)
+        return _umma_linear(_aligned(x), w_raw, type_name, N, _aligned(gamma), eps, epi, status)
     if M >= TENSOR_CORE_MIN_ROWS and K % 64 == 0 and (epi != 1 or (N // 2) % 128 == 0):
         from . import gemm_bf16, rmsnorm, EPI_BF16, EPI_SWIGLU, EPI_F32
         w = _dequant_scratch(w_raw, type_name, N, K)
         xin = x.contiguous() if gamma is None else rmsnorm(x.contiguous(), gamma, mode=2, eps=eps)
-        return gemm_bf16(xin, w, epi={0: EPI_BF16, 1: EPI_SWIGLU, 2: EPI_F32}[epi])
+        return gemm_bf16(xin, w, epi={0: EPI_BF16, 1: EPI_SWIGLU, 2: EPI_F32}[epi], status=status)
     y = torch.empty(M, ncols, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
     step = max(1, min(8, (184 * 1024) // (K * 4)))
     step = 8 if step >= 8 else 4 if step >= 4 else 2 if step >= 2 else 1
@@ -55,7 +59,6 @@ UMMA_TYPES = frozenset({"iq2_xxs", "q4_k", "q5_k"})
 UMMA_MAX_ROWS = 257
 UMMA_SPLIT_ROUTES = 64
 UMMA_MAX_GROUPS = 512
-_status: dict = {}
 
 
 def _umma_takes(w_raw: torch.Tensor, type_name: str, groups: int = 1) -> bool:
@@ -63,11 +66,23 @@ def _umma_takes(w_raw: torch.Tensor, type_name: str, groups: int = 1) -> bool:
     return type_name in UMMA_TYPES and w_raw.data_ptr() % 16 == 0 and w_raw.numel() % (4 * groups) == 0 and w_raw.numel() // groups < 1 << 32
 
 
-def _umma_status(dev) -> torch.Tensor:
-    """Error word of the bounded waits."""
-    if dev.index not in _status:
-        _status[dev.index] = torch.zeros(1, device=dev, dtype=torch.int32)
-    return _status[dev.index]
+class StepWord:
+    """A step's token and the error word of its products in one device buffer, so that one copy reads both."""
+
+    def __init__(self, device):
+        self.buf = torch.zeros(2, dtype=torch.int64, device=device)
+        self.status = self.buf.view(torch.int32)[2:3]
+
+    def pick(self, logits: torch.Tensor) -> None:
+        """The greedy token of `logits` [vocab] goes into the buffer."""
+        torch.argmax(logits, dim=0, out=self.buf[0])
+
+    def read(self) -> tuple[int, int]:
+        """(token, error word); the word is cleared when it was set."""
+        token, failed = self.buf.tolist()
+        if failed:
+            self.status.zero_()
+        return token, failed
 
 
 def _aligned(t: torch.Tensor | None) -> torch.Tensor | None:
@@ -85,6 +100,7 @@ class _Staged:
                  ws_floats: int = 0):
         K = x.shape[1]
         pitch = _lib.kernels().pk_quant_stage_pitch(c_int(DEVICE_TYPE[type_name]), c_int(K))
+        counters += 1       # the last one: the product's error word where the caller has none
         sizes = (rows * terms * pitch * 2, rows * 4, counters * 4, ws_floats * 4)
         offs, at = [], 0
         for n in sizes:
@@ -94,6 +110,7 @@ class _Staged:
         self.rows, self.terms = rows, terms
         p = self.buf.data_ptr()
         self.data, self.scale, self.counters, self.ws = (c_void_p(p + o) for o in offs)
+        self.status = c_void_p(p + offs[2] + 4 * counters - 4)
         _check(_lib.kernels().pk_quant_stage_rows(_ptr(x), c_int(int(x.dtype == torch.float32)), c_int(x.stride(0)), c_int(K), _ptr(index), c_int(rows),
                                                  _ptr(gamma), c_float(eps), c_int(0), c_void_p(0), c_void_p(0), c_void_p(0),
                                                  c_int(DEVICE_TYPE[type_name]), c_int(terms), self.data, self.scale, self.counters, c_int(counters),
@@ -101,10 +118,10 @@ class _Staged:
 
 
 def _umma(st: _Staged, w_raw: torch.Tensor, type_name: str, N: int, K: int, seg, groups: int, epi: int, out: torch.Tensor, limit: float, columns: int,
-          splits: int) -> None:
+          splits: int, status: torch.Tensor | None) -> None:
     _check(_lib.kernels().pk_quant_rows(_ptr(w_raw), c_int(DEVICE_TYPE[type_name]), c_int(N), c_int(K), _ptr(seg), c_int(groups), c_int(st.rows), st.data,
                                        st.scale, c_int(st.terms), c_int(epi), _ptr(out), c_int(out.stride(0)), c_void_p(0), c_float(limit), c_int(columns),
-                                       c_int(splits), st.ws, st.counters, _ptr(_umma_status(out.device)), c_void_p(0), c_int(0),
+                                       c_int(splits), st.ws, st.counters, st.status if status is None else _ptr(status), c_void_p(0), c_int(0),
                                        c_int(_sm_count()), _stream()), "pk_quant_rows")
 
 
@@ -124,19 +141,20 @@ def _umma_slots(type_name: str, columns: int) -> int:
     return _sm_count() * (2 if type_name == "iq2_xxs" and columns < 64 else 1)      # resident CTAs of the kernel
 
 
-def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, gamma, eps: float, epi: int) -> torch.Tensor:
+def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, gamma, eps: float, epi: int,
+                 status: torch.Tensor | None) -> torch.Tensor:
     M, K = x.shape
     columns = 16 if M <= 16 else 32 if M <= 32 else 64
     tiles = (-(-(N // 2) // 64) if epi == 1 else -(-N // 128)) * -(-M // columns)
     splits = _umma_splits(tiles, K, _umma_slots(type_name, columns))
     st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
     y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
-    _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits)
+    _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits, status)
     return y
 
 
 def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, inter: int, routes: "Routes", limit: float,
-                  E: int, expert_offset: int, local: int, terms: int) -> torch.Tensor:
+                  E: int, expert_offset: int, local: int, terms: int, status: torch.Tensor | None) -> torch.Tensor:
     """fp32 [R, H]: every route's expert output, without its weight. `terms`: fp16 terms that a hidden value is multiplied as."""
     seg, tok, _ = routes
     H, R, dev = x.shape[1], tok.numel(), x.device
@@ -153,7 +171,7 @@ def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, 
             splits = _umma_splits(max(1, min(R, local)) * row_tiles, K, _umma_slots(type_name, c))
         tiles = (min(R, local) + R * t // c) * row_tiles if splits > 1 else 0
         st = _Staged(x, type_name, R, t, index=index, counters=tiles, ws_floats=tiles * splits * c * 128)
-        _umma(st, w_raw, type_name, N, K, seg, local, epi, out, limit, c, splits)
+        _umma(st, w_raw, type_name, N, K, seg, local, epi, out, limit, c, splits, status)
 
     h = torch.empty(R, inter, device=dev, dtype=torch.float32)
     y = torch.empty(R, H, device=dev, dtype=torch.float32)
@@ -233,7 +251,8 @@ def group_routes(ids: torch.Tensor, weights: torch.Tensor, E: int) -> Routes:
 
 def gguf_moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, E: int, inter: int,
                      seg: torch.Tensor, tok: torch.Tensor, rw: torch.Tensor, *, limit: float = 0.0, expert_offset: int = 0,
-                     local_experts: int | None = None, out: torch.Tensor | None = None, routes: "Routes | None" = None) -> torch.Tensor:
+                     local_experts: int | None = None, out: torch.Tensor | None = None, routes: "Routes | None" = None,
+                     status: torch.Tensor | None = None) -> torch.Tensor:
     """Routed experts of this rank accumulated into fp32 `out` [T, H] (zeroed when not given). With `routes` (the object
     `group_routes` returned) the per-token sum runs in a fixed order and the result is bitwise reproducible; without it
     the routes are added with atomics."""
@@ -244,7 +263,7 @@ def gguf_moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tenso
         out = torch.zeros(T, H, device=x.device, dtype=torch.float32)
     if routes is not None and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
         # hidden values in two fp16 terms: as good as the fp32 values of the kernels that decode in registers
-        y = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, limit, E, expert_offset, local, 2)
+        y = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, limit, E, expert_offset, local, 2, status)
         return _reduce_routes(y, routes, x.shape, expert_offset, local, out)
     hbuf = torch.empty(R, inter, device=x.device, dtype=torch.float32)
     if routes is not None:
@@ -269,7 +288,7 @@ _GROUPED_SCRATCH: dict = {}
 
 def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, E: int, inter: int,
                              routes: "Routes", *, expert_offset: int = 0, local_experts: int | None = None,
-                             out: torch.Tensor | None = None, peer=None) -> torch.Tensor:
+                             out: torch.Tensor | None = None, peer=None, status: torch.Tensor | None = None) -> torch.Tensor:
     """Routed experts of this rank on the tensor cores, for steps with many routes (prefill). Types in `UMMA_TYPES` are decoded
     inside the product up to `UMMA_MAX_ROUTES_PER_EXPERT`; otherwise the rank's experts are decoded to bf16 once per call
     into a scratch that is reused across layers, token rows are gathered in expert order, and two
@@ -288,7 +307,7 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
         out = torch.zeros(T, H, device=dev, dtype=torch.float32)
     K = _lib.kernels()
     if R <= UMMA_MAX_ROUTES_PER_EXPERT * E and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
-        ybuf = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, 0.0, E, expert_offset, local, 1)
+        ybuf = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, 0.0, E, expert_offset, local, 1, status)
     else:
         key = (dev.index, local, H, inter)
         sc = _GROUPED_SCRATCH.get(key)
@@ -304,7 +323,8 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
         xg = x.index_select(0, tok.long())                                   # [R, H] rows in expert order
         hbuf = torch.empty(R, inter, device=dev, dtype=torch.bfloat16)
         ybuf = torch.empty(R, H, device=dev, dtype=torch.float32)
-        status = torch.zeros(1, device=dev, dtype=torch.int32)
+        if status is None:
+            status = torch.zeros(1, device=dev, dtype=torch.int32)
         segl = seg[expert_offset:]
         _check(K.pk_gemm_bf16_grouped(_ptr(xg), c_int(H), _ptr(w13), _ptr(segl), c_int(local), c_int(R), c_int(2 * inter), c_int(H), c_int(EPI_SWIGLU),
                                       _ptr(hbuf), c_int(inter), _ptr(status), c_int(_sm_count()), _stream()), "pk_gemm_bf16_grouped(w13)")
@@ -328,7 +348,8 @@ GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local exp
 
 
 def moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, E: int, inter: int, routes: "Routes", *,
-                limit: float = 0.0, expert_offset: int = 0, local_experts: int | None = None, peer=None) -> torch.Tensor:
+                limit: float = 0.0, expert_offset: int = 0, local_experts: int | None = None, peer=None,
+                status: torch.Tensor | None = None) -> torch.Tensor:
     """Routed experts of this rank, fp32 [T, H]: the grouped form for steps with many routes per expert (prefill),
     otherwise (decode, clamped SwiGLU) the form that keeps hidden values in fp32."""
     seg, tok, rw = routes
@@ -336,10 +357,10 @@ def moe_forward(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, ty
     H = x.shape[1]
     if (limit == 0.0 and tok.numel() >= GROUPED_MIN_ROUTES_PER_EXPERT * local and inter % 128 == 0 and H % 128 == 0 and local <= 512):
         return gguf_moe_forward_grouped(x, w13_raw, w2_raw, type13, type2, E, inter, routes, expert_offset=expert_offset, local_experts=local,
-                                        peer=peer)
+                                        peer=peer, status=status)
     routes.combined = False
     return gguf_moe_forward(x, w13_raw, w2_raw, type13, type2, E, inter, seg, tok, rw, limit=limit, expert_offset=expert_offset,
-                            local_experts=local, routes=routes)
+                            local_experts=local, routes=routes, status=status)
 
 
 def gguf_dequant_rows(w_raw: torch.Tensor, type_name: str, K: int, rows: torch.Tensor | None = None, *, nrows: int | None = None,

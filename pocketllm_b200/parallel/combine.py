@@ -8,7 +8,8 @@ A peer wait that runs out leaves a sticky status word on the rank that waited; l
 return without reducing, so the step's result is wrong on at least one rank. `check_step()` is therefore called by
 the model runtimes once per forward, after the step's device synchronisation and before any token is returned: it
 takes the MAX of the status words over the group, so every rank reaches the same verdict, and on a failure every
-rank clears its word, drops the peer path (NCCL from then on) and raises `StepFailed`. Reference behaviour:
+rank clears its word, drops the peer path (NCCL from then on) and raises `StepFailed`. The error word of the step's quantised
+products (`ops.gguf_ops`) takes part in the same verdict and leaves the peer path as it is. Reference behaviour:
 src/models/deepseek_v4/runtime.py:4191-4196 (custom all-reduce timeout -> NCCL)."""
 from __future__ import annotations
 
@@ -19,7 +20,7 @@ import torch.distributed as dist
 
 
 class StepFailed(TimeoutError):
-    """The current step must be discarded: a peer all-reduce of some rank gave up waiting."""
+    """The current step must be discarded: a peer all-reduce or a product of some rank gave up waiting."""
 
 
 class ExpertCombine:
@@ -27,6 +28,7 @@ class ExpertCombine:
                  multimem_min_floats: int | None = None, mm=None):
         """`peer` / `mm`: objects with `all_reduce`, `status(clear=False)` and `capacity` (tests inject them)."""
         self.world, self.group = world, group
+        self.products: torch.Tensor | None = None        # error word of the step's products where the runtime has one
         self.peer = peer
         self.mm = mm
         self.calls = {"peer": 0, "nccl": 0, "multimem": 0}
@@ -59,26 +61,36 @@ class ExpertCombine:
         dist.all_reduce(y, group=self.group)
         return y
 
-    def check_step(self, device: torch.device | str | None = None) -> None:
+    def check_step(self, device: torch.device | str | None = None, failed: int | None = None) -> None:
         """Collective over the group (every rank calls it once per forward, also ranks whose own word is clean).
-        Raises `StepFailed` on every rank when any rank's peer wait ran out; the peer path is off afterwards."""
-        if self.world == 1 or (self.peer is None and self.mm is None):
+        Raises `StepFailed` on every rank when any rank's wait ran out; after a peer wait the peer path is off. `failed`: the products'
+        error word where the caller has read (and cleared) it already."""
+        if failed is None and self.products is not None:
+            failed = int(self.products)
+            if failed:
+                self.products.zero_()
+        if self.world == 1:
+            if failed:
+                raise StepFailed(f"a product gave up waiting (status {failed}): the step is discarded")
+            return
+        if self.peer is None and self.mm is None and failed is None:
             return
         local = max(int(self.peer.status()) if self.peer is not None else 0, int(self.mm.status()) if self.mm is not None else 0)
         if device is None:
             device = "cuda" if dist.get_backend(self.group) == "nccl" else "cpu"
-        word = torch.tensor([local], dtype=torch.int32, device=device)
-        dist.all_reduce(word, op=dist.ReduceOp.MAX, group=self.group)
-        worst = int(word.item())
-        if worst == 0:
-            return
-        for path in (self.peer, self.mm):
-            if path is not None:
-                path.status(clear=True)
-        self.peer = self.mm = None
-        self.fallbacks += 1
-        raise StepFailed(f"a peer all-reduce gave up waiting (status {worst}, this rank {local}): the step is discarded "
-                         "and the following steps use NCCL")
+        words = torch.tensor([local, failed or 0], dtype=torch.int32, device=device)
+        dist.all_reduce(words, op=dist.ReduceOp.MAX, group=self.group)
+        worst, product = words.tolist()
+        if worst:
+            for path in (self.peer, self.mm):
+                if path is not None:
+                    path.status(clear=True)
+            self.peer = self.mm = None
+            self.fallbacks += 1
+            raise StepFailed(f"a peer all-reduce gave up waiting (status {worst}, this rank {local}): the step is discarded "
+                             "and the following steps use NCCL")
+        if product:
+            raise StepFailed(f"a product gave up waiting (status {product}, this rank {failed or 0}): the step is discarded")
 
     # kept for callers of the earlier, rank-local API
     def check(self) -> None:

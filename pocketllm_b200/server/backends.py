@@ -90,6 +90,8 @@ class GGUFBackend:
             produced: list[int] = []
             while True:
                 t = sample_token(apply_penalties(raw.clone(), produced, p), p, gen)
+                if hasattr(self.rt, "check_step"):
+                    self.rt.check_step()
                 produced.append(t)
                 yield token_logprobs(raw, t, p.logprobs) if p.logprobs >= 0 else t
                 if len(produced) >= p.max_tokens or t in p.stop_token_ids:

@@ -128,3 +128,48 @@ def test_large_payloads_take_the_in_switch_path_and_its_timeout_fails_the_step_e
         assert routed == (1, 1, [True])                       # 8 floats: unicast kernel; 256 floats: multimem, two shot
         assert s0 == l0 == 3.0
         assert raised and all_off and nccl_calls == 1 and y0 == 3.0
+
+
+def _worker_product(rank, world, port, q):
+    from pocketllm_b200.parallel.combine import ExpertCombine, StepFailed
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
+    dist.init_process_group("gloo", rank=rank, world_size=world)
+    comb = ExpertCombine(world, None, peer=_FakePeer(world))
+    comb.products = torch.zeros(1, dtype=torch.int32)
+    raised = []
+    for failed, word in ((None, 0), (33 if rank == 1 else 0, 0), (None, 31 if rank == 0 else 0), (None, 0)):
+        comb.products.fill_(word)
+        try:
+            comb.check_step("cpu", failed)
+            raised.append(False)
+        except StepFailed:
+            raised.append(True)
+    q.put((rank, raised, comb.peer is not None, int(comb.products)))
+    dist.destroy_process_group()
+
+
+def test_a_product_that_gave_up_on_one_rank_fails_the_step_everywhere():
+    world = 2
+    with socket.socket() as s:
+        s.bind(("127.0.0.1", 0))
+        port = s.getsockname()[1]
+    ctx = mp.get_context("spawn")
+    q = ctx.Queue()
+    ps = [ctx.Process(target=_worker_product, args=(r, world, port, q)) for r in range(world)]
+    for p in ps:
+        p.start()
+    res = [q.get(timeout=180) for _ in range(world)]
+    for p in ps:
+        p.join(60)
+    for rank, raised, peer_kept, word in res:
+        assert raised == [False, True, True, False] and peer_kept and word == 0
+
+
+def test_a_product_that_gave_up_fails_the_step_of_a_single_rank():
+    import pytest
+    from pocketllm_b200.parallel.combine import ExpertCombine, StepFailed
+    comb = ExpertCombine(1)
+    comb.products = torch.tensor([31], dtype=torch.int32)
+    with pytest.raises(StepFailed):
+        comb.check_step("cpu")
+    comb.check_step("cpu")

@@ -63,3 +63,20 @@ def test_experts_staged_from_host_match_resident_experts(tiny_gguf):
     assert ((a2 - b2).norm() / a2.norm()).item() < 1e-2
     cache = staged.layers[0]["cache"]
     assert cache.slab["w13"].shape[0] == slots and cache.bytes_staged > 0 and cache.lru.stats["evictions"] > 0
+
+
+def test_a_product_that_gave_up_fails_the_step(tiny_gguf):
+    """The error word of the products is read with the token: the step raises, the next one runs."""
+    from pocketllm_b200.models import minimax_m2 as mm
+    from pocketllm_b200.parallel.combine import StepFailed
+    model = mm.MiniMaxM2Model(tiny_gguf, max_context=64)
+    prompt = [3, 77, 140, 9, 255]
+    first = model.prefill(prompt)
+    second = model.decode_one(first)
+    for step in (lambda: model.prefill(prompt), lambda: model.decode_one(first), lambda: (model.forward_logits(prompt), model.check_step())):
+        model.reset()
+        model._word.status.fill_(31)
+        with pytest.raises(StepFailed):
+            step()
+    model.reset()
+    assert model.prefill(prompt) == first and model.decode_one(first) == second
