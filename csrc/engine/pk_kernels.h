@@ -96,7 +96,7 @@ int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const int* ind
                         const float* add, void* sum, void* norm, int type, int terms, void* staged, float* row_scale, uint32_t* counters, int n_counters,
                         cudaStream_t stream);
 int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, int n_groups, int rows, const void* staged, const float* row_scale,
-                  int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int splits, float* ws, uint32_t* counters,
+                  int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int parts, int splits, float* ws, uint32_t* counters,
                   uint32_t* status, const float* w_scale, int w_ld, int sm_count, cudaStream_t stream);
 int pk_rows_fp8(const void* W, const float* w_scale, int w_ld, int M, int N, int K, const void* staged, const float* row_scale, int epi, void* y, int ldy,
                 const void* resid, int sm_count, cudaStream_t stream);

@@ -955,7 +955,7 @@ void QwenEngine::quant_product(const Fp8Linear& w, int M, int epi, void* out, in
       splits = s;
     }
   }
-  check(pk_quant_rows(w.w, kQuantType, w.N, w.K, nullptr, 1, M, quant_rows_, quant_scale_, 1, epi, out, ldo, resid, 0.f, columns, splits, quant_ws_,
+  check(pk_quant_rows(w.w, kQuantType, w.N, w.K, nullptr, 1, M, quant_rows_, quant_scale_, 1, epi, out, ldo, resid, 0.f, columns, splits, splits, quant_ws_,
                       quant_counters_, gemm_status_, w.scale, w.K / 128, sm_count_, stream_),
         "quant_rows");
 }

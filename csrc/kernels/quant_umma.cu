@@ -37,6 +37,7 @@ enum : int { T_IQ2_XXS = 0, T_Q4_K = 3, T_Q5_K = 4, T_E4M3 = 20 };
 
 constexpr int BM = 128;
 constexpr int kMaxGroups = 512;
+constexpr uint32_t kDrainPolls = 1u << 14;      // after a wait that ran out: time for copies and products in flight, which take microseconds
 
 template <int TYPE> struct Fmt;
 // `k`: weights under one factor; `cols`: places of a staged token row for them
@@ -63,10 +64,11 @@ struct Params {
   const float* row_scale; // what a token row's products are multiplied by
   const float* w_scale;   // E4M3: [rows / 128][w_ld]
   int w_ld;
-  int splits;             // parts of K, added by the last of a tile's CTAs in their order
+  int parts;              // of K, summed on their own and added in their order: by one CTA (splits 1, 16 columns) or by the last of a tile's CTAs
+  int splits;             // 1 or `parts`
   float* ws;              // [tile][split][column][128]
   uint32_t* counters;     // [tile], zero between launches
-  uint32_t* status;       // first wait that ran out; a launch that finds it set does no work
+  uint32_t* status;       // first wait that ran out; a launch that finds it set gives NaN
 };
 
 // IQ2_XXS with few columns has two CTAs per SM, which hide one another's waits; the others have more bytes per weight and one CTA with
@@ -283,20 +285,67 @@ template <> struct Dec<T_E4M3> {
   }
 };
 
+__host__ __device__ constexpr uint32_t tmem_columns(uint32_t n) {
+  uint32_t c = 32;
+  while (c < n) c *= 2;
+  return c;
+}
+
+// By one thread, behind the CTA's stores of its part: *last says whether the other parts are there.
+__device__ __forceinline__ void count_part(const Params& p, const Item& w, uint32_t* last) {
+  const uint32_t n = atomicAdd(p.counters + w.tile, 1u);
+  *last = n == (uint32_t)p.splits - 1u;
+  if (*last) p.counters[w.tile] = 0u;
+  __threadfence();
+}
+
 template <int WARPS>
 __device__ __forceinline__ void fold_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
 }
 
+// The rest of a fold warp's items, from `i` on, after a wait that ran out: NaN in their places, so that the result cannot be taken
+// for one, and every part counted, so that the counters are back at zero when the launch is over. Kept out of the loop that it ends.
+template <int NT, int TERMS, int WARPS>
+__device__ __noinline__ void give_up(const Params& p, const int* prefix, int row_tiles, int i, int c0, uint32_t* shared_last) {
+  const int tid = threadIdx.x, lr = ((tid >> 5) & 3) * 32 + (tid & 31), cols = WARPS == 8 ? NT / 2 : NT;
+  const float nan = __uint_as_float(0x7fffffffu);
+  Item w;
+  for (; item_at<NT, TERMS>(p, prefix, row_tiles, i, w); i += gridDim.x) {
+    if (p.splits > 1) {
+      float* part = p.ws + ((size_t)w.tile * p.splits + w.split) * NT * BM + lr;
+      for (int c = c0; c < c0 + cols; ++c) __stcg(part + (size_t)c * BM, nan);
+      __threadfence();
+      fold_sync<WARPS>();
+      if (tid == 0) count_part(p, w, shared_last);
+      fold_sync<WARPS>();
+      const uint32_t last = *(volatile uint32_t*)shared_last;
+      fold_sync<WARPS>();
+      if (!last) continue;
+    }
+    const bool glu = p.epi & 1;
+    const int n = glu ? w.rt * 64 + (lr >> 1) : w.rt * BM + lr;
+    if (n >= (glu ? p.rows >> 1 : p.rows)) continue;
+    for (int m = c0 / TERMS; m < min(w.cnt, (c0 + cols) / TERMS); ++m) {
+      const size_t at = (size_t)(w.row0 + m) * p.ldo + n;
+      if (p.epi == OUT_F32 || p.epi == OUT_SWIGLU_F32) ((float*)p.out)[at] = nan;
+      else ((bf16*)p.out)[at] = __float2bfloat16(nan);
+    }
+  }
+}
+
 template <int TYPE, int NT, int TERMS>
 __global__ void __launch_bounds__(Shape<TYPE, NT>::kThreads, Shape<TYPE, NT>::kCtas)
-quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
+quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ Params p) {
   using S = Shape<TYPE, NT>;
   constexpr int kStages = S::kStages, BB = Fmt<TYPE>::bytes;
   constexpr bool MINS = Fmt<TYPE>::mins;
   constexpr int ST = MINS ? 3 : Fmt<TYPE>::k / 128;      // stages of a block; the third one has the minima in its first 16 places
   constexpr uint32_t kBufCols = MINS ? 2 * NT : NT;
-  constexpr uint32_t kTmemCols = 2 * kBufCols < 32 ? 32 : 2 * kBufCols;
+  // One CTA can have several parts of K where a decode step uses it (16 columns; wider tiles have no registers for it): columns of
+  // their sum, behind the two accumulators.
+  constexpr bool kParts = TYPE != T_E4M3 && NT == 16;
+  constexpr uint32_t kSums = 2 * kBufCols, kTmemCols = tmem_columns(kSums + (kParts ? NT : 0));
   extern __shared__ uint8_t smem_raw[];
   using D = Dec<TYPE>;
   using Sm = Smem<S, D::kPitch>;
@@ -304,9 +353,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row_tiles = (p.epi & 1) ? ((p.rows >> 1) + 63) / 64 : (p.rows + BM - 1) / BM;
 
-  uint32_t failed = 0;
   if (tid == 0) {
-    if (p.status != nullptr) failed = *(const volatile uint32_t*)p.status;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&sm.full[s], S::kDecWarps + 1);
       mbar_init(&sm.empty[s], 1);
@@ -316,6 +363,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       mbar_init(&sm.acc_empty[b], S::kFoldWarps);
     }
     mbar_init(&sm.drained, 1);
+    sm.abort_flag = 0;
     mbar_fence_init();
   }
   for (int g = tid; g < p.n_groups; g += S::kThreads) {
@@ -323,7 +371,6 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
     sm.prefix[g] = (n + NT / TERMS - 1) / (NT / TERMS);
   }
   __syncthreads();
-  if (tid == 0) sm.abort_flag = failed;      // the load had the barrier's time
   if (warp == 1) {
     // token tiles before each group, 32 groups at a time
     int run = 0;
@@ -354,13 +401,14 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
 
   if (warp < S::kFoldWarps) {
     // ---------------- fold and epilogue ----------------
-    // A wait that ran out makes NaN of this item and the CTA's later ones, and they are counted all the same: the result cannot be
-    // taken for one, and the counters are back at zero when the launch is over. (A SwiGLU limit takes NaN for the limit.)
     const int q = warp & 3, c0 = (warp >> 2) * S::kFoldCols, lr = q * 32 + lane;
     uint32_t blk = 0;
     Item w;
     bool ok = true;
-    for (int i = blockIdx.x; item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
+    // an earlier product of the step gave up: this one does as if its first wait had
+    const bool dead = p.status != nullptr && __any_sync(0xffffffffu, *(const volatile uint32_t*)p.status);
+    if (dead) sm.abort_flag = 1u;
+    for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
       const uint8_t* row = group_base(p, w) + tile_row(p, w, lr);
       float acc[S::kFoldCols];
 #pragma unroll
@@ -373,12 +421,12 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       }
       auto factor = [&](int b) { return TYPE == T_E4M3 ? __ldg(ws + b) : ld_half(row + b * BB); };
       float d = factor(w.b0), dm = MINS ? ld_half(row + w.b0 * BB + 2) : 0.f;
-      ok = ok && !__any_sync(0xffffffffu, sm.abort_flag);
-      for (int b = w.b0; ok && b < w.b1; ++b, ++blk) {
+      [[maybe_unused]] int part = 0, part_end = kParts && p.splits == 1 && p.parts > 1 ? p.nblk / p.parts : -1;
+      for (int b = w.b0; b < w.b1; ++b, ++blk) {
         const int nb = min(b + 1, p.nblk - 1);
         const float dn = factor(nb), dmn = MINS ? ld_half(row + nb * BB + 2) : 0.f;
         const int buf = blk & 1;
-        if (!mbar_wait_uniform(&sm.acc_full[buf], (blk >> 1) & 1, &sm.abort_flag, p.status, 31)) {
+        if (dead || !mbar_wait_uniform(&sm.acc_full[buf], (blk >> 1) & 1, &sm.abort_flag, p.status, 31)) {
           ok = false;
           break;
         }
@@ -404,10 +452,32 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
         if (lane == 0) mbar_arrive(&sm.acc_empty[buf]);
         d = dn;
         dm = dmn;
+        if constexpr (kParts)
+          if (b + 1 == part_end) {
+            const uint32_t ts = tmem_base + kSums + ((uint32_t)(q * 32) << 16);
+            uint32_t r[16] = {};
+            if (part > 0) {
+              tmem_ld_32x16(ts, r);
+              tmem_ld_wait();
+            }
+            const bool more = b + 1 < w.b1;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              acc[j] += __uint_as_float(r[j]);
+              r[j] = __float_as_uint(acc[j]);
+              if (more) acc[j] = 0.f;
+            }
+            if (more) {
+              tmem_st_32x16(ts, r);
+              tmem_st_wait();
+            }
+            ++part;
+            part_end = p.nblk * (part + 1) / p.parts;
+          }
       }
       if (!ok) {
-#pragma unroll
-        for (int c = 0; c < S::kFoldCols; ++c) acc[c] = __uint_as_float(0x7fffffffu);
+        give_up<NT, TERMS, S::kFoldWarps>(p, sm.prefix, row_tiles, i, c0, &sm.last);
+        break;
       }
       if (p.splits > 1) {
         float* part = p.ws + ((size_t)w.tile * p.splits + w.split) * NT * BM + lr;
@@ -415,12 +485,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
         for (int c = 0; c < S::kFoldCols; ++c) __stcg(part + (size_t)(c0 + c) * BM, acc[c]);
         __threadfence();
         fold_sync<S::kFoldWarps>();
-        if (tid == 0) {
-          const uint32_t n = atomicAdd(p.counters + w.tile, 1u);
-          sm.last = n == (uint32_t)p.splits - 1u;
-          if (sm.last) p.counters[w.tile] = 0u;
-          __threadfence();
-        }
+        if (tid == 0) count_part(p, w, &sm.last);
         fold_sync<S::kFoldWarps>();
         const uint32_t last = sm.last;
         fold_sync<S::kFoldWarps>();
@@ -484,7 +549,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
     const bool leader = elect_one();
     uint32_t st = 0, ph = 0, blk = 0;
     Item w;
-    bool ok = !__any_sync(0xffffffffu, sm.abort_flag);
+    bool ok = true;
     for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
       for (int b = w.b0; ok && b < w.b1; ++b, ++blk) {
         const int buf = blk & 1;
@@ -525,7 +590,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       // gave up: the products in flight end before their tensor memory is freed
       if (leader) umma_commit(&sm.drained);
       __syncwarp();
-      for (uint32_t n = 0; n < (1u << 20) && !mbar_try_wait(&sm.drained, 0); ++n) {}
+      for (uint32_t n = 0; n < kDrainPolls && !mbar_try_wait(&sm.drained, 0); ++n) {}
     }
   } else if (warp == S::kFoldWarps + 1) {
     // ---------------- token tiles ----------------
@@ -533,7 +598,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       tma_prefetch_desc(&tmap);
       uint32_t st = 0, ph = 1, issued = 0;
       Item w;
-      bool ok = !sm.abort_flag;
+      bool ok = true;
       for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x)
         for (int x = w.b0 * Fmt<TYPE>::cols; ok && x < w.b1 * Fmt<TYPE>::cols;) {
 #pragma unroll
@@ -558,7 +623,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
       if (sm.abort_flag) {
         // gave up: copies in flight land before the CTA exits
         for (uint32_t j = issued > (uint32_t)kStages ? issued - kStages : 0; j < issued; ++j)
-          for (uint32_t n = 0; n < (1u << 20); ++n)
+          for (uint32_t n = 0; n < kDrainPolls; ++n)
             if (mbar_try_wait(&sm.full[j % kStages], (j / kStages) & 1)) break;
       }
     }
@@ -613,7 +678,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
     const uint32_t grid = smem_u32(sm.grid);
     uint32_t st = 0, ph = 1, slot = 0;
     Item w;
-    bool ok = !__any_sync(0xffffffffu, sm.abort_flag);
+    bool ok = true;
     for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
       const uint32_t own = tile_row(p, w, lr);
       for (int b = w.b0; ok && b < w.b1; ++b) {
@@ -862,22 +927,23 @@ PK_API int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const i
 
 // out[t, n] = row_scale[t] * staged[t] . W[g(t), n]: W [n_groups * N] raw rows of `type`; token rows seg[g] .. seg[g + 1] belong to
 // group g (seg null: all `rows` to the one group). epi 0 bf16, 1 SwiGLU bf16, 2 fp32, 3 SwiGLU fp32 (N / 2 gate rows, then as
-// many up rows), 4 bf16 with `resid` added. `columns` 16, 32 or 64 of a tile. splits > 1 needs ws (tiles * splits * columns * 128 floats) and one zeroed
-// counter per tile. E4M3 (type 20): W [N, K] codes, w_scale [ceil(N / 128), w_ld] factors of its 128 x 128 blocks;
+// many up rows), 4 bf16 with `resid` added. `columns` 16, 32 or 64 of a tile. K is summed in `parts`,
+// by as many CTAs (splits = parts) or, with 16 columns, by one (splits 1) to the same bits. splits > 1 needs ws (tiles * splits * columns * 128 floats)
+// and one zeroed counter per tile. E4M3 (type 20): W [N, K] codes, w_scale [ceil(N / 128), w_ld] factors of its 128 x 128 blocks;
 // 32 or 64 columns (up to 16 rows are rows_fp8.cu's).
 PK_API int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, int n_groups, int rows, const void* staged, const float* row_scale,
-                         int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int splits, float* ws, uint32_t* counters, uint32_t* status,
+                         int terms, int epi, void* out, int ldo, const void* resid, float limit, int columns, int parts, int splits, float* ws, uint32_t* counters, uint32_t* status,
                          const float* w_scale, int w_ld, int sm_count, cudaStream_t stream) {
   if (W == nullptr || staged == nullptr || row_scale == nullptr || out == nullptr || rows < 1 || N < 1 || n_groups < 1 || n_groups > kMaxGroups ||
-      (seg == nullptr && n_groups != 1) || terms < 1 || terms > 2 || epi < 0 || epi > 4 || (epi == OUT_RESID && resid == nullptr) || ((epi & 1) && (N & 1)) || splits < 1 ||
+      (seg == nullptr && n_groups != 1) || terms < 1 || terms > 2 || epi < 0 || epi > 4 || (epi == OUT_RESID && resid == nullptr) || ((epi & 1) && (N & 1)) || parts < 1 || (splits != parts && (splits != 1 || columns != 16)) ||
       (splits > 1 && (ws == nullptr || counters == nullptr)) || (columns != 16 && columns != 32 && columns != 64) || pk_quant_stage_pitch(type, K) == 0 ||
-      splits > K / type_k(type) || (type == T_E4M3 && (w_scale == nullptr || terms != 1 || n_groups != 1 || columns == 16)) || ((uintptr_t)W & 15) != 0 || ((uintptr_t)staged & 15) != 0)
+      parts > K / type_k(type) || (type == T_E4M3 && (parts != splits || w_scale == nullptr || terms != 1 || n_groups != 1 || columns == 16)) || ((uintptr_t)W & 15) != 0 || ((uintptr_t)staged & 15) != 0)
     return PK_ERR_BAD_ARG;
   const int nblk = K / type_k(type);
   const long long group_bytes = (long long)nblk * type_bytes(type) * N;      // IQ2 blocks are copied by four bytes
   if (group_bytes >= (1ll << 32) || (type == T_IQ2_XXS && (group_bytes & 3) != 0)) return PK_ERR_UNSUPPORTED;
   const Params p{(const uint8_t*)W, (long long)nblk * type_bytes(type), nblk, N, n_groups, seg, rows, epi, limit, out, ldo, (const pk::bf16*)resid, row_scale, w_scale, w_ld,
-                 splits, ws, counters, status};
+                 parts, splits, ws, counters, status};
   const int sms = sm_count > 0 ? sm_count : 148;
   if (type == T_IQ2_XXS) return launch_shape<T_IQ2_XXS>(columns, terms, staged, rows, p, sms, stream);
   if (type == T_Q4_K) return launch_shape<T_Q4_K>(columns, terms, staged, rows, p, sms, stream);

@@ -118,11 +118,16 @@ class _Staged:
 
 
 def _umma(st: _Staged, w_raw: torch.Tensor, type_name: str, N: int, K: int, seg, groups: int, epi: int, out: torch.Tensor, limit: float, columns: int,
-          splits: int, status: torch.Tensor | None) -> None:
+          parts: int, splits: int, status: torch.Tensor | None) -> None:
     _check(_lib.kernels().pk_quant_rows(_ptr(w_raw), c_int(DEVICE_TYPE[type_name]), c_int(N), c_int(K), _ptr(seg), c_int(groups), c_int(st.rows), st.data,
                                        st.scale, c_int(st.terms), c_int(epi), _ptr(out), c_int(out.stride(0)), c_void_p(0), c_float(limit), c_int(columns),
-                                       c_int(splits), st.ws, st.counters, st.status if status is None else _ptr(status), c_void_p(0), c_int(0),
+                                       c_int(parts), c_int(splits), st.ws, st.counters, st.status if status is None else _ptr(status), c_void_p(0), c_int(0),
                                        c_int(_sm_count()), _stream()), "pk_quant_rows")
+
+
+def _fill(items: int, slots: int) -> float:
+    """How full the rounds of `slots` CTAs are with that many items."""
+    return items / (-(-items // slots) * slots)
 
 
 def _umma_splits(tiles: int, K: int, slots: int) -> int:
@@ -130,8 +135,7 @@ def _umma_splits(tiles: int, K: int, slots: int) -> int:
     256-weight blocks in a part at least."""
     best, most = 1, 0.0
     for s in range(1, min(K // 512, 4 * slots // tiles) + 1):
-        items = tiles * s
-        full = items / (-(-items // slots) * slots) - 0.01 * s
+        full = _fill(tiles * s, slots) - 0.01 * s
         if full > most:
             best, most = s, full
     return best
@@ -149,7 +153,7 @@ def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, g
     splits = _umma_splits(tiles, K, _umma_slots(type_name, columns))
     st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
     y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
-    _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits, status)
+    _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits, splits, status)
     return y
 
 
@@ -166,12 +170,20 @@ def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, 
 
     def product(x, w_raw, type_name, N, K, t, epi, out, limit, index):
         c, row_tiles = columns(t), -(-(N // 2) // 64) if epi == 3 else -(-N // 128)
-        splits = 1
-        if R <= UMMA_SPLIT_ROUTES:       # every route may be an expert of its own; beyond, the tiles fill the SMs
-            splits = _umma_splits(max(1, min(R, local)) * row_tiles, K, _umma_slots(type_name, c))
+        slots = _umma_slots(type_name, c)
+        most = max(1, min(R, local)) * row_tiles        # tiles, if every route is an expert of its own
+        parts = splits = 1
+        if c == 16:
+            # K is cut as for one token's routes whatever the step holds and however the experts are split over ranks: a token's sum does
+            # not depend on the tokens beside it. CTAs of their own take the parts where that fills the SMs better.
+            parts = _umma_splits(routes.topk * row_tiles, K, slots)
+            if R <= UMMA_SPLIT_ROUTES and most * parts <= 4 * slots and _fill(most * parts, slots) > _fill(most, slots) + 0.02:
+                splits = parts
+        elif R <= UMMA_SPLIT_ROUTES:       # beyond, the tiles fill the SMs
+            parts = splits = _umma_splits(most, K, slots)
         tiles = (min(R, local) + R * t // c) * row_tiles if splits > 1 else 0
         st = _Staged(x, type_name, R, t, index=index, counters=tiles, ws_floats=tiles * splits * c * 128)
-        _umma(st, w_raw, type_name, N, K, seg, local, epi, out, limit, c, splits, status)
+        _umma(st, w_raw, type_name, N, K, seg, local, epi, out, limit, c, parts, splits, status)
 
     h = torch.empty(R, inter, device=dev, dtype=torch.float32)
     y = torch.empty(R, H, device=dev, dtype=torch.float32)
