@@ -111,7 +111,7 @@ class _Staged:
         p = self.buf.data_ptr()
         self.data, self.scale, self.counters, self.ws = (c_void_p(p + o) for o in offs)
         self.status = c_void_p(p + offs[2] + 4 * counters - 4)
-        _check(_lib.kernels().pk_quant_stage_rows(_ptr(x), c_int(int(x.dtype == torch.float32)), c_int(x.stride(0)), c_int(K), _ptr(index), c_int(rows),
+        _check(_lib.kernels().pk_quant_stage_rows(_ptr(x), c_int(int(x.dtype == torch.float32)), c_int(K), c_int(K), _ptr(index), c_int(rows),
                                                  _ptr(gamma), c_float(eps), c_int(0), c_void_p(0), c_void_p(0), c_void_p(0),
                                                  c_int(DEVICE_TYPE[type_name]), c_int(terms), self.data, self.scale, self.counters, c_int(counters),
                                                  _stream()), "pk_quant_stage_rows")

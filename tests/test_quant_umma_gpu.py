@@ -55,6 +55,15 @@ def test_linear_rows_of_zeros_and_infinities():
     assert _rel(y[0], x[0].double() @ w.T) < TOL and _rel(y[3], x[3].double() @ w.T) < TOL
 
 
+def test_one_row_of_any_stride():
+    """A single row is contiguous whatever its row stride says."""
+    from pocketllm_b200.ops import gguf_ops as go
+    raw, w = _raw("q5_k", 520, 512, 3)
+    x = torch.randn(512, 1, device="cuda").to(torch.bfloat16).t()
+    assert x.stride(0) == 1 and x.is_contiguous()
+    assert _rel(go.gguf_linear(x, raw, "q5_k", 520, epi=2), x.double() @ w.T) < TOL
+
+
 @pytest.mark.parametrize("t13,t2", [("iq2_xxs", "iq2_xxs"), ("q4_k", "iq2_xxs"), ("iq2_xxs", "q5_k")])
 @pytest.mark.parametrize("T,E,topk,limit", [(1, 16, 4, 0.0), (9, 40, 3, 0.0), (17, 40, 4, 0.0), (33, 40, 3, 0.0), (90, 8, 2, 0.5), (300, 5, 2, 0.0)])
 def test_experts(t13, t2, T, E, topk, limit):
