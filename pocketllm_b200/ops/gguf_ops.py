@@ -33,7 +33,7 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     reference switches to its prefill kernels for rows > 1, src/components/gguf/quantized_ops.py:9-76)."""
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
-    if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name):
+    if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name, N, K):
         return _umma_linear(_aligned(x), w_raw, type_name, N, _aligned(gamma), eps, epi, status)
     if M >= TENSOR_CORE_MIN_ROWS and K % 64 == 0 and (epi != 1 or (N // 2) % 128 == 0):
         from . import gemm_bf16, rmsnorm, EPI_BF16, EPI_SWIGLU, EPI_F32
@@ -61,9 +61,12 @@ UMMA_SPLIT_ROUTES = 64
 UMMA_MAX_GROUPS = 512
 
 
-def _umma_takes(w_raw: torch.Tensor, type_name: str, groups: int = 1) -> bool:
-    # whole words: the kernel copies IQ2 blocks by four bytes
-    return type_name in UMMA_TYPES and w_raw.data_ptr() % 16 == 0 and w_raw.numel() % (4 * groups) == 0 and w_raw.numel() // groups < 1 << 32
+def _umma_takes(w_raw: torch.Tensor, type_name: str, rows: int, K: int, groups: int = 1) -> bool:
+    """Whether the kernel takes `groups` groups of `rows` rows, which may be the beginning of a longer buffer."""
+    if type_name not in UMMA_TYPES or w_raw.data_ptr() % 16 != 0 or K % 256 != 0:
+        return False
+    n = rows * row_bytes(type_name, K)
+    return n % 4 == 0 and n < 1 << 32 and w_raw.numel() >= n * groups       # whole words: IQ2 blocks are copied by four bytes
 
 
 class StepWord:
@@ -193,7 +196,7 @@ def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, 
 
 
 def _umma_experts_take(w13_raw: torch.Tensor, w2_raw: torch.Tensor, type13: str, type2: str, H: int, inter: int, local: int) -> bool:
-    return (_umma_takes(w13_raw, type13, local) and _umma_takes(w2_raw, type2, local) and H % 256 == 0 and inter % 256 == 0 and max(H, inter) * 4 <= 200 * 1024
+    return (_umma_takes(w13_raw, type13, 2 * inter, H, local) and _umma_takes(w2_raw, type2, H, inter, local) and max(H, inter) * 4 <= 200 * 1024
             and local <= UMMA_MAX_GROUPS)
 
 

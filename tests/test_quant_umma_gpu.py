@@ -64,6 +64,16 @@ def test_one_row_of_any_stride():
     assert _rel(go.gguf_linear(x, raw, "q5_k", 520, epi=2), x.double() @ w.T) < TOL
 
 
+@pytest.mark.parametrize("M", [1, 20])
+def test_first_rows_of_a_longer_buffer(M):
+    """An odd number of IQ2 blocks is no whole number of words, the buffer behind it is."""
+    from pocketllm_b200.ops import gguf_ops as go
+    raw, w = _raw("iq2_xxs", 130, 256, 4)
+    x = torch.randn(M, 256, device="cuda").to(torch.bfloat16)
+    assert raw.numel() % 4 == 0
+    assert _rel(go.gguf_linear(x, raw, "iq2_xxs", 129, epi=2), x.double() @ w[:129].T) < TOL
+
+
 @pytest.mark.parametrize("t13,t2", [("iq2_xxs", "iq2_xxs"), ("q4_k", "iq2_xxs"), ("iq2_xxs", "q5_k")])
 @pytest.mark.parametrize("T,E,topk,limit", [(1, 16, 4, 0.0), (9, 40, 3, 0.0), (17, 40, 4, 0.0), (33, 40, 3, 0.0), (90, 8, 2, 0.5), (300, 5, 2, 0.0)])
 def test_experts(t13, t2, T, E, topk, limit):
