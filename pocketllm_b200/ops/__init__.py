@@ -249,7 +249,12 @@ def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, *, mode: int = 1, eps: float =
 
 def residual_add(x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
     """bf16(x + y) for bf16 x and fp32 y [M, K]: one launch and one rounding (the sum in fp32 and its conversion are two)."""
+    if x.dtype != torch.bfloat16 or y.dtype != torch.float32 or x.dim() != 2 or x.shape != y.shape or y.device != x.device:
+        raise ValueError(f"residual_add: bf16 and fp32 rows of one shape on one device, not {x.dtype} {tuple(x.shape)} and {y.dtype} {tuple(y.shape)}")
+    x, y = x.contiguous(), y.contiguous()
     out = torch.empty_like(x)
+    if x.numel() == 0:
+        return out
     st = _lib.kernels().pk_rmsnorm(_ptr(x), _ptr(y), c_int(1), c_int(x.shape[0]), c_int(x.shape[1]), _ptr(out), c_void_p(0), c_int(1), c_float(0.0),
                                    c_void_p(0), c_void_p(0), _stream())
     _check(st, "pk_rmsnorm")
