@@ -254,3 +254,15 @@ def test_bf16_rows(M, N, K, split):
     if split:
         want[:, split:] = x2.double() @ w[split:].double().T
         assert _rel(mo.linear2(x, x2, split, w, y(N, torch.float32), st), want) < TOL
+
+
+@pytest.mark.parametrize("K", [4096, 14336])
+def test_bf16_rows_round_their_sums(K):
+    """Tensor cores cut sums off; a running sum of K values would be off by 2^-24 per 16 of them (5e-7 and 2e-6 here). Sums of 16 that
+    are added with rounding stay within a few 2^-24."""
+    from pocketllm_b200.ops import mixer_ops as mo
+    g = torch.Generator("cuda").manual_seed(K)
+    for x in (torch.randn(3, K, device="cuda", generator=g), torch.rand(3, K, device="cuda", generator=g)):
+        x, w = x.to(torch.bfloat16), (torch.randn(256, K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+        y = mo.linear(x, w, torch.empty(3, 256, device="cuda"), torch.zeros(1, device="cuda", dtype=torch.int32))
+        assert _rel(y, x.double() @ w.double().T) < 4 * 2 ** -24
