@@ -11,7 +11,7 @@ using namespace pk;
 
 enum { OUT_BF16 = 0, OUT_SWIGLU = 1, OUT_F32 = 2 };
 constexpr int WARPS = 8;
-constexpr int kMmaRows = 1;      // from here on linear_rows_mma_kernel where K allows it
+constexpr int kMmaK = 512;       // from here on linear_rows_mma_kernel where K allows it: 1024 x 256, 1 / 8 rows 1.8 / 1.8 us, 1.4 / 2.5 without; 512 x 512 1.6 / 1.6 and 1.7 / 3.2
 
 struct RowsParams {
   const bf16* x;
@@ -144,11 +144,13 @@ __global__ void __launch_bounds__(32 * WARPS) linear_rows_kernel(const RowsParam
 // in shared memory that every lane fills for itself (`cp.async`, no barrier): prefetched into registers they were waited for together
 // with the activations, 2.5 TB/s. The tensor cores cut their sums off, so every 16 products have a sum of their own and these are
 // added with rounding: the error of fp32 results against 64 bits is 9e-8 at K = 4096 and 1.2e-7 at 14336 (8e-8 and 1e-7 with a
-// multiply-add per weight; one running sum has 5e-7 and 1.8e-6), at the same time. Nothing is shared between warps but the sums of a K range that was cut, added in their order.
-constexpr int kRing = 6;
-constexpr size_t kMmaSmem = (size_t)WARPS * kRing * 4 * 32 * 16;
+// multiply-add per weight; one running sum has 5e-7 and 1.8e-6), at the same time. Nothing is shared
+// between warps but the sums of a K range that was cut, added in their order.
+constexpr int kRing = 6, kDeepRing = 12;      // steps; two blocks on an SM, or one where no more are launched
+constexpr size_t mma_smem(int ring) { return (size_t)WARPS * ring * 4 * 32 * 16; }
 
-__global__ void __launch_bounds__(32 * WARPS, 2) linear_rows_mma_kernel(const RowsParams p, int M) {
+template <int RING>
+__global__ void __launch_bounds__(32 * WARPS, RING == kRing ? 2 : 1) linear_rows_mma_kernel(const RowsParams p, int M) {
   extern __shared__ __align__(16) uint4 ring_smem[];
   __shared__ float part[WARPS][16][9];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -162,19 +164,19 @@ __global__ void __launch_bounds__(32 * WARPS, 2) linear_rows_mma_kernel(const Ro
   const bf16* wb = p.w + (size_t)r1 * p.K + t * 8;
   const bf16* x = (n0 < p.split ? p.x : p.x2) + (size_t)min(g, M - 1) * p.ldx + t * 8;
   const int steps = live ? (p.K / 64 - sl + ks - 1) / ks : 0, stride = 64 * ks;
-  uint4* ring = ring_smem + warp * kRing * 128 + lane;
+  uint4* ring = ring_smem + warp * RING * 128 + lane;
   auto copy = [&](int s) {
     if (s < steps) {
       const int k = sl * 64 + s * stride;
       const bf16* src[4] = {wa + k, wa + k + 32, wb + k, wb + k + 32};
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + (s % kRing) * 128);
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + (s % RING) * 128);
 #pragma unroll
       for (int i = 0; i < 4; ++i) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 512), "l"(src[i]) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int s = 0; s < kRing - 1; ++s) copy(s);
+  for (int s = 0; s < RING - 1; ++s) copy(s);
   pdl_trigger();
   pdl_wait();
   float c[4] = {}, before[4][4] = {};      // sums of the step before: they are added while this one's are under way
@@ -182,9 +184,9 @@ __global__ void __launch_bounds__(32 * WARPS, 2) linear_rows_mma_kernel(const Ro
   for (int s = 0; s < steps; ++s) {
     const int k = sl * 64 + s * stride;
     const uint4 x0 = *reinterpret_cast<const uint4*>(x + k), x1 = *reinterpret_cast<const uint4*>(x + k + 32);
-    copy(s + kRing - 1);
-    asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
-    const uint4* q = ring + (s % kRing) * 128;
+    copy(s + RING - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
+    const uint4* q = ring + (s % RING) * 128;
     const uint4 a0 = q[0], a1 = q[32], b0 = q[64], b1 = q[96];
     float d[4][4] = {};
     mma16816(d[0], a0.x, b0.x, a0.y, b0.y, x0.x, x0.y);
@@ -230,20 +232,26 @@ PK_API int pk_linear_rows2(const void* x, const void* x2, int split, int ldx, co
   if (M < 1 || M > 8 || N < 1 || K < 8 || (K & 7) != 0 || (ldx & 7) != 0 || ldx < K || epi < 0 || epi > 2) return PK_ERR_BAD_ARG;
   if (((uintptr_t)x & 15) != 0 || ((uintptr_t)w & 15) != 0 || (epi == OUT_SWIGLU && (N & 1) != 0)) return PK_ERR_BAD_ARG;
   if (ldy < (epi == OUT_SWIGLU ? N / 2 : N)) return PK_ERR_BAD_ARG;
-  if (M >= kMmaRows && (K & 63) == 0 && (split >= N || (split & 15) == 0)) {
+  if (K >= kMmaK && (K & 63) == 0 && (split >= N || (split & 15) == 0)) {
     const int outs = epi == OUT_SWIGLU ? N / 2 : N, span = epi == OUT_SWIGLU ? 8 : 16, groups = (outs + span - 1) / span;
     int ks = 1;      // warps for two blocks on every SM, two steps of 64 in a share at least
     while (ks < WARPS && groups * ks < (sm_count > 0 ? sm_count : 148) * 2 * WARPS && K >= 128 * ks * 2) ks *= 2;
     const RowsParams p{(const pk::bf16*)x, (const pk::bf16*)x2, split, ldx, (const pk::bf16*)w, N, K, epi, ks, y, ldy};
     static PkDeviceOnce once;
     if (PkDeviceOnceGuard once_guard{once}; once_guard.needed()) {
-      if (cudaFuncSetAttribute(linear_rows_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem) != cudaSuccess) {
+      if (cudaFuncSetAttribute(linear_rows_mma_kernel<kRing>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem(kRing)) != cudaSuccess ||
+          cudaFuncSetAttribute(linear_rows_mma_kernel<kDeepRing>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem(kDeepRing)) != cudaSuccess) {
         pk_set_last_cuda_error((int)cudaGetLastError());
         return PK_ERR_CUDA;
       }
       once_guard.done();
     }
-    PK_LAUNCH_PDL(linear_rows_mma_kernel, dim3((groups + WARPS / ks - 1) / (WARPS / ks)), dim3(32 * WARPS), kMmaSmem, stream, p, M);
+    // blocks that are alone on their SM hold twice as many steps, if there are so many: 512 x 4096, one row 4.1 -> 2.8 us
+    const int blocks = (groups + WARPS / ks - 1) / (WARPS / ks);
+    if (blocks <= (sm_count > 0 ? sm_count : 148) && K / 64 / ks >= kRing)
+      PK_LAUNCH_PDL(linear_rows_mma_kernel<kDeepRing>, dim3(blocks), dim3(32 * WARPS), mma_smem(kDeepRing), stream, p, M);
+    else
+      PK_LAUNCH_PDL(linear_rows_mma_kernel<kRing>, dim3(blocks), dim3(32 * WARPS), mma_smem(kRing), stream, p, M);
     return PK_OK;
   }
   const int groups = epi == OUT_SWIGLU ? N / 2 : (N + 1) / 2;

@@ -238,7 +238,7 @@ def test_router_logits(T, E, H):
 
 
 @pytest.mark.parametrize("M", [1, 3, 8])
-@pytest.mark.parametrize("N,K,split", [(8, 64, 0), (40, 128, 16), (130, 960, 0), (66, 4096, 32), (4112, 192, 0)])
+@pytest.mark.parametrize("N,K,split", [(8, 64, 0), (40, 128, 16), (130, 960, 0), (66, 4096, 32), (4112, 192, 0), (40, 512, 16), (24, 6144, 0), (300, 3072, 0), (16, 12544, 0)])
 def test_bf16_rows(M, N, K, split):
     """Rows of whole steps of 64: fewer steps than the ring holds and more, K cut over warps, ragged groups, two inputs."""
     from pocketllm_b200.ops import mixer_ops as mo
