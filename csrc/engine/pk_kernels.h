@@ -92,6 +92,7 @@ int pk_gqa_prefill_umma(const void* q, const void* kcache, const void* vcache, c
                         float scale, const void* gate_proj, int ld, void* out, uint32_t* status, cudaStream_t stream);
 int pk_gemm_bf16_grouped(const void* A, int lda, const void* W, const int* seg, int n_groups, int R, int N, int K, int epi, void* C, int ldc,
                          uint32_t* status, int sm_count, cudaStream_t stream);
+int pk_matvec_one_piece(int K, int M);
 int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const int* index, int rows, const float* gamma, float eps, int plus_one,
                         const float* add, void* sum, void* norm, int type, int terms, void* staged, float* row_scale, uint32_t* counters, int n_counters,
                         cudaStream_t stream);

@@ -919,13 +919,28 @@ PkPush QwenEngine::make_push(int site, bool big, int rows_per_rank) const {
 // ---------------------------------------------------------------------------------------
 // few rows on the tensor cores
 
-bool QwenEngine::quant_takes(const Fp8Linear& w, int M) const {
-  // Loops that compare the picks of passes over different numbers of rows keep one order of addition: engines whose single rows take
-  // one launch per projection (also for the predictor or an external drafter's taps), and POCKET_MATVEC_RING=0.
+// Once per pass. Loops that compare the picks of passes over different numbers of rows keep one order of addition: engines whose single rows
+// do take one launch per projection (asked for, for the predictor or an external drafter's taps, or because the persistent kernel
+// does not take the shapes), and POCKET_MATVEC_RING=0.
+void QwenEngine::choose_row_kernels() {
+  few_rows_ = verify_rows_ = false;
+  if (quant_rows_ == nullptr || nccl_mode_ || opt_.mtp || !tap_layers_.empty()) return;
   const char* ring = getenv("POCKET_MATVEC_RING");
-  const char* persistent = getenv("POCKET_DECODE_PERSISTENT");
-  const bool one_order = opt_.mtp || !tap_layers_.empty() || (persistent ? atoi(persistent) : opt_.persistent_decode) == 0 || (ring != nullptr && atoi(ring) == 0);
-  return quant_rows_ != nullptr && !one_order && !nccl_mode_ && w.w != nullptr && w.scale != nullptr && M <= kQuantRows && (w.K & 127) == 0;
+  if (ring != nullptr && ring[0] == '0') return;
+  const char* v = getenv("POCKET_DECODE_PERSISTENT");
+  const int mode = v != nullptr ? atoi(v) : opt_.persistent_decode;
+  if (mode < 0 && !persistent_built_ && peers_set_) build_persistent();
+  few_rows_ = mode > 0 || (mode < 0 && persistent_ok_);
+  // Verified rows of three to eight: while matvec.cu stages them in one piece they are bit by bit what single rows are, and they stay with
+  // it (up to K of about 10000). The other kernels also want weights to hide their launches behind: three rows with an MLP of 38 / 63 / 85
+  // million weights 319 -> 376, 394 -> 407, 439 -> 439 us, of 267 million 835 -> 628 (four layers).
+  int kmax = 0;
+  for (int k : {hidden_, inter_l_, vd_l_, hq_l_ * kHeadDim}) kmax = std::max(kmax, k);
+  verify_rows_ = few_rows_ && !pk_matvec_one_piece(kmax, 3) && 3.0 * hidden_ * inter_l_ >= 72e6;
+}
+
+bool QwenEngine::quant_takes(const Fp8Linear& w, int M) const {
+  return few_rows_ && w.w != nullptr && w.scale != nullptr && M <= kQuantRows && (w.K & 127) == 0;
 }
 
 // fp16 rows of x for the products that follow; gamma: RMSNorm (1 + gamma) with a bf16 result; add: fp32 rows added first, the bf16
@@ -980,7 +995,7 @@ void QwenEngine::run_small(int M, bool all_logits, bool mtp) {
     check(pk_embedding(tokens_dev_, M, embed_, hidden_, 0, (int)cfg_.vocab_size, hidden_buf_[cur_], nullptr, stream_), "embedding");
   }
   int pending = -1;  // site whose partial sums still wait to be added to the residual stream
-  const bool few = M >= 3 && !mtp;     // one and two rows stream through the rings of matvec.cu
+  const bool few = M >= 3 && !mtp && verify_rows_;     // one and two rows stream through the rings of matvec.cu
 
   auto consume = [&](const Fp8Linear* w, const void* wb, int nb, const float* gamma, int epi, void* y, int ldy,
                      const PkPush* push) {
@@ -1347,6 +1362,7 @@ int QwenEngine::prefill(const int* tokens_host, int n) {
       throw std::runtime_error("token id " + std::to_string(tokens_host[t]) + " is outside the vocabulary of " + std::to_string(cfg_.vocab_size));
   if (n < 1) throw std::runtime_error("prefill: empty prompt");
   if (pos_ + n + 1 > opt_.max_context) throw std::runtime_error("prefill: prompt exceeds max_context");
+  choose_row_kernels();
   cuda_check(cudaEventRecord(ev0_, stream_), "event");
   const long long l0 = launches_;
   int done = 0;
@@ -1771,6 +1787,7 @@ void QwenEngine::forward_rows(const int* tokens_host, int M, int* out_tokens_hos
     if (tokens_host[t] < 0 || tokens_host[t] >= cfg_.vocab_size) throw std::runtime_error("forward_rows: token id outside the vocabulary");
   if (M < 1 || M > kSmallRows) throw std::runtime_error("forward_rows: 1..8 rows");
   if (pos_ + M + 1 > opt_.max_context) throw std::runtime_error("forward_rows: exceeds max_context");
+  choose_row_kernels();
   memcpy(pinned_tok_, tokens_host, (size_t)M * sizeof(int));
   cuda_check(cudaMemcpyAsync(tokens_dev_, pinned_tok_, (size_t)M * sizeof(int), cudaMemcpyHostToDevice, stream_), "h2d");
   check(pk_iota_int(pos_dev_, M, nullptr, pos_, stream_), "iota");

@@ -319,6 +319,9 @@ class QwenEngine {
   float* quant_scale_ = nullptr;
   float* quant_ws_ = nullptr;
   uint32_t* quant_counters_ = nullptr;
+  bool few_rows_ = false;        // this pass may use them: chunks
+  bool verify_rows_ = false;     // and passes of up to eight rows
+  void choose_row_kernels();
   bool quant_takes(const Fp8Linear& w, int M) const;
   void quant_stage(const void* x, int ldx, int K, int M, const float* gamma, const float* add, void* sum, void* norm);
   void quant_product(const Fp8Linear& w, int M, int epi, void* out, int ldo, const void* resid);

@@ -1020,6 +1020,9 @@ static bool l2_prefetch_enabled() {
   return on != nullptr && on[0] == '1';
 }
 
+// Whether M rows of K inputs are staged in one piece by the register-streaming kernel, which then adds every row up like a single one.
+PK_API int pk_matvec_one_piece(int K, int M) { return (size_t)M * ((K + 511) & ~511) * 2 + (size_t)K * 4 <= (size_t)kSmemBytes ? 1 : 0; }
+
 // The ring variant is on by default; POCKET_MATVEC_RING=0 keeps every shape on the register-streaming kernel.
 static bool ring_enabled() {
   const char* v = getenv("POCKET_MATVEC_RING");

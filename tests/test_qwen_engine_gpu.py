@@ -206,6 +206,60 @@ def test_speculative_decoding_equals_greedy(tiny):
     e.close()
 
 
+def test_rows_keep_one_order_where_the_persistent_kernel_declines():
+    """Three query heads per key head: single rows take one launch per projection, so several rows keep those kernels too."""
+    from pocketllm_b200.models import qwen_hybrid as qh
+    cfg = qh.QwenHybridConfig.tiny(layers=4)
+    cfg.num_attention_heads = 6
+    rows = []
+    for mode in (None, 0):
+        e = qh.QwenEngine(cfg, max_context=128, prefill_chunk=32, persistent_decode=mode).init_random(seed=1, sigma=0.05)
+        e.prefill(list(range(1, 21)))
+        e.forward_rows([5, 6, 7, 8])
+        rows.append(torch.stack([e.logits(r) for r in range(4)]))
+        assert not e.persistent_decode
+        e.close()
+    assert torch.equal(*rows)
+
+
+def test_verified_rows_at_wide_layers():
+    """Widths whose rows from three on are multiplied on the tensor cores: the same logits as row by row up to the rounding between layers."""
+    from pocketllm_b200.models import qwen_hybrid as qh
+    cfg = qh.QwenHybridConfig.tiny(layers=4, hidden=4096, inter=12288, vocab=2048)
+    tokens, rows = [5, 99, 7, 300, 11, 8], {}
+    e = qh.QwenEngine(cfg, max_context=128, prefill_chunk=32).init_random(seed=2, sigma=0.02)
+    for n in (1, 3, 6):
+        e.reset()
+        e.prefill([1, 2])
+        rows[n] = []
+        for i in range(0, 6, n):
+            e.forward_rows(tokens[i:i + n])
+            rows[n] += [e.logits(r) for r in range(n)]
+    e.close()
+    one, three, six = (torch.stack(rows[n]).double() for n in (1, 3, 6))
+    # single rows are multiplied in halves: 3e-4 per product, and bf16 values that round to the other side (2^-9) in 16 products
+    assert ((three - one).norm() / one.norm()).item() < 3e-2
+    assert ((six - three).norm() / three.norm()).item() < 1e-2 and not torch.equal(three, one)
+
+
+def test_speculation_on_a_default_engine_equals_its_plain_steps(tiny):
+    """Verified rows, replays of one to five rows and plain single rows on the kernels that the engine chooses."""
+    from pocketllm_b200.models import qwen_hybrid as qh
+    from pocketllm_b200.runtime.speculative import ReplayDrafter, speculative_generate
+    cfg, tensors, d = tiny
+    prompt = [3, 1, 4, 1, 5, 9, 2, 6, 5, 3, 5]
+    e = qh.QwenEngine(cfg, max_context=256, prefill_chunk=8).load(d)
+    ref = [e.prefill(prompt)]
+    while len(ref) < 33:
+        ref.append(e.forward_rows([ref[-1]])[0])
+    for wrong_at in (2, 3, 5, 100):          # accepted drafts per round: one to all
+        e.reset()
+        drafts = [t if (i + 1) % wrong_at else (t + 7) % cfg.vocab_size for i, t in enumerate(ref[1:])]
+        out, st = speculative_generate(e, prompt, 33, ReplayDrafter(drafts, len(prompt) + 1), k=6)
+        assert out == ref and st.rounds > 0 and (wrong_at == 100 or st.replays > 0)
+    e.close()
+
+
 def test_native_server_serves_the_engine(tiny):
     """pocket_engine --serve: the tokens behind the HTTP answer are the engine's greedy tokens."""
     import http.client
