@@ -33,7 +33,7 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     reference switches to its prefill kernels for rows > 1, src/components/gguf/quantized_ops.py:9-76)."""
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
-    if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name, N, K):
+    if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name, N, K) and not _registers_faster(type_name, M, N * K):
         return _umma_linear(_aligned(x), w_raw, type_name, N, _aligned(gamma), eps, epi, status)
     if M >= TENSOR_CORE_MIN_ROWS and K % 64 == 0 and (epi != 1 or (N // 2) % 128 == 0):
         from . import gemm_bf16, rmsnorm, EPI_BF16, EPI_SWIGLU, EPI_F32
@@ -54,8 +54,9 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
 
 # Block types whose integer part fits fp16: decoded inside the tensor-core kernel (`csrc/kernels/quant_umma.cu`)
 UMMA_TYPES = frozenset({"iq2_xxs", "q4_k", "q5_k"})
-# Q5_K rows of 8192 x 3072 / 3072 x 6144, us, against decoding per eight rows or (from 32 rows) to a bf16 scratch: 1 row 22 / 21 against
-# 25 / 23, 8 rows 22 / 21 against 93 / 86, 64 rows 27 / 27 against 59 / 65, 256 rows 60 / 54 against 63 / 69.
+# Rows of 8192 x 3072 / 3072 x 6144 / 24576 x 6144, us, against decoding per eight rows or (from 32 rows) to a bf16 scratch. Q5_K: 8 rows
+# 22 / 20 / 74 against 95 / 100 / 526, 64 rows 27 / 27 / 97 against 60 / 65 / 272, 256 rows 60 / 55 / 302 against 63 / 68 / 302;
+# IQ2_XXS, 256 rows: 51 / 48 / 252 against 52 / 59 / 244; Q4_K: 54 / 51 / 268 against 57 / 63 / 270.
 UMMA_MAX_ROWS = 257
 UMMA_SPLIT_ROUTES = 64
 UMMA_MAX_GROUPS = 512
@@ -67,6 +68,18 @@ def _umma_takes(w_raw: torch.Tensor, type_name: str, rows: int, K: int, groups: 
         return False
     n = rows * row_bytes(type_name, K)
     return n % 4 == 0 and n < 1 << 32 and w_raw.numel() >= n * groups       # whole words: IQ2 blocks are copied by four bytes
+
+
+def _registers_faster(type_name: str, rows: int, weights: int) -> bool:
+    """Few rows of a small weight decode faster in registers: one launch there, two and a pipeline to fill here (10 us at least), against
+    a multiply-add per weight and row. One row of 2048 x 2048 / 4096 x 4096 / 8192 x 3072, us: IQ2_XXS 5.2 against 13.5, 12.9 / 19.1,
+    19.1 / 21.7 (12288 x 3072: 26.7 / 24.4); Q4_K 7.1 / 13.2, 16.5 / 17.2, 21.9 / 19.2; Q5_K 8.2 / 14.2, 20.2 / 18.6, 25.6 / 21.2.
+    Four rows of 2048 x 2048: 9.7 / 13.8, 12.0 / 13.5, 12.9 / 14.5; eight 16.8 / 13.9, 17.7 / 13.7, 18.9 / 14.6; eight of
+    1024 x 2048 12.1 / 13.8, 12.0 / 13.0, 12.6 / 13.7."""
+    if rows > 8:
+        return False
+    width = 1 << (rows - 1).bit_length()        # the kernels have one, two, four or eight rows
+    return width * weights <= (1 << 25 if type_name == "iq2_xxs" and rows <= 2 else 1 << 24)
 
 
 class StepWord:
@@ -153,7 +166,9 @@ def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, g
     M, K = x.shape
     columns = 16 if M <= 16 else 32 if M <= 32 else 64
     tiles = (-(-(N // 2) // 64) if epi == 1 else -(-N // 128)) * -(-M // columns)
-    splits = _umma_splits(tiles, K, _umma_slots(type_name, columns))
+    slots = _umma_slots(type_name, columns)
+    # several column tiles that fill the SMs once: parts of 64 columns cost more than the last round saves (192 rows of 8192 x 3072: 59 against 51 us)
+    splits = 1 if M > 64 and tiles >= slots else _umma_splits(tiles, K, slots)
     st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
     y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
     _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits, splits, status)

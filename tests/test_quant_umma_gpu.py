@@ -43,6 +43,39 @@ def test_linear(name, M, N, K):
         assert _rel(go.gguf_linear(xs, raw, name, N, epi=1), torch.nn.functional.silu(a) * b) < 2 ** -8
 
 
+@pytest.mark.parametrize("name", ["iq2_xxs", "q4_k", "q5_k"])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (1, 300, 3072), (5, 64, 768), (8, 2, 2304)])
+def test_few_rows_of_small_weights_on_the_tensor_cores(name, M, N, K):
+    """Sizes that `gguf_linear` decodes in registers, in the kernel all the same; zeros and infinities too."""
+    from pocketllm_b200.ops import gguf_ops as go
+    raw, w = _raw(name, N, K, M + N)
+    g = torch.Generator("cuda").manual_seed(K)
+    x = (torch.randn(M, K, device="cuda", generator=g) * torch.logspace(-4, 4, M, device="cuda")[:, None]).to(torch.bfloat16)
+    gamma = 1 + 0.1 * torch.randn(K, device="cuda", generator=g)
+    run = lambda x, gamma=None, epi=2: go._umma_linear(x, raw, name, N, gamma, 1e-6, epi, None)
+    n = (x.float() * torch.rsqrt((x.float() ** 2).mean(-1, keepdim=True) + 1e-6) * gamma).to(torch.bfloat16).double()
+    assert _rel(run(x), x.double() @ w.T) < TOL and _rel(run(x, gamma), n @ w.T) < 2e-4 and _rel(run(x, epi=0), x.double() @ w.T) < 2 ** -8
+    x[0] = 0
+    x[-1, 3] = float("inf") if M > 1 else 0.0
+    y = run(x)
+    assert (y[0] == 0).all() and (M == 1 or (not torch.isfinite(y[-1]).any() and _rel(y[1:-1], x[1:-1].double() @ w.T) < TOL))
+
+
+@pytest.mark.parametrize("name", ["iq2_xxs", "q4_k", "q5_k"])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 8, 9])
+def test_linear_on_both_sides_of_the_rule(name, M):
+    """Weights of the last size that few rows decode in registers, and one block row more."""
+    from pocketllm_b200.ops import gguf_ops as go
+    K, N = 8192, (1 << 24 if name != "iq2_xxs" or M > 2 else 1 << 25) // (1 << (M - 1).bit_length()) // 8192
+    raw, w = _raw(name, 32, K, M)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    for n in (N, N + 32):
+        assert go._registers_faster(name, M, n * K) == (n == N and M <= 8)
+        y = go.gguf_linear(x, raw.repeat(n // 32), name, n, epi=2).view(M, n // 32, 32)
+        want = x.double() @ w.T
+        assert _rel(y[:, 0], want) < TOL and torch.equal(y[:, :1].expand_as(y), y)
+
+
 def test_linear_rows_of_zeros_and_infinities():
     from pocketllm_b200.ops import gguf_ops as go
     raw, w = _raw("q5_k", 256, 512, 0)
@@ -62,6 +95,7 @@ def test_one_row_of_any_stride():
     x = torch.randn(512, 1, device="cuda").to(torch.bfloat16).t()
     assert x.stride(0) == 1 and x.is_contiguous()
     assert _rel(go.gguf_linear(x, raw, "q5_k", 520, epi=2), x.double() @ w.T) < TOL
+    assert _rel(go._umma_linear(x, raw, "q5_k", 520, None, 0.0, 2, None), x.double() @ w.T) < TOL
 
 
 @pytest.mark.parametrize("M", [1, 20])
