@@ -508,8 +508,19 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
 #pragma unroll
   for (int m = 0; m < 8; ++m) a[m] = 0.f;
   const float* w = rw + (size_t)e * H;
-  if ((H & 3) == 0 && ((uintptr_t)rw & 15) == 0) {
-    // by 16 bytes instead of four, 256 experts of 3072: 1 token 11.3 -> 10.5 us, 23 tokens 22.3 -> 14.2
+  const bool vec = (H & 3) == 0 && ((uintptr_t)rw & 15) == 0;
+  // one token without the loop over eight: the same sums in the same order
+  if (nt == 1 && vec) {
+#pragma unroll 8
+    for (int k = lane * 4; k < H; k += 128) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(w + k));
+      const float4 b = *reinterpret_cast<const float4*>(xs + k);
+      a[0] = fmaf(v.w, b.w, fmaf(v.z, b.z, fmaf(v.y, b.y, fmaf(v.x, b.x, a[0]))));
+    }
+  } else if (nt == 1) {
+    for (int k = lane; k < H; k += 32) a[0] = fmaf(w[k], xs[k], a[0]);
+  } else if (vec) {
+    // by 16 bytes instead of four, 256 experts of 3072: 23 tokens 26.8 -> 18.9 us
 #pragma unroll 4
     for (int k = lane * 4; k < H; k += 128) {
       const float4 v = __ldg(reinterpret_cast<const float4*>(w + k));
@@ -538,8 +549,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
 
 // The same for many tokens: a block has 16 tokens x 64 experts, four groups of 128 threads take a quarter of the K steps each and
 // add up in their order; a thread has 2 x 4 sums, four values of K at a time (shared-memory reads and multiply-adds then take about
-// as long). 256 tokens of 3072 by 256 experts: 76 -> 60 us, 1500 tokens: 365 -> 174 us (the form above reads the router's rows once
-// per 8 tokens).
+// as long). 1500 tokens of 3072 by 256 experts: 361 -> 183 us (the form above, which reads the router's rows once per 8 tokens, 279).
+// The sums are added in another order than above.
 constexpr int kRt = 16, kRe = 64, kRk = 32;
 __global__ void __launch_bounds__(512) router_logits_tile_kernel(const bf16* __restrict__ x, const float* __restrict__ rw, int H, int E, int T, float* logits) {
   __shared__ __align__(16) float ws[4][kRe][kRk + 4];
@@ -834,8 +845,10 @@ static float* router_scratch(size_t floats) {
   return buf[dev];
 }
 
-// From 128 tokens the tiles of 16 tokens fill the SMs; with fewer the form of one warp per expert has more blocks.
-static constexpr int kRouterTileMin = 128;
+// A tile takes the time of its K steps however few there are, so the tiles pay when tokens x experts fill the SMs with them and an
+// expert tile is full. One warp per expert / tiles, us: 256 experts of 3072, 256 tokens 58 / 64, 384 tokens 84 / 64; 128 of 4096, 512 tokens 90 / 83;
+// 64 of 2048, 1024 tokens 41 / 44, 1500 tokens 56 / 48; 8 of 4096, 1500 tokens 33 / 83.
+static constexpr long long kRouterTileMin = 72000;
 
 PK_API int pk_router_topk(const void* x, const float* router_w, const float* bias, int T, int H, int E, int topk,
                           int score_func, int norm_topk, float route_scale, int* ids, float* weights,
@@ -856,7 +869,7 @@ PK_API int pk_router_topk(const void* x, const float* router_w, const float* bia
   }
   float* logits = router_scratch((size_t)T * E);
   if (logits == nullptr) return PK_ERR_CUDA;
-  if (T >= kRouterTileMin)
+  if (E >= kRe && (long long)T * E >= kRouterTileMin)
     router_logits_tile_kernel<<<dim3((E + kRe - 1) / kRe, (T + kRt - 1) / kRt), 512, 0, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);
   else
     router_logits_kernel<<<dim3((E + 7) / 8, (T + 7) / 8), 256, smem_x, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);

@@ -257,7 +257,7 @@ def test_grouped_routes(T, topk, E):
     assert torch.equal(routes.src.cpu().long(), order) and torch.equal(tok.long(), order // topk) and torch.equal(w, weight.view(-1)[order])
 
 
-@pytest.mark.parametrize("T,E,H", [(1, 256, 3072), (3, 33, 1002), (9, 40, 1000), (127, 64, 256), (128, 60, 96), (130, 65, 3072), (300, 256, 1000)])
+@pytest.mark.parametrize("T,E,H", [(1, 256, 3072), (3, 33, 1002), (9, 40, 1000), (127, 64, 256), (128, 60, 96), (130, 65, 3072), (300, 256, 1000), (281, 256, 96), (282, 256, 96), (1130, 64, 132), (2000, 40, 64)])
 def test_router_logits(T, E, H):
     from pocketllm_b200.ops import gguf_ops as go
     g = torch.Generator("cuda").manual_seed(T)
