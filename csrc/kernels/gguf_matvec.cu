@@ -674,7 +674,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, c
 // Group routes by expert, those of an expert in increasing route index (one block). Every warp counts a contiguous share of the
 // routes in counters of its own, the counts become offsets (warp by warp within an expert, expert by expert), and the warps walk
 // their shares again: 32 routes at a time, a route's place among them from a match of the expert ids. The first form scanned all
-// routes once per expert: 122 us for 2048 routes and 720 us for 12000 over 256 experts, against 9 and 26 us.
+// routes once per expert: 238 us for 4096 routes over 256 experts, against 11 us.
 __global__ void __launch_bounds__(1024) group_routes_kernel(const int* ids, const float* weights, int T, int topk, int E,
                                                             int* seg_start, int* route_token, float* route_weight,
                                                             int* route_src) {
@@ -884,7 +884,8 @@ PK_API int pk_group_routes(const int* ids, const float* weights, int T, int topk
                            float* route_weight, int* route_src, cudaStream_t stream) {
   if (E + 1 > 12000) return PK_ERR_UNSUPPORTED;
   const int R = T * topk;
-  int warps = min(32, max(1, (R + 31) / 32));
+  // warps for the routes and, with few of them, for the walk over the experts: one token of 256 / 2000 experts 5.0 / 27.7 -> 3.4 / 8.5 us
+  int warps = min(32, max((E + 63) / 64, (R + 31) / 32));
   while (warps > 4 && (size_t)warps * E * sizeof(int) > 192 * 1024) warps >>= 1;
   const size_t smem = (size_t)warps * E * sizeof(int);
   if (smem > kPlainSmem) {

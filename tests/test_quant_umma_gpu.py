@@ -243,7 +243,7 @@ def test_narrow_linear(M, N, K):
     assert _rel(y[:, :N], x.double() @ w.double().T) < 2 ** -8 and torch.isnan(y[:, N:]).all()
 
 
-@pytest.mark.parametrize("T,topk,E", [(1, 8, 256), (3, 2, 5), (700, 8, 256), (129, 6, 2000), (40, 1, 11000)])
+@pytest.mark.parametrize("T,topk,E", [(1, 8, 256), (3, 2, 5), (700, 8, 256), (129, 6, 2000), (40, 1, 11000), (1, 6, 2000), (2, 3, 65), (1, 4, 11999)])
 def test_grouped_routes(T, topk, E):
     from pocketllm_b200.ops import gguf_ops as go
     g = torch.Generator().manual_seed(T)
