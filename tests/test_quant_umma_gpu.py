@@ -300,3 +300,18 @@ def test_bf16_rows_round_their_sums(K):
         x, w = x.to(torch.bfloat16), (torch.randn(256, K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
         y = mo.linear(x, w, torch.empty(3, 256, device="cuda"), torch.zeros(1, device="cuda", dtype=torch.int32))
         assert _rel(y, x.double() @ w.double().T) < 4 * 2 ** -24
+
+
+@pytest.mark.parametrize("M,K", [(1, 8), (300, 256), (3, 1016), (3, 1024), (2, 1028), (7, 3072), (2, 12296)])
+@pytest.mark.parametrize("mode", [1, 2])
+def test_rmsnorm_by_width(M, K, mode):
+    """On both sides of the 16-byte form's rule, with a residual sum and without."""
+    from pocketllm_b200 import ops
+    g = torch.Generator("cuda").manual_seed(M + K)
+    x, gamma, y = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16), torch.randn(K, device="cuda", generator=g), torch.randn(1, M, K, device="cuda", generator=g)
+    h = torch.empty_like(x)
+    scale = gamma.double() + (1 if mode == 1 else 0)
+    norm = lambda v: v.double() * torch.rsqrt((v.double() ** 2).mean(-1, keepdim=True) + 1e-6) * scale
+    assert _rel(ops.rmsnorm(x, gamma, mode=mode), norm(x)) < 2 ** -8
+    out = ops.rmsnorm(x, gamma, mode=mode, parts=y, hidden_out=h)
+    assert torch.equal(h, (x + y[0]).to(torch.bfloat16)) and _rel(out, norm(h)) < 2 ** -8
