@@ -336,9 +336,9 @@ __global__ void __launch_bounds__(256) full_qk_norm_rope_append_kernel(const Ful
 }
 
 // The same for rows of whole 16-byte pieces whose rotated halves are whole pieces as well: the row is loaded once, eight elements a
-// thread, and kept in shared memory, where an element finds its partner. One row of 48 heads 15 -> 4.8 us, 256 rows 14 -> 9 us; with 1500 rows the form above has
-// enough blocks to hide its loads and fewer threads without an element (30 against 37 us).
-constexpr int kFullQkThreads = 512, kFullQkVecRows = 512;
+// thread, and kept in shared memory, where an element finds its partner. One row of 48 heads 7.7 -> 4.1 us, 64 rows 8.3 -> 4.5; from 256
+// rows on (8.6 against 9.2 us, 512 rows 9.6 against 13.3) the form above has enough blocks to hide its loads and fewer threads without an element.
+constexpr int kFullQkThreads = 512, kFullQkVecRows = 128;
 __global__ void __launch_bounds__(kFullQkThreads) full_qk_norm_rope_append_vec_kernel(const FullQkParams p) {
   extern __shared__ __align__(16) float xs[];      // [heads * D]
   __shared__ float red[40];

@@ -603,3 +603,27 @@ def test_full_qk_norm_rope_append_matches_torch():
     untouched = torch.ones(ctx, dtype=torch.bool, device="cuda")
     untouched[idx] = False
     assert kc[:, untouched].abs().sum() == 0 and vc[:, untouched].abs().sum() == 0
+
+
+@pytest.mark.parametrize("T", [1, 128, 129])
+def test_full_qk_norm_on_both_sides_of_the_rule(T):
+    from pocketllm_b200 import ops
+    g = torch.Generator("cuda").manual_seed(T)
+    Hq, Hkv, rd = 6, 2, 32
+    q, k, v = (torch.randn(T, h * 128, device="cuda", generator=g).to(torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    qg, kg, ang = (torch.randn(n, device="cuda", generator=g) for n in (Hq * 128, Hkv * 128, 200 * rd // 2))
+    cos, sin = ang.cos().view(200, rd // 2), ang.sin().view(200, rd // 2)
+    kc, vc = (torch.zeros(Hkv, 200, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    pos = torch.arange(3, 3 + T, device="cuda", dtype=torch.int32)
+    out = ops.full_qk_norm_rope_append(q, k, v, pos, qg, kg, cos, sin, kc, vc, n_heads=Hq, n_kv_heads=Hkv, rope_dim=rd)
+
+    def want(x, gamma, H):
+        y = (x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-6) * gamma.double()).view(T, H, 128)
+        a, b = y[..., :rd // 2].clone(), y[..., rd // 2:rd].clone()
+        c, s = cos[pos.long(), None].double(), sin[pos.long(), None].double()
+        y[..., :rd // 2], y[..., rd // 2:rd] = a * c - b * s, b * c + a * s
+        return y
+
+    for got, ref in ((out, want(q, qg, Hq)), (kc[:, 3:3 + T].transpose(0, 1), want(k, kg, Hkv))):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+    assert torch.equal(vc[:, 3:3 + T].transpose(0, 1).reshape(T, -1), v)
