@@ -1,17 +1,19 @@
 // Products of few token rows with quantised weights through the 5th-generation tensor cores: linear layers and routed experts on raw
 // GGUF blocks, linear layers in E4M3 with a scale per 128 x 128 block.
 //
-// The weights are the M side of the product: a tile is 128 weight rows times up to 64 token columns, so that a step with one
-// token and a step with hundreds both decode every weight once and none is expanded in HBM. Decode warps write the INTEGER part
+// The weights are the M side of the product: a tile is 128 weight rows times up to 64 token columns (a token row takes one, or two where its
+// values are two terms), so that a step with one token decodes every weight once and one with hundreds once per 64 columns; none is
+// expanded in HBM. Decode warps write the INTEGER part
 // of the weights (codebook entry or code times the sub-block's scale: at most 11 bits) as fp16 into the swizzled A tiles, token
 // rows are fp16 under a power of two per row (`pk_quant_stage_rows`), and the fp32 factor of a block is applied when
-// the block's accumulator is folded from TMEM into registers: every product is exact and every sum is fp32, as in the kernels
-// that decode in registers. K-quants carry a minimum per 32 weights: these are a second, 16-wide product per block, of the
-// minima's codes with the sums of the token values (two fp16 terms each).
+// the block's accumulator is folded from TMEM into registers: every product of a bf16 value within 2^-24 of its row's largest is
+// exact (smaller ones lose bits that fp16 has no place for) and every sum is fp32. K-quants carry a minimum per 32 weights: these
+// are a second, 16-wide product per block, of the minima's codes with the sums of the token values (two fp16 terms each).
 //
 // Measured per layer of the MiniMax-M2 shape (256 experts of 3 x 1536 x 3072 in IQ2_XXS, top 8), experts alone: 23 tokens 1860 -> 650 us
 // (kernels that decode in registers), 256 tokens 4590 -> 1215 us (decode to a bf16 scratch, bf16 GEMM), 1500 tokens 4750 -> 1470 us. Bound by
-// the decode's instructions: 0.14 ms of weights at the copy rate. One token's 8 routes: 50 + 32 -> 39 + 26 us with K in parts. E4M3, 40
+// the shared-memory pipe of the decode (77 % busy, a third of it bank conflicts of the codebook's random 8-byte reads; issue slots 67 %,
+// DRAM 9 %): 0.14 ms of weights at the copy rate. One token's 8 routes: 50 + 32 -> 39 + 26 us with K in parts. E4M3, 40
 // rows of 34816 x 5120: 71 us, 2.5 TB/s.
 //
 //   warps 0-3 (0-7 for 64 columns)  fold: TMEM -> fp32 registers with the block factors, epilogue
@@ -170,7 +172,8 @@ __device__ __forceinline__ uint4 ld_shared4(uint32_t a) {
 }
 
 template <int TYPE> struct Dec;
-// The instructions per weight set the pace of this type (ALU pipe): codebook bytes become halves 1024 + v by one byte permutation a
+// A codebook entry per eight weights is read from a random place in shared memory, which with the instructions sets the pace of this type.
+// Few instructions per weight: codebook bytes become halves 1024 + v by one byte permutation a
 // pair, sign bits reach the tops of the halves by a multiplication, and scale and bias are one fused multiply-add.
 template <> struct Dec<T_IQ2_XXS> {
   // a block of 66 bytes starts on 4 bytes or two behind: 17 words hold it
@@ -727,7 +730,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
 }
 
 // Token rows for the product: fp16 under a power of two per row (1024 at most, so that a bf16 value within 2^-24 of the row's
-// largest keeps all its bits), in one or two terms, in the order of the decoded weights; with `mins` the sums over every 32
+// largest keeps all its bits), in one or two terms (22 to 23 bits of an fp32 value), in the order of the decoded weights; with `mins` the sums over every 32
 // values follow each 256. One block per row.
 struct StageParams {
   const void* x;

@@ -27,7 +27,7 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     `UMMA_TYPES` whose wait ran out gives NaN, and so does one that finds the word set; its owner reads the word once per step
     (`StepWord`) and clears it.
 
-    Up to `UMMA_MAX_ROWS - 1` rows of the types in `UMMA_TYPES` are decoded inside a tensor-core kernel, once for all rows.
+    Up to `UMMA_MAX_ROWS - 1` rows of the types in `UMMA_TYPES` are decoded inside a tensor-core kernel, once per 64 rows.
     Of the other types, up to `TENSOR_CORE_MIN_ROWS - 1` rows decode the blocks in registers (groups of up to 8 rows per
     launch). Above, the weight is decoded once into a bf16 scratch and the product runs on the tcgen05 GEMM (the
     reference switches to its prefill kernels for rows > 1, src/components/gguf/quantized_ops.py:9-76)."""
