@@ -3,23 +3,24 @@
 //
 // The weights are the M side of the product: a tile is 128 weight rows times up to 64 token columns (a token row takes one, or two where its
 // values are two terms), so that a step with one token decodes every weight once and one with hundreds once per 64 columns; none is
-// expanded in HBM. Decode warps write the INTEGER part
-// of the weights (codebook entry or code times the sub-block's scale: at most 11 bits) as fp16 into the swizzled A tiles, token
-// rows are fp16 under a power of two per row (`pk_quant_stage_rows`), and the fp32 factor of a block is applied when
-// the block's accumulator is folded from TMEM into registers: every product of a bf16 value within 2^-24 of its row's largest is
-// exact (smaller ones lose bits that fp16 has no place for) and every sum is fp32. K-quants carry a minimum per 32 weights: these
-// are a second, 16-wide product per block, of the minima's codes with the sums of the token values (two fp16 terms each).
+// expanded in HBM. Decode warps write the INTEGER part of the weights (codebook entry or code times the sub-block's scale: at most 11 bits)
+// as fp16 into tensor memory, from where the products take their A operand: shared memory then holds the raw blocks, the token columns
+// and the lookups only. Token rows are fp16 under a power of two per row (`pk_quant_stage_rows`), and the fp32 factor of a block is
+// applied when the block's accumulator is folded from TMEM into registers: every product of a bf16 value within 2^-24 of its row's
+// largest is exact (smaller ones lose bits that fp16 has no place for) and every sum is fp32. K-quants carry a minimum per 32 weights:
+// these are a second, 16-wide product per block, of the minima's codes with the sums of the token values (two fp16 terms each).
 //
-// Measured per layer of the MiniMax-M2 shape (256 experts of 3 x 1536 x 3072 in IQ2_XXS, top 8), experts alone: 23 tokens 1860 -> 650 us
-// (kernels that decode in registers), 256 tokens 4590 -> 1215 us (decode to a bf16 scratch, bf16 GEMM), 1500 tokens 4750 -> 1470 us. Bound by
-// the shared-memory pipe of the decode (77 % busy, a third of it bank conflicts of the codebook's random 8-byte reads; issue slots 67 %,
-// DRAM 9 %): 0.14 ms of weights at the copy rate. One token's 8 routes: 50 + 32 -> 39 + 26 us with K in parts. E4M3, 40
-// rows of 34816 x 5120: 71 us, 2.5 TB/s.
+// Measured, 256 experts of the MiniMax-M2 shape in IQ2_XXS, gate and up / down, us (before: weights through swizzled shared memory, entries
+// of 8 bytes from one copy of the codebook, whose bank conflicts and the stores kept the shared-memory pipe 77 % busy): 184 routes
+// 410 / 223 -> 215 / 127, 2048 routes 815 / 432 -> 414 / 223, 12000 routes 957 / 510 -> 559 / 289. Bound by the instructions of the decode:
+// 4330 warp instructions per 32768 weights, of which 2450 turn codes into halves; issue slots 75 %, ALU 67 %, shared-memory pipe 35 %. Of
+// Q5_K, 256 rows of 8192 x 3072: 62 -> 43; E4M3, 40 rows of 34816 x 5120: 68 -> 57.
 //
 //   warps 0-3 (0-7 for 64 columns)  fold: TMEM -> fp32 registers with the block factors, epilogue
 //   next warp                       MMA issuer
-//   next warp                       token tiles by TMA (no multicast)
-//   8 warps (16 for 64 columns)     decode
+//   next warp                       token tiles, and raw blocks whose rows are whole 16 bytes, by TMA (no multicast)
+//   next 2 warps                    raw blocks of IQ2_XXS, by cp.async
+//   16 warps                        decode
 //
 // Weights per lane stay in the order 0 2 1 3 within four (what masking two bytes of a word into two halves gives); the staged
 // token rows have the same order.
@@ -39,6 +40,8 @@ enum : int { T_IQ2_XXS = 0, T_Q4_K = 3, T_Q5_K = 4, T_E4M3 = 20 };
 
 constexpr int BM = 128;
 constexpr int kMaxGroups = 512;
+constexpr int kMaxTiles = 1024;      // of token rows whose group and place are looked up
+constexpr int kIq2Table = (256 + 128) * 32;      // words: codes of the codebook's entries, then sign patterns, each once per lane
 constexpr uint32_t kDrainPolls = 1u << 14;      // after a wait that ran out: time for copies and products in flight, which take microseconds
 
 template <int TYPE> struct Fmt;
@@ -71,37 +74,37 @@ struct Params {
   float* ws;              // [tile][split][column][128]
   uint32_t* counters;     // [tile], zero between launches
   uint32_t* status;       // first wait that ran out; a launch that finds it set gives NaN
+  int row_tiles;
+  int step_split, step_rt, step_tt;      // from an item of a CTA to its next one
 };
 
-// IQ2_XXS with few columns has two CTAs per SM, which hide one another's waits; the others have more bytes per weight and one CTA with
-// twice the decode warps and a deeper ring.
+// One CTA per SM. A unit is 256 weights of every row of a tile (a GGUF block, two E4M3 blocks), in four pieces of 64.
 template <int TYPE, int NT>
 struct Shape {
-  static constexpr bool kWide = TYPE != T_IQ2_XXS || NT == 64;
   static constexpr int kFoldWarps = NT == 64 ? 8 : 4;
   static constexpr int kFoldCols = NT == 64 ? 32 : NT;
-  static constexpr int kDecWarps = kWide ? 16 : 8;
-  static constexpr int kRows = BM / kDecWarps;          // of a decode warp
-  static constexpr int kStages = kWide ? 3 : 2;
-  static constexpr int kSlots = TYPE == T_E4M3 ? 4 : 3;
-  static constexpr int kABytes = 2 * BM * 128, kBBytes = 2 * NT * 128;      // a stage: 128 weights of every row, in two slabs of 64
-  static constexpr int kThreads = 32 * (kFoldWarps + 2 + kDecWarps);
-  static constexpr int kCtas = kWide ? 1 : 2;      // resident per SM
+  static constexpr int kDecWarps = 16;                          // four of each quarter of the rows: one per piece
+  static constexpr int kSlots = TYPE == T_IQ2_XXS ? (NT == 64 ? 6 : 8) : TYPE == T_E4M3 ? 4 : 5;      // units of raw blocks
+  static constexpr int kBBytes = NT * 128;                      // token columns of a piece
+  static constexpr int kThreads = 32 * (kFoldWarps + 4 + kDecWarps);
 };
 
-template <class S, int PITCH>
+template <int TYPE, int NT, int PITCH>
 struct __align__(1024) Smem {
-  uint8_t a[S::kStages][S::kABytes];
-  uint8_t b[S::kStages][S::kBBytes];
+  using S = Shape<TYPE, NT>;
+  uint32_t tab[TYPE == T_IQ2_XXS ? kIq2Table : 256];      // first: its lookups count on the place
+  uint8_t b[2][4][S::kBBytes];
+  uint8_t bm[Fmt<TYPE>::mins ? 2 : 1][Fmt<TYPE>::mins ? S::kBBytes : 1024];      // sums of the token values, for the minima
   uint8_t ring[S::kSlots][BM * PITCH];
-  uint64_t grid[PITCH == 68 ? 256 : 1];
-  uint64_t full[S::kStages], empty[S::kStages];
-  uint64_t acc_full[2], acc_empty[2];
+  float factor[4][Fmt<TYPE>::mins ? 2 : 1][BM];      // of a unit's rows, and those of the minima
+  uint64_t raw[S::kSlots], freed[S::kSlots];      // a slot's blocks are there; have been read
+  uint64_t full[2], done[2], folded[2];              // a unit's operands are there, its products are, its accumulator has been read
   uint64_t drained;
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
   uint32_t last;
   int prefix[kMaxGroups + 1];     // token tiles before each group
+  int2 tiles[kMaxTiles];          // `Cursor::place`
 };
 
 // One stretch of work: blocks [b0, b1) of a tile of 128 weight rows and up to NT columns.
@@ -109,29 +112,58 @@ struct Item {
   int group, rt, split, b0, b1, row0, cnt, tile;
 };
 
+// A CTA's items in their order: parts of K within row tiles within token tiles, every gridDim.x-th of them.
 template <int NT, int TERMS>
-__device__ __forceinline__ bool item_at(const Params& p, const int* prefix, int row_tiles, int i, Item& w) {
-  const int total = prefix[p.n_groups];
-  w.split = i % p.splits;
-  i /= p.splits;
-  w.tile = i;
-  w.rt = i % row_tiles;
-  const int tt = i / row_tiles;
-  if (tt >= total) return false;
-  int lo = 0, hi = p.n_groups;      // prefix[lo] <= tt < prefix[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (prefix[mid] <= tt) lo = mid;
-    else hi = mid;
+struct Cursor {
+  int split, rt, tt;
+  __device__ __forceinline__ explicit Cursor(const Params& p) {
+    const int i = blockIdx.x / p.splits;
+    split = blockIdx.x - i * p.splits;
+    tt = i / p.row_tiles;
+    rt = i - tt * p.row_tiles;
   }
-  w.group = lo;
-  const int first = p.seg ? __ldg(p.seg + lo) : 0, end = p.seg ? __ldg(p.seg + lo + 1) : p.M;
-  w.row0 = first + (tt - prefix[lo]) * (NT / TERMS);
-  w.cnt = min(NT / TERMS, end - w.row0);
-  w.b0 = p.nblk * w.split / p.splits;
-  w.b1 = p.nblk * (w.split + 1) / p.splits;
-  return true;
-}
+  __device__ __forceinline__ void next(const Params& p) {
+    split += p.step_split;
+    rt += p.step_rt;
+    tt += p.step_tt;
+    if (split >= p.splits) {
+      split -= p.splits;
+      ++rt;
+    }
+    if (rt >= p.row_tiles) {
+      rt -= p.row_tiles;
+      ++tt;
+    }
+  }
+  template <class Sm>
+  __device__ __forceinline__ bool get(const Params& p, const Sm& sm, Item& w) const {
+    if (tt >= sm.prefix[p.n_groups]) return false;
+    w.split = split;
+    w.rt = rt;
+    w.tile = tt * p.row_tiles + rt;
+    w.b0 = p.splits == 1 ? 0 : p.nblk * split / p.splits;
+    w.b1 = p.splits == 1 ? p.nblk : p.nblk * (split + 1) / p.splits;
+    const int2 t = tt < kMaxTiles ? sm.tiles[tt] : search(p, sm.prefix, tt);
+    w.row0 = t.x;
+    w.cnt = t.y & 255;
+    w.group = t.y >> 8;
+    return true;
+  }
+  static __device__ __forceinline__ int2 search(const Params& p, const int* prefix, int tt) {
+    int lo = 0, hi = p.n_groups;      // prefix[lo] <= tt < prefix[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (prefix[mid] <= tt) lo = mid;
+      else hi = mid;
+    }
+    return place(p, lo, tt - prefix[lo]);
+  }
+  // tile n of a group: first row; group * 256 + rows
+  static __device__ __forceinline__ int2 place(const Params& p, int g, int n) {
+    const int first = p.seg ? __ldg(p.seg + g) : 0, end = p.seg ? __ldg(p.seg + g + 1) : p.M, row0 = first + n * (NT / TERMS);
+    return make_int2(row0, g * 256 + min(NT / TERMS, end - row0));
+  }
+};
 
 // Byte offset, in its group, of the weight row behind row `i` of a tile. SwiGLU tiles alternate gate and up rows, so that a pair
 // sits in neighbouring lanes.
@@ -147,67 +179,92 @@ __device__ __forceinline__ uint32_t tile_row(const Params& p, const Item& w, int
 }
 __device__ __forceinline__ const uint8_t* group_base(const Params& p, const Item& w) { return p.W + (long long)w.group * p.rows * p.rb; }
 
+// `__byte_perm` without its mask over the selector, whose nibbles are 0 to 7 here
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+// A value that is kept in a register, not computed again at every use.
+__device__ __forceinline__ void keep(uint32_t& v) { asm volatile("" : "+r"(v)); }
 __device__ __forceinline__ uint32_t mul2(uint32_t x, __half2 s, __half2 off) {
   const __half2 r = __hfma2(*reinterpret_cast<__half2*>(&x), s, off);
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-__device__ __forceinline__ void st_shared4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-__device__ __forceinline__ float ld_half(const uint8_t* p) { return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short*>(p)))); }
-
-// A decode warp owns RW rows of the tile: it copies their blocks, kSlots - 1 ahead, into a ring of its own (`cp.async`, neighbouring
-// lanes take neighbouring bytes: a load of every lane from a row of its own is an L1 pass per row) and decodes from there; a lane
-// decodes half a slab of one row at a time.
+template <int OFF = 0>
 __device__ __forceinline__ uint32_t ld_shared(uint32_t a) {
   uint32_t v;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  asm volatile("ld.shared.b32 %0, [%1 + %2];" : "=r"(v) : "r"(a), "n"(OFF) : "memory");
   return v;
 }
+__device__ __forceinline__ float half_of(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
 __device__ __forceinline__ uint4 ld_shared4(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
   return v;
 }
 
+// `load`: what piece j of a lane's row needs, from the unit at `src`, whose first byte has the address a16 (mod 16) in memory.
+// `half_piece`: sub-block h of the piece as 16 pairs in the order of the token rows. `factors`: those of the row's block.
 template <int TYPE> struct Dec;
-// A codebook entry per eight weights is read from a random place in shared memory, which with the instructions sets the pace of this type.
-// Few instructions per weight: codebook bytes become halves 1024 + v by one byte permutation a
-// pair, sign bits reach the tops of the halves by a multiplication, and scale and bias are one fused multiply-add.
+// A weight is one of three magnitudes with a sign: a nibble of 0..2 for the magnitude, plus 4 when it is negative. An entry's eight
+// nibbles and a sign pattern's eight come from tables that hold every word once per lane (a random read is then one pass, where entries of
+// 8 bytes read by 32 lanes took six on average), and the sum of the two selects bytes 128 +- magnitude by byte permutation. With 0x64
+// above them these are halves 1024 + 128 +- magnitude; scale and bias are one fused multiply-add.
 template <> struct Dec<T_IQ2_XXS> {
-  // a block of 66 bytes starts on 4 bytes or two behind: 17 words hold it
-  static constexpr int kCopy = 4, kData = 68, kPitch = 68;
-  __device__ static void stage(uint32_t src, int mis, uint32_t dst, int row7, int h, int s, uint32_t grid) {
-    const uint32_t a = src + ((mis + 2 + (2 * s + h) * 8) & ~3);
-    uint32_t w0 = ld_shared(a), w1 = ld_shared(a + 4);
-    if (!mis) {
-      const uint32_t w2 = ld_shared(a + 8);
-      w0 = __byte_perm(w0, w1, 0x5432);
-      w1 = __byte_perm(w1, w2, 0x5432);
-    }
-    // the odd scale 2 s + 1 as a half, from 1024 + it
-    const uint32_t lsw = 0x64016401u + (w1 >> 28) * 0x00020002u;
-    const __half2 s2 = __hadd2(*reinterpret_cast<const __half2*>(&lsw), __float2half2_rn(-1024.f)), o2 = __hmul2(s2, __float2half2_rn(-1024.f));
-    const uint32_t at = dst | (((4 * h) ^ row7) << 4);
-    uint32_t e[4][2];      // all four entries are on their way before the first is used
+  // 66 bytes lie in five of the 16-byte pieces of memory, wherever they begin
+  static constexpr int kPitch = 80, kRegs = 10;
+  static constexpr uint32_t kAlign = 32768;      // of the tables: the place of an entry and of the lane are put together by bits
+  // Rows in the ring: eight rows of 80 bytes are a multiple of all banks; rows of different alignment come to those places.
+  __device__ static int place(int r) { return (r >> 2) | (r & 3) << 3; }
+  __device__ static void load(uint32_t src, uint32_t a16, int j, uint32_t tab, uint32_t (&w)[kRegs]) {
+    const uint32_t o = a16 + 2 + 16 * j, a = src + (o & ~3u), sel = (o & 2) ? 0x5432u : 0x3210u;
+    uint32_t v[5];
 #pragma unroll
-    for (int g = 0; g < 4; ++g)
-      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(e[g][0]), "=r"(e[g][1]) : "r"(grid + ((w0 >> (8 * g)) & 255u) * 8u));
+    for (int i = 0; i < 5; ++i) v[i] = ld_shared(a + 4 * i);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      const uint32_t lo = e[g][0], hi = e[g][1];
-      uint32_t sg = (w1 >> (7 * g)) & 127u;
-      sg += (__popc(sg) & 1u) * 128u;                 // the eighth sign makes their number even
-      uint32_t x0 = mul2(__byte_perm(lo, 0x64646464u, 0x4240), s2, o2), x1 = mul2(__byte_perm(lo, 0x64646464u, 0x4341), s2, o2);
-      uint32_t x2 = mul2(__byte_perm(hi, 0x64646464u, 0x4240), s2, o2), x3 = mul2(__byte_perm(hi, 0x64646464u, 0x4341), s2, o2);
-      x0 ^= (sg * ((1u << 15) + (1u << 29))) & 0x80008000u;
-      x1 ^= (sg * ((1u << 14) + (1u << 28))) & 0x80008000u;
-      x2 ^= (sg * ((1u << 11) + (1u << 25))) & 0x80008000u;
-      x3 ^= (sg * ((1u << 10) + (1u << 24))) & 0x80008000u;
-      st_shared4(at ^ (g << 4), x0, x1, x2, x3);
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t idx = prmt(v[2 * h], v[2 * h + 1], sel), aux = prmt(v[2 * h + 1], v[2 * h + 2], sel), aux2 = aux >> 14;
+      w[8 + h] = aux;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t si = g == 0 ? aux << 7 : g == 1 ? aux : g == 2 ? aux2 << 7 : aux2;
+        w[4 * h + g] = ld_shared(tab + prmt(idx, 0, 0x4440 + g) * 128u) + ld_shared<32768>(tab | (si & 0x3f80u));
+      }
     }
   }
+  __device__ static void half_piece(const uint32_t (&w)[kRegs], int h, uint32_t (&x)[16]) {
+    // the odd scale 2 s + 1 as a half, from 1024 + it
+    const uint32_t lsw = 0x64016401u + (w[8 + h] >> 28) * 0x00020002u;
+    const __half2 s2 = __hadd2(*reinterpret_cast<const __half2*>(&lsw), __float2half2_rn(-1024.f)), o2 = __hmul2(s2, __float2half2_rn(-1152.f));
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      constexpr uint32_t plus = 136u | 153u << 8 | 171u << 16, minus = 120u | 103u << 8 | 85u << 16;      // 128 +- 8, 25, 43
+      const uint32_t c = w[4 * h + g], lo = prmt(plus, minus, c), hi = prmt(plus, minus, c >> 16);
+      x[4 * g] = mul2(prmt(lo, 0x64646464u, 0x4140), s2, o2);
+      x[4 * g + 1] = mul2(prmt(lo, 0x64646464u, 0x4342), s2, o2);
+      x[4 * g + 2] = mul2(prmt(hi, 0x64646464u, 0x4140), s2, o2);
+      x[4 * g + 3] = mul2(prmt(hi, 0x64646464u, 0x4342), s2, o2);
+    }
+  }
+  __device__ static void factors(uint32_t src, uint32_t a16, float* f) { f[0] = 0.125f * half_of(ld_shared(src + (a16 & ~3u)) >> (8 * (a16 & 2))); }
+  // Warp w of twelve writes 32 entries of the table.
+  __device__ static void fill(uint32_t* tab, int w, int lane) {
+    uint32_t c = 0;
+    if (w < 8) {
+      const uint64_t e = kIq2xxsGrid[32 * w + lane] >> 4;      // 8, 25, 43 -> 0, 1, 2
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c |= (uint32_t)(e >> (8 * i) & 3u) << (4 * nibble(i));
+    } else {
+      const uint32_t n = 32 * (w - 8) + lane, sg = n | (__popc(n) & 1u) << 7;      // the eighth sign makes their number even
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c |= (sg >> i & 1u) << (4 * nibble(i) + 2);
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) tab[(32 * w + i) * 32 + lane] = __shfl_sync(0xffffffffu, c, i);
+  }
+  // of weight i of eight
+  __host__ __device__ static constexpr int nibble(int i) { return (i & 4) | (i & 1) << 1 | (i & 2) >> 1; }
 };
 
 // scale (m = 0) or minimum (m = 1) of sub-block j from the twelve bytes of a K-quant's 6-bit pairs
@@ -217,82 +274,101 @@ __device__ __forceinline__ uint32_t k4_field(const uint32_t (&s)[3], int j, int 
   return ((s[2] >> (k + 4 * m)) & 15u) | (((s[m] >> (k + 6)) & 3u) << 4);
 }
 
-// K-quants: low and high nibbles of bytes [16 h, 16 h + 16) of a stage's codes belong to two sub-blocks.
+// K-quants: low and high nibbles of the 32 bytes of a piece are its two sub-blocks.
 template <int TYPE> struct DecK {
-  static constexpr int kCopy = 16, kData = Fmt<TYPE>::bytes, kPitch = Fmt<TYPE>::bytes;
-  __device__ static void stage(uint32_t src, int, uint32_t dst, int row7, int h, int st, uint32_t) {
+  static constexpr int kPitch = Fmt<TYPE>::bytes, kRegs = TYPE == T_Q5_K ? 18 : 10;
+  static constexpr uint32_t kAlign = 1024;
+  __device__ static int place(int r) { return r; }
+  // words 0 to 7: codes; then the scales of the sub-blocks; then Q5_K's high bits, those of the piece lowest in their bytes
+  __device__ static void load(uint32_t src, uint32_t, int j, uint32_t, uint32_t (&w)[kRegs]) {
     const uint4 f = ld_shared4(src);
     const uint32_t s[3] = {f.y, f.z, f.w};
-    if (st == 4) {      // the codes of the eight minima, for the sums' first (h = 0) and second terms
-      uint32_t x[4];
+    w[8] = k4_field(s, 2 * j, 0);
+    w[9] = k4_field(s, 2 * j + 1, 0);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __half2 v = __halves2half2(__uint2half_rn(k4_field(s, 2 * i, 1)), __uint2half_rn(k4_field(s, 2 * i + 1, 1)));
-        x[i] = *reinterpret_cast<const uint32_t*>(&v);
+    for (int i = 0; i < 2; ++i) {
+      const uint4 q = ld_shared4(src + (TYPE == T_Q5_K ? 48 : 16) + 32 * j + 16 * i);
+      w[4 * i] = q.x;
+      w[4 * i + 1] = q.y;
+      w[4 * i + 2] = q.z;
+      w[4 * i + 3] = q.w;
+      if constexpr (TYPE == T_Q5_K) {
+        const uint4 t = ld_shared4(src + 16 + 16 * i);
+        w[10 + 4 * i] = t.x >> (2 * j);
+        w[11 + 4 * i] = t.y >> (2 * j);
+        w[12 + 4 * i] = t.z >> (2 * j);
+        w[13 + 4 * i] = t.w >> (2 * j);
       }
-      st_shared4(dst + ((h ^ row7) << 4), x[0], x[1], x[2], x[3]);
-      return;
     }
-    const uint32_t c0 = k4_field(s, 2 * st, 0), c1 = k4_field(s, 2 * st + 1, 0);
-    const __half2 s0 = __half2half2(__uint2half_rn(c0)), o0 = __half2half2(__int2half_rn(-1024 * (int)c0));
-    const __half2 s1 = __half2half2(__uint2half_rn(c1)), o1 = __half2half2(__int2half_rn(-64 * (int)c1));
-    const uint4 q = ld_shared4(src + (TYPE == T_Q5_K ? 48 : 16) + 32 * st + 16 * h);
-    const uint4 qh = TYPE == T_Q5_K ? ld_shared4(src + 16 + 16 * h) : make_uint4(0, 0, 0, 0);
-    const uint32_t qw[4] = {q.x, q.y, q.z, q.w}, hw[4] = {qh.x, qh.y, qh.z, qh.w};
-    uint32_t lo[8], hi[8];
+  }
+  __device__ static void half_piece(const uint32_t (&w)[kRegs], int h, uint32_t (&x)[16]) {
+    const int c = (int)w[8 + h];
+    const __half2 s2 = __half2half2(__int2half_rn(c)), o2 = __half2half2(__int2half_rn((h ? -64 : -1024) * c));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t q = w[i], q8 = q >> 8;
+      uint32_t a0, a1;
+      if (h == 0) {      // 1024 + code
+        a0 = (q & 0x000f000fu) | 0x64006400u;
+        a1 = (q8 & 0x000f000fu) | 0x64006400u;
+      } else {           // 64 + code
+        a0 = (q & 0x00f000f0u) | 0x54005400u;
+        a1 = (q8 & 0x00f000f0u) | 0x54005400u;
+      }
+      if constexpr (TYPE == T_Q5_K) {
+        const uint32_t t = w[10 + i], t8 = t >> 8;      // bit 0: low sub-block, bit 1: high
+        a0 |= h ? (t << 7) & 0x01000100u : (t << 4) & 0x00100010u;
+        a1 |= h ? (t8 << 7) & 0x01000100u : (t8 << 4) & 0x00100010u;
+      }
+      x[2 * i] = mul2(a0, s2, o2);
+      x[2 * i + 1] = mul2(a1, s2, o2);
+    }
+  }
+  __device__ static void factors(uint32_t src, uint32_t, float* f) {
+    const uint32_t v = ld_shared(src);
+    f[0] = half_of(v);
+    f[BM] = -half_of(v >> 16);
+  }
+  // the codes of the eight minima, for the sums' first and second terms
+  __device__ static void minima(uint32_t src, uint32_t (&x)[8]) {
+    const uint4 f = ld_shared4(src);
+    const uint32_t s[3] = {f.y, f.z, f.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint32_t w = qw[i], w8 = w >> 8;
-      uint32_t a0 = (w & 0x000f000fu) | 0x64006400u, a1 = (w8 & 0x000f000fu) | 0x64006400u;      // 1024 + code
-      uint32_t b0 = (w & 0x00f000f0u) | 0x54005400u, b1 = (w8 & 0x00f000f0u) | 0x54005400u;      // 64 + code
-      if constexpr (TYPE == T_Q5_K) {
-        const uint32_t t = hw[i] >> (2 * st), t8 = t >> 8;      // bit 0: low sub-block, bit 1: high
-        a0 |= (t << 4) & 0x00100010u;
-        a1 |= (t8 << 4) & 0x00100010u;
-        b0 |= (t << 7) & 0x01000100u;
-        b1 |= (t8 << 7) & 0x01000100u;
-      }
-      lo[2 * i] = mul2(a0, s0, o0);
-      lo[2 * i + 1] = mul2(a1, s0, o0);
-      hi[2 * i] = mul2(b0, s1, o1);
-      hi[2 * i + 1] = mul2(b1, s1, o1);
+      const __half2 v = __halves2half2(__uint2half_rn(k4_field(s, 2 * i, 1)), __uint2half_rn(k4_field(s, 2 * i + 1, 1)));
+      x[i] = x[i + 4] = *reinterpret_cast<const uint32_t*>(&v);
     }
-    st_shared4(dst + (((2 * h) ^ row7) << 4), lo[0], lo[1], lo[2], lo[3]);
-    st_shared4(dst + (((2 * h + 1) ^ row7) << 4), lo[4], lo[5], lo[6], lo[7]);
-    st_shared4(dst + (((4 + 2 * h) ^ row7) << 4), hi[0], hi[1], hi[2], hi[3]);
-    st_shared4(dst + (((5 + 2 * h) ^ row7) << 4), hi[4], hi[5], hi[6], hi[7]);
   }
 };
 template <> struct Dec<T_Q4_K> : DecK<T_Q4_K> {};
 template <> struct Dec<T_Q5_K> : DecK<T_Q5_K> {};
 
-// E4M3 codes are fp16 numbers already; the rows of the ring are 16 bytes apart from whole lines (bank conflicts).
+// E4M3 codes are fp16 numbers already; a unit is two tiles of 128 bytes a row in the 128-byte swizzle (bank conflicts).
 template <> struct Dec<T_E4M3> {
-  static constexpr int kCopy = 16, kData = 128, kPitch = 144;
-  __device__ static void stage(uint32_t src, int, uint32_t dst, int row7, int h, int s, uint32_t) {
+  static constexpr int kPitch = 256, kRegs = 16;
+  static constexpr uint32_t kAlign = 1024;
+  __device__ static int place(int r) { return r; }
+  __device__ static void load(uint32_t src, uint32_t, int j, uint32_t, uint32_t (&w)[kRegs]) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint4 v = ld_shared4(src + 64 * s + 32 * h + 16 * i);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      uint32_t x[8];
+    for (int i = 0; i < 4; ++i) {
+      const uint4 v = ld_shared4((src + (j >> 1) * (BM * 128)) + ((64 * (j & 1) + 16 * i) ^ (src >> 3 & 0x70)));
+      w[4 * i] = v.x;
+      w[4 * i + 1] = v.y;
+      w[4 * i + 2] = v.z;
+      w[4 * i + 3] = v.w;
+    }
+  }
+  __device__ static void half_piece(const uint32_t (&w)[kRegs], int h, uint32_t (&x)[16]) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[j] & 0xffffu), __NV_E4M3);
-        const __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[j] >> 16), __NV_E4M3);
-        x[2 * j] = (uint32_t)lo.x | (uint32_t)lo.y << 16;
-        x[2 * j + 1] = (uint32_t)hi.x | (uint32_t)hi.y << 16;
-      }
-      st_shared4(dst + (((4 * h + 2 * i) ^ row7) << 4), x[0], x[1], x[2], x[3]);
-      st_shared4(dst + (((4 * h + 2 * i + 1) ^ row7) << 4), x[4], x[5], x[6], x[7]);
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t v = w[8 * h + i];
+      const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(v & 0xffffu), __NV_E4M3);
+      const __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(v >> 16), __NV_E4M3);
+      x[2 * i] = (uint32_t)lo.x | (uint32_t)lo.y << 16;
+      x[2 * i + 1] = (uint32_t)hi.x | (uint32_t)hi.y << 16;
     }
   }
 };
-
-__host__ __device__ constexpr uint32_t tmem_columns(uint32_t n) {
-  uint32_t c = 32;
-  while (c < n) c *= 2;
-  return c;
-}
 
 // By one thread, behind the CTA's stores of its part: *last says whether the other parts are there.
 __device__ __forceinline__ void count_part(const Params& p, const Item& w, uint32_t* last) {
@@ -307,22 +383,22 @@ __device__ __forceinline__ void fold_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
 }
 
-// The rest of a fold warp's items, from `i` on, after a wait that ran out: NaN in their places, so that the result cannot be taken
+// The rest of a fold warp's items, from `cur` on, after a wait that ran out: NaN in their places, so that the result cannot be taken
 // for one, and every part counted, so that the counters are back at zero when the launch is over. Kept out of the loop that it ends.
-template <int NT, int TERMS, int WARPS>
-__device__ __noinline__ void give_up(const Params& p, const int* prefix, int row_tiles, int i, int c0, uint32_t* shared_last) {
+template <int NT, int TERMS, int WARPS, class Sm>
+__device__ __noinline__ void give_up(const Params& p, Sm& sm, Cursor<NT, TERMS> cur, int c0) {
   const int tid = threadIdx.x, lr = ((tid >> 5) & 3) * 32 + (tid & 31), cols = WARPS == 8 ? NT / 2 : NT;
   const float nan = __uint_as_float(0x7fffffffu);
   Item w;
-  for (; item_at<NT, TERMS>(p, prefix, row_tiles, i, w); i += gridDim.x) {
+  for (; cur.get(p, sm, w); cur.next(p)) {
     if (p.splits > 1) {
       float* part = p.ws + ((size_t)w.tile * p.splits + w.split) * NT * BM + lr;
       for (int c = c0; c < c0 + cols; ++c) __stcg(part + (size_t)c * BM, nan);
       __threadfence();
       fold_sync<WARPS>();
-      if (tid == 0) count_part(p, w, shared_last);
+      if (tid == 0) count_part(p, w, &sm.last);
       fold_sync<WARPS>();
-      const uint32_t last = *(volatile uint32_t*)shared_last;
+      const uint32_t last = *(volatile uint32_t*)&sm.last;
       fold_sync<WARPS>();
       if (!last) continue;
     }
@@ -337,33 +413,45 @@ __device__ __noinline__ void give_up(const Params& p, const int* prefix, int row
   }
 }
 
+// The copies that this thread has begun arrive on `bar` when they are there.
+__device__ __forceinline__ void copies_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(dst)), "l"(map),
+               "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
+
 template <int TYPE, int NT, int TERMS>
-__global__ void __launch_bounds__(Shape<TYPE, NT>::kThreads, Shape<TYPE, NT>::kCtas)
-quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(Shape<TYPE, NT>::kThreads, 1)
+quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ Params p) {
   using S = Shape<TYPE, NT>;
-  constexpr int kStages = S::kStages, BB = Fmt<TYPE>::bytes;
+  constexpr int BB = Fmt<TYPE>::bytes;
   constexpr bool MINS = Fmt<TYPE>::mins;
-  constexpr int ST = MINS ? 3 : Fmt<TYPE>::k / 128;      // stages of a block; the third one has the minima in its first 16 places
-  constexpr uint32_t kBufCols = MINS ? 2 * NT : NT;
-  // One CTA can have several parts of K where a decode step uses it (16 columns; wider tiles have no registers for it): columns of
-  // their sum, behind the two accumulators.
+  constexpr int kPieces = Fmt<TYPE>::k / 64, kUnit = 4 / kPieces;      // pieces of a block, blocks of a unit
+  // One CTA can have several parts of K where a decode step uses it (16 columns; wider tiles have no registers for it).
   constexpr bool kParts = TYPE != T_E4M3 && NT == 16;
-  constexpr uint32_t kSums = 2 * kBufCols, kTmemCols = tmem_columns(kSums + (kParts ? NT : 0));
+  // Tensor memory: accumulators of two units, that of the minima, the sum of the parts, the codes of the minima of two units, the weights of two units.
+  constexpr uint32_t kAccCols = kUnit * NT, kMinCol = 2 * NT, kSumCol = 3 * NT, kACodes = 240, kACol = 256, kTmemCols = 512;
+  static_assert(2 * kAccCols <= kACol && (TYPE == T_E4M3 || 3 * NT + (kParts ? NT : 0) <= kACodes), "tensor memory");
   extern __shared__ uint8_t smem_raw[];
   using D = Dec<TYPE>;
-  using Sm = Smem<S, D::kPitch>;
-  Sm& sm = *reinterpret_cast<Sm*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  using Sm = Smem<TYPE, NT, D::kPitch>;
+  // aligned in the shared window, whose addresses the lookups are made of
+  Sm& sm = *reinterpret_cast<Sm*>(smem_raw + (-smem_u32(smem_raw) & (D::kAlign - 1)));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row_tiles = (p.epi & 1) ? ((p.rows >> 1) + 63) / 64 : (p.rows + BM - 1) / BM;
+  using Cur = Cursor<NT, TERMS>;
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&sm.full[s], S::kDecWarps + 1);
-      mbar_init(&sm.empty[s], 1);
-    }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&sm.acc_full[b], 1);
-      mbar_init(&sm.acc_empty[b], S::kFoldWarps);
+      mbar_init(&sm.full[b], S::kDecWarps + 1);
+      mbar_init(&sm.done[b], 1);
+      mbar_init(&sm.folded[b], S::kFoldWarps);
+    }
+    for (int k = 0; k < S::kSlots; ++k) {
+      mbar_init(&sm.raw[k], TYPE == T_IQ2_XXS ? 64 : 1);
+      mbar_init(&sm.freed[k], 1);
     }
     mbar_init(&sm.drained, 1);
     sm.abort_flag = 0;
@@ -396,23 +484,27 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     tmem_relinquish();
   }
   if constexpr (TYPE == T_IQ2_XXS)
-    for (int i = tid; i < 256; i += S::kThreads) sm.grid[i] = kIq2xxsGrid[i];
+    if (warp >= 4 && warp < 16) D::fill(sm.tab, warp - 4, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
+  for (int g = warp; g < p.n_groups; g += S::kThreads / 32) {
+    const int first = sm.prefix[g], n = min(sm.prefix[g + 1], kMaxTiles) - first;
+    for (int k = lane; k < n; k += 32) sm.tiles[first + k] = Cur::place(p, g, k);
+  }
+  __syncthreads();
 
   if (warp < S::kFoldWarps) {
     // ---------------- fold and epilogue ----------------
     const int q = warp & 3, c0 = (warp >> 2) * S::kFoldCols, lr = q * 32 + lane;
-    uint32_t blk = 0;
+    uint32_t unit = 0;
     Item w;
     bool ok = true;
     // an earlier product of the step gave up: this one does as if its first wait had
     const bool dead = p.status != nullptr && __any_sync(0xffffffffu, *(const volatile uint32_t*)p.status);
     if (dead) sm.abort_flag = 1u;
-    for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
-      const uint8_t* row = group_base(p, w) + tile_row(p, w, lr);
+    for (Cur cur(p); ok && cur.get(p, sm, w); cur.next(p)) {
       float acc[S::kFoldCols];
 #pragma unroll
       for (int c = 0; c < S::kFoldCols; ++c) acc[c] = 0.f;
@@ -422,42 +514,41 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
         const int r = (p.epi & 1) ? min(w.rt * 64 + (lr >> 1), half - 1) + (lr & 1) * half : w.rt * BM;
         ws = p.w_scale + (size_t)(r >> 7) * p.w_ld;
       }
-      auto factor = [&](int b) { return TYPE == T_E4M3 ? __ldg(ws + b) : ld_half(row + b * BB); };
-      float d = factor(w.b0), dm = MINS ? ld_half(row + w.b0 * BB + 2) : 0.f;
       [[maybe_unused]] int part = 0, part_end = kParts && p.splits == 1 && p.parts > 1 ? p.nblk / p.parts : -1;
-      for (int b = w.b0; b < w.b1; ++b, ++blk) {
-        const int nb = min(b + 1, p.nblk - 1);
-        const float dn = factor(nb), dmn = MINS ? ld_half(row + nb * BB + 2) : 0.f;
-        const int buf = blk & 1;
-        if (dead || !mbar_wait_uniform(&sm.acc_full[buf], (blk >> 1) & 1, &sm.abort_flag, p.status, 31)) {
+      for (int b = w.b0; b < w.b1; b += kUnit, ++unit) {
+        const int buf = unit & 1;
+        if (dead || !mbar_wait_uniform(&sm.done[buf], (unit >> 1) & 1, &sm.abort_flag, p.status, 31)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const float f = TYPE == T_IQ2_XXS ? 0.125f * d : d;
-        const uint32_t t = tmem_base + buf * kBufCols + c0 + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+        for (int k = 0; k < kUnit; ++k) {
+          if (kUnit > 1 && b + k >= w.b1) break;
+          const float f = TYPE == T_E4M3 ? __ldg(ws + b + k) : sm.factor[unit & 3][0][lr];
+          const uint32_t t = tmem_base + c0 + ((uint32_t)(q * 32) << 16);
 #pragma unroll
-        for (int c = 0; c < S::kFoldCols; c += 16) {
-          uint32_t r[16];
-          tmem_ld_32x16(t + c, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(f, __uint_as_float(r[j]), acc[c + j]);
-          if constexpr (MINS) {
-            tmem_ld_32x16(t + NT + c, r);
+          for (int c = 0; c < S::kFoldCols; c += 16) {
+            uint32_t r[16];
+            tmem_ld_32x16(t + buf * kAccCols + k * NT + c, r);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(-dm, __uint_as_float(r[j]), acc[c + j]);
+            for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(f, __uint_as_float(r[j]), acc[c + j]);
+            if constexpr (MINS) {
+              const float fm = sm.factor[unit & 3][1][lr];
+              tmem_ld_32x16(t + kMinCol + c, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(fm, __uint_as_float(r[j]), acc[c + j]);
+            }
           }
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.acc_empty[buf]);
-        d = dn;
-        dm = dmn;
+        if (lane == 0) mbar_arrive(&sm.folded[buf]);
         if constexpr (kParts)
           if (b + 1 == part_end) {
-            const uint32_t ts = tmem_base + kSums + ((uint32_t)(q * 32) << 16);
+            const uint32_t ts = tmem_base + kSumCol + ((uint32_t)(q * 32) << 16);
             uint32_t r[16] = {};
             if (part > 0) {
               tmem_ld_32x16(ts, r);
@@ -479,7 +570,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
           }
       }
       if (!ok) {
-        give_up<NT, TERMS, S::kFoldWarps>(p, sm.prefix, row_tiles, i, c0, &sm.last);
+        give_up<NT, TERMS, S::kFoldWarps>(p, sm, cur, c0);
         break;
       }
       if (p.splits > 1) {
@@ -548,45 +639,33 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
     // The whole warp walks the loop and one lane issues: addresses and descriptors are then uniform, which is what the
     // instructions take; computed by a lone lane they cost more than the products.
     constexpr uint32_t idesc = umma_idesc(0, 0, BM, NT);
-    const uint64_t da0 = smem_desc_k_sw128(smem_u32(sm.a[0])), db0 = smem_desc_k_sw128(smem_u32(sm.b[0]));
+    const uint64_t db0 = smem_desc_k_sw128(smem_u32(sm.b[0][0])), dm0 = smem_desc_k_sw128(smem_u32(sm.bm[0]));
     const bool leader = elect_one();
-    uint32_t st = 0, ph = 0, blk = 0;
+    uint32_t unit = 0, slot = 0;
     Item w;
     bool ok = true;
-    for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
-      for (int b = w.b0; ok && b < w.b1; ++b, ++blk) {
-        const int buf = blk & 1;
-        if (!mbar_wait_uniform(&sm.acc_empty[buf], ((blk >> 1) & 1) ^ 1, &sm.abort_flag, p.status, 32)) {
-          ok = false;
-          break;
-        }
+    for (Cur cur(p); ok && cur.get(p, sm, w); cur.next(p)) {
+      for (int b = w.b0; b < w.b1; b += kUnit, ++unit) {
+        const uint32_t buf = unit & 1, ph = (unit >> 1) & 1;
+        // the one accumulator of the minima: the fold is through with the unit before, too
+        ok = mbar_wait_uniform(&sm.folded[buf], ph ^ 1, &sm.abort_flag, p.status, 32) && mbar_wait_uniform(&sm.full[buf], ph, &sm.abort_flag, p.status, 33) &&
+             (!MINS || unit == 0 || mbar_wait_uniform(&sm.folded[buf ^ 1], ((unit - 1) >> 1) & 1, &sm.abort_flag, p.status, 34));
+        if (!ok) break;
+        if (TYPE == T_IQ2_XXS && leader) mbar_arrive(&sm.freed[slot]);      // full: all decode warps have read theirs
+        slot = slot + 1 == S::kSlots ? 0 : slot + 1;
         tc_fence_after();
-        const uint32_t acc = tmem_base + buf * kBufCols;
-#pragma unroll 1
-        for (int s = 0; s < ST; ++s) {
-          if (!mbar_wait_uniform(&sm.full[st], ph, &sm.abort_flag, p.status, 33)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t da = da0 + st * (S::kABytes >> 4), db = db0 + st * (S::kBBytes >> 4);
-          if (leader) {
-            if (s < 2) {
+        const uint32_t acc = tmem_base + buf * kAccCols, ta = tmem_base + kACol + buf * 128;
+        const uint64_t db = db0 + buf * (4 * S::kBBytes >> 4);
+        const int pieces = kUnit == 1 ? 4 : min(4, (w.b1 - b) * kPieces);      // the last unit of an item can be one E4M3 block
+        if (leader) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k)
-                umma_f16(acc, da + (k >> 2) * (BM * 128 >> 4) + (k & 3) * 2, db + (k >> 2) * (NT * 128 >> 4) + (k & 3) * 2, idesc, (s > 0 || k > 0) ? 1u : 0u);
-            } else {
-              umma_f16(acc + NT, da, db, idesc, 0u);
-            }
-            umma_commit(&sm.empty[st]);
-            if (s == ST - 1) umma_commit(&sm.acc_full[buf]);
-          }
-          __syncwarp();
-          if (++st == kStages) {
-            st = 0;
-            ph ^= 1u;
-          }
+          for (int k = 0; k < 16; ++k)
+            if (kUnit == 1 || k / 4 < pieces)
+              umma_f16_ts(acc + (k / (4 * kPieces)) * NT, ta + k * 8, db + (k / 4) * (S::kBBytes >> 4) + (k % 4) * 2, idesc, k % (4 * kPieces) > 0 ? 1u : 0u);
+          if constexpr (MINS) umma_f16_ts(tmem_base + kMinCol, tmem_base + kACodes + buf * 8, dm0 + buf * (S::kBBytes >> 4), idesc, 0u);
+          umma_commit(&sm.done[buf]);
         }
+        __syncwarp();
       }
     }
     if (!ok) {
@@ -596,129 +675,149 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
       for (uint32_t n = 0; n < kDrainPolls && !mbar_try_wait(&sm.drained, 0); ++n) {}
     }
   } else if (warp == S::kFoldWarps + 1) {
-    // ---------------- token tiles ----------------
+    // ---------------- token tiles, raw blocks whose rows are whole 16 bytes ----------------
     if (lane == 0) {
       tma_prefetch_desc(&tmap);
-      uint32_t st = 0, ph = 1, issued = 0;
+      constexpr bool RAW = TYPE != T_IQ2_XXS;
+      constexpr uint32_t kBlockBytes = BM * BB;
+      // Raw blocks run kSlots units ahead, over the ends of the CTA's items.
+      Cur ahead(p);
+      Item c;
+      c.b0 = c.b1 = 0;
+      uint32_t fill = 0, copied = 0;
+      auto copy_next = [&]() {
+        if (c.b0 >= c.b1) {
+          if (!ahead.get(p, sm, c)) return;
+          ahead.next(p);
+        }
+        const int blocks = min(kUnit, c.b1 - c.b0), row = c.rt * ((p.epi & 1) ? 64 : BM);
+        mbar_arrive_expect_tx(&sm.raw[fill], blocks * kBlockBytes);
+        for (int k = 0; k < blocks; ++k) tma_load_4d(sm.ring[fill] + k * kBlockBytes, &wmap, &sm.raw[fill], (c.b0 + k) * BB, 0, row, c.group);
+        c.b0 += kUnit;
+        ++copied;
+        fill = fill + 1 == S::kSlots ? 0 : fill + 1;
+      };
+      if constexpr (RAW)
+        for (int k = 0; k < S::kSlots; ++k) copy_next();
+      uint32_t unit = 0;
       Item w;
       bool ok = true;
-      for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x)
-        for (int x = w.b0 * Fmt<TYPE>::cols; ok && x < w.b1 * Fmt<TYPE>::cols;) {
-#pragma unroll
-          for (int s = 0; s < ST; ++s, ++issued) {
-            if (!mbar_wait(&sm.empty[st], ph, &sm.abort_flag, p.status, 35)) {
-              ok = false;
-              break;
-            }
-            mbar_arrive_expect_tx(&sm.full[st], (s < 2 ? 2 : 1) * NT * 128);
-            tma_load_2d(sm.b[st], &tmap, &sm.full[st], x, w.row0 * TERMS);
-            x += 64;
-            if (s < 2) {
-              tma_load_2d(sm.b[st] + NT * 128, &tmap, &sm.full[st], x, w.row0 * TERMS);
-              x += 64;
-            }
-            if (++st == kStages) {
-              st = 0;
-              ph ^= 1u;
-            }
-          }
-        }
-      if (sm.abort_flag) {
-        // gave up: copies in flight land before the CTA exits
-        for (uint32_t j = issued > (uint32_t)kStages ? issued - kStages : 0; j < issued; ++j)
-          for (uint32_t n = 0; n < kDrainPolls; ++n)
-            if (mbar_try_wait(&sm.full[j % kStages], (j / kStages) & 1)) break;
-      }
-    }
-  } else {
-    // ---------------- decode ----------------
-    constexpr int RW = S::kRows, SB = 16 / RW;            // rows of a warp; slabs of a stage that it decodes side by side
-    constexpr int kRowChunks = D::kData / D::kCopy, kChunks = RW * kRowChunks;      // copies of a block of a row, of the warp's rows
-    constexpr int kCopies = (kChunks + 31) / 32;
-    const int dw = warp - S::kFoldWarps - 2, r = lane % RW, lr = dw * RW + r, h = (lane / RW) & 1, sb = lane / (2 * RW);
-    const uint32_t ring = smem_u32(sm.ring[0]) + dw * RW * D::kPitch;
-    // The copy cursor runs kSlots - 1 blocks ahead of the decoding, over the ends of the CTA's items.
-    int ci = blockIdx.x, cb = 0, cb1 = 0;
-    uint32_t slot_fill = 0;
-    bool more = true;
-    const uint8_t* base = nullptr;
-    uint32_t off[kCopies];
-    auto copy_next = [&]() {
-      if (more && cb == cb1) {
-        Item c;
-        more = item_at<NT, TERMS>(p, sm.prefix, row_tiles, ci, c);
-        ci += gridDim.x;
-        if (more) {
-          base = group_base(p, c);
-          cb = c.b0;
-          cb1 = c.b1;
-#pragma unroll
-          for (int k = 0; k < kCopies; ++k) {
-            const int n = min(lane + 32 * k, kChunks - 1), j = n / kRowChunks;
-            off[k] = tile_row(p, c, dw * RW + j) + (n - j * kRowChunks) * D::kCopy;
-          }
-        }
-      }
-      if (more) {
-#pragma unroll
-        for (int k = 0; k < kCopies; ++k) {
-          uint32_t o = off[k] + (uint32_t)cb * BB;
-          if constexpr (D::kCopy == 4) o &= ~3u;
-          const int n = lane + 32 * k, j = n / kRowChunks;
-          const uint32_t dst = ring + slot_fill * (BM * D::kPitch) + (D::kData == D::kPitch ? n * D::kCopy : j * D::kPitch + (n - j * kRowChunks) * D::kCopy);
-          if ((k + 1) * 32 <= kChunks || n < kChunks) {
-            if constexpr (D::kCopy == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(base + o) : "memory");
-            else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(base + o) : "memory");
-          }
-        }
-        ++cb;
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      slot_fill = slot_fill + 1 == S::kSlots ? 0 : slot_fill + 1;
-    };
-#pragma unroll
-    for (int k = 0; k + 1 < S::kSlots; ++k) copy_next();
-    const uint32_t grid = smem_u32(sm.grid);
-    uint32_t st = 0, ph = 1, slot = 0;
-    Item w;
-    bool ok = true;
-    for (int i = blockIdx.x; ok && item_at<NT, TERMS>(p, sm.prefix, row_tiles, i, w); i += gridDim.x) {
-      const uint32_t own = tile_row(p, w, lr);
-      for (int b = w.b0; ok && b < w.b1; ++b) {
-        __syncwarp();       // the slot that is filled now has been read by all lanes
-        copy_next();
-        asm volatile("cp.async.wait_group %0;" ::"n"(S::kSlots - 1) : "memory");
-        __syncwarp();       // every lane's copies of this block are there
-        const uint32_t src = ring + slot * (BM * D::kPitch) + r * D::kPitch;
-        slot = slot + 1 == S::kSlots ? 0 : slot + 1;
-        const int mis = D::kCopy == 4 ? (int)((own + (uint32_t)b * BB) & 2u) : 0;
-#pragma unroll 1      // code that fits the instruction caches
-        for (int s = 0; s < ST; ++s) {
-          if (!mbar_wait_uniform(&sm.empty[st], ph, &sm.abort_flag, p.status, 36)) {
+      for (Cur cur(p); ok && cur.get(p, sm, w); cur.next(p))
+        for (int b = w.b0; b < w.b1; b += kUnit, ++unit) {
+          const uint32_t buf = unit & 1;
+          if (!mbar_wait(&sm.done[buf], ((unit >> 1) & 1) ^ 1, &sm.abort_flag, p.status, 35)) {
             ok = false;
             break;
           }
-          const uint32_t dst = smem_u32(sm.a[st]) + lr * 128;
-          if (s < 2) {       // two slabs of 64
-#pragma unroll 1
-            for (int e = 0; e < 2; e += SB) {
-              const int slab = SB == 2 ? sb : e;
-              D::stage(src, mis, dst + slab * (BM * 128), lr & 7, h, 2 * s + slab, grid);
-            }
-          } else if (sb == 0) {
-            D::stage(src, mis, dst, lr & 7, h, 4, grid);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.full[st]);
-          if (++st == kStages) {
-            st = 0;
-            ph ^= 1u;
-          }
+          const int pieces = kUnit == 1 ? 4 : min(4, (w.b1 - b) * kPieces), x = b * Fmt<TYPE>::cols;
+          mbar_arrive_expect_tx(&sm.full[buf], (pieces + (MINS ? 1 : 0)) * NT * 128);
+          for (int j = 0; j < pieces; ++j) tma_load_2d(sm.b[buf][j], &tmap, &sm.full[buf], x + 64 * j, w.row0 * TERMS);
+          if constexpr (MINS) tma_load_2d(sm.bm[buf], &tmap, &sm.full[buf], x + 256, w.row0 * TERMS);
+          if (RAW && unit >= 2) copy_next();      // into the slot of the unit that has been multiplied
         }
+      if (sm.abort_flag) {
+        // gave up: copies in flight land before the CTA exits
+        for (uint32_t u = unit > 2 ? unit - 2 : 0; u < unit; ++u)
+          for (uint32_t n = 0; n < kDrainPolls; ++n)
+            if (mbar_try_wait(&sm.full[u & 1], (u >> 1) & 1)) break;
+        if constexpr (RAW)
+          for (uint32_t u = copied > S::kSlots ? copied - S::kSlots : 0; u < copied; ++u)
+            for (uint32_t n = 0; n < kDrainPolls; ++n)
+              if (mbar_try_wait(&sm.raw[u % S::kSlots], (u / S::kSlots) & 1)) break;
       }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp < S::kFoldWarps + 4) {
+    // ---------------- raw blocks of 66 bytes: two warps, 64 rows each ----------------
+    // Five 16-byte pieces of memory hold a block, wherever it begins (those at its ends hold bytes of its neighbours). Bulk copies of 80
+    // bytes take 35 cycles each, several times the decode; as two warps' work `cp.async` costs the decode warps nothing.
+    if constexpr (TYPE == T_IQ2_XXS) {
+      constexpr int kCopies = 10;
+      const int r0 = (warp - S::kFoldWarps - 2) * 64;
+      uint32_t to[kCopies], off[kCopies];
+#pragma unroll
+      for (int k = 0; k < kCopies; ++k) {
+        const int n = lane + 32 * k, r = r0 + n / 5;
+        to[k] = smem_u32(sm.ring[0]) + ((r & ~31) + D::place(r & 31)) * D::kPitch + n % 5 * 16;
+        keep(to[k]);
+      }
+      const uint8_t* pos = p.W;
+      int left = 0;      // blocks of the cursor's item
+      uint32_t fill = 0, turn = 0;
+      Item c;
+      Cur ahead(p);
+      while (true) {
+        if (left == 0) {
+          if (!ahead.get(p, sm, c)) break;
+          ahead.next(p);
+          left = c.b1 - c.b0;
+          pos = group_base(p, c) + c.b0 * BB;
+#pragma unroll
+          for (int k = 0; k < kCopies; ++k) off[k] = tile_row(p, c, r0 + (lane + 32 * k) / 5) + (lane + 32 * k) % 5 * 16;
+        }
+        if (!mbar_wait_uniform(&sm.freed[fill], turn ^ 1, &sm.abort_flag, p.status, 38)) break;
+        const uint32_t at = fill * (BM * D::kPitch);
+#pragma unroll
+        for (int k = 0; k < kCopies; ++k)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to[k] + at), "l"((uintptr_t)(pos + off[k]) & ~(uintptr_t)15) : "memory");
+        copies_arrive(&sm.raw[fill]);
+        --left;
+        pos += BB;
+        if (++fill == S::kSlots) {
+          fill = 0;
+          turn ^= 1u;
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+  } else {
+    // ---------------- decode ----------------
+    // A lane has a row of its warp's quarter, the only rows whose tensor memory the warp can write, and piece j of every unit.
+    const int q = warp & 3, j = (warp - S::kFoldWarps - 4) >> 2, lr = q * 32 + lane;
+    uint32_t tab = smem_u32(sm.tab) + lane * 4, ta0 = tmem_base + kACol + ((uint32_t)(q * 32) << 16) + j * 32;
+    const uint32_t row = smem_u32(sm.ring[0]) + (q * 32 + D::place(lane)) * (TYPE == T_E4M3 ? 128 : D::kPitch);
+    uint32_t unit = 0, slot = 0, turn = 0;
+    keep(tab);
+    keep(ta0);
+    Item w;
+    bool ok = true;
+    for (Cur cur(p); ok && cur.get(p, sm, w); cur.next(p)) {
+      uint32_t at = (uint32_t)(uintptr_t)group_base(p, w) + tile_row(p, w, lr) + w.b0 * BB;      // address of the unit, its last bits
+      for (int b = w.b0; b < w.b1; b += kUnit, ++unit, at += kUnit * BB) {
+        if (!mbar_wait_uniform(&sm.raw[slot], turn, &sm.abort_flag, p.status, 37)) {
+          ok = false;
+          break;
+        }
+        const uint32_t src = row + slot * (BM * D::kPitch), a16 = at & 15u, buf = unit & 1, ta = ta0 + buf * 128;
+        if (++slot == S::kSlots) {
+          slot = 0;
+          turn ^= 1u;
+        }
+        uint32_t raw[D::kRegs], x[16];
+        D::load(src, a16, j, tab, raw);
+        if (!mbar_wait_uniform(&sm.done[buf], ((unit >> 1) & 1) ^ 1, &sm.abort_flag, p.status, 36)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        // four units of factors: the fold has read those of the unit four back when the one two back has been multiplied
+        if constexpr (TYPE != T_E4M3)
+          if (j == 0) D::factors(src, a16, &sm.factor[unit & 3][0][lr]);
+        D::half_piece(raw, 0, x);
+        tmem_st_32x16(ta, x);
+        D::half_piece(raw, 1, x);
+        tmem_st_32x16(ta + 16, x);
+        if constexpr (MINS)
+          if (j == 3) {
+            uint32_t m[8];
+            D::minima(src, m);
+            tmem_st_32x8(tmem_base + kACodes + buf * 8 + ((uint32_t)(q * 32) << 16), m);
+          }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.full[buf]);
+      }
+    }
   }
 
   tc_fence_before();
@@ -854,14 +953,24 @@ template <int TYPE, int NT, int TERMS>
 int launch(const void* staged, int total_rows, const Params& p, int sms, cudaStream_t stream) {
   EncodeTiledFn encode = encode_fn();
   if (encode == nullptr) return PK_ERR_UNSUPPORTED;
-  CUtensorMap map;
+  CUtensorMap map, wmap{};
   const cuuint64_t pitch = (cuuint64_t)p.nblk * Fmt<TYPE>::cols;
   const cuuint64_t gdim[2] = {pitch, (cuuint64_t)total_rows * TERMS}, gstride[1] = {pitch * 2};
-  const cuuint32_t box[2] = {64, NT}, estr[2] = {1, 1};
+  const cuuint32_t box[2] = {64, NT}, estr[4] = {1, 1, 1, 1};
   if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(staged), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return PK_ERR_CUDA;
-  const size_t smem = sizeof(Smem<Shape<TYPE, NT>, Dec<TYPE>::kPitch>) + 1024;
+  if constexpr (TYPE != T_IQ2_XXS) {
+    // bytes of a row, gate and up of a pair (or one), rows, groups; every stride is a multiple of a block's bytes, which are whole 16
+    const cuuint64_t two = (p.epi & 1) ? 2 : 1, rows = p.rows / two, rb = (cuuint64_t)p.rb;
+    const cuuint64_t wdim[4] = {rb, two, rows, (cuuint64_t)p.n_groups}, wstride[3] = {rows * rb, rb, rb * p.rows};
+    const cuuint32_t wbox[4] = {(cuuint32_t)Fmt<TYPE>::bytes, (cuuint32_t)two, (cuuint32_t)(BM / two), 1};
+    if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<uint8_t*>(p.W), wdim, wstride, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               TYPE == T_E4M3 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return PK_ERR_CUDA;
+  }
+  constexpr size_t smem = sizeof(Smem<TYPE, NT, Dec<TYPE>::kPitch>) + Dec<TYPE>::kAlign;
+  static_assert(smem <= 227 * 1024, "shared memory");
   static PkDeviceOnce once;
   if (PkDeviceOnceGuard once_guard{once}; once_guard.needed()) {
     if (cudaFuncSetAttribute(quant_umma_kernel<TYPE, NT, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -870,7 +979,7 @@ int launch(const void* staged, int total_rows, const Params& p, int sms, cudaStr
     }
     once_guard.done();
   }
-  quant_umma_kernel<TYPE, NT, TERMS><<<sms * Shape<TYPE, NT>::kCtas, Shape<TYPE, NT>::kThreads, smem, stream>>>(map, p);
+  quant_umma_kernel<TYPE, NT, TERMS><<<sms, Shape<TYPE, NT>::kThreads, smem, stream>>>(map, wmap, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -945,9 +1054,10 @@ PK_API int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, 
   const int nblk = K / type_k(type);
   const long long group_bytes = (long long)nblk * type_bytes(type) * N;      // IQ2 blocks are copied by four bytes
   if (group_bytes >= (1ll << 32) || (type == T_IQ2_XXS && (group_bytes & 3) != 0)) return PK_ERR_UNSUPPORTED;
-  const Params p{(const uint8_t*)W, (long long)nblk * type_bytes(type), nblk, N, n_groups, seg, rows, epi, limit, out, ldo, (const pk::bf16*)resid, row_scale, w_scale, w_ld,
-                 parts, splits, ws, counters, status};
   const int sms = sm_count > 0 ? sm_count : 148;
+  const int row_tiles = (epi & 1) ? (N / 2 + 63) / 64 : (N + BM - 1) / BM;
+  const Params p{(const uint8_t*)W, (long long)nblk * type_bytes(type), nblk, N, n_groups, seg, rows, epi, limit, out, ldo, (const pk::bf16*)resid, row_scale, w_scale, w_ld,
+                 parts, splits, ws, counters, status, row_tiles, sms % splits, sms / splits % row_tiles, sms / splits / row_tiles};
   if (type == T_IQ2_XXS) return launch_shape<T_IQ2_XXS>(columns, terms, staged, rows, p, sms, stream);
   if (type == T_Q4_K) return launch_shape<T_Q4_K>(columns, terms, staged, rows, p, sms, stream);
   if (type == T_Q5_K) return launch_shape<T_Q5_K>(columns, terms, staged, rows, p, sms, stream);

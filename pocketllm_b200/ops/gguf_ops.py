@@ -158,7 +158,7 @@ def _umma_splits(tiles: int, K: int, slots: int) -> int:
 
 
 def _umma_slots(type_name: str, columns: int) -> int:
-    return _sm_count() * (2 if type_name == "iq2_xxs" and columns < 64 else 1)      # resident CTAs of the kernel
+    return _sm_count()      # resident CTAs of the kernel
 
 
 def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, gamma, eps: float, epi: int,

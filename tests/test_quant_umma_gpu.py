@@ -315,3 +315,28 @@ def test_rmsnorm_by_width(M, K, mode):
     assert _rel(ops.rmsnorm(x, gamma, mode=mode), norm(x)) < 2 ** -8
     out = ops.rmsnorm(x, gamma, mode=mode, parts=y, hidden_out=h)
     assert torch.equal(h, (x + y[0]).to(torch.bfloat16)) and _rel(out, norm(h)) < 2 ** -8
+
+
+@pytest.mark.parametrize("name,N,K,rows,E", [("iq2_xxs", 130, 256, 40, 7), ("iq2_xxs", 2, 768, 25, 5), ("q4_k", 130, 512, 40, 7), ("iq2_xxs", 6, 256, 16500, 1), ("q5_k", 4, 256, 16500, 3)])
+@pytest.mark.parametrize("columns", [16, 64])
+def test_groups_at_any_place(name, N, K, rows, E, columns):
+    """Groups that begin on any four bytes, and more token tiles than are looked up."""
+    from ctypes import c_float, c_int, c_void_p
+    from pocketllm_b200 import ops
+    from pocketllm_b200.ops import gguf_ops as go
+    raw, w = _raw(name, E * N, K, rows)
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, K, generator=g).to(torch.bfloat16).cuda()
+    cut = torch.sort(torch.randint(0, rows + 1, (E - 1,), generator=g)).values
+    seg = torch.cat([torch.zeros(1, dtype=torch.long), cut, torch.tensor([rows])])
+    st = go._Staged(x, name, rows, 1)
+    for epi in (2, 3):
+        y = torch.full((rows, N if epi == 2 else N // 2), float("nan"), device="cuda")
+        go._umma(st, raw, name, N, K, seg.int().cuda(), E, epi, y, 0.0, columns, 1, 1, None)
+        for e in range(E):
+            a, b = int(seg[e]), int(seg[e + 1])
+            want = x[a:b].double() @ w[e * N:(e + 1) * N].T
+            if epi == 3:
+                u, v = want.chunk(2, -1)
+                want = torch.nn.functional.silu(u) * v
+            assert a == b or _rel(y[a:b], want) < TOL * (1 if epi == 2 else 4)      # the exponential of a SiLU and its product
