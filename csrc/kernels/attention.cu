@@ -111,32 +111,46 @@ struct DecodeParams {
   const float* vscale;
 };
 
-// Eight consecutive channels of one cached row as floats. bf16: one 16-byte load; fp8: one 8-byte load and the scale of
-// the 64-channel group the lane's channels belong to.
-__device__ __forceinline__ void load_kv8(const void* base, const float* scale, size_t row, int l16, bool fp8, float (&f)[8]) {
+// Eight consecutive channels of one cached row as they lie in memory (bf16: one 16-byte load; fp8: one 8-byte load and the scale of the
+// 64-channel group the lane's channels belong to), and as floats.
+struct Kv8 {
+  uint4 w;
+  float scale;
+};
+__device__ __forceinline__ Kv8 load_kv8(const void* base, const float* scale, size_t row, int l16, bool fp8) {
+  Kv8 r;
   if (!fp8) {
-    const uint4 r = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(base) + row * kD + l16 * 8);
-    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+    r.w = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(base) + row * kD + l16 * 8);
+    r.scale = 0.f;
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(base) + row * kD + l16 * 8);
+    r.w = make_uint4(v.x, v.y, 0u, 0u);
+    r.scale = scale[row * 2 + (l16 >> 3)];
+  }
+  return r;
+}
+__device__ __forceinline__ void unpack_kv8(const Kv8& r, bool fp8, float (&f)[8]) {
+  const uint32_t w[4] = {r.w.x, r.w.y, r.w.z, r.w.w};
+  if (!fp8) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       f[2 * j] = __uint_as_float(w[j] << 16);
       f[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
     }
   } else {
-    const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(base) + row * kD + l16 * 8);
-    const float sc = scale[row * 2 + (l16 >> 3)];
-    const uint32_t w[2] = {r.x, r.y};
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const float2 a = e4m3x2_to_float2((uint16_t)(w[j] & 0xffffu)), b = e4m3x2_to_float2((uint16_t)(w[j] >> 16));
-      f[4 * j] = a.x * sc;
-      f[4 * j + 1] = a.y * sc;
-      f[4 * j + 2] = b.x * sc;
-      f[4 * j + 3] = b.y * sc;
+      f[4 * j] = a.x * r.scale;
+      f[4 * j + 1] = a.y * r.scale;
+      f[4 * j + 2] = b.x * r.scale;
+      f[4 * j + 3] = b.y * r.scale;
     }
   }
 }
 
+// A split has few keys per warp, and its time was that of one load after the other: the keys and values of the two next steps are on
+// their way while one is worked on. One row, 48 heads of 8 key heads, 210 keys in 8 splits: 11.5 -> 7.9 us.
 template <int G>
 __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParams p) {
   pk::pdl_wait();
@@ -172,15 +186,30 @@ __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParam
 
   const size_t head_row0 = (size_t)hk * p.ctx_cap;
   const bool fp8 = p.kv_fp8 != 0;
+  constexpr int kAhead = 2;
+  Kv8 kr[kAhead + 1], vr[kAhead + 1];
+  auto in_range = [&](int t) { return t < end && (p.window == 0 || t >= win_lo || t < p.sink); };
+  auto fetch = [&](int t, Kv8& k, Kv8& v) {
+    k.w = v.w = make_uint4(0u, 0u, 0u, 0u);
+    k.scale = v.scale = 0.f;
+    if (in_range(t)) {
+      k = load_kv8(p.kcache, p.kscale, head_row0 + t, l16, fp8);
+      v = load_kv8(p.vcache, p.vscale, head_row0 + t, l16, fp8);
+    }
+  };
+#pragma unroll
+  for (int a = 0; a < kAhead; ++a) fetch(start + warp * 2 + khalf + 8 * a, kr[a], vr[a]);
   for (int t0 = start + warp * 2; t0 < end; t0 += 8) {
     const int t = t0 + khalf;
-    const bool valid = t < end && (p.window == 0 || t >= win_lo || t < p.sink);
+    const bool valid = in_range(t);
+    fetch(t + 8 * kAhead, kr[kAhead], vr[kAhead]);
     float kf[8], vf[8];
+    unpack_kv8(kr[0], fp8, kf);
+    unpack_kv8(vr[0], fp8, vf);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) kf[j] = vf[j] = 0.f;
-    if (valid) {
-      load_kv8(p.kcache, p.kscale, head_row0 + t, l16, fp8, kf);
-      load_kv8(p.vcache, p.vscale, head_row0 + t, l16, fp8, vf);
+    for (int a = 0; a < kAhead; ++a) {
+      kr[a] = kr[a + 1];
+      vr[a] = vr[a + 1];
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -256,25 +285,41 @@ struct MergeParams {
   bf16* out;         // [M, Hq*D]
 };
 
+// Eight splits at a time, all their loads on the way together: one after the other they were the kernel's time. One row of 48 heads in 8
+// splits 11.7 -> 7.4 us.
 __global__ void __launch_bounds__(kD) gqa_merge_kernel(const MergeParams p) {
   pk::pdl_wait();
   pk::pdl_trigger();
   const int m = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const float* w = p.ws + ((size_t)m * p.Hq + h) * p.nsplit * (kD + 2);
-  float nm = -INFINITY;
-  for (int s = 0; s < p.nsplit; ++s) nm = fmaxf(nm, w[s * (kD + 2) + kD]);
-  float l = 0.f, a = 0.f;
-  for (int s = 0; s < p.nsplit; ++s) {
-    const float ms = w[s * (kD + 2) + kD];
-    const float c = ms == -INFINITY ? 0.f : __expf(ms - nm);
-    l += w[s * (kD + 2) + kD + 1] * c;
-    a += w[s * (kD + 2) + d] * c;
+  const float gate = p.proj != nullptr ? __bfloat162float(p.proj[(size_t)m * p.ld + h * 2 * kD + kD + d]) : 0.f;
+  float mx = -INFINITY, l = 0.f, a = 0.f;
+  for (int s0 = 0; s0 < p.nsplit; s0 += 8) {
+    float ms[8], ls[8], as[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const bool in = s0 + s < p.nsplit;
+      const float* ws = w + (size_t)(in ? s0 + s : 0) * (kD + 2);
+      ms[s] = in ? ws[kD] : -INFINITY;
+      ls[s] = in ? ws[kD + 1] : 0.f;
+      as[s] = in ? ws[d] : 0.f;
+    }
+    float nm = mx;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) nm = fmaxf(nm, ms[s]);
+    const float c0 = mx == -INFINITY ? 0.f : __expf(mx - nm);
+    l *= c0;
+    a *= c0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const float c = ms[s] == -INFINITY ? 0.f : __expf(ms[s] - nm);
+      l += ls[s] * c;
+      a += as[s] * c;
+    }
+    mx = nm;
   }
   float o = l > 0.f ? a / l : 0.f;
-  if (p.proj != nullptr) {
-    const float gate = __bfloat162float(p.proj[(size_t)m * p.ld + h * 2 * kD + kD + d]);
-    o *= sigmoidf_(gate);
-  }
+  if (p.proj != nullptr) o *= sigmoidf_(gate);
   p.out[((size_t)m * p.Hq + h) * kD + d] = __float2bfloat16(o);
 }
 
