@@ -958,15 +958,15 @@ void QwenEngine::quant_product(const Fp8Linear& w, int M, int epi, void* out, in
   }
   const int columns = M <= 32 ? 32 : 64;
   const int tiles = epi == 1 ? (w.N / 2 + 63) / 64 : (w.N + 127) / 128;
-  // More than 16 rows. Parts of K: the fewest with which the last round of CTAs is about as full as it gets, four 128-wide blocks in a part at least.
-  // 40 tiles of a 5120-row projection leave most SMs idle without.
+  // More than 16 rows. Parts of K: rounds of CTAs, each with its blocks and, with parts, the exchange of a part (in blocks of 256 weights),
+  // four 128-wide blocks in a part at least. 5120 x 17408 (40 tiles), 24 rows, us: 2 / 3 / 4 / 6 / 11 parts 45 / 39 / 57 / 53 / 76; 34816 x 5120:
+  // 1 / 2 / 4 parts 54 / 72 / 105.
   int splits = 1;
-  double best = 0;
-  for (int s = 1; s <= w.K / 512 && tiles * s <= kQuantItems; ++s) {
-    const int items = tiles * s;
-    const double full = (double)items / ((items + sm_count_ - 1) / sm_count_ * sm_count_) - 0.01 * s;
-    if (full > best) {
-      best = full;
+  double best = 1e30;
+  for (int s = 1; s == 1 || (s <= w.K / 512 && tiles * s <= std::min(kQuantItems, 4 * sm_count_)); ++s) {
+    const double cost = ((tiles * s + sm_count_ - 1) / sm_count_) * (w.K / 256.0 / s + (s > 1 ? 3 + s * columns / 32.0 : 0.0));
+    if (cost < best) {
+      best = cost;
       splits = s;
     }
   }

@@ -102,7 +102,7 @@ struct __align__(1024) Smem {
   uint64_t drained;
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
-  uint32_t last;
+  uint32_t last[4];
   int prefix[kMaxGroups + 1];     // token tiles before each group
   int2 tiles[kMaxTiles];          // `Cursor::place`
 };
@@ -370,17 +370,24 @@ template <> struct Dec<T_E4M3> {
   }
 };
 
-// By one thread, behind the CTA's stores of its part: *last says whether the other parts are there.
-__device__ __forceinline__ void count_part(const Params& p, const Item& w, uint32_t* last) {
-  const uint32_t n = atomicAdd(p.counters + w.tile, 1u);
-  *last = n == (uint32_t)p.splits - 1u;
-  if (*last) p.counters[w.tile] = 0u;
-  __threadfence();
-}
-
+// By the fold warps of a quarter of the rows, behind their stores of a part: whether the other parts of these rows are there. A byte
+// of the tile's counter per quarter, so that quarters do not wait for one another.
 template <int WARPS>
-__device__ __forceinline__ void fold_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
+__device__ __forceinline__ bool count_part(const Params& p, const Item& w, uint32_t* last) {
+  const int q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  auto sync = [&]() {
+    if constexpr (WARPS == 8) asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+    else __syncwarp();
+  };
+  sync();
+  if (threadIdx.x < 128 && lane == 0) {
+    uint32_t n;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(n) : "l"(p.counters + w.tile), "r"(1u << (8 * q)) : "memory");
+    last[q] = ((n >> (8 * q)) & 255u) == (uint32_t)p.splits - 1u;
+    if (last[q]) atomicSub(p.counters + w.tile, (uint32_t)p.splits << (8 * q));
+  }
+  sync();
+  return *(volatile uint32_t*)&last[q];
 }
 
 // The rest of a fold warp's items, from `cur` on, after a wait that ran out: NaN in their places, so that the result cannot be taken
@@ -394,13 +401,7 @@ __device__ __noinline__ void give_up(const Params& p, Sm& sm, Cursor<NT, TERMS> 
     if (p.splits > 1) {
       float* part = p.ws + ((size_t)w.tile * p.splits + w.split) * NT * BM + lr;
       for (int c = c0; c < c0 + cols; ++c) __stcg(part + (size_t)c * BM, nan);
-      __threadfence();
-      fold_sync<WARPS>();
-      if (tid == 0) count_part(p, w, &sm.last);
-      fold_sync<WARPS>();
-      const uint32_t last = *(volatile uint32_t*)&sm.last;
-      fold_sync<WARPS>();
-      if (!last) continue;
+      if (!count_part<WARPS>(p, w, sm.last)) continue;
     }
     const bool glu = p.epi & 1;
     const int n = glu ? w.rt * 64 + (lr >> 1) : w.rt * BM + lr;
@@ -577,14 +578,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
         float* part = p.ws + ((size_t)w.tile * p.splits + w.split) * NT * BM + lr;
 #pragma unroll
         for (int c = 0; c < S::kFoldCols; ++c) __stcg(part + (size_t)(c0 + c) * BM, acc[c]);
-        __threadfence();
-        fold_sync<S::kFoldWarps>();
-        if (tid == 0) count_part(p, w, &sm.last);
-        fold_sync<S::kFoldWarps>();
-        const uint32_t last = sm.last;
-        fold_sync<S::kFoldWarps>();
-        if (!last) continue;
-        __threadfence();
+        if (!count_part<S::kFoldWarps>(p, w, sm.last)) continue;
         const float* all = p.ws + (size_t)w.tile * p.splits * NT * BM + lr;
 #pragma unroll
         for (int c = 0; c < S::kFoldCols; ++c) acc[c] = 0.f;
@@ -1054,6 +1048,7 @@ PK_API int pk_quant_rows(const void* W, int type, int N, int K, const int* seg, 
   const int nblk = K / type_k(type);
   const long long group_bytes = (long long)nblk * type_bytes(type) * N;      // IQ2 blocks are copied by four bytes
   if (group_bytes >= (1ll << 32) || (type == T_IQ2_XXS && (group_bytes & 3) != 0)) return PK_ERR_UNSUPPORTED;
+  if (splits > 255) parts = splits = 255;      // a byte counts them
   const int sms = sm_count > 0 ? sm_count : 148;
   const int row_tiles = (epi & 1) ? (N / 2 + 63) / 64 : (N + BM - 1) / BM;
   const Params p{(const uint8_t*)W, (long long)nblk * type_bytes(type), nblk, N, n_groups, seg, rows, epi, limit, out, ldo, (const pk::bf16*)resid, row_scale, w_scale, w_ld,

@@ -141,20 +141,19 @@ def _umma(st: _Staged, w_raw: torch.Tensor, type_name: str, N: int, K: int, seg,
                                        c_int(_sm_count()), _stream()), "pk_quant_rows")
 
 
-def _fill(items: int, slots: int) -> float:
-    """How full the rounds of `slots` CTAs are with that many items."""
-    return items / (-(-items // slots) * slots)
+def _umma_cost(tiles: int, K: int, parts: int, slots: int, columns: int) -> float:
+    """What `tiles` tiles with K in `parts` take on `slots` CTAs, in blocks of 256 weights: rounds of CTAs, each with its blocks and, with
+    parts, the exchange of a part: its 128 x `columns` sums and the counter, then all parts by the last CTA. 128-row tiles, us by parts:
+    IQ2_XXS, 192 tiles of K = 3072 22.5 / 26.6 / 29.4 (1 / 2 / 3), 24 tiles 20.5 / 18.4 / 16.4 / 16.4 (1 / 2 / 4 / 6); Q5_K, 24 tiles of K =
+    6144, 16 columns 32.7 / 23.4 / 19.2 / 17.2 / 22.6 (1 / 2 / 4 / 6 / 8), 64 columns 36.9 / 27.6 / 24.6 / 25.4 / 36.8; 64 tiles of K = 3072
+    22.5 / 18.5 / 22.5 (1 / 2 / 3); Q4_K, 256 tiles 28.7 / 38.9 / 43.0."""
+    return -(-tiles * parts // slots) * (K / 256 / parts + (3 + parts * columns / 32 if parts > 1 and columns else 0))
 
 
-def _umma_splits(tiles: int, K: int, slots: int) -> int:
-    """Parts of K for `tiles` tiles on `slots` CTAs: the fewest with which the last round of CTAs is about as full as it gets, two
-    256-weight blocks in a part at least."""
-    best, most = 1, 0.0
-    for s in range(1, min(K // 512, 4 * slots // tiles) + 1):
-        full = _fill(tiles * s, slots) - 0.01 * s
-        if full > most:
-            best, most = s, full
-    return best
+def _umma_splits(tiles: int, K: int, slots: int, columns: int = 0) -> int:
+    """Parts of K for `tiles` tiles of `columns` columns on `slots` CTAs (columns 0: as if the exchange cost nothing), two 256-weight blocks in
+    a part at least."""
+    return min(range(1, max(1, min(K // 512, 4 * slots // tiles)) + 1), key=lambda s: _umma_cost(tiles, K, s, slots, columns))
 
 
 def _umma_slots(type_name: str, columns: int) -> int:
@@ -167,8 +166,7 @@ def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, g
     columns = 16 if M <= 16 else 32 if M <= 32 else 64
     tiles = (-(-(N // 2) // 64) if epi == 1 else -(-N // 128)) * -(-M // columns)
     slots = _umma_slots(type_name, columns)
-    # several column tiles that fill the SMs once: parts of 64 columns cost more than the last round saves (192 rows of 8192 x 3072: 59 against 51 us)
-    splits = 1 if M > 64 and tiles >= slots else _umma_splits(tiles, K, slots)
+    splits = _umma_splits(tiles, K, slots, columns)
     st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
     y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
     _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits, splits, status)
@@ -194,11 +192,11 @@ def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, 
         if c == 16:
             # K is cut as for one token's routes whatever the step holds and however the experts are split over ranks: a token's sum does
             # not depend on the tokens beside it. CTAs of their own take the parts where that fills the SMs better.
-            parts = _umma_splits(routes.topk * row_tiles, K, slots)
-            if R <= UMMA_SPLIT_ROUTES and most * parts <= 4 * slots and _fill(most * parts, slots) > _fill(most, slots) + 0.02:
+            parts = _umma_splits(routes.topk * row_tiles, K, slots, c)
+            if R <= UMMA_SPLIT_ROUTES and most * parts <= 4 * slots and _umma_cost(most, K, parts, slots, c) < _umma_cost(most, K, 1, slots, c):
                 splits = parts
         elif R <= UMMA_SPLIT_ROUTES:       # beyond, the tiles fill the SMs
-            parts = splits = _umma_splits(most, K, slots)
+            parts = splits = _umma_splits(most, K, slots, c)
         tiles = (min(R, local) + R * t // c) * row_tiles if splits > 1 else 0
         st = _Staged(x, type_name, R, t, index=index, counters=tiles, ws_floats=tiles * splits * c * 128)
         _umma(st, w_raw, type_name, N, K, seg, local, epi, out, limit, c, parts, splits, status)
