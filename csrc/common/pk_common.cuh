@@ -158,6 +158,15 @@ __device__ __forceinline__ float e2m1_to_float(uint32_t nib) {
 // this one retire. Both are no-ops for a launch without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+// Waits, and ties the pointers to the wait: loads through `__ldg` or `const __restrict__` count as reads of what no one writes, and
+// could otherwise be moved before it.
+template <class P>
+__device__ __forceinline__ void pdl_after(P& p) { asm volatile("" : "+l"(p)); }
+template <class... P>
+__device__ __forceinline__ void pdl_wait_for(P&... p) {
+  pdl_wait();
+  (pdl_after(p), ...);
+}
 
 __device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }

@@ -346,6 +346,8 @@ struct FullQkParams {
 };
 
 __global__ void __launch_bounds__(256) full_qk_norm_rope_append_kernel(const FullQkParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   __shared__ float red[40];
   const int t = blockIdx.x, is_k = blockIdx.y, tid = threadIdx.x;
   const int H = is_k ? p.Hkv : p.Hq, n = H * kD;
@@ -385,6 +387,8 @@ __global__ void __launch_bounds__(256) full_qk_norm_rope_append_kernel(const Ful
 // rows on (8.6 against 9.2 us, 512 rows 9.6 against 13.3) the form above has enough blocks to hide its loads and fewer threads without an element.
 constexpr int kFullQkThreads = 512, kFullQkVecRows = 128;
 __global__ void __launch_bounds__(kFullQkThreads) full_qk_norm_rope_append_vec_kernel(const FullQkParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ __align__(16) float xs[];      // [heads * D]
   __shared__ float red[40];
   const int t = blockIdx.x, is_k = blockIdx.y, tid = threadIdx.x;
@@ -456,9 +460,9 @@ PK_API int pk_full_qk_norm_rope_append(const void* q, int ldq, const void* k, in
   const uintptr_t at = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)q_out | (uintptr_t)kcache | (uintptr_t)vcache;
   const size_t smem = (size_t)(Hq > Hkv ? Hq : Hkv) * kD * sizeof(float);
   if ((at & 15) == 0 && ((ldq | ldk | ldv) & 7) == 0 && (rope_dim & 15) == 0 && smem <= kPlainSmem && T <= kFullQkVecRows)
-    full_qk_norm_rope_append_vec_kernel<<<dim3(T, 2), kFullQkThreads, smem, stream>>>(p);
+    PK_LAUNCH_PDL(full_qk_norm_rope_append_vec_kernel, dim3(T, 2), dim3(kFullQkThreads), smem, stream, p);
   else
-    full_qk_norm_rope_append_kernel<<<dim3(T, 2), 256, 0, stream>>>(p);
+    PK_LAUNCH_PDL(full_qk_norm_rope_append_kernel, dim3(T, 2), dim3(256), 0, stream, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

@@ -475,6 +475,8 @@ __global__ void moe_reduce_routes_kernel(const float* __restrict__ ybuf, const i
 __global__ void moe_reduce_routes_weighted_kernel(const float* __restrict__ ybuf, const float* __restrict__ route_weight,
                                                   const int* __restrict__ route_pos, const int* __restrict__ seg_start, int topk, int H,
                                                   int expert_offset, int local_experts, float* y) {
+  pk::pdl_wait_for(ybuf, route_weight, route_pos, seg_start);
+  pk::pdl_trigger();
   const int t = blockIdx.y, n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= H) return;
   const int lo = seg_start[expert_offset], hi = seg_start[expert_offset + local_experts];
@@ -487,6 +489,8 @@ __global__ void moe_reduce_routes_weighted_kernel(const float* __restrict__ ybuf
 }
 
 __global__ void invert_routes_kernel(const int* __restrict__ route_src, int R, int* route_pos) {
+  pk::pdl_wait_for(route_src);
+  pk::pdl_trigger();
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos < R) route_pos[route_src[pos]] = pos;
 }
@@ -496,6 +500,8 @@ __global__ void invert_routes_kernel(const int* __restrict__ route_src, int R, i
 // once for the tile's tokens. A single token spreads over E / 8 blocks instead of streaming the whole router matrix
 // through one block.
 __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const float* rw, int H, int E, int T, float* logits) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ __align__(16) float xs[];  // [tokens of the tile][H]
   const int t0 = blockIdx.y * 8, nt = min(8, T - t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -553,6 +559,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
 // The sums are added in another order than above.
 constexpr int kRt = 16, kRe = 64, kRk = 32;
 __global__ void __launch_bounds__(512) router_logits_tile_kernel(const bf16* __restrict__ x, const float* __restrict__ rw, int H, int E, int T, float* logits) {
+  pk::pdl_wait_for(x);
+  pk::pdl_trigger();
   __shared__ __align__(16) float ws[4][kRe][kRk + 4];
   __shared__ __align__(16) float xs[4][kRt][kRk + 4];
   const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, tx = t & 15, ty = t >> 4;      // experts tx + 16 j, tokens 2 ty ..
@@ -614,6 +622,8 @@ __global__ void __launch_bounds__(512) router_logits_tile_kernel(const bf16* __r
 __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, const float* bias, int E,
                                                           int topk, int score_func, int norm_topk, float route_scale,
                                                           int* ids, float* weights) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ float sm[];  // [E] scores, [E] selection keys
   float* sc = sm;
   float* key = sc + E;
@@ -678,6 +688,8 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, c
 __global__ void __launch_bounds__(1024) group_routes_kernel(const int* ids, const float* weights, int T, int topk, int E,
                                                             int* seg_start, int* route_token, float* route_weight,
                                                             int* route_src) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ int cnt[];  // [warps][E]
   __shared__ int part[33];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5, R = T * topk;
@@ -745,6 +757,8 @@ __global__ void __launch_bounds__(1024) group_routes_kernel(const int* ids, cons
 // Quantised embedding: decode selected rows to bf16 (one warp per 256 weights).
 __global__ void __launch_bounds__(256) gguf_dequant_rows_kernel(const uint8_t* W, int type, const int* rows, int nrows,
                                                                 int K, int row_offset, int table_rows, bf16* out) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   // one warp per 256-weight block, walking (row, block) units with a grid stride; a lane's eight weights leave as one
   // 16-byte store
   const int lane = threadIdx.x & 31;
@@ -870,11 +884,11 @@ PK_API int pk_router_topk(const void* x, const float* router_w, const float* bia
   float* logits = router_scratch((size_t)T * E);
   if (logits == nullptr) return PK_ERR_CUDA;
   if (E >= kRe && (long long)T * E >= kRouterTileMin)
-    router_logits_tile_kernel<<<dim3((E + kRe - 1) / kRe, (T + kRt - 1) / kRt), 512, 0, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);
+    PK_LAUNCH_PDL(router_logits_tile_kernel, dim3((E + kRe - 1) / kRe, (T + kRt - 1) / kRt), dim3(512), 0, stream, (const pk::bf16*)x, router_w, H, E, T, logits);
   else
-    router_logits_kernel<<<dim3((E + 7) / 8, (T + 7) / 8), 256, smem_x, stream>>>((const pk::bf16*)x, router_w, H, E, T, logits);
+    PK_LAUNCH_PDL(router_logits_kernel, dim3((E + 7) / 8, (T + 7) / 8), dim3(256), smem_x, stream, (const pk::bf16*)x, router_w, H, E, T, logits);
   PK_CHECK_LAUNCH();
-  router_topk_kernel<<<T, 256, (size_t)2 * E * sizeof(float), stream>>>(logits, bias, E, topk, score_func, norm_topk, route_scale, ids,
+  PK_LAUNCH_PDL(router_topk_kernel, dim3(T), dim3(256), (size_t)2 * E * sizeof(float), stream, logits, bias, E, topk, score_func, norm_topk, route_scale, ids,
                                                                         weights);
   PK_CHECK_LAUNCH();
   return PK_OK;
@@ -898,7 +912,7 @@ PK_API int pk_group_routes(const int* ids, const float* weights, int T, int topk
       once_guard.done();
     }
   }
-  group_routes_kernel<<<1, warps * 32, smem, stream>>>(ids, weights, T, topk, E, seg_start, route_token, route_weight, route_src);
+  PK_LAUNCH_PDL(group_routes_kernel, dim3(1), dim3(warps * 32), smem, stream, ids, weights, T, topk, E, seg_start, route_token, route_weight, route_src);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -912,9 +926,9 @@ PK_API int pk_moe_reduce_routes(const float* ybuf, const float* route_weight, co
   if (ybuf == nullptr || route_weight == nullptr || route_src == nullptr || seg_start == nullptr || route_pos == nullptr || y == nullptr || T < 1 || topk < 1)
     return PK_ERR_BAD_ARG;
   const int R = T * topk;
-  invert_routes_kernel<<<(R + 255) / 256, 256, 0, stream>>>(route_src, R, route_pos);
+  PK_LAUNCH_PDL(invert_routes_kernel, dim3((R + 255) / 256), dim3(256), 0, stream, route_src, R, route_pos);
   PK_CHECK_LAUNCH();
-  moe_reduce_routes_weighted_kernel<<<dim3((H + 255) / 256, T), 256, 0, stream>>>(ybuf, route_weight, route_pos, seg_start, topk, H, expert_offset,
+  PK_LAUNCH_PDL(moe_reduce_routes_weighted_kernel, dim3((H + 255) / 256, T), dim3(256), 0, stream, ybuf, route_weight, route_pos, seg_start, topk, H, expert_offset,
                                                                                   local_experts, y);
   PK_CHECK_LAUNCH();
   return PK_OK;
@@ -923,7 +937,7 @@ PK_API int pk_moe_reduce_routes(const float* ybuf, const float* route_weight, co
 // route_pos[route_src[pos]] = pos: where route (t, k) sits in the expert-sorted order.
 PK_API int pk_invert_routes(const int* route_src, int R, int* route_pos, cudaStream_t stream) {
   if (route_src == nullptr || route_pos == nullptr || R < 1) return PK_ERR_BAD_ARG;
-  invert_routes_kernel<<<(R + 255) / 256, 256, 0, stream>>>(route_src, R, route_pos);
+  PK_LAUNCH_PDL(invert_routes_kernel, dim3((R + 255) / 256), dim3(256), 0, stream, route_src, R, route_pos);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -953,7 +967,7 @@ PK_API int pk_gguf_moe_forward_det(const void* W13, const void* W2, int type13, 
   const int rc = moe_forward_impl(W13, W2, type13, type2, E, H, I, x, seg_start, route_token, route_weight, hbuf, y, limit,
                                   expert_offset, local_experts, sm_count, ybuf, stream, R);
   if (rc != PK_OK) return rc;
-  invert_routes_kernel<<<(R + 255) / 256, 256, 0, stream>>>(route_src, R, route_pos);
+  PK_LAUNCH_PDL(invert_routes_kernel, dim3((R + 255) / 256), dim3(256), 0, stream, route_src, R, route_pos);
   PK_CHECK_LAUNCH();
   moe_reduce_routes_kernel<<<dim3((H + 255) / 256, T), 256, 0, stream>>>(ybuf, route_pos, seg_start, topk, H, expert_offset,
                                                                          local_experts, y);
@@ -1010,7 +1024,7 @@ PK_API int pk_gguf_dequant_rows(const void* W, int type, const int* rows, int nr
   const long long units = (long long)nrows * (K >> 8);
   const long long want = (units + 7) / 8;
   const int grid = (int)(want < 148LL * 32 ? want : 148LL * 32);
-  gguf_dequant_rows_kernel<<<grid, 256, 0, stream>>>((const uint8_t*)W, type, rows, nrows, K, row_offset, table_rows,
+  PK_LAUNCH_PDL(gguf_dequant_rows_kernel, dim3(grid), dim3(256), 0, stream, (const uint8_t*)W, type, rows, nrows, K, row_offset, table_rows,
                                                     (pk::bf16*)out);
   PK_CHECK_LAUNCH();
   return PK_OK;

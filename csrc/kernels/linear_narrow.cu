@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(32 * kWarps) linear_narrow_kernel(const Narrow
   float acc[kRows / 8][4] = {};
   const bf16* xa = p.x + (size_t)min(m0 + g, p.M - 1) * p.ldx + t * 8;
   const bf16* xb = p.x + (size_t)min(m0 + g + 8, p.M - 1) * p.ldx + t * 8;
+  pk::pdl_wait_for(xa, xb);
+  pk::pdl_trigger();
   const bf16* wr[kRows / 8];
 #pragma unroll
   for (int j = 0; j < kRows / 8; ++j) wr[j] = p.w + (size_t)min(n0 + j * 8 + g, p.N - 1) * p.K + t * 8;
@@ -78,7 +80,7 @@ PK_API int pk_linear_narrow(const void* x, int ldx, const void* w, int M, int N,
       ((uintptr_t)x & 15) != 0 || ((uintptr_t)w & 15) != 0 || (N + kRows - 1) / kRows > 65535)
     return PK_ERR_BAD_ARG;
   const NarrowParams p{(const pk::bf16*)x, ldx, (const pk::bf16*)w, M, N, K, (pk::bf16*)y, ldy};
-  linear_narrow_kernel<<<dim3((M + kTok - 1) / kTok, (N + kRows - 1) / kRows), 32 * kWarps, 0, stream>>>(p);
+  PK_LAUNCH_PDL(linear_narrow_kernel, dim3((M + kTok - 1) / kTok, (N + kRows - 1) / kRows), dim3(32 * kWarps), 0, stream, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

@@ -46,6 +46,8 @@ struct NormParams {
 };
 
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const NormParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ float row[];
   __shared__ float red[40];
   const int m = blockIdx.x;
@@ -77,6 +79,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const NormParams p) {
 // its loads of an iteration under way together. One row of 3072: 9.3 -> 3.3 us, 1500 rows 23 -> 13 us (the form above loads
 // two bytes, waits and goes on).
 __global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const NormParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ __align__(16) float row[];
   __shared__ float red[40];
   const size_t base = (size_t)blockIdx.x * p.K;
@@ -148,6 +152,8 @@ struct NormQuantParams {
 };
 
 __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const NormQuantParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ __align__(16) float row[];
   __shared__ float red[40];
   const int m = blockIdx.x, tid = threadIdx.x, nvec = p.K >> 3;
@@ -413,8 +419,8 @@ PK_API int pk_rmsnorm(const void* x, const float* parts, int nparts, int M, int 
       return PK_ERR_CUDA;
     }
   }
-  if (vec) PK_LAUNCH(rmsnorm_vec_kernel, dim3(M), dim3(256), smem, stream, p);
-  else PK_LAUNCH(rmsnorm_kernel, dim3(M), dim3(256), smem, stream, p);
+  if (vec) PK_LAUNCH_PDL(rmsnorm_vec_kernel, dim3(M), dim3(256), smem, stream, p);
+  else PK_LAUNCH_PDL(rmsnorm_kernel, dim3(M), dim3(256), smem, stream, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -436,7 +442,7 @@ PK_API int pk_rmsnorm_quant(const void* x, int M, int K, const float* gamma, int
     pk_set_last_cuda_error((int)cudaGetLastError());
     return PK_ERR_CUDA;
   }
-  rmsnorm_quant_kernel<<<M, 256, smem, stream>>>(p);
+  PK_LAUNCH_PDL(rmsnorm_quant_kernel, dim3(M), dim3(256), smem, stream, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

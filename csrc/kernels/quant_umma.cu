@@ -424,6 +424,8 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
                : "memory");
 }
 
+// Before `pdl_wait` the kernel reads the weights and the route segments: its predecessor in the stream is the staging of its rows (or
+// another product of them), which lets it begin only when everything before itself is complete.
 template <int TYPE, int NT, int TERMS>
 __global__ void __launch_bounds__(Shape<TYPE, NT>::kThreads, 1)
 quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ Params p) {
@@ -498,6 +500,8 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
 
   if (warp < S::kFoldWarps) {
     // ---------------- fold and epilogue ----------------
+    pk::pdl_wait();
+    pk::pdl_trigger();
     const int q = warp & 3, c0 = (warp >> 2) * S::kFoldCols, lr = q * 32 + lane;
     uint32_t unit = 0;
     Item w;
@@ -594,7 +598,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
       const int m0 = c0 / TERMS;
 #pragma unroll
       for (int m = 0; m < kRows; ++m)
-        if (m0 + m < w.cnt) v[m] *= __ldg(p.row_scale + w.row0 + m0 + m);
+        if (m0 + m < w.cnt) v[m] *= p.row_scale[w.row0 + m0 + m];
       if (p.epi & 1) {
         // gate and up of an output sit in a pair of lanes, of which each takes every second token row
         const int j = w.rt * 64 + (lr >> 1);
@@ -693,6 +697,7 @@ quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constan
       };
       if constexpr (RAW)
         for (int k = 0; k < S::kSlots; ++k) copy_next();
+      pk::pdl_wait();      // the staged rows
       uint32_t unit = 0;
       Item w;
       bool ok = true;
@@ -843,6 +848,8 @@ struct StageParams {
 };
 
 __global__ void __launch_bounds__(1024) quant_stage_rows_kernel(const StageParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ __align__(16) float xs[];      // [K]
   __shared__ float red[40];
   const int r = blockIdx.x, tid = threadIdx.x, stride = blockDim.x * 4;
@@ -973,7 +980,7 @@ int launch(const void* staged, int total_rows, const Params& p, int sms, cudaStr
     }
     once_guard.done();
   }
-  quant_umma_kernel<TYPE, NT, TERMS><<<sms, Shape<TYPE, NT>::kThreads, smem, stream>>>(map, wmap, p);
+  PK_LAUNCH_PDL((quant_umma_kernel<TYPE, NT, TERMS>), dim3(sms), dim3(Shape<TYPE, NT>::kThreads), smem, stream, map, wmap, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -1026,7 +1033,7 @@ PK_API int pk_quant_stage_rows(const void* x, int x_f32, int ldx, int K, const i
   const StageParams p{x, x_f32, ldx, K, index, gamma, eps, plus_one, add, (pk::bf16*)sum, (pk::bf16*)norm, terms, has_mins(type) ? 1 : 0, type == T_E4M3 ? 1 : 0, (__half*)staged, row_scale, counters, n_counters};
   // a block per row: with few rows a thread per four elements (13 rows of 5120 to 17408: mean 6.2 -> 4.6 us, one of 3072: 3.8 -> 2.9), with many the blocks hide one another
   const int threads = rows <= 148 ? min(1024, (K / 4 + 31) / 32 * 32) : 256;
-  quant_stage_rows_kernel<<<rows, threads, smem, stream>>>(p);
+  PK_LAUNCH_PDL(quant_stage_rows_kernel, dim3(rows), dim3(threads), smem, stream, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
