@@ -23,6 +23,9 @@ int pk_gemm_umma(const void* A, int lda, const void* W, const float* scale, int 
                  int epi, void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push,
                  cudaStream_t stream);
 
+void pk_gemm_reserve(int sm_count, cudaStream_t stream);
+void pk_gemm_release(cudaStream_t stream);
+
 int pk_deltanet_seq(const void* proj, int ld, int T, int key_heads, int value_heads, int key_dim,
                     int value_dim, const float* conv_w, float* conv_state, const float* A_log,
                     const float* dt_bias, const float* norm_w, float eps, float* state, void* out,

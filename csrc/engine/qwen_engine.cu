@@ -190,6 +190,7 @@ QwenEngine::QwenEngine(const QwenConfig& cfg, const QwenEngineOptions& opt) : cf
   cudaDeviceProp prop;
   cuda_check(cudaGetDeviceProperties(&prop, opt.device), "props");
   sm_count_ = prop.multiProcessorCount;
+  pk_gemm_reserve(sm_count_, stream_);
   cuda_check(cudaEventCreate(&ev0_), "event");
   cuda_check(cudaEventCreate(&ev1_), "event");
 
@@ -399,7 +400,10 @@ QwenEngine::~QwenEngine() {
   }
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
-  if (stream_) cudaStreamDestroy(stream_);
+  if (stream_) {
+    pk_gemm_release(stream_);
+    cudaStreamDestroy(stream_);
+  }
 }
 
 // ---------------------------------------------------------------------------------------

@@ -50,6 +50,8 @@ __device__ __forceinline__ float2 conv_input2(const PrepParams& p, int t, int ch
 // One block per (token, key head): 64 threads per 128-channel segment (q, k, then the head's value heads), two
 // adjacent channels per thread.
 __global__ void __launch_bounds__(256) deltanet_prep_kernel(const PrepParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   const int t = blockIdx.x, hk = blockIdx.y;
   const int rep = p.Hv / p.Hk;
   const int seg = threadIdx.x >> 6, d = (threadIdx.x & 63) * 2;  // seg 0: q, 1: k, 2+: value heads
@@ -94,6 +96,8 @@ __global__ void __launch_bounds__(256) deltanet_prep_kernel(const PrepParams p) 
 
 // New conv tail = inputs of the last three tokens. Runs after prep (which reads the old tail).
 __global__ void deltanet_tail_kernel(const bf16* proj, int ld, int T, int channels, float* conv_state) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= channels) return;
   float nv[3];
@@ -119,6 +123,8 @@ struct ChunkParams {
 };
 
 __global__ void __launch_bounds__(256) deltanet_chunk_kernel(const ChunkParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   extern __shared__ float smem[];
   float* Ks = smem;                  // [64][129]
   float* Qs = Ks + CH * KS;          // [64][129]
@@ -236,6 +242,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // Before: loads, then arithmetic, per chunk (20 us per chunk step, a third of it exposed load latency).
 template <int ST>
 __global__ void __launch_bounds__(ST) deltanet_state_kernel(const StateParams p) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   constexpr int RW = CH / (ST / 32);   // chunk rows per warp
   constexpr int SW = D / (ST / 32);    // state rows per warp
   extern __shared__ __align__(16) float smem[];
@@ -383,6 +391,8 @@ __global__ void __launch_bounds__(ST) deltanet_state_kernel(const StateParams p)
 // One warp per (token, value head), four channels per lane.
 __global__ void __launch_bounds__(256) deltanet_out_kernel(const float* O, const bf16* proj, int ld, int Hk, int Hv, int T,
                                                            const float* norm_w, float eps, bf16* out) {
+  pk::pdl_wait();
+  pk::pdl_trigger();
   const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (unit >= T * Hv) return;
   const int t = unit / Hv, h = unit - t * Hv, d = (threadIdx.x & 31) * 4;
@@ -438,10 +448,10 @@ PK_API int pk_deltanet_chunked(const void* proj, int ld, int T, int key_heads, i
 
   PrepParams pp{(const pk::bf16*)proj, ld, T, Tpad, key_heads, value_heads, conv_w, conv_state, A_log, dt_bias,
                 qn, kn, v, g, beta};
-  deltanet_prep_kernel<<<dim3(Tpad, key_heads), 64 * (2 + rep), 0, stream>>>(pp);
+  PK_LAUNCH_PDL(deltanet_prep_kernel, dim3(Tpad, key_heads), dim3(64 * (2 + rep)), 0, stream, pp);
   PK_CHECK_LAUNCH();
   const int channels = (2 * key_heads + value_heads) * D;
-  deltanet_tail_kernel<<<(channels + 255) / 256, 256, 0, stream>>>((const pk::bf16*)proj, ld, T, channels, conv_state);
+  PK_LAUNCH_PDL(deltanet_tail_kernel, dim3((channels + 255) / 256), dim3(256), 0, stream, (const pk::bf16*)proj, ld, T, channels, conv_state);
   PK_CHECK_LAUNCH();
 
   static PkDeviceOnce once;
@@ -457,17 +467,17 @@ PK_API int pk_deltanet_chunked(const void* proj, int ld, int T, int key_heads, i
     once_guard.done();
   }
   ChunkParams cp{qn, kn, v, g, beta, key_heads, value_heads, Tpad, U, W, P, G};
-  deltanet_chunk_kernel<<<dim3(nchunks, value_heads), 256, smem_chunk, stream>>>(cp);
+  PK_LAUNCH_PDL(deltanet_chunk_kernel, dim3(nchunks, value_heads), dim3(256), smem_chunk, stream, cp);
   PK_CHECK_LAUNCH();
   StateParams sp{qn, kn, U, W, P, G, key_heads, value_heads, Tpad, nchunks, state, O};
   static const int state_threads = [] {
     const char* e = getenv("POCKET_DELTANET_STATE_THREADS");
     return e && atoi(e) == 256 ? 256 : 512;
   }();
-  if (state_threads == 256) deltanet_state_kernel<256><<<dim3(value_heads, D / SL), 256, smem_state, stream>>>(sp);
-  else deltanet_state_kernel<512><<<dim3(value_heads, D / SL), 512, smem_state, stream>>>(sp);
+  if (state_threads == 256) PK_LAUNCH_PDL(deltanet_state_kernel<256>, dim3(value_heads, D / SL), dim3(256), smem_state, stream, sp);
+  else PK_LAUNCH_PDL(deltanet_state_kernel<512>, dim3(value_heads, D / SL), dim3(512), smem_state, stream, sp);
   PK_CHECK_LAUNCH();
-  deltanet_out_kernel<<<(T * value_heads + 7) / 8, 256, 0, stream>>>(O, (const pk::bf16*)proj, ld, key_heads, value_heads, T,
+  PK_LAUNCH_PDL(deltanet_out_kernel, dim3((T * value_heads + 7) / 8), dim3(256), 0, stream, O, (const pk::bf16*)proj, ld, key_heads, value_heads, T,
                                                                      norm_w, eps, (pk::bf16*)out);
   PK_CHECK_LAUNCH();
   return PK_OK;

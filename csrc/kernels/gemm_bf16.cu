@@ -13,11 +13,15 @@
 //   warps 2-9   epilogue (tcgen05.ld, then bf16 store / residual add / SiLU(gate)*up / fp32 / push to peers)
 //
 // Every mbarrier wait is bounded (status word + CTA-wide abort flag), as in gemm_umma.cu.
+//
+// us (before: a lone lane computed descriptors and issued, partial tiles and residuals were read a row at a time, stream-K from 96 k steps a group
+// on): 1900 rows of 5120 x 4096 96 -> 78, 4096 x 4096 with a residual 90 -> 70, 10304 x 4096 159 -> 133; 512 rows of 5120 x 17408 122 -> 92.
 #include <cstdlib>
 #include <mutex>
 
 #include "../common/pk_comm.cuh"
 #include "../common/pk_sm100.cuh"
+#include "../common/pk_streamk.hpp"
 
 namespace {
 
@@ -29,7 +33,7 @@ constexpr int kStages = 4;
 constexpr int kABytes = BM * BK * 2;      // 16 KB
 constexpr int kBBytes = BN * BK * 2;      // 32 KB
 constexpr int kEpiWarps = 8;
-constexpr int kThreads = 64 + kEpiWarps * 32;
+constexpr int kEpiThreads = kEpiWarps * 32, kThreads = 64 + kEpiThreads;
 constexpr uint32_t kTmemCols = 512;       // two accumulators of 256 columns
 
 enum { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_RESID = 2, EPI_F32 = 3, EPI_PUSH = 4, EPI_RELU2 = 5 };
@@ -136,8 +140,8 @@ __device__ __forceinline__ void tile_coords(const Params& p, const Smem& sm, int
     if (sm.mt_prefix[mid] <= g) lo = mid;
     else hi = mid;
   }
-  a_row = __ldg(p.seg + lo) + (g - sm.mt_prefix[lo]) * BM;
-  rows = __ldg(p.seg + lo + 1) - a_row;
+  a_row = p.seg[lo] + (g - sm.mt_prefix[lo]) * BM;
+  rows = p.seg[lo + 1] - a_row;
   w_off = lo * p.N;
 }
 
@@ -176,18 +180,28 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     sm.abort_flag = 0;
     sm.part_done = 0;
     mbar_fence_init();
-    if (p.seg != nullptr) {
-      int run = 0;
-      for (int g = 0; g < p.n_groups; ++g) {
-        sm.mt_prefix[g] = run;
-        run += (p.seg[g + 1] - p.seg[g] + BM - 1) / BM;
-      }
-      sm.mt_prefix[p.n_groups] = run;
-    }
   }
   if (warp == 1) {
     tmem_alloc(&sm.tmem_base, kTmemCols);
     tmem_relinquish();
+  }
+  if (p.seg != nullptr && warp == 2) {
+    // m-tiles before each group, 32 groups at a time
+    pk::pdl_wait();
+    int run = 0;
+    for (int g0 = 0; g0 < p.n_groups; g0 += 32) {
+      const int g = g0 + lane;
+      const int n = g < p.n_groups ? (p.seg[g + 1] - p.seg[g] + BM - 1) / BM : 0;
+      int inc = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (g < p.n_groups) sm.mt_prefix[g] = run + inc - n;
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) sm.mt_prefix[p.n_groups] = run;
   }
   tc_fence_before();
   __syncthreads();
@@ -200,9 +214,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (lane == 0) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_w);
-      uint32_t it = 0, issued = 0;
+      uint32_t it = 0, issued = 0, ahead = 0;
       WorkIter work(p, num_kb, tiles_m);
       Seg sg;
+      {
+        // the first weight tiles are requested before the rows of A are there (route segments, when there are any, are)
+        WorkIter first = work;
+        if (first.next(sg)) {
+          int tn, a_row, w_off, rows, r0, r1;
+          tile_coords(p, sm, sg.tile, tiles_m, tn, a_row, w_off, rows);
+          weight_rows(p, tn, r0, r1);
+          for (; ahead < (uint32_t)kStages && sg.kb0 + (int)ahead < sg.kb1; ++ahead) {
+            mbar_arrive_expect_tx(&sm.full[ahead], kABytes + kBBytes);
+            tma_load_2d(sm.b[ahead], &tmap_w, &sm.full[ahead], (sg.kb0 + (int)ahead) * BK, w_off + r0);
+            tma_load_2d(sm.b[ahead] + kBBytes / 2, &tmap_w, &sm.full[ahead], (sg.kb0 + (int)ahead) * BK, w_off + r1);
+          }
+        }
+      }
+      pk::pdl_wait();
       while (!sm.abort_flag && work.next(sg)) {
         int tn, a_row, w_off, rows;
         tile_coords(p, sm, sg.tile, tiles_m, tn, a_row, w_off, rows);
@@ -213,10 +242,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
           const int s = it % kStages;
           if (!mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1, &sm.abort_flag, p.status, 21)) break;
-          mbar_arrive_expect_tx(&sm.full[s], kABytes + kBBytes);
+          if (it >= ahead) {
+            mbar_arrive_expect_tx(&sm.full[s], kABytes + kBBytes);
+            tma_load_2d(sm.b[s], &tmap_w, &sm.full[s], kb * BK, r0);
+            tma_load_2d(sm.b[s] + kBBytes / 2, &tmap_w, &sm.full[s], kb * BK, r1);
+          }
           tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * BK, a_row);
-          tma_load_2d(sm.b[s], &tmap_w, &sm.full[s], kb * BK, r0);
-          tma_load_2d(sm.b[s] + kBBytes / 2, &tmap_w, &sm.full[s], kb * BK, r1);
           issued = it + 1;
         }
       }
@@ -231,36 +262,50 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(1, 1, BM, BN);
-      uint32_t it = 0;
-      int local = 0;
-      WorkIter work(p, num_kb, tiles_m);
-      Seg sg;
-      for (; !sm.abort_flag && work.next(sg); ++local) {
-        const int buf = local & 1;
-        const uint32_t use = (uint32_t)local >> 1;
-        // the epilogue must have drained this accumulator (passes at once for its first use)
-        if (!mbar_wait(&sm.acc_empty[buf], (use & 1) ^ 1, &sm.abort_flag, p.status, 22)) break;
+    // The whole warp walks the loop and one lane issues: addresses and descriptors are then uniform, which is what the
+    // instructions take.
+    constexpr uint32_t idesc = umma_idesc(1, 1, BM, BN);
+    const uint64_t da0 = smem_desc_k_sw128(smem_u32(sm.a[0])), db0 = smem_desc_k_sw128(smem_u32(sm.b[0]));
+    const bool leader = elect_one();
+    uint32_t s = 0, ph = 0;
+    int local = 0;
+    WorkIter work(p, num_kb, tiles_m);
+    Seg sg;
+    bool ok = true;
+    for (; ok && work.next(sg); ++local) {
+      const int buf = local & 1;
+      const uint32_t use = (uint32_t)local >> 1;
+      // the epilogue must have drained this accumulator (passes at once for its first use)
+      if (!mbar_wait_uniform(&sm.acc_empty[buf], (use & 1) ^ 1, &sm.abort_flag, p.status, 22)) break;
+      tc_fence_after();
+      const uint32_t tmem_acc = tmem_base + (uint32_t)buf * BN;
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+        if (!mbar_wait_uniform(&sm.full[s], ph, &sm.abort_flag, p.status, 23)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t tmem_acc = tmem_base + (uint32_t)buf * BN;
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          if (!mbar_wait(&sm.full[s], (it / kStages) & 1, &sm.abort_flag, p.status, 23)) break;
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(sm.a[s]), b_addr = smem_u32(sm.b[s]);
+        const uint64_t da = da0 + s * (uint32_t)(kABytes >> 4), db = db0 + s * (uint32_t)(kBBytes >> 4);
+        if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_f16(tmem_acc, smem_desc_k_sw128(a_addr + k * 32), smem_desc_k_sw128(b_addr + k * 32), idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k) umma_f16(tmem_acc, da + (k * 32 >> 4), db + (k * 32 >> 4), idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
           umma_commit(&sm.empty[s]);
+          if (kb + 1 == sg.kb1) umma_commit(&sm.acc_full[buf]);
         }
-        umma_commit(&sm.acc_full[buf]);
+        __syncwarp();
+        if (++s == (uint32_t)kStages) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
     }
   } else {
     // ---------------- epilogue ----------------
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     const int ch = (warp - 2) >> 2;         // which half of the tile's columns
+    // Partial sums of a row and 32 columns are the pieces v of the thread that has them: neighbouring threads have neighbouring pieces.
+    auto part_at = [&](int slot, int c0, int v) {
+      return reinterpret_cast<float4*>(p.ws + (size_t)slot * BM * BN) + (((c0 & 127) >> 5) * 8 + v) * kEpiThreads + (c0 >> 7) * 128 + q * 32 + lane;
+    };
+    pk::pdl_wait();
+    pk::pdl_trigger();
     int local = 0;
     WorkIter work(p, num_kb, tiles_m);
     Seg sg;
@@ -274,17 +319,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const int m = a_row + q * 32 + lane;
       const bool row_ok = q * 32 + lane < rows;
       const uint32_t lane_addr = tmem_base + (uint32_t)buf * BN + ((uint32_t)(q * 32) << 16);
-      const int row_in_tile = q * 32 + lane;
       if (sg.kb0 > 0) {
         // Not the owner of this tile: park the fp32 partial in this CTA's workspace slot and publish it.
-        float* dst = p.ws + ((size_t)blockIdx.x * BM + row_in_tile) * BN + ch * 128;
 #pragma unroll 1
         for (int cc = 0; cc < 4; ++cc) {
           uint32_t r[32];
           tmem_ld_32x32(lane_addr + ch * 128 + cc * 32, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int v = 0; v < 8; ++v) *reinterpret_cast<uint4*>(dst + cc * 32 + v * 4) = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
+          for (int v = 0; v < 8; ++v) *reinterpret_cast<uint4*>(part_at(blockIdx.x, ch * 128 + cc * 32, v)) = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
         }
         __threadfence();
         tc_fence_before();
@@ -323,14 +366,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
         if (!ok) n_parts = 0;
       }
-      const float* part0 = p.ws + ((size_t)(blockIdx.x + p.tiles_m) * BM + row_in_tile) * BN;
       // adds the parked partials of the following CTAs to one 32-column chunk
       auto add_parts = [&](int c0, uint32_t (&r)[32]) {
         for (int j = 0; j < n_parts; ++j) {
-          const float* src = part0 + (size_t)j * p.tiles_m * BM * BN + c0;
+          const int slot = blockIdx.x + (j + 1) * p.tiles_m;
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
-            const float4 x = __ldcg(reinterpret_cast<const float4*>(src + v * 4));
+            const float4 x = __ldcg(part_at(slot, c0, v));
             r[v * 4] = __float_as_uint(__uint_as_float(r[v * 4]) + x.x);
             r[v * 4 + 1] = __float_as_uint(__uint_as_float(r[v * 4 + 1]) + x.y);
             r[v * 4 + 2] = __float_as_uint(__uint_as_float(r[v * 4 + 2]) + x.z);
@@ -353,7 +395,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           if (!row_ok) continue;
           if (p.row_scale) {
-            const float s = __ldg(p.row_scale + m);
+            const float s = p.row_scale[m];
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               u[i] = __float_as_uint(__uint_as_float(u[i]) * s);
@@ -417,7 +459,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           } else {
             if (p.epi == EPI_RELU2) {
-              const float s = p.row_scale ? __ldg(p.row_scale + m) : 1.f;
+              const float s = p.row_scale ? p.row_scale[m] : 1.f;
               const float s0 = p.scale_after ? 1.f : s, s1 = p.scale_after ? s : 1.f;
 #pragma unroll
               for (int i = 0; i < 32; ++i) {
@@ -428,14 +470,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             bf16* dst = p.C + (size_t)m * p.ldc + n;
             const bf16* rs = p.epi == EPI_RESID ? p.resid + (size_t)m * p.ldc + n : nullptr;
             if (n + 32 <= p.N) {
+              // all pieces of the residual are on their way before the first store (which may go to the same memory: a thread's own elements)
+              uint4 rr[4];
+#pragma unroll
+              for (int v = 0; v < 4; ++v) rr[v] = rs ? *reinterpret_cast<const uint4*>(rs + v * 8) : make_uint4(0, 0, 0, 0);
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
                 float f[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[v * 8 + e]);
                 if (rs) {
-                  const uint4 rr = *reinterpret_cast<const uint4*>(rs + v * 8);
-                  const uint32_t w[4] = {rr.x, rr.y, rr.z, rr.w};
+                  const uint32_t w[4] = {rr[v].x, rr[v].y, rr[v].z, rr[v].w};
 #pragma unroll
                   for (int e = 0; e < 4; ++e) {
                     f[2 * e] += __uint_as_float(w[e] << 16);
@@ -484,45 +529,7 @@ EncodeTiledFn encode_fn() {
 }
 
 // Per-device stream-K scratch: one fp32 tile and one flag per CTA. Allocated on first use.
-struct StreamKBuffers {
-  float* ws = nullptr;
-  uint32_t* flags = nullptr;
-  uint32_t seq = 0;
-  int ctas = 0;
-};
 
-// Stream-K mode: 0 = never (POCKET_GEMM_NO_STREAMK, or POCKET_GEMM_STREAMK=0), 2 = whenever the schedule allows it
-// (POCKET_GEMM_STREAMK=1: tests), 1 = only with long k ranges (default). Measured at M = 512 on B200: K = 12288, N = 5120
-// gains 7 % (104 k-steps per CTA group), K = 5120, N = 4096 loses 25 % (35 k-steps per group: the fix-up dominates).
-static int streamk_mode() {
-  if (getenv("POCKET_GEMM_NO_STREAMK") != nullptr) return 0;
-  const char* v = getenv("POCKET_GEMM_STREAMK");
-  if (v == nullptr) return 1;
-  return v[0] == '1' ? 2 : 0;
-}
-
-
-StreamKBuffers* streamk_buffers(int ctas) {
-  static StreamKBuffers per_device[64];
-  static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  StreamKBuffers& b = per_device[dev];
-  if (b.ws == nullptr || b.ctas < ctas) {
-    if (b.ws) cudaFree(b.ws);
-    if (b.flags) cudaFree(b.flags);
-    b = StreamKBuffers();
-    if (cudaMalloc(&b.ws, (size_t)ctas * BM * BN * sizeof(float)) != cudaSuccess) return nullptr;
-    if (cudaMalloc(&b.flags, (size_t)ctas * sizeof(uint32_t)) != cudaSuccess || cudaMemset(b.flags, 0, (size_t)ctas * sizeof(uint32_t)) != cudaSuccess) {
-      cudaFree(b.ws);
-      b = StreamKBuffers();
-      return nullptr;
-    }
-    b.ctas = ctas;
-  }
-  return &b;
-}
 
 bool encode_bf16_2d(EncodeTiledFn encode, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
                     uint32_t box_inner, uint32_t box_outer) {
@@ -580,7 +587,7 @@ PK_API int pk_gemm_bf16_grouped_scaled(const void* A, int lda, const void* W, co
     }
     once_guard.done();
   }
-  gemm_bf16_kernel<<<sm_count > 0 ? sm_count : 148, kThreads, smem, stream>>>(tmap_a, tmap_w, p);
+  PK_LAUNCH_PDL(gemm_bf16_kernel, dim3(sm_count > 0 ? sm_count : 148), dim3(kThreads), smem, stream, tmap_a, tmap_w, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -638,19 +645,17 @@ PK_API int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int
   const double eff = rounds / (double)((tiles + sms - 1) / sms);
   p.streamk = 0;
   const int groups = p.tiles_m <= sms ? sms / p.tiles_m : 0;
-  if (eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 8 && streamk_mode() != 0 &&
-      (streamk_mode() == 2 || (long long)p.tiles_n * num_kb >= (long long)groups * 96)) {
-    StreamKBuffers* b = streamk_buffers(sms);
-    if (b != nullptr) {
-      p.streamk = 1;
-      p.ws = b->ws;
-      p.flags = b->flags;
-      p.seq = ++b->seq;
-      p.timeout_us = 2000000;
-      grid = groups * p.tiles_m;
-    }
+  // us without and with (eight k steps to a group of CTAs at least): 512 rows, N = 5120, K = 4096 43 / 42, 168 rows, N = 10304 45 / 43. (Before the
+  // parts were laid out by threads, the exchange took 20 us and paid only from 96 k steps on.)
+  if (pk::StreamK b; eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 8 && pk::streamk_allowed() && pk::streamk_take(sms, stream, b)) {
+    p.streamk = 1;
+    p.ws = b.ws;
+    p.flags = b.flags;
+    p.seq = b.seq;
+    p.timeout_us = 2000000;
+    grid = groups * p.tiles_m;
   }
-  gemm_bf16_kernel<<<grid, kThreads, smem, stream>>>(tmap_a, tmap_w, p);
+  PK_LAUNCH_PDL(gemm_bf16_kernel, dim3(grid), dim3(kThreads), smem, stream, tmap_a, tmap_w, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

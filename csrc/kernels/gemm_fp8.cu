@@ -22,8 +22,12 @@
 //
 // Every wait is bounded (status word + CTA-wide abort flag), as in gemm_bf16.cu.
 //
-// Measured on B200 (M = 2048, N = 34816, K = 5120, SwiGLU epilogue): 1.57 PFLOP/s with one term, 1.15 with two (counting
-// the product once), against 1.48 for the bf16 kernel on bf16 copies and 2.9 for the library's per-tensor-scaled FP8 GEMM.
+// Measured on B200 (M = 2048, N = 34816, K = 5120, SwiGLU epilogue): 1.57 PFLOP/s with one term, 1.43 with two (counting
+// the product once), against 1.58 for the bf16 kernel on bf16 copies and 2.9 for the library's per-tensor-scaled FP8 GEMM.
+// With two terms, us (before: partial tiles and residuals a row at a time, stream-K from 48 k blocks a group on): 512 rows of 34816 x 5120
+// 163 -> 141, 5120 x 17408 108 -> 88, 12288 x 5120 82 -> 68, 5120 x 4096 49 -> 43. A k block takes 1230 cycles and more where its
+// products take 1024: the fold's reads and the hand-over do not quite hide behind one block. Pairs of CTAs (M 256, half of the weight
+// tile each) have a quarter less to load and are as fast or 3 % slower.
 // The same loop without the per-block hand-over of the accumulator streams at 2.4 (one term): the four-stage ring is
 // bound by the latency of the tile loads, so every wait between "tile landed" and "stage released" lowers the bytes in
 // flight. Tried and slower: one MMA group per 128-column half (N = 128 instructions re-read the A tile and run into
@@ -38,6 +42,7 @@
 
 #include "../common/pk_comm.cuh"
 #include "../common/pk_sm100.cuh"
+#include "../common/pk_streamk.hpp"
 
 namespace {
 
@@ -48,7 +53,7 @@ constexpr int BM = 128, BN = 256, BK = 128;
 constexpr int kABytes = BM * BK;          // 16 KB per term
 constexpr int kBBytes = BN * BK;          // 32 KB
 constexpr int kEpiWarps = 16;
-constexpr int kThreads = 64 + kEpiWarps * 32;
+constexpr int kFoldThreads = kEpiWarps * 32, kThreads = 64 + kFoldThreads;
 constexpr uint32_t kTmemCols = 512;       // two accumulators of 256 columns
 
 enum { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_RESID = 2, EPI_F32 = 3, EPI_PUSH = 4, EPI_SCORE = 5 };
@@ -179,14 +184,17 @@ __device__ __forceinline__ void emit32(const Params& p, int m, int n, const floa
     bf16* dst = p.C + (size_t)m * p.ldc + n;
     const bf16* rs = p.epi == EPI_RESID ? p.resid + (size_t)m * p.ldc + n : nullptr;
     if (n + 32 <= p.N) {
+      // all pieces of the residual are on their way before the first store (which may go to the same memory: a thread's own elements)
+      uint4 rr[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) rr[v] = rs ? *reinterpret_cast<const uint4*>(rs + v * 8) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         float f[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) f[e] = r[v * 8 + e];
         if (rs) {
-          const uint4 rr = *reinterpret_cast<const uint4*>(rs + v * 8);
-          const uint32_t w[4] = {rr.x, rr.y, rr.z, rr.w};
+          const uint32_t w[4] = {rr[v].x, rr[v].y, rr[v].z, rr[v].w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             f[2 * e] += __uint_as_float(w[e] << 16);
@@ -240,9 +248,23 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     if (lane == 0) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_w);
-      uint32_t it = 0, issued = 0;
+      uint32_t it = 0, issued = 0, ahead = 0;
       WorkIter work(p, num_kb);
       Seg sg;
+      {
+        // the first weight tiles are requested before the activations are there
+        WorkIter first = work;
+        if (first.next(sg)) {
+          int r0, r1;
+          weight_rows(p, sg.tile / p.tiles_m, r0, r1);
+          for (; ahead < (uint32_t)kStages && sg.kb0 + (int)ahead < sg.kb1; ++ahead) {
+            mbar_arrive_expect_tx(&sm.full[ahead], TERMS * kABytes + kBBytes);
+            tma_load_2d(sm.b[ahead], &tmap_w, &sm.full[ahead], (sg.kb0 + (int)ahead) * BK, r0);
+            tma_load_2d(sm.b[ahead] + kBBytes / 2, &tmap_w, &sm.full[ahead], (sg.kb0 + (int)ahead) * BK, r1);
+          }
+        }
+      }
+      pk::pdl_wait();
       while (!sm.abort_flag && work.next(sg)) {
         const int tm = sg.tile % p.tiles_m, tn = sg.tile / p.tiles_m;
         int r0, r1;
@@ -250,11 +272,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
           const int s = it % kStages;
           if (!mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1, &sm.abort_flag, p.status, 31)) break;
-          mbar_arrive_expect_tx(&sm.full[s], TERMS * kABytes + kBBytes);
+          if (it >= ahead) {
+            mbar_arrive_expect_tx(&sm.full[s], TERMS * kABytes + kBBytes);
+            tma_load_2d(sm.b[s], &tmap_w, &sm.full[s], kb * BK, r0);
+            tma_load_2d(sm.b[s] + kBBytes / 2, &tmap_w, &sm.full[s], kb * BK, r1);
+          }
 #pragma unroll
           for (int t = 0; t < TERMS; ++t) tma_load_2d(sm.a[s] + t * kABytes, &tmap_a, &sm.full[s], kb * BK, t * p.m_pad + tm * BM);
-          tma_load_2d(sm.b[s], &tmap_w, &sm.full[s], kb * BK, r0);
-          tma_load_2d(sm.b[s] + kBBytes / 2, &tmap_w, &sm.full[s], kb * BK, r1);
           issued = it + 1;
         }
       }
@@ -307,6 +331,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     // ---------------- per-block fold, then the tile's epilogue ----------------
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     const int cq = (warp - 2) >> 2;         // columns cq * 32 .. + 32 of both 128-column halves
+    const int fold_thread = threadIdx.x - 64;
+    const float* a_scale = p.a_scale;
+    pk::pdl_wait_for(a_scale);
+    pk::pdl_trigger();
     uint32_t it = 0;
     WorkIter work(p, num_kb);
     Seg sg;
@@ -318,7 +346,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const int row_in_tile = q * 32 + lane;
       const int m = tm * BM + row_in_tile;
       const bool row_ok = m < p.M;
-      const float* as_ptr = p.a_scale + (row_ok ? m : p.M - 1);
+      const float* as_ptr = a_scale + (row_ok ? m : p.M - 1);
       const int nb_last = (p.N - 1) >> 7;
       const float* ws0_ptr = p.w_scale + (size_t)min(r0 >> 7, nb_last) * p.w_ld;
       const float* ws1_ptr = p.w_scale + (size_t)min(r1 >> 7, nb_last) * p.w_ld;
@@ -364,11 +392,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
       if (sg.kb0 > 0) {
         // Not the owner of this tile: park the fp32 partial in this CTA's workspace slot and publish it.
-        float* dst = p.ws + ((size_t)blockIdx.x * BM + row_in_tile) * BN + cq * 32;
+        // (A thread's sums are read by the thread of the same place: neighbouring threads have neighbouring pieces.)
+        float4* dst = reinterpret_cast<float4*>(p.ws + (size_t)blockIdx.x * BM * BN) + fold_thread;
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
-          *reinterpret_cast<float4*>(dst + v * 4) = make_float4(acc0[v * 4], acc0[v * 4 + 1], acc0[v * 4 + 2], acc0[v * 4 + 3]);
-          *reinterpret_cast<float4*>(dst + 128 + v * 4) = make_float4(acc1[v * 4], acc1[v * 4 + 1], acc1[v * 4 + 2], acc1[v * 4 + 3]);
+          dst[v * kFoldThreads] = make_float4(acc0[v * 4], acc0[v * 4 + 1], acc0[v * 4 + 2], acc0[v * 4 + 3]);
+          dst[(8 + v) * kFoldThreads] = make_float4(acc1[v * 4], acc1[v * 4 + 1], acc1[v * 4 + 2], acc1[v * 4 + 3]);
         }
         __threadfence();
         __syncwarp();
@@ -402,13 +431,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
         got = __shfl_sync(0xffffffffu, (int)got, 0) != 0;
         if (!got) n_parts = 0;
-        const float* part0 = p.ws + ((size_t)(blockIdx.x + p.tiles_m) * BM + row_in_tile) * BN + cq * 32;
+        const float4* part0 = reinterpret_cast<const float4*>(p.ws + (size_t)(blockIdx.x + p.tiles_m) * BM * BN) + fold_thread;
         for (int j = 0; j < n_parts; ++j) {
-          const float* src = part0 + (size_t)j * p.tiles_m * BM * BN;
+          const float4* src = part0 + (size_t)j * p.tiles_m * BM * BN / 4;
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
-            const float4 x = __ldcg(reinterpret_cast<const float4*>(src + v * 4));
-            const float4 y = __ldcg(reinterpret_cast<const float4*>(src + 128 + v * 4));
+            const float4 x = __ldcg(src + v * kFoldThreads);
+            const float4 y = __ldcg(src + (8 + v) * kFoldThreads);
             acc0[v * 4] += x.x; acc0[v * 4 + 1] += x.y; acc0[v * 4 + 2] += x.z; acc0[v * 4 + 3] += x.w;
             acc1[v * 4] += y.x; acc1[v * 4 + 1] += y.y; acc1[v * 4 + 2] += y.z; acc1[v * 4 + 3] += y.w;
           }
@@ -464,6 +493,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 __global__ void __launch_bounds__(256)
 quant_act_fp8_kernel(const bf16* __restrict__ x, int ldx, int M, int K, int terms, uint8_t* __restrict__ q, int m_pad, float* __restrict__ scale_t,
                      int s_ld) {
+  pk::pdl_wait_for(x);
+  pk::pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int nkb = K >> 7;
   const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -506,44 +537,6 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-struct StreamKBuffers {
-  float* ws = nullptr;
-  uint32_t* flags = nullptr;
-  uint32_t seq = 0;
-  int ctas = 0;
-};
-
-StreamKBuffers* streamk_buffers(int ctas) {
-  static StreamKBuffers per_device[64];
-  static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  StreamKBuffers& b = per_device[dev];
-  if (b.ws == nullptr || b.ctas < ctas) {
-    if (b.ws) cudaFree(b.ws);
-    if (b.flags) cudaFree(b.flags);
-    b = StreamKBuffers();
-    if (cudaMalloc(&b.ws, (size_t)ctas * BM * BN * sizeof(float)) != cudaSuccess) return nullptr;
-    if (cudaMalloc(&b.flags, (size_t)ctas * sizeof(uint32_t)) != cudaSuccess || cudaMemset(b.flags, 0, (size_t)ctas * sizeof(uint32_t)) != cudaSuccess) {
-      cudaFree(b.ws);
-      b = StreamKBuffers();
-      return nullptr;
-    }
-    b.ctas = ctas;
-  }
-  return &b;
-}
-
-// Stream-K: 0 never (POCKET_GEMM_NO_STREAMK or POCKET_GEMM_STREAMK=0), 2 whenever the schedule allows it
-// (POCKET_GEMM_STREAMK=1: tests), 1 only with long k ranges (default).
-int streamk_mode() {
-  if (getenv("POCKET_GEMM_NO_STREAMK") != nullptr) return 0;
-  const char* v = getenv("POCKET_GEMM_STREAMK");
-  if (v == nullptr) return 1;
-  return v[0] == '1' ? 2 : 0;
-}
-
 bool encode_u8_2d(EncodeTiledFn encode, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes) {
   const cuuint64_t gdim[2] = {inner, outer};
   const cuuint64_t gstride[1] = {row_stride_bytes};
@@ -564,7 +557,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tw, const Params& p, int gr
     }
     once_guard.done();
   }
-  gemm_fp8_kernel<TERMS><<<grid, kThreads, smem, stream>>>(ta, tw, p);
+  PK_LAUNCH_PDL(gemm_fp8_kernel<TERMS>, dim3(grid), dim3(kThreads), smem, stream, ta, tw, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -577,7 +570,7 @@ PK_API int pk_quant_act_fp8(const void* x, int ldx, int M, int K, int terms, voi
   if (M < 1 || K < 128 || (K & 127) != 0 || (terms != 1 && terms != 2) || m_pad < M || s_ld < M) return PK_ERR_BAD_ARG;
   if (((uintptr_t)x & 7) != 0 || (ldx & 3) != 0 || ((uintptr_t)q & 3) != 0) return PK_ERR_BAD_ARG;
   const long long units = (long long)M * (K >> 7);
-  quant_act_fp8_kernel<<<(unsigned)((units + 7) / 8), 256, 0, stream>>>((const pk::bf16*)x, ldx, M, K, terms, (uint8_t*)q, m_pad, scale_t, s_ld);
+  PK_LAUNCH_PDL(quant_act_fp8_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, (const pk::bf16*)x, ldx, M, K, terms, (uint8_t*)q, m_pad, scale_t, s_ld);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -626,19 +619,31 @@ PK_API int pk_gemm_fp8(const void* Aq, int terms, int m_pad, const float* a_scal
   const double rounds = (double)tiles / sms;
   const double eff = rounds / (double)((tiles + sms - 1) / sms);
   const int groups = p.tiles_m <= sms ? sms / p.tiles_m : 0;
-  if (eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 4 && streamk_mode() != 0 &&
-      (streamk_mode() == 2 || (long long)p.tiles_n * num_kb >= (long long)groups * 48)) {
-    StreamKBuffers* b = streamk_buffers(sms);
-    if (b != nullptr) {
-      p.streamk = 1;
-      p.ws = b->ws;
-      p.flags = b->flags;
-      p.seq = ++b->seq;
-      p.timeout_us = 2000000;
-      grid = groups * p.tiles_m;
-    }
+  // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time), four k blocks to a group of CTAs at least.
+  // us without and with: 512 rows, N = 5120, K = 4096 45 / 43, K = 5120 51 / 48; 128 rows, N = 5120, K = 17408 123 / 59, N = 12288, K = 5120
+  // 47 / 41. (Before the parts were laid out by threads, the exchange took 15 us and paid only from 48 k blocks on.)
+  if (pk::StreamK b; eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 4 && pk::streamk_allowed() && pk::streamk_take(sms, stream, b)) {
+    p.streamk = 1;
+    p.ws = b.ws;
+    p.flags = b.flags;
+    p.seq = b.seq;
+    p.timeout_us = 2000000;
+    grid = groups * p.tiles_m;
   }
   return terms == 1 ? launch<1>(tmap_a, tmap_w, p, grid, stream) : launch<2>(tmap_a, tmap_w, p, grid, stream);
+}
+
+// The stream-K work space of `stream`, allocated now instead of by the first product on it (1 ms and more), and given back: by the owner of
+// the stream, when nothing runs on it any more.
+PK_API void pk_gemm_reserve(int sm_count, cudaStream_t stream) {
+  pk::StreamKPool& pool = pk::streamk_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  if (pk::streamk_allowed()) pool.of(stream, sm_count > 0 ? sm_count : 148, true);
+}
+PK_API void pk_gemm_release(cudaStream_t stream) {
+  pk::StreamKPool& pool = pk::streamk_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  if (pk::StreamKPool::Entry* e = pool.of(stream, 0, false)) e->id = pk::kStreamKFree;
 }
 
 // Chunk scorer of the long-context retriever as one FP8 GEMM: keys [n_chunks, 128] E4M3 codes with one fp32 scale per

@@ -294,6 +294,32 @@ def test_gemm_fp8_stream_k_and_many_tiles(M, N, K, epi):
     assert _rel_err(c2, planes @ wd2.t()) < 6e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 5120, 1024), (200, 2304, 3072)])
+def test_stream_k_on_several_streams_and_under_capture(M, N, K):
+    """Tiles whose K is shared: launches on more streams than there are work spaces, and replays of a captured launch with new rows."""
+    from pocketllm_b200 import ops
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    xs = [torch.randn(M, K, device="cuda").to(torch.bfloat16) for _ in range(10)]
+    want = [x.float() @ w.float().t() for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = []
+    for x, st in zip(xs, streams):
+        with torch.cuda.stream(st):
+            got.append([ops.gemm_bf16(x, w) for _ in range(3)])
+    torch.cuda.synchronize()
+    for g, r in zip(got, want):
+        assert all(_rel_err(y, r) < 6e-3 for y in g) and torch.equal(g[0], g[1]) and torch.equal(g[1], g[2])
+    x = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ops.gemm_bf16(x, w)
+    for new, r in zip(xs, want):
+        x.copy_(new)
+        graph.replay()
+        assert _rel_err(y, r) < 6e-3
+
+
 def test_rmsnorm_embedding_argmax():
     from pocketllm_b200 import ops
     x = torch.randn(5, 640, device="cuda").to(torch.bfloat16)
