@@ -12,8 +12,10 @@
 // The reference engine has only the token-serial form for prefill
 // (cpp_engine/cuda/qwen_half_ops.cu:858-930, one 128-float state column per thread).
 //
-// All matrix products here are fp32 SIMT; they are the next candidates for tcgen05 tiles.
-#include <cstdlib>
+// All matrix products here are fp32 multiply-adds, a thread with 4 x 4 sums, so that shared-memory reads (which set the pace of one row or
+// column a thread) take less time than they do.
+#include <type_traits>
+
 #include "../common/pk_common.cuh"
 
 namespace {
@@ -22,7 +24,7 @@ using namespace pk;
 
 constexpr int CH = 64;   // chunk length
 constexpr int D = 128;   // key and value head dim
-constexpr int KS = 129;  // padded row stride of K / Q tiles in shared memory
+constexpr int KS = 132;  // padded row stride of 128-wide tiles in shared memory: neighbouring rows are four banks apart
 
 // ---------------------------------------------------------------------------------------
 // prep: conv + SiLU, L2 norms, gates, for every token in parallel
@@ -111,7 +113,8 @@ __global__ void deltanet_tail_kernel(const bf16* proj, int ld, int T, int channe
 }
 
 // ---------------------------------------------------------------------------------------
-// per (chunk, value head): G, A, U, W, P
+// per (chunk, value head): G, A, U, W, P. 8 chunks of 32 heads 68 -> 37 us: the products read shared memory a value a multiply-add, and
+// the substitution loaded each right-hand side behind the store of the solution before it.
 
 struct ChunkParams {
   const float* qn; const float* kn; const float* v; const float* g; const float* beta;
@@ -122,12 +125,12 @@ struct ChunkParams {
   float* G;   // [Hv, Tpad] running log decay inside the chunk
 };
 
-__global__ void __launch_bounds__(256) deltanet_chunk_kernel(const ChunkParams p) {
+__global__ void __launch_bounds__(256, 2) deltanet_chunk_kernel(const ChunkParams p) {
   pk::pdl_wait();
   pk::pdl_trigger();
   extern __shared__ float smem[];
-  float* Ks = smem;                  // [64][129]
-  float* Qs = Ks + CH * KS;          // [64][129]
+  float* Ks = smem;                  // [64][132]
+  float* Qs = Ks + CH * KS;          // [64][132]
   float* As = Qs + CH * KS;          // [64][64]
   float* Gs = As + CH * CH;          // [64]
   float* Bs = Gs + CH;               // [64]
@@ -135,10 +138,11 @@ __global__ void __launch_bounds__(256) deltanet_chunk_kernel(const ChunkParams p
   const int hk = h / (p.Hv / p.Hk);
   const int t0 = c * CH;
 
-  for (int i = tid; i < CH * D; i += 256) {
-    const int r = i >> 7, d = i & 127;
-    Ks[r * KS + d] = p.kn[((size_t)(t0 + r) * p.Hk + hk) * D + d];
-    Qs[r * KS + d] = p.qn[((size_t)(t0 + r) * p.Hk + hk) * D + d];
+#pragma unroll 4
+  for (int i = tid; i < CH * D / 4; i += 256) {
+    const int r = i >> 5, d = (i & 31) * 4;
+    *reinterpret_cast<float4*>(Ks + r * KS + d) = *reinterpret_cast<const float4*>(p.kn + ((size_t)(t0 + r) * p.Hk + hk) * D + d);
+    *reinterpret_cast<float4*>(Qs + r * KS + d) = *reinterpret_cast<const float4*>(p.qn + ((size_t)(t0 + r) * p.Hk + hk) * D + d);
   }
   if (tid < 32) {
     // inclusive scan of g over the 64 tokens (two per lane)
@@ -163,15 +167,23 @@ __global__ void __launch_bounds__(256) deltanet_chunk_kernel(const ChunkParams p
     float accA[16], accP[16];
 #pragma unroll
     for (int n = 0; n < 16; ++n) { accA[n] = 0.f; accP[n] = 0.f; }
-    for (int k = 0; k < D; ++k) {
-      const float kj = Ks[j * KS + k];
+    // columns 32 to 63 have nothing above row 32
+    auto products = [&](auto first) {
+      constexpr int N0 = decltype(first)::value;
+#pragma unroll 2
+      for (int k = 0; k < D; k += 4) {
+        const float4 kj = *reinterpret_cast<const float4*>(Ks + j * KS + k);
 #pragma unroll
-      for (int n = 0; n < 16; ++n) {
-        const int i = ig + 4 * n;
-        accA[n] = fmaf(Ks[i * KS + k], kj, accA[n]);
-        accP[n] = fmaf(Qs[i * KS + k], kj, accP[n]);
+        for (int n = N0; n < 16; ++n) {
+          const int i = ig + 4 * n;
+          const float4 a = *reinterpret_cast<const float4*>(Ks + i * KS + k), b = *reinterpret_cast<const float4*>(Qs + i * KS + k);
+          accA[n] = fmaf(a.w, kj.w, fmaf(a.z, kj.z, fmaf(a.y, kj.y, fmaf(a.x, kj.x, accA[n]))));
+          accP[n] = fmaf(b.w, kj.w, fmaf(b.z, kj.z, fmaf(b.y, kj.y, fmaf(b.x, kj.x, accP[n]))));
+        }
       }
-    }
+    };
+    if (j < 32) products(std::integral_constant<int, 0>());
+    else products(std::integral_constant<int, 8>());
     float* Pout = p.P + (((size_t)h * (p.Tpad / CH) + c) * CH) * CH;
 #pragma unroll
     for (int n = 0; n < 16; ++n) {
@@ -189,12 +201,12 @@ __global__ void __launch_bounds__(256) deltanet_chunk_kernel(const ChunkParams p
     const int col = tid & 127;
     const bool isW = tid >= 128;
     float X[CH];
+    // the right-hand sides first: behind the stores of the solution the loads would wait for one another
+#pragma unroll
+    for (int i = 0; i < CH; ++i) X[i] = isW ? Ks[i * KS + col] : p.v[((size_t)(t0 + i) * p.Hv + h) * D + col];
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
-      float b;
-      if (isW) b = Bs[i] * __expf(Gs[i]) * Ks[i * KS + col];
-      else b = Bs[i] * p.v[((size_t)(t0 + i) * p.Hv + h) * D + col];
-      float acc = b;
+      float acc = X[i] * (isW ? Bs[i] * __expf(Gs[i]) : Bs[i]);
 #pragma unroll
       for (int j4 = 0; j4 < (i + 3) / 4; ++j4) {
         const float4 a = *reinterpret_cast<const float4*>(As + i * CH + j4 * 4);
@@ -232,157 +244,179 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// ST threads per block: with 512 (16 warps) warp w owns 4 chunk rows and 8 state rows, with 256 it owns 8 and 16.
-// One block per SM (137 KB of shared memory). The three operand tiles of a chunk (W, q, k: 32 KB each) and P arrive by
-// cp.async straight into the buffer that the matching phase of the PREVIOUS chunk has just finished with, so every load
-// has two phases of arithmetic to land in: W(c+1) is issued after the Delta phase of chunk c, q and P after the output
-// phase, k after the state phase. Three groups are always in flight in that order, so "all but the two newest groups
-// have landed" is the right wait before every phase. q and k stay unscaled in shared memory: e^{G_i} multiplies the
-// q.S sums, e^{G_C - G_j} multiplies Delta_j on the way into the state update.
-// Before: loads, then arithmetic, per chunk (20 us per chunk step, a third of it exposed load latency).
-template <int ST>
+// One block of 16 warps per SM (190 KB of shared memory). A thread has 4 x 4 sums: lane = 4 row groups x 8 column groups, a warp 16 rows of the
+// slice's 32 columns, and the warps that are left share the sums' K, whose parts are added through shared memory. A step of four
+// K then takes 8 reads of 16 bytes for 64 multiply-adds (a row and a column a thread took 8 for 16). q S runs with W S, on the same
+// reads of S. The operands of a chunk arrive by cp.async in the buffers that the chunk before has just finished with: W and q behind
+// its Delta, P and k behind its state. q and k stay unscaled in shared memory: e^{G_i} multiplies the q S sums, e^{G_C - G_j} Delta_j.
+// Bound by shared-memory reads (a 16-byte read is four passes, whatever lanes share: some 7 of 9 us a chunk, the multiply-adds 3.8) and six
+// barriers. 8 chunks of 32 heads: 110 -> 75 us.
+constexpr int ST = 512, PS = 68;
+struct StateSmem {
+  float W[CH * KS], Q[CH * KS], K[CH * KS], P[CH * PS];
+  float Dl[CH * SL], Dk[CH * SL];      // Delta, e^{G_C - G} Delta
+  float S[D * SL];
+  float R[4 * CH * SL];                // parts of sums: [4][64][32] or [2][128][32]
+  float Eq[CH], Ek[CH];
+};
+
+__device__ __forceinline__ void fma4(float (&acc)[4], float a, const float4& b) {
+  acc[0] = fmaf(a, b.x, acc[0]);
+  acc[1] = fmaf(a, b.y, acc[1]);
+  acc[2] = fmaf(a, b.z, acc[2]);
+  acc[3] = fmaf(a, b.w, acc[3]);
+}
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+
 __global__ void __launch_bounds__(ST) deltanet_state_kernel(const StateParams p) {
   pk::pdl_wait();
   pk::pdl_trigger();
-  constexpr int RW = CH / (ST / 32);   // chunk rows per warp
-  constexpr int SW = D / (ST / 32);    // state rows per warp
   extern __shared__ __align__(16) float smem[];
-  float* Ws = smem;               // [64][128]
-  float* Qs = Ws + CH * D;        // [64][128]  q_i (unscaled)
-  float* Ks = Qs + CH * D;        // [64][128]  k_i (unscaled)
-  float* Ps = Ks + CH * D;        // [64][64]
-  float* Ds = Ps + CH * CH;       // [64][32]   Delta
-  float* Ss = Ds + CH * SL;       // [128][32]  state slice
-  float* Gs = Ss + D * SL;        // [64]
-  float* Eq = Gs + CH;            // [64] e^{G_i}
-  float* Ek = Eq + CH;            // [64] e^{G_C - G_i}
-  const int h = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
+  StateSmem& m = *reinterpret_cast<StateSmem*>(smem);
+  const int h = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hk = h / (p.Hv / p.Hk);
-  const int tx = tid & 31, ty = tid >> 5;
+  const int rg = lane >> 3, cg = (lane & 7) * 4;                       // rows 4 e + rg of a tile, columns cg ..
+  const int rt = (warp & 3) * 16, kg = warp >> 2;                      // 64 x 32 sums: row tile, quarter of K
+  const int st = (warp & 7) * 16, jh = warp >> 3;                      // 128 x 32 sums: row tile, half of K
+  const int orow = tid >> 3, ocol = (tid & 7) * 4;                     // a thread's place when parts are added
   float* sp = p.state + (size_t)h * D * D + sl * SL;
 
-  auto issue_w = [&](int c) {
+  auto rows128 = [&](float* dst, const float* src, size_t ld) {
+    for (int i = tid; i < CH * D / 4; i += ST) cp_async16(dst + (i >> 5) * KS + (i & 31) * 4, src + (i >> 5) * ld + (i & 31) * 4);
+  };
+  auto issue_wq = [&](int c) {
     if (c < p.nchunks) {
-      const float* src = p.W + ((size_t)h * p.Tpad + (size_t)c * CH) * D;
-      for (int i = tid; i < CH * D / 4; i += ST) cp_async16(Ws + i * 4, src + i * 4);
+      rows128(m.W, p.W + ((size_t)h * p.Tpad + (size_t)c * CH) * D, D);
+      rows128(m.Q, p.qn + ((size_t)c * CH * p.Hk + hk) * D, (size_t)p.Hk * D);
     }
     cp_async_commit();
   };
-  auto issue_qp = [&](int c) {
+  auto issue_pk = [&](int c) {
     if (c < p.nchunks) {
-      for (int i = tid; i < CH * D / 4; i += ST) {
-        const int r = i >> 5, d4 = (i & 31) * 4;
-        cp_async16(Qs + r * D + d4, p.qn + ((size_t)(c * CH + r) * p.Hk + hk) * D + d4);
-      }
       const float* src = p.P + (((size_t)h * p.nchunks + c) * CH) * CH;
-      for (int i = tid; i < CH * CH / 4; i += ST) cp_async16(Ps + i * 4, src + i * 4);
-    }
-    cp_async_commit();
-  };
-  auto issue_k = [&](int c) {
-    if (c < p.nchunks) {
-      for (int i = tid; i < CH * D / 4; i += ST) {
-        const int r = i >> 5, d4 = (i & 31) * 4;
-        cp_async16(Ks + r * D + d4, p.kn + ((size_t)(c * CH + r) * p.Hk + hk) * D + d4);
-      }
+      for (int i = tid; i < CH * CH / 4; i += ST) cp_async16(m.P + (i >> 4) * PS + (i & 15) * 4, src + i * 4);
+      rows128(m.K, p.kn + ((size_t)c * CH * p.Hk + hk) * D, (size_t)p.Hk * D);
     }
     cp_async_commit();
   };
 
-  issue_w(0);
-  issue_qp(0);
-  issue_k(0);
-  for (int i = tid; i < D * SL; i += ST) Ss[i] = sp[(size_t)(i >> 5) * D + (i & 31)];
-  float gnext = tid < CH ? p.G[(size_t)h * p.Tpad + tid] : 0.f;
+  issue_wq(0);
+  issue_pk(0);
+  for (int i = tid; i < D * SL / 4; i += ST) *reinterpret_cast<float4*>(m.S + i * 4) = load4(sp + (size_t)(i >> 3) * D + (i & 7) * 4);
+  const float* Uc = p.U + ((size_t)h * p.Tpad + orow) * D + sl * SL + ocol;
+  const float* Gc = p.G + (size_t)h * p.Tpad;
+  float4 u = load4(Uc);
+  float g = tid < CH ? Gc[tid] : 0.f, gC = Gc[CH - 1];
 
   for (int c = 0; c < p.nchunks; ++c) {
     const int t0 = c * CH;
-    if (tid < CH) Gs[tid] = gnext;
-    if (tid < CH && c + 1 < p.nchunks) gnext = p.G[(size_t)h * p.Tpad + t0 + CH + tid];
-    float acc[RW];
-#pragma unroll
-    for (int r = 0; r < RW; ++r) acc[r] = p.U[((size_t)h * p.Tpad + t0 + ty * RW + r) * D + sl * SL + tx];
-    __syncthreads();
-    const float gC = Gs[CH - 1];
+    const float eC = __expf(gC);
     if (tid < CH) {
-      Eq[tid] = __expf(Gs[tid]);
-      Ek[tid] = __expf(gC - Gs[tid]);
+      m.Eq[tid] = __expf(g);
+      m.Ek[tid] = __expf(gC - g);
     }
-    cp_async_wait<2>();   // W of this chunk
+    cp_async_wait<1>();   // W and q of this chunk
     __syncthreads();
 
-    // Delta = U - W S, rows ty*RW .. ty*RW+RW-1
-    for (int k = 0; k < D; k += 4) {
-      const float s0 = Ss[(k + 0) * SL + tx], s1 = Ss[(k + 1) * SL + tx], s2 = Ss[(k + 2) * SL + tx],
-                  s3 = Ss[(k + 3) * SL + tx];
+    // W S and q S
+    float aw[4][4] = {}, aq[4][4] = {};
+#pragma unroll 2
+    for (int k = kg * 32; k < kg * 32 + 32; k += 4) {
+      const float4 s0 = load4(m.S + k * SL + cg), s1 = load4(m.S + (k + 1) * SL + cg), s2 = load4(m.S + (k + 2) * SL + cg), s3 = load4(m.S + (k + 3) * SL + cg);
 #pragma unroll
-      for (int r = 0; r < RW; ++r) {
-        const float4 w = *reinterpret_cast<const float4*>(Ws + (ty * RW + r) * D + k);
-        acc[r] -= w.x * s0 + w.y * s1 + w.z * s2 + w.w * s3;
+      for (int e = 0; e < 4; ++e) {
+        const float4 w = load4(m.W + (rt + 4 * e + rg) * KS + k), q = load4(m.Q + (rt + 4 * e + rg) * KS + k);
+        fma4(aw[e], w.x, s0);
+        fma4(aw[e], w.y, s1);
+        fma4(aw[e], w.z, s2);
+        fma4(aw[e], w.w, s3);
+        fma4(aq[e], q.x, s0);
+        fma4(aq[e], q.y, s1);
+        fma4(aq[e], q.z, s2);
+        fma4(aq[e], q.w, s3);
       }
     }
 #pragma unroll
-    for (int r = 0; r < RW; ++r) Ds[(ty * RW + r) * SL + tx] = acc[r];
+    for (int e = 0; e < 4; ++e) store4(m.R + (kg * CH + rt + 4 * e + rg) * SL + cg, aw[e]);
     __syncthreads();
-    issue_w(c + 1);       // Ws is free
-    cp_async_wait<2>();   // q and P of this chunk
+    issue_wq(c + 1);
+
+    // Delta = U - W S
+    {
+      float4 d = u;
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const float4 r = load4(m.R + (n * CH + orow) * SL + ocol);
+        d = make_float4(d.x - r.x, d.y - r.y, d.z - r.z, d.w - r.w);
+      }
+      const float ek = m.Ek[orow];
+      *reinterpret_cast<float4*>(m.Dl + orow * SL + ocol) = d;
+      *reinterpret_cast<float4*>(m.Dk + orow * SL + ocol) = make_float4(d.x * ek, d.y * ek, d.z * ek, d.w * ek);
+    }
+    if (c + 1 < p.nchunks) {
+      u = load4(Uc + (size_t)(t0 + CH) * D);
+      g = tid < CH ? Gc[t0 + CH + tid] : 0.f;
+      gC = Gc[t0 + 2 * CH - 1];
+    }
+    cp_async_wait<1>();   // P and k of this chunk
     __syncthreads();
 
     // O = e^{G} (q S) + P Delta
 #pragma unroll
-    for (int r = 0; r < RW; ++r) acc[r] = 0.f;
-    for (int k = 0; k < D; k += 4) {
-      const float s0 = Ss[(k + 0) * SL + tx], s1 = Ss[(k + 1) * SL + tx], s2 = Ss[(k + 2) * SL + tx],
-                  s3 = Ss[(k + 3) * SL + tx];
+    for (int e = 0; e < 4; ++e) {
+      const float f = m.Eq[rt + 4 * e + rg];
 #pragma unroll
-      for (int r = 0; r < RW; ++r) {
-        const float4 w = *reinterpret_cast<const float4*>(Qs + (ty * RW + r) * D + k);
-        acc[r] += w.x * s0 + w.y * s1 + w.z * s2 + w.w * s3;
+      for (int i = 0; i < 4; ++i) aq[e][i] *= f;
+    }
+#pragma unroll
+    for (int j = kg * 16; j < kg * 16 + 16; j += 4) {
+      const float4 d0 = load4(m.Dl + j * SL + cg), d1 = load4(m.Dl + (j + 1) * SL + cg), d2 = load4(m.Dl + (j + 2) * SL + cg), d3 = load4(m.Dl + (j + 3) * SL + cg);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 w = load4(m.P + (rt + 4 * e + rg) * PS + j);
+        fma4(aq[e], w.x, d0);
+        fma4(aq[e], w.y, d1);
+        fma4(aq[e], w.z, d2);
+        fma4(aq[e], w.w, d3);
       }
     }
 #pragma unroll
-    for (int r = 0; r < RW; ++r) acc[r] *= Eq[ty * RW + r];
-    for (int j = 0; j < CH; j += 4) {
-      const float d0 = Ds[(j + 0) * SL + tx], d1 = Ds[(j + 1) * SL + tx], d2 = Ds[(j + 2) * SL + tx],
-                  d3 = Ds[(j + 3) * SL + tx];
-#pragma unroll
-      for (int r = 0; r < RW; ++r) {
-        const float4 w = *reinterpret_cast<const float4*>(Ps + (ty * RW + r) * CH + j);
-        acc[r] += w.x * d0 + w.y * d1 + w.z * d2 + w.w * d3;
-      }
+    for (int e = 0; e < 4; ++e) store4(m.R + (kg * CH + rt + 4 * e + rg) * SL + cg, aq[e]);
+    // S: k^T (e^{G_C - G} Delta), rows st + 4 rg + e
+    float as[4][4] = {};
+#pragma unroll 4
+    for (int j = jh * 32; j < jh * 32 + 32; ++j) {
+      const float4 k = load4(m.K + j * KS + st + 4 * rg), d = load4(m.Dk + j * SL + cg);
+      fma4(as[0], k.x, d);
+      fma4(as[1], k.y, d);
+      fma4(as[2], k.z, d);
+      fma4(as[3], k.w, d);
     }
-#pragma unroll
-    for (int r = 0; r < RW; ++r)
-      p.O[((size_t)(t0 + ty * RW + r) * p.Hv + h) * D + sl * SL + tx] = acc[r];
     __syncthreads();
-    issue_qp(c + 1);      // Qs and Ps are free
-    cp_async_wait<2>();   // k of this chunk
-    __syncthreads();
-
-    // S <- e^{G_C} S + k^T (e^{G_C - G} Delta), rows ty*SW .. ty*SW+SW-1
-    float sn[SW];
-    const float eC = __expf(gC);
+    issue_pk(c + 1);
+    {
+      float4 o = load4(m.R + orow * SL + ocol);
 #pragma unroll
-    for (int r = 0; r < SW; ++r) sn[r] = eC * Ss[(ty * SW + r) * SL + tx];
-    for (int j = 0; j < CH; ++j) {
-      const float dj = Ds[j * SL + tx] * Ek[j];
-#pragma unroll
-      for (int r4 = 0; r4 < SW / 4; ++r4) {
-        const float4 k = *reinterpret_cast<const float4*>(Ks + j * D + ty * SW + r4 * 4);
-        sn[r4 * 4 + 0] = fmaf(k.x, dj, sn[r4 * 4 + 0]);
-        sn[r4 * 4 + 1] = fmaf(k.y, dj, sn[r4 * 4 + 1]);
-        sn[r4 * 4 + 2] = fmaf(k.z, dj, sn[r4 * 4 + 2]);
-        sn[r4 * 4 + 3] = fmaf(k.w, dj, sn[r4 * 4 + 3]);
+      for (int n = 1; n < 4; ++n) {
+        const float4 r = load4(m.R + (n * CH + orow) * SL + ocol);
+        o = make_float4(o.x + r.x, o.y + r.y, o.z + r.z, o.w + r.w);
       }
+      *reinterpret_cast<float4*>(p.O + ((size_t)(t0 + orow) * p.Hv + h) * D + sl * SL + ocol) = o;
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < SW; ++r) Ss[(ty * SW + r) * SL + tx] = sn[r];
-    issue_k(c + 1);       // Ks is free
+    for (int e = 0; e < 4; ++e) store4(m.R + (jh * D + st + 4 * rg + e) * SL + cg, as[e]);
     __syncthreads();
+    for (int i = tid; i < D * SL / 4; i += ST) {
+      const float4 a = load4(m.R + i * 4), b = load4(m.R + D * SL + i * 4), s = load4(m.S + i * 4);
+      *reinterpret_cast<float4*>(m.S + i * 4) =
+          make_float4(fmaf(eC, s.x, a.x + b.x), fmaf(eC, s.y, a.y + b.y), fmaf(eC, s.z, a.z + b.z), fmaf(eC, s.w, a.w + b.w));
+    }
   }
   cp_async_wait<0>();
-  for (int i = tid; i < D * SL; i += ST) sp[(size_t)(i >> 5) * D + (i & 31)] = Ss[i];
+  __syncthreads();
+  for (int i = tid; i < D * SL / 4; i += ST) *reinterpret_cast<float4*>(sp + (size_t)(i >> 3) * D + (i & 7) * 4) = load4(m.S + i * 4);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -456,11 +490,10 @@ PK_API int pk_deltanet_chunked(const void* proj, int ld, int T, int key_heads, i
 
   static PkDeviceOnce once;
   const size_t smem_chunk = (size_t)(2 * CH * KS + CH * CH + 2 * CH) * sizeof(float);
-  const size_t smem_state = (size_t)(3 * CH * D + CH * CH + CH * SL + D * SL + 3 * CH) * sizeof(float);
+  const size_t smem_state = sizeof(StateSmem);
   if (PkDeviceOnceGuard once_guard{once}; once_guard.needed()) {
     if (cudaFuncSetAttribute(deltanet_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_chunk) != cudaSuccess ||
-        cudaFuncSetAttribute(deltanet_state_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_state) != cudaSuccess ||
-        cudaFuncSetAttribute(deltanet_state_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_state) != cudaSuccess) {
+        cudaFuncSetAttribute(deltanet_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_state) != cudaSuccess) {
       pk_set_last_cuda_error((int)cudaGetLastError());
       return PK_ERR_CUDA;
     }
@@ -470,12 +503,7 @@ PK_API int pk_deltanet_chunked(const void* proj, int ld, int T, int key_heads, i
   PK_LAUNCH_PDL(deltanet_chunk_kernel, dim3(nchunks, value_heads), dim3(256), smem_chunk, stream, cp);
   PK_CHECK_LAUNCH();
   StateParams sp{qn, kn, U, W, P, G, key_heads, value_heads, Tpad, nchunks, state, O};
-  static const int state_threads = [] {
-    const char* e = getenv("POCKET_DELTANET_STATE_THREADS");
-    return e && atoi(e) == 256 ? 256 : 512;
-  }();
-  if (state_threads == 256) PK_LAUNCH_PDL(deltanet_state_kernel<256>, dim3(value_heads, D / SL), dim3(256), smem_state, stream, sp);
-  else PK_LAUNCH_PDL(deltanet_state_kernel<512>, dim3(value_heads, D / SL), dim3(512), smem_state, stream, sp);
+  PK_LAUNCH_PDL(deltanet_state_kernel, dim3(value_heads, D / SL), dim3(ST), smem_state, stream, sp);
   PK_CHECK_LAUNCH();
   PK_LAUNCH_PDL(deltanet_out_kernel, dim3((T * value_heads + 7) / 8), dim3(256), 0, stream, O, (const pk::bf16*)proj, ld, key_heads, value_heads, T,
                                                                      norm_w, eps, (pk::bf16*)out);
