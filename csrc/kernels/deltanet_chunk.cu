@@ -49,49 +49,62 @@ __device__ __forceinline__ float2 conv_input2(const PrepParams& p, int t, int ch
   return make_float2(p.conv_state[(size_t)ch * 3 + (3 + t)], p.conv_state[(size_t)(ch + 1) * 3 + (3 + t)]);
 }
 
-// One block per (token, key head): 64 threads per 128-channel segment (q, k, then the head's value heads), two
-// adjacent channels per thread.
+// One block per (eight tokens, key head): 64 threads per 128-channel segment (q, k, then the head's value heads), two adjacent channels per
+// thread. A token's inputs serve the conv of the three after it, the conv's weights all eight: 512 tokens 24 -> 15 us (a block per token
+// read four rows and all weights for one).
+constexpr int kPrepTokens = 8;
 __global__ void __launch_bounds__(256) deltanet_prep_kernel(const PrepParams p) {
   pk::pdl_wait();
   pk::pdl_trigger();
-  const int t = blockIdx.x, hk = blockIdx.y;
+  const int t0 = blockIdx.x * kPrepTokens, hk = blockIdx.y;
   const int rep = p.Hv / p.Hk;
-  const int seg = threadIdx.x >> 6, d = (threadIdx.x & 63) * 2;  // seg 0: q, 1: k, 2+: value heads
+  const int seg = threadIdx.x >> 6, th = threadIdx.x & 63, d = th * 2;  // seg 0: q, 1: k, 2+: value heads
   const int KD = p.Hk * D, VD = p.Hv * D;
-  __shared__ float s_sum[4][2];
+  __shared__ float s_sum[kPrepTokens][2][2];
   const int h = hk * rep + (seg - 2);
-  float y0 = 0.f, y1 = 0.f;
-  if (t < p.T) {
-    const int ch = seg == 0 ? hk * D + d : seg == 1 ? KD + hk * D + d : 2 * KD + h * D + d;
-    const float4 w0 = *reinterpret_cast<const float4*>(p.conv_w + (size_t)ch * 4);
-    const float4 w1 = *reinterpret_cast<const float4*>(p.conv_w + (size_t)(ch + 1) * 4);
-    const float2 a = conv_input2(p, t - 3, ch), b = conv_input2(p, t - 2, ch), c = conv_input2(p, t - 1, ch), e = conv_input2(p, t, ch);
-    y0 = w0.x * a.x + w0.y * b.x + w0.z * c.x + w0.w * e.x;
-    y1 = w1.x * a.y + w1.y * b.y + w1.z * c.y + w1.w * e.y;
-    y0 = __bfloat162float(__float2bfloat16(silu(y0)));
-    y1 = __bfloat162float(__float2bfloat16(silu(y1)));
+  const int ch = seg == 0 ? hk * D + d : seg == 1 ? KD + hk * D + d : 2 * KD + h * D + d;
+  const float4 w0 = *reinterpret_cast<const float4*>(p.conv_w + (size_t)ch * 4);
+  const float4 w1 = *reinterpret_cast<const float4*>(p.conv_w + (size_t)(ch + 1) * 4);
+  float2 x[kPrepTokens + 3];
+#pragma unroll
+  for (int i = 0; i < kPrepTokens + 3; ++i) x[i] = t0 + i - 3 < p.T ? conv_input2(p, t0 + i - 3, ch) : make_float2(0.f, 0.f);
+  if (seg >= 2 && th < kPrepTokens) {
+    const int t = t0 + th;
+    float gg = 0.f, bb = 0.f;
+    if (t < p.T) {
+      const bf16* row = p.proj + (size_t)t * p.ld;
+      const float a = __bfloat162float(row[2 * KD + 2 * VD + h]);
+      const float b = __bfloat162float(row[2 * KD + 2 * VD + p.Hv + h]);
+      gg = -__expf(p.A_log[h]) * softplusf_(a + p.dt_bias[h]);
+      bb = sigmoidf_(b);
+    }
+    p.g[(size_t)t * p.Hv + h] = gg;
+    p.beta[(size_t)t * p.Hv + h] = bb;
   }
-  const float ss = warp_sum(y0 * y0 + y1 * y1);
-  if ((threadIdx.x & 31) == 0) s_sum[seg][(threadIdx.x >> 5) & 1] = ss;
+  float2 y[kPrepTokens];
+#pragma unroll
+  for (int i = 0; i < kPrepTokens; ++i) {
+    const float y0 = w0.x * x[i].x + w0.y * x[i + 1].x + w0.z * x[i + 2].x + w0.w * x[i + 3].x;
+    const float y1 = w1.x * x[i].y + w1.y * x[i + 1].y + w1.z * x[i + 2].y + w1.w * x[i + 3].y;
+    y[i] = t0 + i < p.T ? make_float2(__bfloat162float(__float2bfloat16(silu(y0))), __bfloat162float(__float2bfloat16(silu(y1)))) : make_float2(0.f, 0.f);
+  }
+  if (seg >= 2) {
+#pragma unroll
+    for (int i = 0; i < kPrepTokens; ++i) *reinterpret_cast<float2*>(p.v + ((size_t)(t0 + i) * p.Hv + h) * D + d) = y[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < kPrepTokens; ++i) {
+      const float ss = warp_sum(y[i].x * y[i].x + y[i].y * y[i].y);
+      if ((th & 31) == 0) s_sum[i][seg][th >> 5] = ss;
+    }
+  }
   __syncthreads();
   if (seg < 2) {
-    const float tot = s_sum[seg][0] + s_sum[seg][1];
-    const float n = rsqrtf(tot + 1e-6f) * (seg == 0 ? rsqrtf((float)D) : 1.f);
-    float* dst = (seg == 0 ? p.qn : p.kn) + ((size_t)t * p.Hk + hk) * D + d;
-    *reinterpret_cast<float2*>(dst) = make_float2(y0 * n, y1 * n);
-  } else {
-    *reinterpret_cast<float2*>(p.v + ((size_t)t * p.Hv + h) * D + d) = make_float2(y0, y1);
-    if (d == 0) {
-      float gg = 0.f, bb = 0.f;
-      if (t < p.T) {
-        const bf16* row = p.proj + (size_t)t * p.ld;
-        const float a = __bfloat162float(row[2 * KD + 2 * VD + h]);
-        const float b = __bfloat162float(row[2 * KD + 2 * VD + p.Hv + h]);
-        gg = -__expf(p.A_log[h]) * softplusf_(a + p.dt_bias[h]);
-        bb = sigmoidf_(b);
-      }
-      p.g[(size_t)t * p.Hv + h] = gg;
-      p.beta[(size_t)t * p.Hv + h] = bb;
+    float* dst = seg == 0 ? p.qn : p.kn;
+#pragma unroll
+    for (int i = 0; i < kPrepTokens; ++i) {
+      const float n = rsqrtf(s_sum[i][seg][0] + s_sum[i][seg][1] + 1e-6f) * (seg == 0 ? rsqrtf((float)D) : 1.f);
+      *reinterpret_cast<float2*>(dst + ((size_t)(t0 + i) * p.Hk + hk) * D + d) = make_float2(y[i].x * n, y[i].y * n);
     }
   }
 }
@@ -482,7 +495,7 @@ PK_API int pk_deltanet_chunked(const void* proj, int ld, int T, int key_heads, i
 
   PrepParams pp{(const pk::bf16*)proj, ld, T, Tpad, key_heads, value_heads, conv_w, conv_state, A_log, dt_bias,
                 qn, kn, v, g, beta};
-  PK_LAUNCH_PDL(deltanet_prep_kernel, dim3(Tpad, key_heads), dim3(64 * (2 + rep)), 0, stream, pp);
+  PK_LAUNCH_PDL(deltanet_prep_kernel, dim3(Tpad / kPrepTokens, key_heads), dim3(64 * (2 + rep)), 0, stream, pp);
   PK_CHECK_LAUNCH();
   const int channels = (2 * key_heads + value_heads) * D;
   PK_LAUNCH_PDL(deltanet_tail_kernel, dim3((channels + 255) / 256), dim3(256), 0, stream, (const pk::bf16*)proj, ld, T, channels, conv_state);
