@@ -1,15 +1,20 @@
 // Causal GQA attention for prefill chunks on the 5th-generation tensor cores.
 //
-// One CTA works one (query head, tile of 128 query rows). For every tile of 128 cached positions up to the causal limit:
-//   S  = Q K^T          tcgen05.mma kind::f16, both operands K-major (head dim contiguous), fp32 S in TMEM
-//   P  = exp2(S - m)    four softmax warps, one query row per thread: tcgen05.ld, mask, running max / sum, bf16 P written
-//                       into shared memory in the K-major 128-byte-swizzle operand layout
-//   PV = P V            tcgen05.mma with V as an MN-major operand (the cache stores a position's 128 channels
-//                       contiguously, which is the MN direction of this product), fresh accumulator in TMEM
-//   O  = O * alpha + PV folded into fp32 registers of the softmax warps (the same hand-over as the FP8 GEMM's k blocks)
-// K and V tiles arrive by TMA (no multicast) into two alternating buffers, the next tile's loads in flight during the
-// current tile's arithmetic. The output is divided by the row sum, gated (sigmoid of the projection's gate half) and
-// written as bf16.
+// One CTA works one (query head, tile of 128 query rows). For every 64 cached positions up to the causal limit:
+//   S  = Q K^T          tcgen05.mma kind::f16, both operands K-major (head dim contiguous), fp32 S in TMEM (two buffers: S of the next
+//                       step is computed while the softmax warps work on this one)
+//   P  = exp2(S - m)    four softmax warps, one query row per thread: tcgen05.ld, mask, maximum, exponentials; bf16 P goes to the
+//                       columns that S had, from where the next product takes it
+//   O += P V            V as an MN-major operand (the cache stores a position's 128 channels contiguously, which is the MN direction
+//                       of this product), O in TMEM. The reference m of a row only moves when its maximum has grown by more than a
+//                       factor of 2^8; its warp then rescales O in TMEM
+// K and V arrive by TMA (no multicast) into two alternating buffers each. Two CTAs are resident per SM (98 KB of shared and half of the tensor
+// memory each): one's products run under the other's softmax. The output is divided by the row sum, gated (sigmoid of the projection's
+// gate half) and written as bf16.
+//
+// Bound by the softmax (16 exponentials a cycle and SM). 1500 rows of 48 heads 155 -> 43 us, 441 rows of 40 heads behind 2560 positions 219 -> 65.
+// (Before: one CTA per SM, one tile of 128 positions after the other through S, softmax with P through shared memory, P V and a fold of every
+// tile's output into registers.)
 //
 // Every wait is bounded (status word + CTA-wide abort flag).
 //
@@ -23,11 +28,13 @@ using namespace pk;
 using namespace pk::sm100;
 
 constexpr int kD = 128;
-constexpr int kTile = 128;
-constexpr int kPanel = kTile * 128;        // bytes of one 64-element-wide panel of a 128-row bf16 tile
-constexpr int kTileBytes = 2 * kPanel;     // 32 KB
-constexpr int kThreads = 32 + 128;         // warp 0: TMA + MMA issue; warps 1-4: softmax, fold, epilogue
-constexpr uint32_t kTmemCols = 256;        // S and PV, 128 fp32 columns each
+constexpr int kTile = 128;                 // query rows
+constexpr int kKV = 64;                    // positions of a step
+constexpr int kQPanel = kTile * 128;       // bytes of one 64-element-wide panel of the query tile
+constexpr int kKPanel = kKV * 128;
+constexpr int kThreads = 64 + 128;         // warp 0: MMA issue; warp 1: TMA; warps 2-5: softmax, epilogue
+constexpr uint32_t kTmemCols = 256;        // S in two buffers of 64 columns, O
+constexpr float kSlack = 8.f;              // log2 of how far a row's maximum may run ahead of its reference
 
 struct Params {
   int M, Hq, Hkv, cap;
@@ -40,11 +47,10 @@ struct Params {
 };
 
 struct __align__(1024) Smem {
-  uint8_t q[kTileBytes];
-  uint8_t k[2][kTileBytes];
-  uint8_t v[2][kTileBytes];
-  uint8_t p[kTileBytes];
-  uint64_t q_full, kv_full[2], s_full, p_ready, pv_full;
+  uint8_t q[2 * kQPanel];
+  uint8_t k[2][2 * kKPanel];
+  uint8_t v[2][2 * kKPanel];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_full[2];
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
 };
@@ -61,26 +67,32 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t smem_addr, uint3
   return d;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
 gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         const Params p) {
   extern __shared__ uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, row0 = blockIdx.x * kTile;
+  const int h = blockIdx.x, row0 = (int)(gridDim.y - 1 - blockIdx.y) * kTile;      // the last rows see most: they go first
   const int kvh = h / (p.Hq / p.Hkv);
-  // positions are consecutive: the last row of this tile decides how far the cache is read
-  const int pos0 = __ldg(p.pos);
-  const int last_row = min(row0 + kTile, p.M) - 1;
-  const int n_tiles = (pos0 + last_row) / kTile + 1;
 
   if (threadIdx.x == 0) {
     mbar_init(&sm.q_full, 1);
-    mbar_init(&sm.kv_full[0], 1);
-    mbar_init(&sm.kv_full[1], 1);
-    mbar_init(&sm.s_full, 1);
-    mbar_init(&sm.p_ready, 4);
-    mbar_init(&sm.pv_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sm.k_full[i], 1);
+      mbar_init(&sm.k_empty[i], 1);
+      mbar_init(&sm.v_full[i], 1);
+      mbar_init(&sm.v_empty[i], 1);
+      mbar_init(&sm.s_full[i], 1);
+      mbar_init(&sm.p_ready[i], 4);      // one per buffer: a warp can be a step ahead of the others
+      mbar_init(&sm.pv_full[i], 1);
+    }
     sm.abort_flag = 0;
     mbar_fence_init();
   }
@@ -91,147 +103,197 @@ gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_s = sm.tmem_base, tmem_pv = sm.tmem_base + 128;
+  pk::pdl_wait();
+  pk::pdl_trigger();
+  const uint32_t tmem_s = sm.tmem_base, tmem_o = sm.tmem_base + 2 * kKV;
+  // positions are consecutive: the last row of this tile decides how far the cache is read
+  const int pos0 = p.pos[0];
+  const int last_row = min(row0 + kTile, p.M) - 1;
+  const int n_steps = (pos0 + last_row) / kKV + 1;
 
-  if (warp == 0) {
+  if (warp == 1) {
+    // ---------------- TMA producer ----------------
     if (lane == 0) {
       tma_prefetch_desc(&tmap_q);
       tma_prefetch_desc(&tmap_k);
       tma_prefetch_desc(&tmap_v);
-      auto load_kv = [&](int t) {
-        const int b = t & 1;
-        mbar_arrive_expect_tx(&sm.kv_full[b], 2 * kTileBytes);
-        const int y = kvh * p.cap + t * kTile;
-        tma_load_2d(sm.k[b], &tmap_k, &sm.kv_full[b], 0, y);
-        tma_load_2d(sm.k[b] + kPanel, &tmap_k, &sm.kv_full[b], 64, y);
-        tma_load_2d(sm.v[b], &tmap_v, &sm.kv_full[b], 0, y);
-        tma_load_2d(sm.v[b] + kPanel, &tmap_v, &sm.kv_full[b], 64, y);
-      };
-      mbar_arrive_expect_tx(&sm.q_full, kTileBytes);
-      tma_load_2d(sm.q, &tmap_q, &sm.q_full, h * kD, row0);
-      tma_load_2d(sm.q + kPanel, &tmap_q, &sm.q_full, h * kD + 64, row0);
-      load_kv(0);
-      constexpr uint32_t idesc_s = umma_idesc(1, 1, kTile, kTile);                  // bf16 x bf16, both K-major
-      constexpr uint32_t idesc_pv = umma_idesc(1, 1, kTile, kD) | (1u << 16);       // B (= V) MN-major
-      bool ok = mbar_wait(&sm.q_full, 0, &sm.abort_flag, p.status, 41);
-      int issued = 1;     // K/V tiles whose loads were issued
-      for (int t = 0; t < n_tiles && ok; ++t) {
-        const int b = t & 1;
-        if (!mbar_wait(&sm.kv_full[b], (t >> 1) & 1, &sm.abort_flag, p.status, 42)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sm.q), ka = smem_u32(sm.k[b]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          umma_f16(tmem_s, smem_desc_k_sw128(qa + (j >> 2) * kPanel + (j & 3) * 32), smem_desc_k_sw128(ka + (j >> 2) * kPanel + (j & 3) * 32), idesc_s, j > 0 ? 1u : 0u);
-        umma_commit(&sm.s_full);
-        // the other buffer was last read by the PV product of tile t - 1, whose completion the loop waited for below
-        if (t + 1 < n_tiles) {
-          load_kv(t + 1);
-          issued = t + 2;
-        }
-        if (!mbar_wait(&sm.p_ready, t & 1, &sm.abort_flag, p.status, 43)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t pa = smem_u32(sm.p), va = smem_u32(sm.v[b]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          umma_f16(tmem_pv, smem_desc_k_sw128(pa + (j >> 2) * kPanel + (j & 3) * 32), smem_desc_mn_sw128(va + j * 2048, kPanel, 1024), idesc_pv, j > 0 ? 1u : 0u);
-        umma_commit(&sm.pv_full);
-        // S of the next tile overwrites the S columns (read before p_ready), its loads reuse this tile's buffers only
-        // after the PV product is done
-        if (!mbar_wait(&sm.pv_full, t & 1, &sm.abort_flag, p.status, 44)) { ok = false; break; }
+      mbar_arrive_expect_tx(&sm.q_full, 2 * kQPanel);
+      for (int i = 0; i < 4; ++i) tma_load_2d(sm.q + i * kQPanel / 2, &tmap_q, &sm.q_full, h * kD + (i >> 1) * 64, row0 + (i & 1) * kKV);
+      int k_issued = 0, v_issued = 0;
+      for (int t = 0; t < n_steps; ++t) {
+        const int b = t & 1, y = kvh * p.cap + t * kKV;
+        if (t >= 2 && !mbar_wait(&sm.k_empty[b], ((t - 2) >> 1) & 1, &sm.abort_flag, p.status, 41)) break;
+        mbar_arrive_expect_tx(&sm.k_full[b], 2 * kKPanel);
+        tma_load_2d(sm.k[b], &tmap_k, &sm.k_full[b], 0, y);
+        tma_load_2d(sm.k[b] + kKPanel, &tmap_k, &sm.k_full[b], 64, y);
+        k_issued = t + 1;
+        if (t >= 2 && !mbar_wait(&sm.v_empty[b], ((t - 2) >> 1) & 1, &sm.abort_flag, p.status, 42)) break;
+        mbar_arrive_expect_tx(&sm.v_full[b], 2 * kKPanel);
+        tma_load_2d(sm.v[b], &tmap_v, &sm.v_full[b], 0, y);
+        tma_load_2d(sm.v[b] + kKPanel, &tmap_v, &sm.v_full[b], 64, y);
+        v_issued = t + 1;
       }
-      if (!ok) {
-        // gave up: let the tile loads in flight land before the CTA exits
-        for (int t = max(issued - 2, 0); t < issued; ++t)
+      if (sm.abort_flag) {
+        // gave up: let the loads in flight land before the CTA exits
+        for (uint32_t i = 0; i < (1u << 20); ++i)
+          if (mbar_try_wait(&sm.q_full, 0)) break;
+        for (int t = max(k_issued - 2, 0); t < k_issued; ++t)
           for (uint32_t i = 0; i < (1u << 20); ++i)
-            if (mbar_try_wait(&sm.kv_full[t & 1], (t >> 1) & 1)) break;
+            if (mbar_try_wait(&sm.k_full[t & 1], (t >> 1) & 1)) break;
+        for (int t = max(v_issued - 2, 0); t < v_issued; ++t)
+          for (uint32_t i = 0; i < (1u << 20); ++i)
+            if (mbar_try_wait(&sm.v_full[t & 1], (t >> 1) & 1)) break;
       }
     }
+    __syncwarp();
+  } else if (warp == 0) {
+    // ---------------- MMA issuer ----------------
+    // The whole warp walks the loop and one lane issues: addresses and descriptors are then uniform, which is what the
+    // instructions take.
+    constexpr uint32_t idesc_s = umma_idesc(1, 1, kTile, kKV);                    // bf16 x bf16, both K-major
+    constexpr uint32_t idesc_pv = umma_idesc(1, 1, kTile, kD) | (1u << 16);       // V MN-major
+    const uint64_t dq = smem_desc_k_sw128(smem_u32(sm.q)), dk = smem_desc_k_sw128(smem_u32(sm.k[0])), dv = smem_desc_mn_sw128(smem_u32(sm.v[0]), kKPanel, 1024);
+    const bool leader = elect_one();
+    auto issue_s = [&](int t) {
+      const uint32_t b = t & 1;
+      if (leader) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          umma_f16(tmem_s + b * kKV, dq + ((j >> 2) * kQPanel + (j & 3) * 32 >> 4), dk + b * (2 * kKPanel >> 4) + ((j >> 2) * kKPanel + (j & 3) * 32 >> 4), idesc_s,
+                   j > 0 ? 1u : 0u);
+        umma_commit(&sm.s_full[b]);
+        if (t + 2 < n_steps) umma_commit(&sm.k_empty[b]);
+      }
+      __syncwarp();
+    };
+    bool ok = mbar_wait_uniform(&sm.q_full, 0, &sm.abort_flag, p.status, 43) && mbar_wait_uniform(&sm.k_full[0], 0, &sm.abort_flag, p.status, 44);
+    if (ok) {
+      tc_fence_after();
+      issue_s(0);
+    }
+    for (int t = 0; t < n_steps && ok; ++t) {
+      const uint32_t b = t & 1;
+      if (t + 1 < n_steps) {
+        // the S buffer of step t + 1 is free when the product with the weights of step t - 1 is done
+        if ((t > 0 && !mbar_wait_uniform(&sm.pv_full[b ^ 1], ((t - 1) >> 1) & 1, &sm.abort_flag, p.status, 45)) ||
+            !mbar_wait_uniform(&sm.k_full[b ^ 1], ((t + 1) >> 1) & 1, &sm.abort_flag, p.status, 46))
+          break;
+        tc_fence_after();
+        issue_s(t + 1);
+      }
+      if (!mbar_wait_uniform(&sm.v_full[b], (t >> 1) & 1, &sm.abort_flag, p.status, 47) || !mbar_wait_uniform(&sm.p_ready[b], (t >> 1) & 1, &sm.abort_flag, p.status, 48)) break;
+      tc_fence_after();
+      if (leader) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          umma_f16_ts(tmem_o, tmem_s + b * kKV + j * 8, dv + b * (2 * kKPanel >> 4) + (j * 2048 >> 4), idesc_pv, t > 0 || j > 0 ? 1u : 0u);
+        umma_commit(&sm.pv_full[b]);
+        if (t + 2 < n_steps) umma_commit(&sm.v_empty[b]);
+      }
+      __syncwarp();
+    }
   } else {
+    // ---------------- softmax ----------------
     const int q4 = warp & 3;                       // TMEM lane quarter of this warp
     const int r = q4 * 32 + lane;                  // query row inside the tile
     const int m = row0 + r;
     const bool row_ok = m < p.M;
     const int q_pos = pos0 + (row_ok ? m : p.M - 1);
-    const uint32_t lane_off = (uint32_t)(q4 * 32) << 16;
-    float o[kD];
-#pragma unroll
-    for (int i = 0; i < kD; ++i) o[i] = 0.f;
-    float mx = -INFINITY, sum = 0.f;
+    const uint32_t lane_off = (uint32_t)(q4 * 32) << 16, ts = tmem_s + lane_off, to = tmem_o + lane_off;
+    float ref = -INFINITY, sum = 0.f;              // the row's reference (log2 units) and the sum of its weights
     bool ok = true;
-    for (int t = 0; t < n_tiles && ok; ++t) {
-      if (!mbar_wait(&sm.s_full, t & 1, &sm.abort_flag, p.status, 45)) { ok = false; break; }
+    for (int t = 0; t < n_steps; ++t) {
+      if (!mbar_wait_warp(&sm.s_full[t & 1], (t >> 1) & 1, &sm.abort_flag, p.status, 49)) {
+        ok = false;
+        break;
+      }
       tc_fence_after();
-      const int kv0 = t * kTile;
-      // pass 1: the row's maximum over the positions it may see
-      float tmax = -INFINITY;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t s[32];
-        tmem_ld_32x32(tmem_s + lane_off + c * 32, s);
-        tmem_ld_wait();
+      uint32_t s[2][32];
+      tmem_ld_32x32(ts + (t & 1) * kKV, s[0]);
+      tmem_ld_32x32(ts + (t & 1) * kKV + 32, s[1]);
+      tmem_ld_wait();
+      const int c_hi = q_pos - t * kKV;            // last visible column of this row in this step
+      if (__any_sync(0xffffffffu, c_hi < kKV - 1)) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (kv0 + c * 32 + i <= q_pos) tmax = fmaxf(tmax, __uint_as_float(s[i]));
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i > c_hi) s[c][i] = 0xff800000u;
       }
-      const float m_new = fmaxf(mx, tmax * p.scale_log2);
-      const float alpha = mx == -INFINITY ? 0.f : exp2f(mx - m_new);
-      const float base = m_new == -INFINITY ? 0.f : m_new;
-      // pass 2: probabilities, row sum, bf16 P into the operand layout
-      float tsum = 0.f;
+      float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t4[i & 3] = fmaxf(t4[i & 3], __uint_as_float(s[c][i]));
+      const float top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * p.scale_log2;
+      if (ref == -INFINITY) ref = top;             // nothing was visible so far: sum and O are zero
+      const bool grow = top > ref + kSlack;
+      if (__any_sync(0xffffffffu, grow)) {
+        const float alpha = grow ? exp2_approx(ref - top) : 1.f;
+        if (t > 0) {
+          if (!mbar_wait_warp(&sm.pv_full[(t - 1) & 1], ((t - 1) >> 1) & 1, &sm.abort_flag, p.status, 50)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t s[32];
-        tmem_ld_32x32(tmem_s + lane_off + c * 32, s);
-        tmem_ld_wait();
-        uint32_t packed[16];
+          for (int c = 0; c < kD / 32; ++c) {
+            uint32_t x[32];
+            tmem_ld_32x32(to + c * 32, x);
+            tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float a = kv0 + c * 32 + i <= q_pos ? exp2f(__uint_as_float(s[i]) * p.scale_log2 - base) : 0.f;
-          const float b2 = kv0 + c * 32 + i + 1 <= q_pos ? exp2f(__uint_as_float(s[i + 1]) * p.scale_log2 - base) : 0.f;
-          const __nv_bfloat162 pr = __floats2bfloat162_rn(a, b2);
-          // the sum runs over the rounded values, which are what the PV product multiplies
-          tsum += __bfloat162float(pr.x) + __bfloat162float(pr.y);
-          packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&pr);
+            for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(__uint_as_float(x[i]) * alpha);
+            tmem_st_32x32(to + c * 32, x);
+          }
+          tmem_st_wait();
         }
-        uint8_t* prow = sm.p + (c >> 1) * kPanel + r * 128;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int chunk = ((c & 1) * 4 + g) ^ (r & 7);
-          *reinterpret_cast<uint4*>(prow + chunk * 16) = make_uint4(packed[g * 4], packed[g * 4 + 1], packed[g * 4 + 2], packed[g * 4 + 3]);
-        }
+        sum *= alpha;
+        if (grow) ref = top;
       }
-      sum = sum * alpha + tsum;
-      mx = m_new;
-      // P is complete for this warp's rows and S has been read: let the MMA thread go on
-      fence_proxy_async_smem();
+      const float mb = ref == -INFINITY ? 0.f : ref;
+      float u4[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t w[32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(exp2_approx(fmaf(__uint_as_float(s[c][2 * e]), p.scale_log2, -mb)),
+                                                          exp2_approx(fmaf(__uint_as_float(s[c][2 * e + 1]), p.scale_log2, -mb)));
+          const uint32_t b2 = *reinterpret_cast<const uint32_t*>(&pr);
+          // the sum runs over the rounded values, which are what the product multiplies
+          u4[e & 3] += __uint_as_float(b2 << 16) + __uint_as_float(b2 & 0xffff0000u);
+          w[c * 16 + e] = b2;
+        }
+      sum += (u4[0] + u4[1]) + (u4[2] + u4[3]);
+      tmem_st_32x32(ts + (t & 1) * kKV, w);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.p_ready);
-      if (!mbar_wait(&sm.pv_full, t & 1, &sm.abort_flag, p.status, 46)) { ok = false; break; }
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t pv[32];
-        tmem_ld_32x32(tmem_pv + lane_off + c * 32, pv);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], alpha, __uint_as_float(pv[i]));
-      }
-      tc_fence_before();
+      if (lane == 0) mbar_arrive(&sm.p_ready[t & 1]);
     }
-    if (ok && row_ok) {
-      const float inv = sum > 0.f ? 1.f / sum : 0.f;
-      bf16* dst = p.out + (size_t)m * p.Hq * kD + h * kD;
-      const bf16* g = p.gate ? p.gate + (size_t)m * p.ld + h * 2 * kD + kD : nullptr;
+    // Of the products before the last only those up to the third last are known to be complete here: with a barrier for
+    // even and one for odd steps that is the phase before the one waited for.
+    if (ok && !mbar_wait_warp(&sm.pv_full[(n_steps - 1) & 1], ((n_steps - 1) >> 1) & 1, &sm.abort_flag, p.status, 51)) ok = false;
+    tc_fence_after();
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    bf16* dst = p.out + (size_t)m * p.Hq * kD + h * kD;
+    const bf16* g = p.gate ? p.gate + (size_t)m * p.ld + h * 2 * kD + kD : nullptr;
+#pragma unroll 1
+    for (int c = 0; c < kD / 32; ++c) {
+      uint32_t x[32];
+      tmem_ld_32x32(to + c * 32, x);      // all lanes of the warp take part
+      tmem_ld_wait();
+      if (!ok || !row_ok) continue;
+      uint4 gg[4];
 #pragma unroll
-      for (int v = 0; v < 16; ++v) {
+      for (int v = 0; v < 4; ++v) gg[v] = g ? *reinterpret_cast<const uint4*>(g + c * 32 + v * 8) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
         float f[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = o[v * 8 + e] * inv;
+        for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(x[v * 8 + e]) * inv;
         if (g) {
-          const uint4 gg = *reinterpret_cast<const uint4*>(g + v * 8);
-          const uint32_t w[4] = {gg.x, gg.y, gg.z, gg.w};
+          const uint32_t w[4] = {gg[v].x, gg[v].y, gg[v].z, gg[v].w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             f[2 * e] *= 1.f / (1.f + __expf(-__uint_as_float(w[e] << 16)));
@@ -244,7 +306,7 @@ gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           const __nv_bfloat162 pr = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
           o4[e] = *reinterpret_cast<const uint32_t*>(&pr);
         }
-        *reinterpret_cast<uint4*>(dst + v * 8) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+        *reinterpret_cast<uint4*>(dst + c * 32 + v * 8) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
       }
     }
   }
@@ -275,7 +337,7 @@ EncodeTiledFn encode_fn() {
 bool encode_rows(EncodeTiledFn encode, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer) {
   const cuuint64_t gdim[2] = {inner, outer};
   const cuuint64_t gstride[1] = {inner * 2};
-  const cuuint32_t box[2] = {64, kTile};
+  const cuuint32_t box[2] = {64, kKV};
   const cuuint32_t estr[2] = {1, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -308,7 +370,7 @@ PK_API int pk_gqa_prefill_umma(const void* q, const void* kcache, const void* vc
     }
     once_guard.done();
   }
-  gqa_prefill_umma_kernel<<<dim3((M + kTile - 1) / kTile, Hq), kThreads, smem, stream>>>(tq, tk, tv, p);
+  PK_LAUNCH_PDL(gqa_prefill_umma_kernel, dim3(Hq, (M + kTile - 1) / kTile), dim3(kThreads), smem, stream, tq, tk, tv, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

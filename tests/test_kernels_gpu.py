@@ -605,6 +605,35 @@ def test_gqa_prefill_tensor_core_attention_matches_fp32(M, pos0, Hq, Hkv):
     assert _rel_err(gated, simt) < 1e-2
 
 
+@pytest.mark.parametrize("M,pos0", [(1, 0), (64, 0), (65, 63), (129, 0), (130, 64), (200, 191), (128, 704)])
+@pytest.mark.parametrize("growth", [0.0, 0.4, -0.4])
+def test_gqa_prefill_with_maxima_that_move(M, pos0, growth):
+    """Steps of 64 positions around 1, 2, 3 .. of them, and keys that grow or shrink along the context, so that the reference of a row
+    moves in every step, in some, or never. Weights are rounded to bf16 before the sum and the product (2^-9 each, in numerator
+    and denominator) and so is the output: |error| <= 2^-8 (sum of p |v| + |result|)."""
+    from pocketllm_b200 import ops
+    torch.manual_seed(M + pos0)
+    D, cap, Hq, Hkv = 128, 1024, 4, 2
+    ctx = pos0 + M
+    kc = torch.zeros(Hkv, cap, D, device="cuda", dtype=torch.bfloat16)
+    vc = torch.zeros_like(kc)
+    ramp = torch.arange(ctx, device="cuda", dtype=torch.float32)[None, :, None] * growth / D ** 0.5
+    kc[:, :ctx] = (torch.randn(Hkv, ctx, D, device="cuda") + ramp).to(torch.bfloat16)
+    vc[:, :ctx] = torch.randn(Hkv, ctx, D, device="cuda").to(torch.bfloat16)
+    q = (torch.randn(M, Hq, D, device="cuda") * 0.5 + 0.7).to(torch.bfloat16)
+    pos = torch.arange(pos0, pos0 + M, device="cuda", dtype=torch.int32)
+    K, V = kc[:, :ctx].double().repeat_interleave(Hq // Hkv, 0), vc[:, :ctx].double().repeat_interleave(Hq // Hkv, 0)
+    sc = torch.einsum("mhd,htd->mht", q.double(), K) * D ** -0.5
+    pr = torch.softmax(sc.masked_fill(torch.arange(ctx, device="cuda")[None, None, :] > pos[:, None, None], float("-inf")), -1)
+    want, scale = torch.einsum("mht,htd->mhd", pr, V), torch.einsum("mht,htd->mhd", pr, V.abs())
+    for _ in range(3):
+        status = torch.zeros(1, device="cuda", dtype=torch.int32)
+        got = ops.gqa_prefill(q, kc, vc, pos, status=status)
+        torch.cuda.synchronize()
+        assert status.item() == 0
+        assert ((got.view(M, Hq, D).double() - want).abs() <= 2 ** -8 * (scale + want.abs()) + 1e-6).all()
+
+
 def test_full_qk_norm_rope_append_matches_torch():
     """Whole-vector RMS (one gamma per element) + half-split rotation from tables + KV append, against plain PyTorch."""
     from pocketllm_b200 import ops

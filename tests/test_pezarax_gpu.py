@@ -36,6 +36,68 @@ def oracle(cfg, t, seq, key):
 
 # ---- kernels ----
 
+@pytest.mark.parametrize("M,pos0", [(1, 0), (64, 0), (65, 63), (129, 0), (130, 64), (200, 191), (128, 704)])
+@pytest.mark.parametrize("maps,D,V,window,growth", [(1, 64, 64, 0, 0.4), (1, 128, 128, 100, 0.4), (2, 32, 48, 0, -0.4), (2, 96, 128, 65, 0.4), (1, 128, 200, 64, 0.0)])
+def test_long_portions_with_maxima_that_move(M, pos0, maps, D, V, window, growth):
+    """Steps of 64 positions around 1, 2, 3 .. of them, and keys that grow or shrink along the context, so that the reference of a row
+    moves in every step, in some, or never; sinks that count and one without weight. Weights are sums of two bf16 terms (2^-17 left) and
+    finished outputs are rounded to bf16; scores are sums in fp32, a few 2^-23 of the largest s, in numerator and denominator:
+    |error| <= 2^-8 |result| + (2^-15 + 2^-20 max |s|) sum of p |v|."""
+    from pocketllm_b200.ops import mixer_ops as mo
+    torch.manual_seed(M + D)
+    H, G, lam, dev = 4, 2, 0.4, "cuda"
+    ctx, up8 = pos0 + M, lambda n: (n + 7) // 8 * 8
+    dp, vp, q_ld = up8(D), up8(V), (D + 63) // 64 * 64
+    row, pages = G * (maps * dp + vp), (ctx + 63) // 64 + 2
+    ramp = torch.arange(ctx, device=dev, dtype=torch.float32)[:, None, None] * growth / D ** 0.5
+    k = (torch.randn(ctx, G * maps, D, device=dev) + ramp).to(torch.bfloat16)
+    v = torch.randn(ctx, G, V, device=dev).to(torch.bfloat16)
+    q = (torch.randn(M, H * maps, D, device=dev) * 0.5 + 0.7).to(torch.bfloat16)
+    table = torch.randperm(pages, device=dev).to(torch.int32)[None]
+    cache = torch.zeros(pages, 64, row, device=dev, dtype=torch.bfloat16)
+    t = torch.arange(ctx, device=dev)
+    flat = torch.zeros(ctx, row, device=dev, dtype=torch.bfloat16)
+    flat[:, :G * maps * dp].view(ctx, G * maps, dp)[..., :D] = k
+    flat[:, G * maps * dp:].view(ctx, G, vp)[..., :V] = v
+    cache[table[0, t // 64].long(), t % 64] = flat
+    qf = torch.zeros(M, H * maps, q_ld, device=dev, dtype=torch.bfloat16)
+    qf[..., :D] = q
+    sink = torch.randn(H * maps, device=dev)
+    sink[1] = float("-inf")
+    pos = torch.arange(pos0, ctx, device=dev, dtype=torch.int32)
+    K = k.double().view(ctx, G, maps, D).repeat_interleave(H // G, 1)
+    sc = torch.einsum("mhad,thad->mhat", q.double().view(M, H, maps, D), K) * D ** -0.5
+    mask = t[None] > pos[:, None]
+    if window:
+        mask = mask | (t[None] <= pos[:, None] - window)
+    sc = torch.cat((sc.masked_fill(mask[:, None, None], float("-inf")), sink.double().view(1, H, maps, 1).expand(M, -1, -1, -1)), -1)
+    pr_ = torch.softmax(sc, -1)[..., :-1]
+    rel = 2 ** -15 + 2 ** -20 * sc[sc > float("-inf")].abs().max()
+    VV = v.double().repeat_interleave(H // G, 1)
+    form = mo.paged_prefill_form(maps, D, V)
+    comb = torch.tensor([1.0, -lam][:maps], device=dev, dtype=torch.float64)
+    if form == 0:
+        want, size = (torch.einsum("mhat,thv->mhav", pr_, x) for x in (VV, VV.abs()))
+    else:
+        want, size = (torch.einsum("mhat,thv,a->mhv", pr_, x, c) for x, c in ((VV, comb), (VV.abs(), comb.abs())))
+    n = (M + 127) // 128
+    tiles = torch.tensor([[128 * i, min(128, M - 128 * i), 0, 0] for i in range(n)], device=dev, dtype=torch.int32)
+    seqs = torch.tensor([[0, M, 0, pos0]], device=dev, dtype=torch.int32)
+    out = torch.empty(M, H * V, device=dev, dtype=torch.bfloat16)
+    part = torch.empty(M, H * maps, V, device=dev)
+    status = torch.zeros(1, device=dev, dtype=torch.int32)
+    slot = torch.zeros(M, device=dev, dtype=torch.int32)
+    d = mo.PagedAttention(pos=pos.data_ptr(), slot=slot.data_ptr(), table=table.data_ptr(), table_ld=pages, cache=cache.data_ptr(), qf=qf.data_ptr(), q_ld=q_ld,
+                          out=out.data_ptr(), ldo=H * V, width=H * V, status=status.data_ptr(), sink=sink.data_ptr(), H=H, G=G, maps=maps, D=D, V=V, dp=dp, vp=vp,
+                          row=row, window=window, gate=-1, nsplit=1, scale=D ** -0.5, lambda_=lam, post=1.0, part_o=part.data_ptr() if form == 0 else 0)
+    for _ in range(3):
+        mo.paged_prefill(d, M, pages, tiles, n, seqs)
+        torch.cuda.synchronize()
+        assert status.item() == 0
+        got = (part if form == 0 else out).double().view(want.shape)
+        assert ((got - want).abs() <= 2 ** -8 * want.abs() + rel * size + 1e-6).all()
+
+
 @pytest.mark.parametrize("W", [24, 300, 2048])
 def test_residual_steps_without_post_norm(W):
     """Plain addition of a sublayer's output, of the sum of a token's expert rows, of the scaled embedding row."""
