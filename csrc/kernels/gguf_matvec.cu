@@ -10,6 +10,8 @@
 // q2_k 1, iq1_m 2, q4_k 3, q5_k 4, iq2_xs 5, iq3_xxs 6, iq4_xs 7, q6_k 8, plus q8_0 9 and
 // bf16 10 here. Replaces its DP4A / float kernels (src/csrc/cuda_kernel_impl.cu:6545-6632,
 // 7039-8275: gguf_quant_gemm*, gguf_moe_w13*, gguf_moe_w2*, gguf_moe_single_*).
+#include <cooperative_groups.h>
+#include <algorithm>
 #include <mutex>
 
 #include "../common/pk_common.cuh"
@@ -553,68 +555,173 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
   }
 }
 
-// The same for many tokens: a block has 16 tokens x 64 experts, four groups of 128 threads take a quarter of the K steps each and
-// add up in their order; a thread has 2 x 4 sums, four values of K at a time (shared-memory reads and multiply-adds then take about
-// as long). 1500 tokens of 3072 by 256 experts: 361 -> 183 us (the form above, which reads the router's rows once per 8 tokens, 279).
-// The sums are added in another order than above.
-constexpr int kRt = 16, kRe = 64, kRk = 32;
-__global__ void __launch_bounds__(512) router_logits_tile_kernel(const bf16* __restrict__ x, const float* __restrict__ rw, int H, int E, int T, float* logits) {
-  pk::pdl_wait_for(x);
-  pk::pdl_trigger();
-  __shared__ __align__(16) float ws[4][kRe][kRk + 4];
-  __shared__ __align__(16) float xs[4][kRt][kRk + 4];
-  const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, tx = t & 15, ty = t >> 4;      // experts tx + 16 j, tokens 2 ty ..
-  const int t0 = blockIdx.y * kRt, e0 = blockIdx.x * kRe;
-  float acc[2][4] = {};
-  const int steps = (H + kRk - 1) / kRk;
-  float wn[16], xn[4];      // the next step's share of the tiles, on its way while this one is multiplied
-  auto fetch = [&](int s) {
-    const int k = s * kRk + (t & 31);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int r = e0 + (t >> 5) + 4 * i;
-      wn[i] = s < steps && r < E && k < H ? __ldg(rw + (size_t)r * H + k) : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = t0 + (t >> 5) + 4 * i;
-      xn[i] = s < steps && r < T && k < H ? __bfloat162float(x[(size_t)r * H + k]) : 0.f;
+// The same for many tokens: a block has 64 tokens x 64 experts, a thread 8 x 8 sums: 16 reads of shared memory then feed 128
+// multiply-adds, which bound it. Four groups of 64 threads take a quarter of every 64 values of K each; where the tiles leave SMs idle the
+// blocks of a cluster take a part of K each. All add up in their order (another one than above). The router's rows of the first
+// steps are requested before the predecessor is complete. A row that cannot be copied by 16 bytes is loaded by elements (V = false).
+// 1500 tokens of 3072 by 256 experts: 73 us (2 x 4 sums a thread, 16 tokens a block: 174; the form above, which reads
+// the router's rows once per 8 tokens, 279). 56 % of the rate of fp32 multiply-adds, with one or two blocks on an SM alike.
+constexpr int kRt = 64, kRe = 64, kRk = 64, kRs = 3;      // tile, values of K per step, steps in shared memory
+constexpr int kRw = kRk + 4, kRx = kRk + 8, kRo = kRe + 8;      // pitches: rows of eight consecutive threads start in different banks
+constexpr int kRouterSmem = kRs * (kRe * kRw * 4 + kRt * kRx * 2);
+static_assert(4 * kRt * kRo * 4 <= kRouterSmem, "the groups' sums take the place of the tiles");
+template <bool V>
+__global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* x, const float* rw, int H, int E, int T, float* logits) {
+  extern __shared__ __align__(16) uint8_t router_smem[];
+  float* ws = reinterpret_cast<float*>(router_smem);                            // [kRs][kRe][kRw]
+  bf16* xs = reinterpret_cast<bf16*>(router_smem + kRs * kRe * kRw * 4);        // [kRs][kRt][kRx]
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int parts = gridDim.x, part = blockIdx.x;      // a cluster is one tile
+  const int tid = threadIdx.x, lane = tid & 31, grp = tid >> 6, tx = lane & 7, ty = (lane >> 3) + 4 * ((tid >> 5) & 1);
+  const int e0 = blockIdx.y * kRe, t0 = blockIdx.z * kRt;
+  const int steps = (H + kRk - 1) / kRk, per = (steps + parts - 1) / parts;
+  const int first = min(part * per, steps), n = min(per, steps - first);
+  auto fetch_w = [&](int i) {
+    float* dst = ws + (i % kRs) * kRe * kRw;
+    const int k0 = (first + i) * kRk;
+    if constexpr (V) {
+#pragma unroll 1
+      for (int c = tid; c < kRe * (kRk / 4); c += 256) {
+        const int r = c / (kRk / 4), k = (c & (kRk / 4 - 1)) * 4;
+        const bool in = e0 + r < E && k0 + k < H;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * kRw + k)),
+                     "l"(in ? rw + (size_t)(e0 + r) * H + k0 + k : rw), "r"(in ? 16 : 0) : "memory");
+      }
+    } else {
+      for (int c = tid; c < kRe * kRk; c += 256) {
+        const int r = c / kRk, k = c & (kRk - 1);
+        dst[r * kRw + k] = e0 + r < E && k0 + k < H ? rw[(size_t)(e0 + r) * H + k0 + k] : 0.f;
+      }
     }
   };
-  fetch(grp);
-  for (int s = grp; s - grp < steps; s += 4) {      // every group takes part in the barriers
+  auto fetch_x = [&](int i) {
+    bf16* dst = xs + (i % kRs) * kRt * kRx;
+    const int k0 = (first + i) * kRk;
+    if constexpr (V) {
+#pragma unroll 1
+      for (int c = tid; c < kRt * (kRk / 8); c += 256) {
+        const int r = c / (kRk / 8), k = (c & (kRk / 8 - 1)) * 8;
+        const bool in = t0 + r < T && k0 + k < H;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * kRx + k)),
+                     "l"(in ? x + (size_t)(t0 + r) * H + k0 + k : x), "r"(in ? 16 : 0) : "memory");
+      }
+    } else {
+      for (int c = tid; c < kRt * kRk; c += 256) {
+        const int r = c / kRk, k = c & (kRk - 1);
+        dst[r * kRx + k] = t0 + r < T && k0 + k < H ? x[(size_t)(t0 + r) * H + k0 + k] : __float2bfloat16(0.f);
+      }
+    }
+  };
+  for (int i = 0; i < kRs - 1; ++i)
+    if (i < n) fetch_w(i);
+  pk::pdl_wait_for(x);
+  pk::pdl_trigger();
+  for (int i = 0; i < kRs - 1; ++i) {
+    if (i < n) fetch_x(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float2 acc[4][8] = {};      // tokens ty + 16 m and ty + 16 m + 8
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRs - 2) : "memory");
     __syncthreads();
+    if (i + kRs - 1 < n) {      // into the buffer that all have read before this barrier
+      fetch_w(i + kRs - 1);
+      fetch_x(i + kRs - 1);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* w = ws + (i % kRs) * kRe * kRw + tx * kRw + grp * 16;
+    const bf16* a = xs + (i % kRs) * kRt * kRx + ty * kRx + grp * 16;
+#pragma unroll 2
+    for (int k = 0; k < 16; k += 2) {      // two values at a time and no more unrolled: the sums would spill
+      float2 v[4][2];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) ws[grp][(t >> 5) + 4 * i][t & 31] = wn[i];
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t u = *reinterpret_cast<const uint32_t*>(a + m * 16 * kRx + k), l = *reinterpret_cast<const uint32_t*>(a + (m * 16 + 8) * kRx + k);
+        v[m][0] = make_float2(__uint_as_float(u << 16), __uint_as_float(l << 16));
+        v[m][1] = make_float2(__uint_as_float(u & 0xffff0000u), __uint_as_float(l & 0xffff0000u));
+      }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) xs[grp][(t >> 5) + 4 * i][t & 31] = xn[i];
-    fetch(s + 4);
-    __syncthreads();
-    if (s < steps) {
+      for (int j = 0; j < 8; ++j) {
+        const float2 b = *reinterpret_cast<const float2*>(w + j * 8 * kRw + k);
 #pragma unroll
-      for (int k = 0; k < kRk; k += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&xs[grp][ty * 2][k]), b = *reinterpret_cast<const float4*>(&xs[grp][ty * 2 + 1][k]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 w = *reinterpret_cast<const float4*>(&ws[grp][tx + 16 * j][k]);
-          acc[0][j] = fmaf(w.w, a.w, fmaf(w.z, a.z, fmaf(w.y, a.y, fmaf(w.x, a.x, acc[0][j]))));
-          acc[1][j] = fmaf(w.w, b.w, fmaf(w.z, b.z, fmaf(w.y, b.y, fmaf(w.x, b.x, acc[1][j]))));
-        }
+        for (int m = 0; m < 4; ++m) acc[m][j] = __ffma2_rn(make_float2(b.y, b.y), v[m][1], __ffma2_rn(make_float2(b.x, b.x), v[m][0], acc[m][j]));
       }
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  float* sums = &ws[0][0][0];      // [4][kRt][kRe]
+  float* sums = ws;      // [4][kRt][kRo]
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int m = 0; m < 4; ++m)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sums[(grp * kRt + ty * 2 + i) * kRe + tx + 16 * j] = acc[i][j];
+    for (int j = 0; j < 8; ++j) {
+      sums[(grp * kRt + ty + 16 * m) * kRo + tx + 8 * j] = acc[m][j].x;
+      sums[(grp * kRt + ty + 16 * m + 8) * kRo + tx + 8 * j] = acc[m][j].y;
+    }
   __syncthreads();
-  for (int o = threadIdx.x; o < kRt * kRe; o += 512) {
-    const int r = o / kRe, e = o - r * kRe;
-    if (t0 + r < T && e0 + e < E)
-      logits[(size_t)(t0 + r) * E + e0 + e] = (sums[o] + sums[kRt * kRe + o]) + (sums[2 * kRt * kRe + o] + sums[3 * kRt * kRe + o]);
+  for (int o = tid; o < kRt * kRe; o += 256) {
+    const int r = o / kRe, e = o - r * kRe, at = r * kRo + e;
+    const float v = (sums[at] + sums[kRt * kRo + at]) + (sums[2 * kRt * kRo + at] + sums[3 * kRt * kRo + at]);
+    if (parts > 1)
+      sums[at] = v;
+    else if (t0 + r < T && e0 + e < E)
+      logits[(size_t)(t0 + r) * E + e0 + e] = v;
   }
+  if (parts == 1) return;
+  cluster.sync();
+  for (int o = part * 256 + tid; o < kRt * kRe; o += parts * 256) {
+    const int r = o / kRe, e = o - r * kRe, at = r * kRo + e;
+    float v = *cluster.map_shared_rank(sums + at, 0);
+    for (int q = 1; q < parts; ++q) v += *cluster.map_shared_rank(sums + at, q);
+    if (t0 + r < T && e0 + e < E) logits[(size_t)(t0 + r) * E + e0 + e] = v;
+  }
+  cluster.sync();      // the last sums have been read
+}
+
+template <bool V>
+static int launch_router_tiles(const bf16* x, const float* rw, int H, int E, int T, int sms, float* logits, cudaStream_t stream) {
+  static PkDeviceOnce once;
+  if (PkDeviceOnceGuard g{once}; g.needed()) {
+    if (cudaFuncSetAttribute(router_logits_tile_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRouterSmem) != cudaSuccess) {
+      pk_set_last_cuda_error((int)cudaGetLastError());
+      return PK_ERR_CUDA;
+    }
+    g.done();
+  }
+  const int et = (E + kRe - 1) / kRe, tt = (T + kRt - 1) / kRt, steps = (H + kRk - 1) / kRk;
+  // A block alone keeps its SM as busy as two do, so the time is that of the fullest SM: blocks of it x (steps of a block + what a block
+  // costs besides, 2.5 steps). 256 experts of 3072, tiles with 1 / 2 / 4 / 8 parts, us (all measured with a form
+  // 10 % slower): 96 tiles 108 / 106 / 83 / 92, 64 tiles 107 / 60 / 57 / 64,
+  // 32 tiles 106 / 58 / 33 / 32, 256 tiles 200 / 204 / 208 / 219.
+  int parts = 1;
+  double best = 0.;
+  for (int c = 1; c <= 8 && c <= steps; c *= 2) {
+    const double cost = (double)(((long long)et * tt * c + sms - 1) / sms) * ((steps + c - 1) / c + 2.5);
+    if (c == 1 || cost < best) {
+      best = cost;
+      parts = c;
+    }
+  }
+  pk_prefer_max_smem((const void*)router_logits_tile_kernel<V>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(parts, et, tt);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = kRouterSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pk_pdl_enabled() ? 2 : 1;
+  if (const cudaError_t e = cudaLaunchKernelEx(&cfg, router_logits_tile_kernel<V>, x, rw, H, E, T, logits); e != cudaSuccess) {
+    pk_set_last_cuda_error((int)e);
+    return PK_ERR_CUDA;
+  }
+  return PK_OK;
 }
 
 // One block per token: scores from the logits, top-k with lowest-id tie break.
@@ -859,10 +966,14 @@ static float* router_scratch(size_t floats) {
   return buf[dev];
 }
 
-// A tile takes the time of its K steps however few there are, so the tiles pay when tokens x experts fill the SMs with them and an
-// expert tile is full. One warp per expert / tiles, us: 256 experts of 3072, 256 tokens 58 / 64, 384 tokens 84 / 64; 128 of 4096, 512 tokens 90 / 83;
-// 64 of 2048, 1024 tokens 41 / 44, 1500 tokens 56 / 48; 8 of 4096, 1500 tokens 33 / 83.
-static constexpr long long kRouterTileMin = 72000;
+// The blocks of the form with one warp per expert keep eight tokens of H floats each in shared memory; when they are more than are
+// resident at once, the tiles are faster, if an expert tile is full. One warp per expert / tiles, us: 256 experts of 3072 (256 blocks for
+// 64 tokens, 296 resident), 64 tokens 15 / 17, 96 tokens 28 / 17, 256 tokens 56 / 27; 128 of 4096 (148 resident), 64 tokens 13 / 21, 96 tokens
+// 27 / 21, 512 tokens 86 / 34; 64 of 2048 (444 resident), 384 tokens 13 / 13, 512 tokens 26 / 13.
+static bool router_tiles(int T, int E, int H, int sms) {
+  const long long resident = std::min(8, (227 * 1024) / (32 * H + 1024));
+  return E >= kRe && (long long)((E + 7) / 8) * ((T + 7) / 8) > resident * sms;
+}
 
 PK_API int pk_router_topk(const void* x, const float* router_w, const float* bias, int T, int H, int E, int topk,
                           int score_func, int norm_topk, float route_scale, int* ids, float* weights,
@@ -883,9 +994,14 @@ PK_API int pk_router_topk(const void* x, const float* router_w, const float* bia
   }
   float* logits = router_scratch((size_t)T * E);
   if (logits == nullptr) return PK_ERR_CUDA;
-  if (E >= kRe && (long long)T * E >= kRouterTileMin)
-    PK_LAUNCH_PDL(router_logits_tile_kernel, dim3((E + kRe - 1) / kRe, (T + kRt - 1) / kRt), dim3(512), 0, stream, (const pk::bf16*)x, router_w, H, E, T, logits);
-  else
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return PK_ERR_CUDA;
+  if (router_tiles(T, E, H, sms)) {
+    const bool v = (H & 7) == 0 && (((uintptr_t)x | (uintptr_t)router_w) & 15) == 0;
+    if (const int rc = v ? launch_router_tiles<true>((const pk::bf16*)x, router_w, H, E, T, sms, logits, stream)
+                         : launch_router_tiles<false>((const pk::bf16*)x, router_w, H, E, T, sms, logits, stream))
+      return rc;
+  } else
     PK_LAUNCH_PDL(router_logits_kernel, dim3((E + 7) / 8, (T + 7) / 8), dim3(256), smem_x, stream, (const pk::bf16*)x, router_w, H, E, T, logits);
   PK_CHECK_LAUNCH();
   PK_LAUNCH_PDL(router_topk_kernel, dim3(T), dim3(256), (size_t)2 * E * sizeof(float), stream, logits, bias, E, topk, score_func, norm_topk, route_scale, ids,

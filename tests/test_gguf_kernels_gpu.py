@@ -92,6 +92,26 @@ def test_router_topk(score, norm):
     assert torch.allclose(w, ref_w * 1.5, rtol=2e-3, atol=1e-5)
 
 
+@pytest.mark.parametrize("T,H,E", [(1024, 64, 96), (700, 3072, 64), (128, 3072, 128), (97, 4104, 96), (1500, 1001, 65), (257, 2052, 160)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_router_of_many_tokens(T, H, E, offset):
+    """Tiles of 64 x 64 with ragged edges, rows that cannot be copied by 16 bytes, parts of K in a cluster, against float64: fp32 sums of
+    H products are off by at most (H + 8) 2^-24 sum |x w|, a quarter of that behind the sigmoid, whose own error is a few 2^-24."""
+    from pocketllm_b200.ops import gguf_ops as go
+    torch.manual_seed(T + H)
+    x = torch.randn(T * H + offset, device="cuda").to(torch.bfloat16)[offset:].view(T, H)
+    rw = (torch.randn(E * H + offset, device="cuda") / H ** 0.5)[offset:].view(E, H)
+    logits, size = x.double() @ rw.double().t(), x.double().abs() @ rw.double().abs().t()
+    for e0 in range(0, E, 32):      # the bias selects 32 experts, whose scores come back
+        pick = torch.arange(e0, min(e0 + 32, E), device="cuda")
+        bias = torch.zeros(E, device="cuda")
+        bias[pick] = 8.0
+        ids, w = go.router_topk(x, rw, len(pick), bias=bias, score_func="sigmoid", norm_topk=False)
+        assert torch.equal(ids.long().sort(-1).values, pick.expand(T, -1))
+        want = torch.sigmoid(logits.gather(1, ids.long()))
+        assert ((w.double() - want).abs() <= 0.25 * (H + 8) * 2 ** -24 * size.gather(1, ids.long()) + 2 ** -20).all()
+
+
 @pytest.mark.parametrize("t13,t2,T", [("iq2_xxs", "q2_k", 1), ("iq2_xxs", "iq2_xxs", 40), ("iq1_m", "iq1_m", 9)])
 def test_moe_forward_matches_dequantised_reference(t13, t2, T):
     from pocketllm_b200.ops import gguf_ops as go
