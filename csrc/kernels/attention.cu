@@ -47,7 +47,6 @@ __global__ void __launch_bounds__(32 * kQkWarps) qk_norm_rope_append_kernel(cons
   const bf16* row = p.proj + (size_t)m * p.ld;
   const int pos = p.pos[m], hr = p.rotary_dim >> 1;
   const bool in_cache = pos >= 0 && pos < p.ctx_cap;
-  if (!in_cache && threadIdx.x == 0) PK_DEBUG_RECORD(101, pos, p.ctx_cap);   // the row is not written (below)
   for (int i = threadIdx.x; i < hr; i += 32 * kQkWarps) {
     const double inv_freq = pow((double)p.theta, -2.0 * (double)i / (double)p.rotary_dim);
     double sn, cs;
@@ -98,6 +97,7 @@ __global__ void __launch_bounds__(32 * kQkWarps) qk_norm_rope_append_kernel(cons
       store4(p.q_out + ((size_t)m * p.Hq + hh) * kD + d, y);
       continue;
     }
+    if (!in_cache && lane == 0) PK_DEBUG_RECORD(101, pos, p.ctx_cap);   // the row is not written (below)
     const float4 v4 = load4(row + p.Hq * 2 * kD + p.Hkv * kD + hk * kD + d);
     const float v[4] = {v4.x, v4.y, v4.z, v4.w};
     const size_t ri = (size_t)hk * p.ctx_cap + pos;
