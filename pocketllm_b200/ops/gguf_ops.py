@@ -27,13 +27,15 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
     `UMMA_TYPES` whose wait ran out gives NaN, and so does one that finds the word set; its owner reads the word once per step
     (`StepWord`) and clears it.
 
-    Up to `UMMA_MAX_ROWS - 1` rows of the types in `UMMA_TYPES` are decoded inside a tensor-core kernel, once per 64 rows.
+    Up to `UMMA_MAX_ROWS - 1` rows (of more than 2^24 weights `UMMA_MAX_ROWS_LARGE - 1`) of the types in `UMMA_TYPES` are decoded inside a
+    tensor-core kernel, once per 64 rows.
     Of the other types, up to `TENSOR_CORE_MIN_ROWS - 1` rows decode the blocks in registers (groups of up to 8 rows per
     launch). Above, the weight is decoded once into a bf16 scratch and the product runs on the tcgen05 GEMM (the
     reference switches to its prefill kernels for rows > 1, src/components/gguf/quantized_ops.py:9-76)."""
     M, K = x.shape
     ncols = N // 2 if epi == 1 else N
-    if 0 < M < UMMA_MAX_ROWS and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name, N, K) and not _registers_faster(type_name, M, N * K):
+    most = UMMA_MAX_ROWS if N * K <= 1 << 24 else UMMA_MAX_ROWS_LARGE
+    if 0 < M < most and K * 4 <= 200 * 1024 and _umma_takes(w_raw, type_name, N, K) and not _registers_faster(type_name, M, N * K):
         return _umma_linear(_aligned(x), w_raw, type_name, N, _aligned(gamma), eps, epi, status)
     if M >= TENSOR_CORE_MIN_ROWS and K % 64 == 0 and (epi != 1 or (N // 2) % 128 == 0):
         from . import gemm_bf16, rmsnorm, EPI_BF16, EPI_SWIGLU, EPI_F32
@@ -54,10 +56,11 @@ def gguf_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, *,
 
 # Block types whose integer part fits fp16: decoded inside the tensor-core kernel (`csrc/kernels/quant_umma.cu`)
 UMMA_TYPES = frozenset({"iq2_xxs", "q4_k", "q5_k"})
-# Rows of 8192 x 3072 / 3072 x 6144 / 24576 x 6144, us, against decoding per eight rows or (from 32 rows) to a bf16 scratch. Q5_K: 8 rows
-# 22 / 20 / 74 against 95 / 100 / 526, 64 rows 27 / 27 / 97 against 60 / 65 / 272, 256 rows 60 / 55 / 302 against 63 / 68 / 302;
-# IQ2_XXS, 256 rows: 51 / 48 / 252 against 52 / 59 / 244; Q4_K: 54 / 51 / 268 against 57 / 63 / 270.
-UMMA_MAX_ROWS = 257
+# Against decoding per eight rows or (from 32 rows) to a bf16 scratch, 4096 x 4096 / 8192 x 3072 / 24576 x 6144, us: IQ2_XXS, 256 rows
+# 28 / 36 / 187 against 47 / 58 / 244, 384 rows 45 / 54 / 242 against 47 / 60 / 288, 512 rows 48 / 72 / 310 against 50 / 66 / 285; Q4_K, 384 rows
+# 44 / 57 / 226 against 51 / 65 / 308; Q5_K, 256 rows 30 / 45 / 220 against 54 / 73 / 297, 384 rows 58 / 70 / 280 against 54 / 81 / 339, 512 rows
+# 63 / 90 / 365 against 61 / 78 / 337. Up to 2^24 weights their tiles fill the SMs a second time from 257 rows on.
+UMMA_MAX_ROWS, UMMA_MAX_ROWS_LARGE = 257, 385
 UMMA_SPLIT_ROUTES = 64
 UMMA_MAX_GROUPS = 512
 
@@ -71,11 +74,11 @@ def _umma_takes(w_raw: torch.Tensor, type_name: str, rows: int, K: int, groups: 
 
 
 def _registers_faster(type_name: str, rows: int, weights: int) -> bool:
-    """Few rows of a small weight decode faster in registers: one launch there, two and a pipeline to fill here (10 us at least), against
-    a multiply-add per weight and row. One row of 2048 x 2048 / 4096 x 4096 / 8192 x 3072, us: IQ2_XXS 5.2 against 13.5, 12.9 / 19.1,
-    19.1 / 21.7 (12288 x 3072: 26.7 / 24.4); Q4_K 7.1 / 13.2, 16.5 / 17.2, 21.9 / 19.2; Q5_K 8.2 / 14.2, 20.2 / 18.6, 25.6 / 21.2.
-    Four rows of 2048 x 2048: 9.7 / 13.8, 12.0 / 13.5, 12.9 / 14.5; eight 16.8 / 13.9, 17.7 / 13.7, 18.9 / 14.6; eight of
-    1024 x 2048 12.1 / 13.8, 12.0 / 13.0, 12.6 / 13.7."""
+    """Few rows of a small weight decode faster in registers: one launch there, two and a pipeline to fill here (12 us at least), against
+    a multiply-add per weight and row. Weights from memory, us: one row of 2048 x 2048 / 4096 x 4096 / 8192 x 3072, IQ2_XXS 6.5 against
+    13.3, 14.2 / 15.9, 20.4 / 16.9; Q4_K 7.9 / 11.9, 17.4 / 15.0, 23.5 / 16.3; Q5_K 8.8 / 12.8, 21.2 / 16.6, 27.4 / 17.9. Four rows of
+    2048 x 2048: 12.3 / 13.6, 13.2 / 12.1, 14.1 / 12.5; eight 19.9 / 13.5, 20.1 / 12.3, 21.1 / 12.9. Lines at half these
+    sizes would be up to 3 us faster; they stay, and with them the order in which single rows and pairs of rows have been added."""
     if rows > 8:
         return False
     width = 1 << (rows - 1).bit_length()        # the kernels have one, two, four or eight rows
@@ -370,10 +373,10 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     return _reduce_routes(ybuf, routes, x.shape, expert_offset, local, out)
 
 
-UMMA_MAX_ROUTES_PER_EXPERT = 192      # above this a decode per 64 routes costs more than one decode to a bf16 scratch: 128 routes 4.2 against
-#                                        5.4 ms, 192 6.0 against 5.9, 256 7.7 against 6.5 (256 experts of the MiniMax-M2 shape)
-#                                        64 experts of 2 x 1536 x 3072 / 2 x 1024 x 2048, 192 routes, us: IQ2_XXS 1353 against 1491 / 716 against 717,
-#                                        Q4_K 1492 / 1650 and 807 / 788, Q5_K 1614 / 1844 and 865 / 871; 256 routes 6 to 18 % slower in all
+UMMA_MAX_ROUTES_PER_EXPERT = 384      # far above this a decode per 64 routes costs more than one decode to a bf16 scratch, us: 256 experts of the
+#                                        MiniMax-M2 shape, IQ2_XXS, 192 routes 3081 against 6452, 384 6342 / 7867, 512 8399 / 8999; 64 experts of
+#                                        2 x 1536 x 3072, 384 routes, IQ2_XXS 1602 / 2029, Q4_K 1666 / 2151, Q5_K 1991 / 2357; of 2 x 1024 x 2048, 384
+#                                        routes, IQ2_XXS 910 / 999, Q5_K 1089 / 1145, 512 routes 1186 / 1127, 1419 / 1275
 GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local expert costs more than the route kernels' per-route decode
 
 

@@ -76,6 +76,21 @@ def test_linear_on_both_sides_of_the_rule(name, M):
         assert _rel(y[:, 0], want) < TOL and torch.equal(y[:, :1].expand_as(y), y)
 
 
+@pytest.mark.parametrize("name", ["iq2_xxs", "q4_k", "q5_k"])
+@pytest.mark.parametrize("M,N", [(256, 2048), (257, 2048), (384, 2080), (385, 2080)])
+def test_linear_on_both_sides_of_the_row_limits(name, M, N):
+    """Up to 2^24 weights 256 rows are the most, above 384; beyond that the weight is rounded to bf16, whose 2^-9 a sum takes over."""
+    from pocketllm_b200.ops import gguf_ops as go
+    K = 8192
+    raw, w = _raw(name, 32, K, M)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    y = go.gguf_linear(x, raw.repeat(N // 32), name, N, epi=2).view(M, N // 32, 32)
+    inside = M < (go.UMMA_MAX_ROWS if N * K <= 1 << 24 else go.UMMA_MAX_ROWS_LARGE)
+    assert inside == (M in (256, 384))
+    want = (x.double() @ w.T)[:, None].expand(-1, N // 32, -1)
+    assert _rel(y, want) < (TOL if inside else 2 ** -8)
+
+
 def test_linear_rows_of_zeros_and_infinities():
     from pocketllm_b200.ops import gguf_ops as go
     raw, w = _raw("q5_k", 256, 512, 0)
