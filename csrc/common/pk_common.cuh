@@ -280,7 +280,15 @@ inline cudaError_t pk_launch_ex(bool pdl, void (*kernel)(KArgs...), dim3 grid, d
       return PK_ERR_CUDA;                                                                           \
     }                                                                                               \
   } while (0)
-// for kernels that begin with pdl_wait()
+// A kernel launched this way may begin as soon as every block of the launch before it has triggered (or ended). Where that one triggers before its own
+// wait, the launches ahead of it can still be running too. So
+//   - what any launch writes is read, and what any launch reads is written, behind `pdl_wait()`; some warp of every block comes to it, or the next
+//     launch's wait would be over too early;
+//   - before it a kernel reads only what the program holds: weights and tables that were finished before the step's first launch. A buffer that is
+//     filled on the stream (a decoded weight, staged rows, route segments) is not held. It may be read early only behind a launch whose blocks wait
+//     before they trigger: when its dependents begin, everything ahead of it is complete. A launcher that cannot tell takes it from its caller
+//     (`pk_gemm_bf16` / `pk_gemm_bf16_held`);
+//   - a wait with a limit begins behind `pdl_wait()`, or its limit would count the time of the launches ahead.
 #define PK_LAUNCH_PDL(kernel, grid, block, smem, stream, ...) PK_LAUNCH_EX_(true, kernel, grid, block, smem, stream, __VA_ARGS__)
 // plain stream order
 #define PK_LAUNCH(kernel, grid, block, smem, stream, ...) PK_LAUNCH_EX_(false, kernel, grid, block, smem, stream, __VA_ARGS__)

@@ -89,8 +89,8 @@ int pk_fp8_to_bf16(const void* w, const float* scale, int N, int K, void* out, c
 int pk_rmsnorm_quant(const void* x, int M, int K, const float* gamma, int mode, float eps, void* y, int terms, void* q, int m_pad,
                      float* scale_t, int s_ld, cudaStream_t stream);
 int pk_quant_act_fp8(const void* x, int ldx, int M, int K, int terms, void* q, int m_pad, float* scale_t, int s_ld, cudaStream_t stream);
-int pk_gemm_fp8(const void* Aq, int terms, int m_pad, const float* a_scale, int a_ld, const void* W, const float* w_scale, int M, int N,
-                int K, int epi, void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream);
+int pk_gemm_fp8_held(const void* Aq, int terms, int m_pad, const float* a_scale, int a_ld, const void* W, const float* w_scale, int M, int N,
+                     int K, int epi, void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream);
 int pk_gqa_prefill_umma(const void* q, const void* kcache, const void* vcache, const int* pos, int M, int Hq, int Hkv, int head_dim, int ctx_cap,
                         float scale, const void* gate_proj, int ld, void* out, uint32_t* status, cudaStream_t stream);
 int pk_gemm_bf16_grouped(const void* A, int lda, const void* W, const int* seg, int n_groups, int R, int N, int K, int epi, void* C, int ldc,
@@ -108,6 +108,6 @@ int pk_linear_rows(const void* x, int ldx, const void* w, int M, int N, int K, i
 int pk_linear_narrow(const void* x, int ldx, const void* w, int M, int N, int K, void* y, int ldy, cudaStream_t stream);
 int pk_scatter_rows(const void* src, const int* slots, int n, int row_bytes, void* pool, cudaStream_t stream);
 int pk_topk_select(const float* score, const int* lengths, int M, int n, int ld, int k, int* out, cudaStream_t stream);
-int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int K, int epi, void* C, const void* resid, int ldc,
-                 uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream);
+int pk_gemm_bf16_held(const void* A, int lda, const void* W, int M, int N, int K, int epi, void* C, const void* resid, int ldc,
+                      uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream);
 }

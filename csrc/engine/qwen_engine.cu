@@ -1167,7 +1167,7 @@ void QwenEngine::run_chunk(int M, bool mtp, bool more) {
   if (W > 1) check(pk_bump_epoch((uint32_t*)((char*)arena_ + off_epoch_), stream_), "epoch");
   if (mtp) {
     check(pk_mtp_concat_norm(mtp_tok_dev_, M, embed_, mtp_in_, hidden_, mtp_norm_e_, mtp_norm_h_, eps, mtp_cat_, stream_), "mtp_concat_norm");
-    int rc = pk_gemm_bf16(mtp_cat_, 2 * hidden_, mtp_fc_, M, hidden_, 2 * hidden_, 0, hid, nullptr, hidden_, gemm_status_, nullptr, sm_count_, stream_);
+    int rc = pk_gemm_bf16_held(mtp_cat_, 2 * hidden_, mtp_fc_, M, hidden_, 2 * hidden_, 0, hid, nullptr, hidden_, gemm_status_, nullptr, sm_count_, stream_);
     if (rc == 4) rc = pk_gemm_umma(mtp_cat_, 2 * hidden_, mtp_fc_, nullptr, 1, M, hidden_, 2 * hidden_, 0, hid, nullptr, hidden_, gemm_status_, nullptr, stream_);
     check(rc, "gemm(mtp fc)");
   } else {
@@ -1187,7 +1187,7 @@ void QwenEngine::run_chunk(int M, bool mtp, bool more) {
       check(pk_quant_act_fp8(A, lda, M, w.K, terms, act_q_, act_rows_, act_scale_, act_rows_, stream_), "quant_act_fp8");
       xn_quantised = false;
     }
-    check(pk_gemm_fp8(act_q_, terms, act_rows_, act_scale_, act_rows_, w.w, w.scale, M, w.N, w.K, epi, C, resid, ldc, gemm_status_, ps, sm_count_,
+    check(pk_gemm_fp8_held(act_q_, terms, act_rows_, act_scale_, act_rows_, w.w, w.scale, M, w.N, w.K, epi, C, resid, ldc, gemm_status_, ps, sm_count_,
                       stream_), "gemm_fp8");
     return true;
   };
@@ -1201,7 +1201,7 @@ void QwenEngine::run_chunk(int M, bool mtp, bool more) {
     if (gemm_native(A, lda, w, epi, C, resid, ldc, nullptr)) return;
     if (w.wb != nullptr) {
       // persistent 128x256 kernel; shapes it does not take (SwiGLU halves not a multiple of 128) go to the 128x128 one
-      int rc = pk_gemm_bf16(A, lda, w.wb, M, w.N, w.K, epi, C, resid, ldc, gemm_status_, nullptr, sm_count_, stream_);
+      int rc = pk_gemm_bf16_held(A, lda, w.wb, M, w.N, w.K, epi, C, resid, ldc, gemm_status_, nullptr, sm_count_, stream_);
       if (rc == 4) rc = pk_gemm_umma(A, lda, w.wb, nullptr, 1, M, w.N, w.K, epi, C, resid, ldc, gemm_status_, nullptr, stream_);
       check(rc, "gemm_bf16");
     } else
@@ -1227,7 +1227,7 @@ void QwenEngine::run_chunk(int M, bool mtp, bool more) {
       PkPush ps = make_push(site, true, rpr);
       if (gemm_native(A, lda, w, 4, nullptr, nullptr, hidden_, &ps)) {
       } else if (w.wb != nullptr)
-        check(pk_gemm_bf16(A, lda, w.wb, M, w.N, w.K, 4, nullptr, nullptr, hidden_, gemm_status_, &ps, sm_count_, stream_), "gemm_bf16(push)");
+        check(pk_gemm_bf16_held(A, lda, w.wb, M, w.N, w.K, 4, nullptr, nullptr, hidden_, gemm_status_, &ps, sm_count_, stream_), "gemm_bf16(push)");
       else
         check(pk_gemm_umma(A, lda, w.w, w.scale, 0, M, w.N, w.K, 4, nullptr, nullptr, hidden_, gemm_status_, &ps, stream_), "gemm_umma(push)");
       pending = site;

@@ -62,6 +62,7 @@ struct Params {
   // silu(gate * s) * up * s, or silu(gate) * up * s (scale_after)
   const float* row_scale;
   int scale_after;
+  int w_held;             // W may be read before the launches ahead of this one are done
 };
 
 constexpr int kMaxGroups = 512;
@@ -218,7 +219,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       WorkIter work(p, num_kb, tiles_m);
       Seg sg;
       {
-        // the first weight tiles are requested before the rows of A are there (route segments, when there are any, are)
+        // the first weight tiles are requested before the rows of A are there (route segments, when there are any, are), if no one can be writing them
+        if (!p.w_held) pk::pdl_wait();
         WorkIter first = work;
         if (first.next(sg)) {
           int tn, a_row, w_off, rows, r0, r1;
@@ -598,10 +600,8 @@ PK_API int pk_gemm_bf16_grouped(const void* A, int lda, const void* W, const int
   return pk_gemm_bf16_grouped_scaled(A, lda, W, seg, n_groups, R, N, K, epi, C, ldc, nullptr, 0, status, sm_count, stream);
 }
 
-// A [M, K] bf16 (row stride lda elements), W [N, K] bf16 row-major, K a multiple of 64. Epilogues as in pk_gemm_umma;
-// for SwiGLU (epi 1) W holds N/2 gate rows then N/2 up rows and N/2 must be a multiple of 128 (else PK_ERR_UNSUPPORTED).
-PK_API int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int K, int epi, void* C, const void* resid, int ldc,
-                        uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream) {
+static int gemm(const void* A, int lda, const void* W, bool w_held, int M, int N, int K, int epi, void* C, const void* resid, int ldc, uint32_t* status,
+                const PkPush* push, int sm_count, cudaStream_t stream) {
   if (M < 1 || N < 1 || K < BK || (K % BK) != 0) return PK_ERR_BAD_ARG;
   if (((uintptr_t)A & 15) != 0 || ((size_t)lda * 2) % 16 != 0 || ((uintptr_t)W & 15) != 0) return PK_ERR_BAD_ARG;
   if (epi < EPI_BF16 || epi > EPI_PUSH) return PK_ERR_BAD_ARG;
@@ -626,6 +626,7 @@ PK_API int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int
   p.tiles_m = (M + BM - 1) / BM;
   p.tiles_n = epi == EPI_SWIGLU ? ((N >> 1) + 127) / 128 : (N + BN - 1) / BN;
   p.status = status;
+  p.w_held = w_held;
   if (push) p.push = *push;
   const size_t smem = sizeof(Smem) + 1024;
   static PkDeviceOnce once;
@@ -658,4 +659,16 @@ PK_API int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int
   PK_LAUNCH_PDL(gemm_bf16_kernel, dim3(grid), dim3(kThreads), smem, stream, tmap_a, tmap_w, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
+}
+
+// A [M, K] bf16 (row stride lda elements), W [N, K] bf16 row-major, K a multiple of 64. Epilogues as in pk_gemm_umma;
+// for SwiGLU (epi 1) W holds N/2 gate rows then N/2 up rows and N/2 must be a multiple of 128 (else PK_ERR_UNSUPPORTED).
+PK_API int pk_gemm_bf16(const void* A, int lda, const void* W, int M, int N, int K, int epi, void* C, const void* resid, int ldc,
+                        uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream) {
+  return gemm(A, lda, W, false, M, N, K, epi, C, resid, ldc, status, push, sm_count, stream);
+}
+// The same with a W that the program holds (PK_LAUNCH_PDL): its first tiles are read while the launch before this one ends.
+PK_API int pk_gemm_bf16_held(const void* A, int lda, const void* W, int M, int N, int K, int epi, void* C, const void* resid, int ldc,
+                             uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream) {
+  return gemm(A, lda, W, true, M, N, K, epi, C, resid, ldc, status, push, sm_count, stream);
 }

@@ -67,6 +67,7 @@ struct Params {
   int ldc;
   int tiles_m, tiles_n;
   int m_pad;               // rows of one term plane in the A tensor map
+  int w_held;              // W may be read before the launches ahead of this one are done
   const float* a_scale;    // [K / 128][a_ld]
   int a_ld;
   const float* w_scale;    // [ceil(N / 128)][w_ld]
@@ -252,7 +253,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       WorkIter work(p, num_kb);
       Seg sg;
       {
-        // the first weight tiles are requested before the activations are there
+        // the first weight tiles are requested before the activations are there, if no one can be writing them
+        if (!p.w_held) pk::pdl_wait();
         WorkIter first = work;
         if (first.next(sg)) {
           int r0, r1;
@@ -575,12 +577,8 @@ PK_API int pk_quant_act_fp8(const void* x, int ldx, int M, int K, int terms, voi
   return PK_OK;
 }
 
-// Aq: [terms][m_pad][K] E4M3 codes from pk_quant_act_fp8 (m_pad a multiple of 128 when terms == 2), a_scale [K / 128][a_ld];
-// W [N, K] E4M3 codes, w_scale [ceil(N / 128)][K / 128] fp32. Epilogues as in pk_gemm_bf16; for SwiGLU (epi 1) W holds
-// N / 2 gate rows then N / 2 up rows and N / 2 must be a multiple of 128 (else PK_ERR_UNSUPPORTED).
-PK_API int pk_gemm_fp8(const void* Aq, int terms, int m_pad, const float* a_scale, int a_ld, const void* W, const float* w_scale, int M, int N,
-                       int K, int epi, void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push, int sm_count,
-                       cudaStream_t stream) {
+static int gemm(const void* Aq, int terms, int m_pad, const float* a_scale, int a_ld, const void* W, bool w_held, const float* w_scale, int M, int N, int K, int epi,
+                void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push, int sm_count, cudaStream_t stream) {
   if (M < 1 || N < 1 || K < BK || (K % BK) != 0 || (terms != 1 && terms != 2)) return PK_ERR_BAD_ARG;
   if (m_pad < M || a_ld < M || (terms == 2 && (m_pad % BM) != 0)) return PK_ERR_BAD_ARG;
   if (((uintptr_t)Aq & 15) != 0 || ((uintptr_t)W & 15) != 0 || a_scale == nullptr || w_scale == nullptr) return PK_ERR_BAD_ARG;
@@ -610,6 +608,7 @@ PK_API int pk_gemm_fp8(const void* Aq, int terms, int m_pad, const float* a_scal
   p.a_ld = a_ld;
   p.w_scale = w_scale;
   p.w_ld = K / BK;
+  p.w_held = w_held;
   p.status = status;
   if (push) p.push = *push;
   const int tiles = p.tiles_m * p.tiles_n;
@@ -631,6 +630,21 @@ PK_API int pk_gemm_fp8(const void* Aq, int terms, int m_pad, const float* a_scal
     grid = groups * p.tiles_m;
   }
   return terms == 1 ? launch<1>(tmap_a, tmap_w, p, grid, stream) : launch<2>(tmap_a, tmap_w, p, grid, stream);
+}
+
+// Aq: [terms][m_pad][K] E4M3 codes from pk_quant_act_fp8 (m_pad a multiple of 128 when terms == 2), a_scale [K / 128][a_ld];
+// W [N, K] E4M3 codes, w_scale [ceil(N / 128)][K / 128] fp32. Epilogues as in pk_gemm_bf16; for SwiGLU (epi 1) W holds
+// N / 2 gate rows then N / 2 up rows and N / 2 must be a multiple of 128 (else PK_ERR_UNSUPPORTED).
+PK_API int pk_gemm_fp8(const void* Aq, int terms, int m_pad, const float* a_scale, int a_ld, const void* W, const float* w_scale, int M, int N,
+                       int K, int epi, void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push, int sm_count,
+                       cudaStream_t stream) {
+  return gemm(Aq, terms, m_pad, a_scale, a_ld, W, false, w_scale, M, N, K, epi, C, resid, ldc, status, push, sm_count, stream);
+}
+// The same with a W that the program holds (PK_LAUNCH_PDL): its first tiles are read while the launch before this one ends.
+PK_API int pk_gemm_fp8_held(const void* Aq, int terms, int m_pad, const float* a_scale, int a_ld, const void* W, const float* w_scale, int M, int N,
+                            int K, int epi, void* C, const void* resid, int ldc, uint32_t* status, const PkPush* push, int sm_count,
+                            cudaStream_t stream) {
+  return gemm(Aq, terms, m_pad, a_scale, a_ld, W, true, w_scale, M, N, K, epi, C, resid, ldc, status, push, sm_count, stream);
 }
 
 // The stream-K work space of `stream`, allocated now instead of by the first product on it (1 ms and more), and given back: by the owner of

@@ -355,3 +355,25 @@ def test_groups_at_any_place(name, N, K, rows, E, columns):
                 u, v = want.chunk(2, -1)
                 want = torch.nn.functional.silu(u) * v
             assert a == b or _rel(y[a:b], want) < TOL * (1 if epi == 2 else 4)      # the exponential of a SiLU and its product
+
+
+@pytest.mark.parametrize("name,M,N,K", [("q8_0", 64, 32768, 3072), ("q5_k", 400, 6400, 3072)])
+def test_product_behind_the_decode_of_its_weight(name, M, N, K):
+    """The decode to the scratch is the launch directly before the product (no norm, status given): a weight tile read before it is
+    written has the NaN that the scratch is filled with, or the other weight. Weights are rounded to bf16: 2^-9 of each, 2^-8 of a sum."""
+    from pocketllm_b200.ops import gguf_ops as go
+    sides = []
+    for seed in (M, M + 1):
+        raw, w = _raw(name, 32, K, seed)
+        x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+        sides.append((raw.repeat(N // 32), x, (x.double() @ w.T)[:, None].expand(-1, N // 32, -1)))
+    status = torch.zeros(1, device="cuda", dtype=torch.int32)
+    go.gguf_linear(sides[0][1], sides[0][0], name, N, epi=2, status=status)
+    (scratch,) = (b for k, b in go._scratch.items() if k[1] == torch.cuda.current_stream().cuda_stream)
+    for i in range(20):
+        raw, x, want = sides[i % 2]
+        if i % 4 < 2:
+            scratch.fill_(float("nan"))
+        y = go.gguf_linear(x, raw, name, N, epi=2, status=status)
+        assert _rel(y.view(want.shape), want) < 2 ** -8
+    assert status.item() == 0
