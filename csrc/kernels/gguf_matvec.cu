@@ -557,8 +557,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
 
 // The same for many tokens: a block has 64 tokens x 64 experts, a thread 8 x 8 sums: 16 reads of shared memory then feed 128
 // multiply-adds, which bound it. Four groups of 64 threads take a quarter of every 64 values of K each; where the tiles leave SMs idle the
-// blocks of a cluster take a part of K each. All add up in their order (another one than above). The router's rows of the first
-// steps are requested before the predecessor is complete. A row that cannot be copied by 16 bytes is loaded by elements (V = false).
+// blocks of a cluster take a part of K each. All add up in their order (another one than above). A row that cannot be copied by 16 bytes
+// is loaded by elements (V = false).
 // 1500 tokens of 3072 by 256 experts: 73 us (2 x 4 sums a thread, 16 tokens a block: 174; the form above, which reads
 // the router's rows once per 8 tokens, 279). 56 % of the rate of fp32 multiply-adds, with one or two blocks on an SM alike.
 constexpr int kRt = 64, kRe = 64, kRk = 64, kRs = 3;      // tile, values of K per step, steps in shared memory
@@ -612,12 +612,13 @@ __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* 
       }
     }
   };
-  for (int i = 0; i < kRs - 1; ++i)
-    if (i < n) fetch_w(i);
-  pk::pdl_wait_for(x);
+  pk::pdl_wait_for(x, rw);      // the router's rows can be the result of the launch before, too
   pk::pdl_trigger();
   for (int i = 0; i < kRs - 1; ++i) {
-    if (i < n) fetch_x(i);
+    if (i < n) {
+      fetch_w(i);
+      fetch_x(i);
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   float2 acc[4][8] = {};      // tokens ty + 16 m and ty + 16 m + 8

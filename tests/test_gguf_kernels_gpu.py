@@ -112,6 +112,21 @@ def test_router_of_many_tokens(T, H, E, offset):
         assert ((w.double() - want).abs() <= 0.25 * (H + 8) * 2 ** -24 * size.gather(1, ids.long()) + 2 ** -20).all()
 
 
+def test_router_behind_the_launch_that_makes_its_weights():
+    """Logits of a router whose rows the launch directly before writes, over rows of NaN."""
+    from pocketllm_b200.ops import gguf_ops as go
+    T, H, E = 600, 3072, 256
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    sides = [torch.randn(E, H, device="cuda") / H ** 0.5 for _ in range(2)]
+    want = [go.router_topk(x, w, 8) for w in sides]
+    rw = torch.empty_like(sides[0])
+    for i in range(20):
+        rw.fill_(float("nan"))
+        rw.copy_(sides[i % 2])
+        ids, w = go.router_topk(x, rw, 8)
+        assert torch.equal(ids, want[i % 2][0]) and torch.equal(w, want[i % 2][1])
+
+
 @pytest.mark.parametrize("t13,t2,T", [("iq2_xxs", "q2_k", 1), ("iq2_xxs", "iq2_xxs", 40), ("iq1_m", "iq1_m", 9)])
 def test_moe_forward_matches_dequantised_reference(t13, t2, T):
     from pocketllm_b200.ops import gguf_ops as go
