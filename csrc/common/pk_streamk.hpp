@@ -21,23 +21,28 @@ inline bool streamk_allowed() {
   return v == nullptr || v[0] != '0';
 }
 
+// Allocations that another thread's capture does not mind.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Work spaces by stream, since launches on several streams can run at the same time: at most `kStreamKStreams` per device (19 MB each with
-// 148 SMs). An owner of a stream can reserve one and gives it back when the stream has ended; otherwise a stream's first launch
-// allocates one or, when there are no more, takes that of a stream which has not been used for some time, after waiting for the device.
-constexpr int kStreamKStreams = 8, kStreamKIdle = 64;
-constexpr unsigned long long kStreamKFree = ~0ull;
+// 148 SMs), one for each of the first streams that ask. The streams after them work whole tiles, and so does every stream under capture (a
+// replay would find the flags of the one before it): no launch waits for another stream. An owner of a stream can have its work space
+// allocated ahead, and frees it when the stream has ended; the others live as long as the process, like the streams of torch's pool that have them.
+constexpr int kStreamKStreams = 8;
 struct StreamKPool {
   struct Entry {
-    unsigned long long id = kStreamKFree, last = 0;
-    StreamK b;
+    unsigned long long id = 0;
+    StreamK b;      // b.ws null: no one's
     int ctas = 0;
   };
   std::mutex mu;
   Entry entries[64][kStreamKStreams];
-  unsigned long long launches = 0;
 
-  // The stream's entry, a new one where it has none; null without one, and under capture (a replay would find the flags of the one
-  // before it). With `mu` held.
+  // The stream's entry, a new one where it has none and `make`; null without one. With `mu` held.
   Entry* of(cudaStream_t stream, int ctas, bool make) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     int dev = 0;
@@ -47,43 +52,34 @@ struct StreamKPool {
       return nullptr;
     }
     if (capture != cudaStreamCaptureStatusNone || dev < 0 || dev >= 64) return nullptr;
-    Entry *unowned = nullptr, *empty = nullptr, *oldest = entries[dev];
+    Entry* empty = nullptr;
     for (Entry& x : entries[dev]) {
       if (x.b.ws != nullptr && x.id == id) return &x;
       if (x.b.ws == nullptr) empty = &x;
-      else if (x.id == kStreamKFree) unowned = &x;
-      if (x.last < oldest->last) oldest = &x;
     }
-    if (!make) return nullptr;
-    Entry* e = unowned != nullptr ? unowned : empty;
-    if (e == nullptr && oldest->last + kStreamKIdle > launches) return nullptr;
-    if (unowned == nullptr) {
-      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // another thread may be capturing
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      bool ok = true;
-      if (e == nullptr) {
-        e = oldest;
-        ok = cudaDeviceSynchronize() == cudaSuccess;
-      } else {
-        const int n = ctas > 148 ? ctas : 148;
-        StreamK b;
-        ok = cudaMalloc(&b.ws, (size_t)n * 128 * 256 * sizeof(float)) == cudaSuccess && cudaMalloc(&b.flags, n * sizeof(uint32_t)) == cudaSuccess &&
-             cudaMemset(b.flags, 0, n * sizeof(uint32_t)) == cudaSuccess;
-        if (ok) {
-          e->b = b;
-          e->ctas = n;
-        } else {
-          cudaFree(b.ws);
-          cudaFree(b.flags);
-        }
-      }
-      if (!ok) cudaGetLastError();
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      if (!ok) return nullptr;
+    if (!make || empty == nullptr) return nullptr;
+    RelaxedCapture relaxed;
+    const int n = ctas > 148 ? ctas : 148;
+    StreamK b;
+    // cleared on the stream itself: its launches come behind, whatever the others do
+    const bool ok = cudaMalloc(&b.ws, (size_t)n * 128 * 256 * sizeof(float)) == cudaSuccess && cudaMalloc(&b.flags, n * sizeof(uint32_t)) == cudaSuccess &&
+                    cudaMemsetAsync(b.flags, 0, n * sizeof(uint32_t), stream) == cudaSuccess;
+    if (!ok) {
+      cudaGetLastError();
+      cudaFree(b.ws);
+      cudaFree(b.flags);
+      return nullptr;
     }
-    e->id = id;
-    e->last = launches;
-    return e;
+    empty->id = id;
+    empty->b = b;
+    empty->ctas = n;
+    return empty;
+  }
+  void free(Entry& e) {
+    RelaxedCapture relaxed;
+    cudaFree(e.b.ws);
+    cudaFree(e.b.flags);
+    e = Entry();
   }
 };
 inline StreamKPool& streamk_pool() {
@@ -95,10 +91,8 @@ inline StreamKPool& streamk_pool() {
 inline bool streamk_take(int ctas, cudaStream_t stream, StreamK& out) {
   StreamKPool& pool = streamk_pool();
   std::lock_guard<std::mutex> lock(pool.mu);
-  ++pool.launches;
   StreamKPool::Entry* e = pool.of(stream, ctas, true);
   if (e == nullptr || e->ctas < ctas) return false;
-  e->last = pool.launches;
   ++e->b.seq;
   out = e->b;
   return true;

@@ -657,7 +657,7 @@ PK_API void pk_gemm_reserve(int sm_count, cudaStream_t stream) {
 PK_API void pk_gemm_release(cudaStream_t stream) {
   pk::StreamKPool& pool = pk::streamk_pool();
   std::lock_guard<std::mutex> lock(pool.mu);
-  if (pk::StreamKPool::Entry* e = pool.of(stream, 0, false)) e->id = pk::kStreamKFree;
+  if (pk::StreamKPool::Entry* e = pool.of(stream, 0, false)) pool.free(*e);
 }
 
 // Chunk scorer of the long-context retriever as one FP8 GEMM: keys [n_chunks, 128] E4M3 codes with one fp32 scale per

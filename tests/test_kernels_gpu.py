@@ -320,6 +320,74 @@ def test_stream_k_on_several_streams_and_under_capture(M, N, K):
         assert _rel_err(y, r) < 6e-3
 
 
+STREAM_K_CHILD = """
+import ctypes, torch
+from pocketllm_b200 import ops
+rt = ctypes.CDLL("libcudart.so.12")
+def stream():
+    h = ctypes.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(ctypes.byref(h), 1) == 0      # does not wait for the default stream
+    return torch.cuda.ExternalStream(h.value)
+M, N, K = 128, 5120, 1024
+w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+want = x.float() @ w.float().t()
+streams, outs = [stream() for _ in range(12)], []
+def launches(which, rounds):
+    for _ in range(rounds):
+        for st in which:
+            with torch.cuda.stream(st):
+                outs.append(ops.gemm_bf16(x, w, status=status))
+def busy(st):
+    with torch.cuda.stream(st):
+        torch.cuda._sleep(4_000_000_000)      # two seconds
+        e = torch.cuda.Event()
+        e.record()
+    return e
+# kernels are loaded and torch has memory for every stream before the waits are looked at
+status = torch.zeros(1, device="cuda", dtype=torch.int32)
+ops.gemm_bf16(x, w, status=status)
+for st in streams:
+    with torch.cuda.stream(st):
+        kept = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(24)]
+torch.cuda._sleep(1000)
+torch.cuda.synchronize()
+# memory that an earlier owner left full of ones: the number of a work space's first launch
+ones, freed = (ctypes.c_uint32 * 148)(*[1] * 148), []
+for _ in range(16):
+    d = ctypes.c_void_p()
+    assert rt.cudaMalloc(ctypes.byref(d), ctypes.c_size_t(592)) == 0 and rt.cudaMemcpy(d, ones, ctypes.c_size_t(592), 1) == 0
+    freed.append(d)
+assert all(rt.cudaFree(d) == 0 for d in freed)
+# clearing the flags does not wait behind the default stream
+e = busy(torch.cuda.default_stream())
+launches(streams, 1)
+for st in streams:
+    st.synchronize()
+assert not e.query(), "a launch waited for the default stream"
+torch.cuda.synchronize()
+assert all((c.float() - want).norm() / want.norm() < 6e-3 for c in outs), "parts were missing"
+# and more streams than work spaces take turns without a wait for the device
+e = busy(streams[0])
+launches(streams[1:], 20)
+for st in streams[1:]:
+    st.synchronize()
+assert not e.query(), "a launch waited for another stream"
+torch.cuda.synchronize()
+assert all((c.float() - want).norm() / want.norm() < 6e-3 for c in outs) and status.item() == 0
+print("streams ok")
+"""
+
+
+def test_stream_k_work_spaces_of_new_streams():
+    """Streams that get their work space now, in memory full of ones and beside a busy default stream; twelve streams in turn."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    r = subprocess.run([sys.executable, "-c", STREAM_K_CHILD], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "streams ok" in r.stdout, r.stderr[-2000:]
+
+
 def test_rmsnorm_embedding_argmax():
     from pocketllm_b200 import ops
     x = torch.randn(5, 640, device="cuda").to(torch.bfloat16)
