@@ -254,8 +254,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
       }
       if (sm.abort_flag) {
-        // Gave up: let the copies already in flight land before the CTA exits.
-        for (uint32_t j = issued > (uint32_t)kStages ? issued - kStages : 0; j < issued; ++j) {
+        // Gave up: let the copies already in flight land before the CTA exits (stages of weights alone do not fill up: a limit's time for them).
+        const uint32_t end = issued > ahead ? issued : ahead;
+        for (uint32_t j = end > (uint32_t)kStages ? end - kStages : 0; j < end; ++j) {
           const int s = j % kStages;
           for (uint32_t i = 0; i < (1u << 20); ++i)
             if (mbar_try_wait(&sm.full[s], (j / kStages) & 1)) break;
@@ -269,6 +270,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     constexpr uint32_t idesc = umma_idesc(1, 1, BM, BN);
     const uint64_t da0 = smem_desc_k_sw128(smem_u32(sm.a[0])), db0 = smem_desc_k_sw128(smem_u32(sm.b[0]));
     const bool leader = elect_one();
+    pk::pdl_wait();      // the limits of the waits count this launch's time only
     uint32_t s = 0, ph = 0;
     int local = 0;
     WorkIter work(p, num_kb, tiles_m);

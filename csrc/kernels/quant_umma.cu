@@ -425,7 +425,8 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
 }
 
 // Before `pdl_wait` the kernel reads the weights and the route segments: its predecessor in the stream is the staging of its rows (or
-// another product of them), which lets it begin only when everything before itself is complete.
+// another product of them), which lets it begin only when everything before itself is complete. What is left of that launch, a few us, counts in the limits
+// of the waits.
 template <int TYPE, int NT, int TERMS>
 __global__ void __launch_bounds__(Shape<TYPE, NT>::kThreads, 1)
 quant_umma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ Params p) {
