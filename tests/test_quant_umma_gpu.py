@@ -162,8 +162,10 @@ def test_experts(t13, t2, T, E, topk, limit):
         assert _rel(go.gguf_moe_forward_grouped(x, raw13, raw2, t13, t2, E, I, routes), want) < 5e-4
 
 
-@pytest.mark.parametrize("t13,t2,E,topk,H,I", [("iq2_xxs", "iq2_xxs", 64, 8, 1536, 768), ("q4_k", "q5_k", 16, 2, 2048, 1280), ("iq2_xxs", "q4_k", 40, 3, 3072, 512)])
-def test_a_token_gives_the_same_bits_in_any_company(t13, t2, E, topk, H, I):
+@pytest.mark.parametrize("t13,t2,E,topk,H,I,cut", [("iq2_xxs", "iq2_xxs", 64, 8, 1536, 768, (False, False)), ("iq2_xxs", "iq2_xxs", 64, 2, 4096, 1024, (True, False)),
+                                                   ("iq2_xxs", "iq2_xxs", 64, 2, 1024, 3072, (False, True)),
+                                                   ("q4_k", "q5_k", 16, 2, 2048, 1280, (True, False)), ("iq2_xxs", "q4_k", 40, 3, 3072, 512, (True, False))])
+def test_a_token_gives_the_same_bits_in_any_company(t13, t2, E, topk, H, I, cut, monkeypatch):
     """One token alone (K in parts over CTAs) and the same token among others (all parts in one CTA), up to the four routes per expert
     from which prompts take the grouped form."""
     from pocketllm_b200.ops import gguf_ops as go
@@ -179,7 +181,8 @@ def test_a_token_gives_the_same_bits_in_any_company(t13, t2, E, topk, H, I):
     x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
     ids = torch.stack([torch.randperm(E, generator=g)[:topk] for _ in range(T)]).int().cuda()
     weight = torch.rand(T, topk, generator=g).cuda()
-    assert go._umma_splits(topk * (2 * I // 128), H, go._umma_slots(t13, 16)) > 1
+    calls, product = [], go._umma
+    monkeypatch.setattr(go, "_umma", lambda *a: (calls.append(a[10:13]), product(*a)))      # columns, parts, splits
 
     def run(n, **k):
         routes = go.group_routes(ids[:n].contiguous(), weight[:n].contiguous(), E)
@@ -187,9 +190,13 @@ def test_a_token_gives_the_same_bits_in_any_company(t13, t2, E, topk, H, I):
 
     half, n13, n2 = E // 2, raw13.numel() // 2, raw2.numel() // 2
     for kw in ({}, dict(a=raw13[n13:].clone(), b=raw2[n2:].clone(), expert_offset=half, local_experts=half)):
+        calls.clear()
         alone = run(1, **kw)
+        assert [(c, p > 1, s == p) for c, p, s in calls] == [(16, b, True) for b in cut]      # which products are cut, into CTAs of their own
         for n in (2, 3, 5, 8, 17, T):
+            calls.clear()
             assert torch.equal(run(n, **kw)[:1], alone), n
+        assert [(c, p > 1, s) for c, p, s in calls] == [(16, b, 1) for b in cut]                # and with all tokens all parts are one CTA's
 
 
 def _e4m3(x, w, scale, epi, resid, columns, splits, failed=0):
