@@ -316,7 +316,11 @@ __global__ void __launch_bounds__(ST) deltanet_state_kernel(const StateParams p)
 
   issue_wq(0);
   issue_pk(0);
-  for (int i = tid; i < D * SL / 4; i += ST) *reinterpret_cast<float4*>(m.S + i * 4) = load4(sp + (size_t)(i >> 3) * D + (i & 7) * 4);
+  const bool whole = ((uintptr_t)p.state & 15) == 0;      // a caller's state can begin on any float
+  for (int i = tid; i < D * SL / 4; i += ST) {
+    const float* s = sp + (size_t)(i >> 3) * D + (i & 7) * 4;
+    *reinterpret_cast<float4*>(m.S + i * 4) = whole ? load4(s) : make_float4(s[0], s[1], s[2], s[3]);
+  }
   const float* Uc = p.U + ((size_t)h * p.Tpad + orow) * D + sl * SL + ocol;
   const float* Gc = p.G + (size_t)h * p.Tpad;
   float4 u = load4(Uc);
@@ -429,7 +433,18 @@ __global__ void __launch_bounds__(ST) deltanet_state_kernel(const StateParams p)
   }
   cp_async_wait<0>();
   __syncthreads();
-  for (int i = tid; i < D * SL / 4; i += ST) *reinterpret_cast<float4*>(sp + (size_t)(i >> 3) * D + (i & 7) * 4) = load4(m.S + i * 4);
+  for (int i = tid; i < D * SL / 4; i += ST) {
+    float* s = sp + (size_t)(i >> 3) * D + (i & 7) * 4;
+    const float4 v = load4(m.S + i * 4);
+    if (whole) {
+      *reinterpret_cast<float4*>(s) = v;
+    } else {
+      s[0] = v.x;
+      s[1] = v.y;
+      s[2] = v.z;
+      s[3] = v.w;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -478,7 +493,8 @@ PK_API int pk_deltanet_chunked(const void* proj, int ld, int T, int key_heads, i
                                float* ws, cudaStream_t stream) {
   if (key_dim != D || value_dim != D) return PK_ERR_UNSUPPORTED;
   if (T < 1 || key_heads < 1 || value_heads % key_heads != 0 || ((uintptr_t)ws & 15) != 0) return PK_ERR_BAD_ARG;   // cp.async of 16 bytes
-  if ((ld & 3) != 0 || ((uintptr_t)proj & 7) != 0 || ((uintptr_t)out & 7) != 0 || ((uintptr_t)norm_w & 15) != 0) return PK_ERR_BAD_ARG;   // 8-byte row accesses
+  if ((ld & 3) != 0 || ((uintptr_t)proj & 7) != 0 || ((uintptr_t)out & 7) != 0 || ((uintptr_t)norm_w & 15) != 0 || ((uintptr_t)conv_w & 15) != 0)
+    return PK_ERR_BAD_ARG;   // row accesses of 8 bytes, a channel's four weights at once
   const int rep = value_heads / key_heads;
   if (rep > 2) return PK_ERR_UNSUPPORTED;
   const int nchunks = (T + CH - 1) / CH, Tpad = nchunks * CH;

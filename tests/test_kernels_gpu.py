@@ -481,6 +481,11 @@ def test_deltanet_chunked_matches_serial_recurrence(Hk, Hv, T):
     S3, cs3 = S.clone(), conv_state.clone()
     out3 = ops.deltanet_seq(proj, Hk, Hv, conv_w, cs3, A_log, dt_bias, norm_w, 1e-6, S3)
     assert _rel_err(out, out3) < 1e-2 and _rel_err(S2, S3) < 2e-3
+    # a state that begins on any float
+    for off in (1, 2, 3):
+        S4, cs4 = torch.cat((S.new_zeros(off), S.flatten(), S.new_zeros(1))), conv_state.clone()
+        out4 = ops.deltanet_chunked(proj, Hk, Hv, conv_w, cs4, A_log, dt_bias, norm_w, 1e-6, S4[off:-1].view_as(S))
+        assert torch.equal(out4, out) and torch.equal(S4[off:-1].view_as(S), S2) and S4[0] == 0 and S4[-1] == 0
 
 
 @pytest.mark.parametrize("M,ctx,Hq,Hkv,nsplit", [(1, 1, 4, 2, 4), (1, 700, 10, 2, 8), (5, 300, 5, 1, 3), (8, 64, 8, 8, 2)])
