@@ -47,7 +47,8 @@ struct StreamKPool {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     int dev = 0;
     unsigned long long id = 0;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetId(stream, &id) != cudaSuccess) {
+    // (under capture nothing else is asked of the stream: its number would end the capture)
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || (capture == cudaStreamCaptureStatusNone && (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetId(stream, &id) != cudaSuccess))) {
       cudaGetLastError();
       return nullptr;
     }

@@ -294,9 +294,10 @@ def test_gemm_fp8_stream_k_and_many_tiles(M, N, K, epi):
     assert _rel_err(c2, planes @ wd2.t()) < 6e-3
 
 
-@pytest.mark.parametrize("M,N,K", [(128, 5120, 1024), (200, 2304, 3072)])
-def test_stream_k_on_several_streams_and_under_capture(M, N, K):
-    """Tiles whose K is shared: launches on more streams than there are work spaces, and replays of a captured launch with new rows."""
+@pytest.mark.parametrize("M,N,K", [(128, 5120, 4096), (200, 2304, 4352)])
+def test_stream_k_on_several_streams_and_under_capture(M, N, K, monkeypatch):
+    """Tiles whose K is shared: launches on more streams than there are work spaces, and replays of a captured launch with new rows, which
+    is the schedule of whole tiles to the bit."""
     from pocketllm_b200 import ops
     w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
     xs = [torch.randn(M, K, device="cuda").to(torch.bfloat16) for _ in range(10)]
@@ -306,38 +307,50 @@ def test_stream_k_on_several_streams_and_under_capture(M, N, K):
     got = []
     for x, st in zip(xs, streams):
         with torch.cuda.stream(st):
-            got.append([ops.gemm_bf16(x, w) for _ in range(3)])
+            got.append([ops.gemm_bf16(x, w, epi=ops.EPI_F32) for _ in range(3)])
     torch.cuda.synchronize()
-    for g, r in zip(got, want):
-        assert all(_rel_err(y, r) < 6e-3 for y in g) and torch.equal(g[0], g[1]) and torch.equal(g[1], g[2])
     x = xs[0].clone()
-    graph = torch.cuda.CUDAGraph()
+    graph, graph8 = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        y = ops.gemm_bf16(x, w)
-    for new, r in zip(xs, want):
+        y = ops.gemm_bf16(x, w, epi=ops.EPI_F32)
+    replayed = []
+    for new in xs:
         x.copy_(new)
         graph.replay()
-        assert _rel_err(y, r) < 6e-3
+        replayed.append(y.clone())
+    aq, asc = ops.quant_act_fp8(xs[0], 2)
+    wq, ws = torch.randint(0, 120, (N, K), device="cuda", dtype=torch.uint8), torch.ones(N // 128, K // 128, device="cuda")
+    with torch.cuda.graph(graph8):
+        y8 = ops.gemm_fp8(aq, asc, M, wq, ws, epi=ops.EPI_F32)
+    graph8.replay()
+    monkeypatch.setenv("POCKET_GEMM_NO_STREAMK", "1")
+    whole = [ops.gemm_bf16(x, w, epi=ops.EPI_F32) for x in xs]
+    assert torch.equal(y8, ops.gemm_fp8(aq, asc, M, wq, ws, epi=ops.EPI_F32))
+    for g, r, t, c in zip(got, want, whole, replayed):
+        assert all(_rel_err(y, r) < 1e-5 for y in g) and torch.equal(g[0], g[1]) and torch.equal(g[1], g[2]) and torch.equal(c, t)
 
 
 STREAM_K_CHILD = """
-import ctypes, torch
+import ctypes, os, torch
 from pocketllm_b200 import ops
 rt = ctypes.CDLL("libcudart.so.12")
 def stream():
     h = ctypes.c_void_p()
     assert rt.cudaStreamCreateWithFlags(ctypes.byref(h), 1) == 0      # does not wait for the default stream
     return torch.cuda.ExternalStream(h.value)
-M, N, K = 128, 5120, 1024
+M, N, K = 128, 5120, 4096
 w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
 x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
 want = x.float() @ w.float().t()
+os.environ["POCKET_GEMM_NO_STREAMK"] = "1"
+whole = ops.gemm_bf16(x, w, epi=ops.EPI_F32)
+del os.environ["POCKET_GEMM_NO_STREAMK"]
 streams, outs = [stream() for _ in range(12)], []
 def launches(which, rounds):
     for _ in range(rounds):
         for st in which:
             with torch.cuda.stream(st):
-                outs.append(ops.gemm_bf16(x, w, status=status))
+                outs.append(ops.gemm_bf16(x, w, epi=ops.EPI_F32, status=status))
 def busy(st):
     with torch.cuda.stream(st):
         torch.cuda._sleep(4_000_000_000)      # two seconds
@@ -346,10 +359,11 @@ def busy(st):
     return e
 # kernels are loaded and torch has memory for every stream before the waits are looked at
 status = torch.zeros(1, device="cuda", dtype=torch.int32)
-ops.gemm_bf16(x, w, status=status)
+shared = ops.gemm_bf16(x, w, epi=ops.EPI_F32, status=status)
+assert not torch.equal(shared, whole) and (shared - want).norm() < 1e-5 * want.norm()       # K in parts, another order
 for st in streams:
     with torch.cuda.stream(st):
-        kept = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(24)]
+        kept = [torch.empty(M, N, device="cuda") for _ in range(24)]
 torch.cuda._sleep(1000)
 torch.cuda.synchronize()
 # memory that an earlier owner left full of ones: the number of a work space's first launch
@@ -366,7 +380,8 @@ for st in streams:
     st.synchronize()
 assert not e.query(), "a launch waited for the default stream"
 torch.cuda.synchronize()
-assert all((c.float() - want).norm() / want.norm() < 6e-3 for c in outs), "parts were missing"
+# the default stream has one of the eight work spaces, the first seven of these the others
+assert all(torch.equal(c, shared) for c in outs[:7]) and all(torch.equal(c, whole) for c in outs[7:]), "parts were missing"
 # and more streams than work spaces take turns without a wait for the device
 e = busy(streams[0])
 launches(streams[1:], 20)
@@ -374,7 +389,9 @@ for st in streams[1:]:
     st.synchronize()
 assert not e.query(), "a launch waited for another stream"
 torch.cuda.synchronize()
-assert all((c.float() - want).norm() / want.norm() < 6e-3 for c in outs) and status.item() == 0
+for i, c in enumerate(outs[12:]):
+    assert torch.equal(c, shared if i % 11 < 6 else whole), i
+assert status.item() == 0
 print("streams ok")
 """
 
