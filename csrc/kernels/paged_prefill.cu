@@ -7,7 +7,8 @@
 //   S  = Q K^T       tcgen05.mma kind::f16, both operands K-major, fp32 S in TMEM (two buffers: S of the next step is
 //                    computed while the softmax warps work on this one)
 //   P  = exp2(S-m)   four softmax warps, one query row per thread; fp32 weights, handed to the tensor cores as the sum of two
-//                    bf16 terms (16 significant bits) in tensor memory, in the columns that S had
+//                    bf16 terms (16 significant bits): with one map in tensor memory, in the columns that S had, with two
+//                    in shared memory
 //   O += P V         V as an MN-major operand, O in TMEM. The reference m of a row only moves when its maximum has grown by
 //                    more than a factor of 2^8; its warp then rescales O in TMEM (weights up to 2^8 lose nothing in fp32)
 // With NMAP = 2 the maps share the loads of V, and while one map's warps are in their exponentials the other map's products
@@ -16,7 +17,9 @@
 // merge kernel.
 //
 // Bound by the exponentials and conversions of the softmax warps: without P in shared memory two CTAs of one map are resident, and one's
-// products run under the other's softmax. 1900 rows of 32 heads, window 1024: 101 -> 69 us.
+// products run under the other's softmax. 1900 rows of 32 heads, window 1024: 101 -> 69 us. Two maps fill the tensor memory, so one CTA
+// is resident either way, and with P in the columns of S the next S would wait for this step's products: 1900 rows of 16 heads of two maps of
+// 64 / 128 channels 81 / 95 us against 72 / 86 with P in shared memory, 512 rows behind 3000 positions 144 / 169 against 126 / 151.
 //
 // Positions outside a row's view are masked; what a page holds behind the last position is finite (zeros or older rows).
 // Every wait is bounded (status word + CTA-wide abort flag).
@@ -82,9 +85,11 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int NV = VP / 64;
   constexpr uint32_t kTmemCols = NMAP == 2 ? 512 : 256;
+  constexpr bool kShared = NMAP == 2;                   // P in shared memory
   const PkPagedAttention& a = p.a;
   const int qp = p.qk_panels;
-  uint8_t* sq = base;                                   // [NMAP][qp] panels of 128 rows (1024-byte aligned panels throughout)
+  uint8_t* sp = base;                                   // kShared: [NMAP][2 terms] of 128 rows (1024-byte aligned panels throughout)
+  uint8_t* sq = sp + (kShared ? NMAP * 2 * kQPanel : 0);      // [NMAP][qp] panels of 128 rows
   uint8_t* sk = sq + NMAP * qp * kQPanel;               // [2][NMAP][qp] panels of 64 rows
   uint8_t* sv = sk + 2 * NMAP * qp * kKPanel;           // [2][NV]
   Ctl& ct = *reinterpret_cast<Ctl*>(sv + 2 * NV * kKPanel);
@@ -191,8 +196,9 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       for (int t = 0; t < n_tiles && ok; ++t) {
         const int b = t & 1;
         if (t + 1 < n_tiles) {
-          // the S buffers of step t + 1 are free when the products with the weights of step t - 1 are done
-          for (int m = 0; m < NMAP && t > 0 && ok; ++m) ok = mbar_wait(&ct.pv_full[m][b ^ 1], ((t - 1) >> 1) & 1, &ct.abort_flag, a.status, 68);
+          // The S buffers of step t + 1 are free when the products with the weights of step t - 1 are done, or, with P in shared
+          // memory, when S has been read: p_ready of step t - 1 was waited for.
+          for (int m = 0; m < NMAP && !kShared && t > 0 && ok; ++m) ok = mbar_wait(&ct.pv_full[m][b ^ 1], ((t - 1) >> 1) & 1, &ct.abort_flag, a.status, 68);
           if (!ok || !mbar_wait(&ct.k_full[b ^ 1], ((t + 1) >> 1) & 1, &ct.abort_flag, a.status, 74)) break;
           tc_fence_after();
           issue_s(t + 1);
@@ -204,10 +210,13 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             break;
           }
           tc_fence_after();
-          const uint32_t pa = tmem_s + m * 128 + b * 64, va = smem_u32(sv + b * NV * kKPanel);
+          const uint32_t va = smem_u32(sv + b * NV * kKPanel), ps = smem_u32(sp + m * 2 * kQPanel);
 #pragma unroll
-          for (int j = 0; j < 8; ++j)   // four k-steps of the leading bf16 term, then four of the remainder
-            umma_f16_ts(tmem_o + m * VP, pa + j * 8, desc_mn_sw128(va + (j & 3) * 2048, kKPanel, 1024), idesc_pv, t > 0 || j > 0 ? 1u : 0u);
+          for (int j = 0; j < 8; ++j) {   // four k-steps of the leading bf16 term, then four of the remainder
+            const uint64_t dv = desc_mn_sw128(va + (j & 3) * 2048, kKPanel, 1024);
+            if constexpr (kShared) umma_f16(tmem_o + m * VP, smem_desc_k_sw128(ps + (j >> 2) * kQPanel + (j & 3) * 32), dv, idesc_pv, t > 0 || j > 0 ? 1u : 0u);
+            else umma_f16_ts(tmem_o + m * VP, tmem_s + m * 128 + b * 64 + j * 8, dv, idesc_pv, t > 0 || j > 0 ? 1u : 0u);
+          }
           umma_commit(&ct.pv_full[m][b]);
         }
         if (ok && t + 2 < n_tiles) umma_commit(&ct.v_empty[b]);
@@ -304,9 +313,25 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           rest[c * 16 + e] = *reinterpret_cast<const uint32_t*>(&pl);
         }
       sum += (u4[0] + u4[1]) + (u4[2] + u4[3]);
-      tmem_st_32x32(ts + (t & 1) * 64, hi);
-      tmem_st_32x32(ts + (t & 1) * 64 + 32, rest);
-      tmem_st_wait();
+      if constexpr (kShared) {
+        // the P buffers are free once the product of the step before is done
+        if (t > 0 && !mbar_wait_warp(&ct.pv_full[m][(t - 1) & 1], ((t - 1) >> 1) & 1, &ct.abort_flag, a.status, 79)) {
+          ok = false;
+          break;
+        }
+        uint8_t* prow = sp + m * 2 * kQPanel + r * 128;
+#pragma unroll
+        for (int g8 = 0; g8 < 8; ++g8) {
+          const int piece = g8 ^ (r & 7);
+          *reinterpret_cast<uint4*>(prow + piece * 16) = make_uint4(hi[4 * g8], hi[4 * g8 + 1], hi[4 * g8 + 2], hi[4 * g8 + 3]);
+          *reinterpret_cast<uint4*>(prow + kQPanel + piece * 16) = make_uint4(rest[4 * g8], rest[4 * g8 + 1], rest[4 * g8 + 2], rest[4 * g8 + 3]);
+        }
+        fence_proxy_async_smem();
+      } else {
+        tmem_st_32x32(ts + (t & 1) * 64, hi);
+        tmem_st_32x32(ts + (t & 1) * 64 + 32, rest);
+        tmem_st_wait();
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ct.p_ready[m][t & 1]);
@@ -318,7 +343,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     float inv = sum > 0.f ? 1.f / sum : 0.f;
     const bool row_ok = ok && r < tile.y;
     const int nv = min(VP, a.V - vs * 128);
-    float* xch = reinterpret_cast<float*>(base);        // [VP][128 rows]: queries, keys and values take at least as much
+    float* xch = reinterpret_cast<float*>(base);        // [VP][128 rows]: with two maps the weights take as much
     if (NMAP == 2) {
       // every product of this CTA is done once both groups have waited for their last one: their operands' buffers are free
       asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -430,9 +455,9 @@ bool encode_rows64(EncodeTiledFn encode, CUtensorMap* map, const void* base, uin
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-size_t smem_bytes(int qp, int vpan, int nmap) { return 1024 + (size_t)nmap * qp * kQPanel + 2 * (size_t)(nmap * qp + vpan) * kKPanel + sizeof(Ctl); }
-// Which widths go which way was decided with P in shared memory as well.
-size_t form_bytes(int qp, int vpan, int nmap) { return smem_bytes(qp, vpan, nmap) + (size_t)nmap * 2 * kQPanel; }
+size_t smem_bytes(int qp, int vpan, int nmap) {
+  return 1024 + (nmap == 2 ? 4 * (size_t)kQPanel : 0) + (size_t)nmap * qp * kQPanel + 2 * (size_t)(nmap * qp + vpan) * kKPanel + sizeof(Ctl);
+}
 
 template <int VP, int NMAP>
 int launch(const CUtensorMap& tq, const CUtensorMap& tc, const Params& p, dim3 grid, cudaStream_t stream) {
@@ -455,9 +480,9 @@ int launch(const CUtensorMap& tq, const CUtensorMap& tc, const Params& p, dim3 g
 // pk_paged_merge (nsplit 1, no part_ml), -1 when keys are too wide for it.
 PK_API int pk_paged_prefill_form(int maps, int D, int V) {
   const int qp = (D + 63) / 64;
-  if (qp > 4 || form_bytes(qp, V <= 64 ? 1 : 2, 1) > 227 * 1024) return -1;
+  if (qp > 4 || smem_bytes(qp, V <= 64 ? 1 : 2, 1) > 227 * 1024) return -1;
   if (V > 128) return 0;
-  return maps == 1 || form_bytes(qp, V <= 64 ? 1 : 2, 2) <= 227 * 1024 ? 1 : 0;
+  return maps == 1 || smem_bytes(qp, V <= 64 ? 1 : 2, 2) <= 227 * 1024 ? 1 : 0;
 }
 
 // Long portions (bf16): qf [rows, H x maps, q_ld] with q_ld a multiple of 64, cache of `pages` pages; tiles [ntiles] and seqs as in
