@@ -200,9 +200,9 @@ __device__ __forceinline__ void unpack_kv8(const Kv8& r, bool fp8, float (&f)[8]
   }
 }
 
-// A split has few keys per warp, and its time was that of one load after the other: the keys and values of the two next steps are on
-// their way while one is worked on. One row, 48 heads of 8 key heads, 210 keys in 8 splits: 11.5 -> 7.9 us.
-template <int G>
+// A split has few keys per warp, and its time was that of one load after the other: the keys and values of the AHEAD next steps are on
+// their way while one is worked on. One row, 48 heads of 8 key heads, 210 keys in 8 splits: 11.5 -> 7.9 us. (The same sums in the same order.)
+template <int G, int AHEAD>
 __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParams p) {
   pk::pdl_wait();
   pk::pdl_trigger();
@@ -237,8 +237,7 @@ __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParam
 
   const size_t head_row0 = (size_t)hk * p.ctx_cap;
   const bool fp8 = p.kv_fp8 != 0;
-  constexpr int kAhead = 2;
-  Kv8 kr[kAhead + 1], vr[kAhead + 1];
+  Kv8 kr[AHEAD + 1], vr[AHEAD + 1];
   auto in_range = [&](int t) { return t < end && (p.window == 0 || t >= win_lo || t < p.sink); };
   auto fetch = [&](int t, Kv8& k, Kv8& v) {
     k.w = v.w = make_uint4(0u, 0u, 0u, 0u);
@@ -249,16 +248,16 @@ __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParam
     }
   };
 #pragma unroll
-  for (int a = 0; a < kAhead; ++a) fetch(start + warp * 2 + khalf + 8 * a, kr[a], vr[a]);
+  for (int a = 0; a < AHEAD; ++a) fetch(start + warp * 2 + khalf + 8 * a, kr[a], vr[a]);
   for (int t0 = start + warp * 2; t0 < end; t0 += 8) {
     const int t = t0 + khalf;
     const bool valid = in_range(t);
-    fetch(t + 8 * kAhead, kr[kAhead], vr[kAhead]);
+    fetch(t + 8 * AHEAD, kr[AHEAD], vr[AHEAD]);
     float kf[8], vf[8];
     unpack_kv8(kr[0], fp8, kf);
     unpack_kv8(vr[0], fp8, vf);
 #pragma unroll
-    for (int a = 0; a < kAhead; ++a) {
+    for (int a = 0; a < AHEAD; ++a) {
       kr[a] = kr[a + 1];
       vr[a] = vr[a + 1];
     }
@@ -326,6 +325,15 @@ __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParam
       o[kD + 1] = l;
     }
   }
+}
+
+// Up to two blocks on an SM loads ahead pay (6000 keys, 256 blocks, one / four / six query heads to a key head: 1.2, 1.11, 1.05 times as fast). More blocks hide
+// one another's loads, and the registers of the loads cost some of them: 512 blocks, 1000 keys in 8 splits, without / with, one to five heads .97, .95, .93, .92, .66 of
+// the speed. From six heads on as many blocks are resident either way, and it pays throughout (1.04 there).
+template <int G>
+cudaError_t launch_split(const DecodeParams& p, dim3 grid, cudaStream_t stream) {
+  const bool ahead = G >= 6 || (long long)grid.x * grid.y * grid.z <= 2 * 148;
+  return ahead ? pk_launch_ex(true, gqa_decode_split_kernel<G, 2>, grid, dim3(128), 0, stream, p) : pk_launch_ex(true, gqa_decode_split_kernel<G, 0>, grid, dim3(128), 0, stream, p);
 }
 
 struct MergeParams {
@@ -568,15 +576,20 @@ PK_API int pk_gqa_decode_kv(const void* q, const void* kcache, const void* vcach
   DecodeParams p{(const pk::bf16*)q, (const pk::bf16*)kcache, (const pk::bf16*)vcache, pos, M, Hq, Hkv,
                  ctx_cap, scale, nsplit, window, sink, ws, kscale != nullptr ? 1 : 0, kscale, vscale};
   const dim3 grid(Hkv, nsplit, M);
+  cudaError_t e = cudaSuccess;
   switch (Hq / Hkv) {
-    case 1: PK_LAUNCH_PDL(gqa_decode_split_kernel<1>, grid, dim3(128), 0, stream, p); break;
-    case 2: PK_LAUNCH_PDL(gqa_decode_split_kernel<2>, grid, dim3(128), 0, stream, p); break;
-    case 3: PK_LAUNCH_PDL(gqa_decode_split_kernel<3>, grid, dim3(128), 0, stream, p); break;
-    case 4: PK_LAUNCH_PDL(gqa_decode_split_kernel<4>, grid, dim3(128), 0, stream, p); break;
-    case 5: PK_LAUNCH_PDL(gqa_decode_split_kernel<5>, grid, dim3(128), 0, stream, p); break;
-    case 6: PK_LAUNCH_PDL(gqa_decode_split_kernel<6>, grid, dim3(128), 0, stream, p); break;
-    case 8: PK_LAUNCH_PDL(gqa_decode_split_kernel<8>, grid, dim3(128), 0, stream, p); break;
+    case 1: e = launch_split<1>(p, grid, stream); break;
+    case 2: e = launch_split<2>(p, grid, stream); break;
+    case 3: e = launch_split<3>(p, grid, stream); break;
+    case 4: e = launch_split<4>(p, grid, stream); break;
+    case 5: e = launch_split<5>(p, grid, stream); break;
+    case 6: e = launch_split<6>(p, grid, stream); break;
+    case 8: e = launch_split<8>(p, grid, stream); break;
     default: return PK_ERR_UNSUPPORTED;
+  }
+  if (e != cudaSuccess) {
+    pk_set_last_cuda_error((int)e);
+    return PK_ERR_CUDA;
   }
   PK_CHECK_LAUNCH();
   MergeParams mp{ws, nsplit, Hq, (const pk::bf16*)gate_proj, ld, (pk::bf16*)out};

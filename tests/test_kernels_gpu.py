@@ -724,6 +724,21 @@ def test_gqa_prefill_with_maxima_that_move(M, pos0, growth):
         assert ((got.view(M, Hq, D).double() - want).abs() <= 2 ** -8 * (scale + want.abs()) + 1e-6).all()
 
 
+@pytest.mark.parametrize("G", [1, 2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("ctx,window", [(1, 0), (9, 0), (300, 0), (300, 64)])
+def test_gqa_decode_of_many_rows_is_that_of_each(G, ctx, window):
+    """Rows of one launch with more than two blocks to an SM, and row by row: loads ahead change no bit."""
+    from pocketllm_b200 import ops
+    Hkv, M, D, cap, nsplit = 2, 40, 128, 512, 4
+    kc, vc = (torch.randn(Hkv, cap, D, device="cuda").to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(M, G * Hkv, D, device="cuda").to(torch.bfloat16)
+    pos = torch.arange(ctx - 1, ctx - 1 + M, device="cuda", dtype=torch.int32)
+    kw = dict(nsplit=nsplit, window=window, sink=4 if window else 0)
+    all_rows = ops.gqa_decode(q, kc, vc, pos, **kw)
+    assert M * Hkv * nsplit > 296 and Hkv * nsplit <= 296
+    assert torch.equal(all_rows, torch.cat([ops.gqa_decode(q[i:i + 1], kc, vc, pos[i:i + 1], **kw) for i in range(M)]))
+
+
 def test_full_qk_norm_rope_append_matches_torch():
     """Whole-vector RMS (one gamma per element) + half-split rotation from tables + KV append, against plain PyTorch."""
     from pocketllm_b200 import ops
