@@ -967,12 +967,13 @@ static float* router_scratch(size_t floats) {
   return buf[dev];
 }
 
-// The blocks of the form with one warp per expert keep eight tokens of H floats each in shared memory; when they are more than are
+// The blocks of the form with one warp per expert keep up to eight tokens of H floats each in shared memory; when they are more than are
 // resident at once, the tiles are faster, if an expert tile is full. One warp per expert / tiles, us: 256 experts of 3072 (256 blocks for
 // 64 tokens, 296 resident), 64 tokens 15 / 17, 96 tokens 28 / 17, 256 tokens 56 / 27; 128 of 4096 (148 resident), 64 tokens 13 / 21, 96 tokens
-// 27 / 21, 512 tokens 86 / 34; 64 of 2048 (444 resident), 384 tokens 13 / 13, 512 tokens 26 / 13.
+// 27 / 21, 512 tokens 86 / 34; 64 of 2048 (444 resident), 384 tokens 13 / 13, 512 tokens 26 / 13;
+// one token by 256 experts of 8192 9 / 39.
 static bool router_tiles(int T, int E, int H, int sms) {
-  const long long resident = std::min(8, (227 * 1024) / (32 * H + 1024));
+  const long long resident = std::max(1, std::min(8, (227 * 1024) / (4 * std::min(T, 8) * H + 1024)));
   return E >= kRe && (long long)((E + 7) / 8) * ((T + 7) / 8) > resident * sms;
 }
 

@@ -112,6 +112,21 @@ def test_router_of_many_tokens(T, H, E, offset):
         assert ((w.double() - want).abs() <= 0.25 * (H + 8) * 2 ** -24 * size.gather(1, ids.long()) + 2 ** -20).all()
 
 
+@pytest.mark.parametrize("T", [1, 3, 6])
+def test_router_of_few_wide_rows(T):
+    """Rows too wide for eight tokens in shared memory keep the form with one warp per expert: zeros behind a narrow row leave every bit as it
+    is there, where a lane adds its values in order."""
+    from pocketllm_b200.ops import gguf_ops as go
+    H, E = 8192, 256
+    torch.manual_seed(T)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    rw = torch.randn(E, H, device="cuda") / H ** 0.5
+    x[:, H // 2:] = 0
+    wide = go.router_topk(x, rw, 32, norm_topk=False)
+    narrow = go.router_topk(x[:, :H // 2].contiguous(), rw[:, :H // 2].contiguous(), 32, norm_topk=False)
+    assert torch.equal(wide[0], narrow[0]) and torch.equal(wide[1], narrow[1])
+
+
 def test_router_behind_the_launch_that_makes_its_weights():
     """Logits of a router whose rows the launch directly before writes, over rows of NaN."""
     from pocketllm_b200.ops import gguf_ops as go
