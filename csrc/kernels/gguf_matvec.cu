@@ -557,15 +557,22 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const bf16* x, const
 
 // The same for many tokens: a block has 64 tokens x 64 experts, a thread 8 x 8 sums: 16 reads of shared memory then feed 128
 // multiply-adds, which bound it. Four groups of 64 threads take a quarter of every 64 values of K each; where the tiles leave SMs idle the
-// blocks of a cluster take a part of K each. All add up in their order (another one than above). A row that cannot be copied by 16 bytes
-// is loaded by elements (V = false).
+// blocks of a cluster take a part of K each. All add up in their order (another one than above). Rows come by 16-byte copies where
+// they are aligned to that (V = 8), by 4-byte copies where the rows of x are aligned to them (V = 2), and with rows of x at odd addresses those wait in
+// registers while a step is multiplied (V = 1). 256 experts, 512 tokens, us: H = 3072 33, 3070 44, 3071 54 (2 x 4 sums a thread 63 each).
 // 1500 tokens of 3072 by 256 experts: 73 us (2 x 4 sums a thread, 16 tokens a block: 174; the form above, which reads
 // the router's rows once per 8 tokens, 279). 56 % of the rate of fp32 multiply-adds, with one or two blocks on an SM alike.
 constexpr int kRt = 64, kRe = 64, kRk = 64, kRs = 3;      // tile, values of K per step, steps in shared memory
 constexpr int kRw = kRk + 4, kRx = kRk + 8, kRo = kRe + 8;      // pitches: rows of eight consecutive threads start in different banks
 constexpr int kRouterSmem = kRs * (kRe * kRw * 4 + kRt * kRx * 2);
 static_assert(4 * kRt * kRo * 4 <= kRouterSmem, "the groups' sums take the place of the tiles");
-template <bool V>
+template <int B>
+__device__ __forceinline__ void router_copy(void* dst, const void* src, bool in) {      // B bytes, zeros unless `in`
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), n = in ? B : 0;
+  if constexpr (B == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+template <int V>
 __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* x, const float* rw, int H, int E, int T, float* logits) {
   extern __shared__ __align__(16) uint8_t router_smem[];
   float* ws = reinterpret_cast<float*>(router_smem);                            // [kRs][kRe][kRw]
@@ -576,39 +583,46 @@ __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* 
   const int e0 = blockIdx.y * kRe, t0 = blockIdx.z * kRt;
   const int steps = (H + kRk - 1) / kRk, per = (steps + parts - 1) / parts;
   const int first = min(part * per, steps), n = min(per, steps - first);
+  constexpr int WV = V == 8 ? 4 : 1;      // floats of a copy
   auto fetch_w = [&](int i) {
     float* dst = ws + (i % kRs) * kRe * kRw;
     const int k0 = (first + i) * kRk;
-    if constexpr (V) {
 #pragma unroll 1
-      for (int c = tid; c < kRe * (kRk / 4); c += 256) {
-        const int r = c / (kRk / 4), k = (c & (kRk / 4 - 1)) * 4;
-        const bool in = e0 + r < E && k0 + k < H;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * kRw + k)),
-                     "l"(in ? rw + (size_t)(e0 + r) * H + k0 + k : rw), "r"(in ? 16 : 0) : "memory");
-      }
-    } else {
-      for (int c = tid; c < kRe * kRk; c += 256) {
-        const int r = c / kRk, k = c & (kRk - 1);
-        dst[r * kRw + k] = e0 + r < E && k0 + k < H ? rw[(size_t)(e0 + r) * H + k0 + k] : 0.f;
-      }
+    for (int c = tid; c < kRe * (kRk / WV); c += 256) {
+      const int r = c / (kRk / WV), k = (c & (kRk / WV - 1)) * WV;
+      const bool in = e0 + r < E && k0 + k < H;
+      router_copy<4 * WV>(dst + r * kRw + k, in ? rw + (size_t)(e0 + r) * H + k0 + k : rw, in);
     }
   };
   auto fetch_x = [&](int i) {
-    bf16* dst = xs + (i % kRs) * kRt * kRx;
-    const int k0 = (first + i) * kRk;
-    if constexpr (V) {
+    if constexpr (V > 1) {
+      bf16* dst = xs + (i % kRs) * kRt * kRx;
+      const int k0 = (first + i) * kRk;
 #pragma unroll 1
-      for (int c = tid; c < kRt * (kRk / 8); c += 256) {
-        const int r = c / (kRk / 8), k = (c & (kRk / 8 - 1)) * 8;
+      for (int c = tid; c < kRt * (kRk / V); c += 256) {
+        const int r = c / (kRk / V), k = (c & (kRk / V - 1)) * V;
         const bool in = t0 + r < T && k0 + k < H;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * kRx + k)),
-                     "l"(in ? x + (size_t)(t0 + r) * H + k0 + k : x), "r"(in ? 16 : 0) : "memory");
+        router_copy<2 * V>(dst + r * kRx + k, in ? x + (size_t)(t0 + r) * H + k0 + k : x, in);
       }
-    } else {
-      for (int c = tid; c < kRt * kRk; c += 256) {
-        const int r = c / kRk, k = c & (kRk - 1);
-        dst[r * kRx + k] = t0 + r < T && k0 + k < H ? x[(size_t)(t0 + r) * H + k0 + k] : __float2bfloat16(0.f);
+    }
+  };
+  // V = 1: element tid & 63 of every fourth row, two rows in a register
+  uint32_t held[V == 1 ? 8 : 1];
+  auto load_x = [&](int i) {
+    if constexpr (V == 1) {
+      const int k = (first + i) * kRk + (tid & 63);
+      auto at = [&](int r) -> uint32_t { return t0 + r < T && k < H ? reinterpret_cast<const uint16_t*>(x)[(size_t)(t0 + r) * H + k] : 0; };
+#pragma unroll
+      for (int j = 0; j < 8; ++j) held[j] = at(grp + 8 * j) | at(grp + 8 * j + 4) << 16;
+    }
+  };
+  auto store_x = [&](int i) {
+    if constexpr (V == 1) {
+      uint16_t* dst = reinterpret_cast<uint16_t*>(xs) + (i % kRs) * kRt * kRx + (tid & 63);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        dst[(grp + 8 * j) * kRx] = (uint16_t)held[j];
+        dst[(grp + 8 * j + 4) * kRx] = (uint16_t)(held[j] >> 16);
       }
     }
   };
@@ -618,6 +632,8 @@ __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* 
     if (i < n) {
       fetch_w(i);
       fetch_x(i);
+      load_x(i);
+      store_x(i);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -629,6 +645,7 @@ __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* 
     if (i + kRs - 1 < n) {      // into the buffer that all have read before this barrier
       fetch_w(i + kRs - 1);
       fetch_x(i + kRs - 1);
+      load_x(i + kRs - 1);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* w = ws + (i % kRs) * kRe * kRw + tx * kRw + grp * 16;
@@ -649,6 +666,7 @@ __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* 
         for (int m = 0; m < 4; ++m) acc[m][j] = __ffma2_rn(make_float2(b.y, b.y), v[m][1], __ffma2_rn(make_float2(b.x, b.x), v[m][0], acc[m][j]));
       }
     }
+    if (i + kRs - 1 < n) store_x(i + kRs - 1);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
@@ -680,7 +698,7 @@ __global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const bf16* 
   cluster.sync();      // the last sums have been read
 }
 
-template <bool V>
+template <int V>
 static int launch_router_tiles(const bf16* x, const float* rw, int H, int E, int T, int sms, float* logits, cudaStream_t stream) {
   static PkDeviceOnce once;
   if (PkDeviceOnceGuard g{once}; g.needed()) {
@@ -999,10 +1017,9 @@ PK_API int pk_router_topk(const void* x, const float* router_w, const float* bia
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return PK_ERR_CUDA;
   if (router_tiles(T, E, H, sms)) {
-    const bool v = (H & 7) == 0 && (((uintptr_t)x | (uintptr_t)router_w) & 15) == 0;
-    if (const int rc = v ? launch_router_tiles<true>((const pk::bf16*)x, router_w, H, E, T, sms, logits, stream)
-                         : launch_router_tiles<false>((const pk::bf16*)x, router_w, H, E, T, sms, logits, stream))
-      return rc;
+    const bool by16 = (H & 7) == 0 && (((uintptr_t)x | (uintptr_t)router_w) & 15) == 0, by4 = (H & 1) == 0 && ((uintptr_t)x & 3) == 0;
+    const auto launch = by16 ? launch_router_tiles<8> : by4 ? launch_router_tiles<2> : launch_router_tiles<1>;
+    if (const int rc = launch((const pk::bf16*)x, router_w, H, E, T, sms, logits, stream)) return rc;
   } else
     PK_LAUNCH_PDL(router_logits_kernel, dim3((E + 7) / 8, (T + 7) / 8), dim3(256), smem_x, stream, (const pk::bf16*)x, router_w, H, E, T, logits);
   PK_CHECK_LAUNCH();
