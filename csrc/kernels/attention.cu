@@ -6,6 +6,8 @@
 //
 // Positions are read from device memory so that one captured CUDA graph serves every
 // decode step; the split count is a launch constant and empty splits return at once.
+#include <algorithm>
+
 #include "../common/pk_common.cuh"
 
 namespace {
@@ -47,6 +49,24 @@ __global__ void __launch_bounds__(32 * kQkWarps) qk_norm_rope_append_kernel(cons
   const bf16* row = p.proj + (size_t)m * p.ld;
   const int pos = p.pos[m], hr = p.rotary_dim >> 1;
   const bool in_cache = pos >= 0 && pos < p.ctx_cap;
+  auto load4 = [](const bf16* x) {
+    if (((uintptr_t)x & 7) == 0) return *reinterpret_cast<const uint2*>(x);
+    const uint16_t* u = reinterpret_cast<const uint16_t*>(x);
+    return make_uint2(u[0] | (uint32_t)u[1] << 16, u[2] | (uint32_t)u[3] << 16);
+  };
+  auto unpack4 = [](const uint2& u) {
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+  };
+  // A head's channels, and a key head's values: the first one's are on their way while the angles are computed.
+  uint2 xn = make_uint2(0u, 0u), vn = make_uint2(0u, 0u);
+  auto fetch = [&](int hh) {
+    if (hh >= p.Hq + p.Hkv) return;
+    const bf16* at = row + (hh < p.Hq ? hh * 2 * kD : p.Hq * kD + hh * kD) + d;
+    xn = load4(at);
+    if (hh >= p.Hq) vn = load4(at + p.Hkv * kD);
+  };
+  const int first = blockIdx.y * kQkWarps + warp;
+  fetch(first);
   for (int i = threadIdx.x; i < hr; i += 32 * kQkWarps) {
     const double inv_freq = pow((double)p.theta, -2.0 * (double)i / (double)p.rotary_dim);
     double sn, cs;
@@ -54,17 +74,11 @@ __global__ void __launch_bounds__(32 * kQkWarps) qk_norm_rope_append_kernel(cons
     s_cs[i] = make_float2((float)cs, (float)sn);
   }
   __syncthreads();
-  auto load4 = [](const bf16* x) {
-    if (((uintptr_t)x & 7) == 0) {
-      const uint2 u = *reinterpret_cast<const uint2*>(x);
-      return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
-    }
-    return make_float4(__bfloat162float(x[0]), __bfloat162float(x[1]), __bfloat162float(x[2]), __bfloat162float(x[3]));
-  };
-  for (int hh = blockIdx.y * kQkWarps + warp; hh < p.Hq + p.Hkv; hh += gridDim.y * kQkWarps) {
+  for (int hh = first; hh < p.Hq + p.Hkv; hh += gridDim.y * kQkWarps) {
     const bool is_q = hh < p.Hq;
     const int hk = hh - p.Hq;
-    const float4 x = load4(row + (is_q ? hh * 2 * kD : p.Hq * 2 * kD + hk * kD) + d);
+    if (hh != first) fetch(hh);
+    const float4 x = unpack4(xn), v4 = unpack4(vn);
     const float* gamma = (is_q ? p.q_gamma : p.k_gamma) + d;
     const float r = rsqrtf(warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w) / (float)kD + p.eps);
     float y[4] = {x.x * r * (1.f + gamma[0]), x.y * r * (1.f + gamma[1]), x.z * r * (1.f + gamma[2]), x.w * r * (1.f + gamma[3])};
@@ -98,7 +112,6 @@ __global__ void __launch_bounds__(32 * kQkWarps) qk_norm_rope_append_kernel(cons
       continue;
     }
     if (!in_cache && lane == 0) PK_DEBUG_RECORD(101, pos, p.ctx_cap);   // the row is not written (below)
-    const float4 v4 = load4(row + p.Hq * 2 * kD + p.Hkv * kD + hk * kD + d);
     const float v[4] = {v4.x, v4.y, v4.z, v4.w};
     const size_t ri = (size_t)hk * p.ctx_cap + pos;
     if (p.kv_fp8) {
@@ -539,8 +552,10 @@ PK_API int pk_qk_norm_rope_append_kv(const void* proj, int ld, int M, int Hq, in
   if (M < 1 || rotary_dim < 0 || rotary_dim > kD || (rotary_dim & 1) || (kscale == nullptr) != (vscale == nullptr)) return PK_ERR_BAD_ARG;
   QkParams p{(const pk::bf16*)proj, ld, M, Hq, Hkv, pos, q_gamma, k_gamma, eps, rotary_dim, theta,
              (pk::bf16*)q_out, (pk::bf16*)kcache, (pk::bf16*)vcache, ctx_cap, kscale != nullptr ? 1 : 0, kscale, vscale};
-  // few rows: a row's heads over several blocks
-  const int per_row = M <= 37 ? (Hq + Hkv + kQkWarps - 1) / kQkWarps : M <= 148 ? 2 : 1;
+  // Few rows: a row's heads over several blocks, up to four to an SM; more blocks cost more in angles than they gain. 40 + 8 heads, us by blocks to
+  // a row (1 / 2 / 3 / 6): 38 rows 6.2 / 4.2 / 3.6 / 3.0, 64 rows 6.2 / 4.2 / 3.9 / 3.6, 149 rows 6.5 / 5.7 / 4.7 / 5.9, 256 rows 7.0 / 5.8 / 7.6 / 8.5, 400 rows
+  // 9.1 / 9.3 / 10.3 / 12.8.
+  const int per_row = std::max(1, std::min((Hq + Hkv + kQkWarps - 1) / kQkWarps, 4 * 148 / M));
   PK_LAUNCH_PDL(qk_norm_rope_append_kernel, dim3(M, per_row), dim3(32 * kQkWarps), 0, stream, p);
   return PK_OK;
 }
