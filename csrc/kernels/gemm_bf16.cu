@@ -16,6 +16,10 @@
 //
 // us (before: a lone lane computed descriptors and issued, partial tiles and residuals were read a row at a time, stream-K from 96 k steps a group
 // on): 1900 rows of 5120 x 4096 96 -> 78, 4096 x 4096 with a residual 90 -> 70, 10304 x 4096 159 -> 133; 512 rows of 5120 x 17408 122 -> 92.
+//
+// Launches over groups request a stage's rows of A before its weights and let their dependents start when they end, plain ones the other way round.
+// Medians, us, weights first and early start / weights first / rows first / neither: 64 groups, 24000 rows, 2048 x 2048 291 / 268 / 289 / 265, 8 groups, 12000
+// rows, 4096 x 4096 411 / 408 / 390 / 399; 512 rows of 5120 x 17408 without groups 108 / 108 / 111 / 112.
 #include <cstdlib>
 #include <mutex>
 
@@ -244,12 +248,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
           const int s = it % kStages;
           if (!mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1, &sm.abort_flag, p.status, 21)) break;
+          if (it >= ahead) mbar_arrive_expect_tx(&sm.full[s], kABytes + kBBytes);
+          if (p.seg != nullptr) tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * BK, a_row);
           if (it >= ahead) {
-            mbar_arrive_expect_tx(&sm.full[s], kABytes + kBBytes);
             tma_load_2d(sm.b[s], &tmap_w, &sm.full[s], kb * BK, r0);
             tma_load_2d(sm.b[s] + kBBytes / 2, &tmap_w, &sm.full[s], kb * BK, r1);
           }
-          tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * BK, a_row);
+          if (p.seg == nullptr) tma_load_2d(sm.a[s], &tmap_a, &sm.full[s], kb * BK, a_row);
           issued = it + 1;
         }
       }
@@ -309,7 +314,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       return reinterpret_cast<float4*>(p.ws + (size_t)slot * BM * BN) + (((c0 & 127) >> 5) * 8 + v) * kEpiThreads + (c0 >> 7) * 128 + q * 32 + lane;
     };
     pk::pdl_wait();
-    pk::pdl_trigger();
+    if (p.seg == nullptr) pk::pdl_trigger();
     int local = 0;
     WorkIter work(p, num_kb, tiles_m);
     Seg sg;
