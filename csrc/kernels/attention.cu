@@ -218,7 +218,7 @@ __device__ __forceinline__ void unpack_kv8(const Kv8& r, bool fp8, float (&f)[8]
 template <int G, int AHEAD>
 __global__ void __launch_bounds__(128) gqa_decode_split_kernel(const DecodeParams p) {
   pk::pdl_wait();
-  pk::pdl_trigger();
+  pk::pdl_trigger_few();      // 8 rows of 40 heads, 20 keys in 8 splits, with the merge: 8.0 -> 6.1 us; 5 rows, 210 keys in 16 12.1 -> 9.4
   const int hk = blockIdx.x, split = blockIdx.y, m = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int l16 = lane & 15, khalf = lane >> 4;
@@ -419,7 +419,7 @@ struct FullQkParams {
 
 __global__ void __launch_bounds__(256) full_qk_norm_rope_append_kernel(const FullQkParams p) {
   pk::pdl_wait();
-  pk::pdl_trigger();
+  pk::pdl_trigger_few();
   __shared__ float red[40];
   const int t = blockIdx.x, is_k = blockIdx.y, tid = threadIdx.x;
   const int H = is_k ? p.Hkv : p.Hq, n = H * kD;
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(256) full_qk_norm_rope_append_kernel(const Ful
 constexpr int kFullQkThreads = 512, kFullQkVecRows = 128;
 __global__ void __launch_bounds__(kFullQkThreads) full_qk_norm_rope_append_vec_kernel(const FullQkParams p) {
   pk::pdl_wait();
-  pk::pdl_trigger();
+  pk::pdl_trigger_few();
   extern __shared__ __align__(16) float xs[];      // [heads * D]
   __shared__ float red[40];
   const int t = blockIdx.x, is_k = blockIdx.y, tid = threadIdx.x;

@@ -749,10 +749,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* logits, c
                                                           int topk, int score_func, int norm_topk, float route_scale,
                                                           int* ids, float* weights) {
   pk::pdl_wait();
-  // Of many tokens the blocks that wait here fill their SMs, and blocks of a launch behind them would come to lie several to an SM where some have
-  // gone first while other SMs stay empty (routing the same tokens again and again, 592 by 8 experts of 1024 13.2 -> 11.7 us, 1000 by 256 of 3072 95 -> 57):
-  // those begin as these end.
-  if (gridDim.x <= 2 * 148) pk::pdl_trigger();
+  pk::pdl_trigger_few();      // routing the same tokens again and again: 592 by 8 experts of 1024 13.2 -> 11.2 us, 1000 by 256 of 3072 95 -> 57
   extern __shared__ float sm[];  // [E] scores, [E] selection keys
   float* sc = sm;
   float* key = sc + E;

@@ -47,7 +47,7 @@ struct NormParams {
 
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const NormParams p) {
   pk::pdl_wait();
-  pk::pdl_trigger();
+  pk::pdl_trigger_few();
   extern __shared__ float row[];
   __shared__ float red[40];
   const int m = blockIdx.x;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const NormParams p) {
 // two bytes, waits and goes on).
 __global__ void __launch_bounds__(256) rmsnorm_vec_kernel(const NormParams p) {
   pk::pdl_wait();
-  pk::pdl_trigger();
+  pk::pdl_trigger_few();
   extern __shared__ __align__(16) float row[];
   __shared__ float red[40];
   const size_t base = (size_t)blockIdx.x * p.K;
