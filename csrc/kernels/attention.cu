@@ -534,7 +534,7 @@ PK_API int pk_full_qk_norm_rope_append(const void* q, int ldq, const void* k, in
   if ((at & 15) == 0 && ((ldq | ldk | ldv) & 7) == 0 && (rope_dim & 15) == 0 && smem <= kPlainSmem && T <= kFullQkVecRows)
     PK_LAUNCH_PDL(full_qk_norm_rope_append_vec_kernel, dim3(T, 2), dim3(kFullQkThreads), smem, stream, p);
   else
-    PK_LAUNCH_PDL(full_qk_norm_rope_append_kernel, dim3(T, 2), dim3(256), 0, stream, p);
+    PK_LAUNCH_PDL_L1(full_qk_norm_rope_append_kernel, dim3(T, 2), dim3(256), 0, stream, p);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }

@@ -1047,7 +1047,7 @@ PK_API int pk_group_routes(const int* ids, const float* weights, int T, int topk
       once_guard.done();
     }
   }
-  PK_LAUNCH_PDL(group_routes_kernel, dim3(1), dim3(warps * 32), smem, stream, ids, weights, T, topk, E, seg_start, route_token, route_weight, route_src);
+  PK_LAUNCH_PDL_L1(group_routes_kernel, dim3(1), dim3(warps * 32), smem, stream, ids, weights, T, topk, E, seg_start, route_token, route_weight, route_src);
   PK_CHECK_LAUNCH();
   return PK_OK;
 }
@@ -1063,7 +1063,7 @@ PK_API int pk_moe_reduce_routes(const float* ybuf, const float* route_weight, co
   const int R = T * topk;
   PK_LAUNCH_PDL(invert_routes_kernel, dim3((R + 255) / 256), dim3(256), 0, stream, route_src, R, route_pos);
   PK_CHECK_LAUNCH();
-  PK_LAUNCH_PDL(moe_reduce_routes_weighted_kernel, dim3((H + 255) / 256, T), dim3(256), 0, stream, ybuf, route_weight, route_pos, seg_start, topk, H, expert_offset,
+  PK_LAUNCH_PDL_L1(moe_reduce_routes_weighted_kernel, dim3((H + 255) / 256, T), dim3(256), 0, stream, ybuf, route_weight, route_pos, seg_start, topk, H, expert_offset,
                                                                                   local_experts, y);
   PK_CHECK_LAUNCH();
   return PK_OK;
@@ -1159,7 +1159,7 @@ PK_API int pk_gguf_dequant_rows(const void* W, int type, const int* rows, int nr
   const long long units = (long long)nrows * (K >> 8);
   const long long want = (units + 7) / 8;
   const int grid = (int)(want < 148LL * 32 ? want : 148LL * 32);
-  PK_LAUNCH_PDL(gguf_dequant_rows_kernel, dim3(grid), dim3(256), 0, stream, (const uint8_t*)W, type, rows, nrows, K, row_offset, table_rows,
+  PK_LAUNCH_PDL_L1(gguf_dequant_rows_kernel, dim3(grid), dim3(256), 0, stream, (const uint8_t*)W, type, rows, nrows, K, row_offset, table_rows,
                                                     (pk::bf16*)out);
   PK_CHECK_LAUNCH();
   return PK_OK;
