@@ -31,14 +31,13 @@ struct RelaxedCapture {
 };
 
 // Whether sharing pays: what whole tiles take against what the groups of CTAs take, in blocks of K, against the exchange of the parts. The
-// constants are fits to 174 (FP8, 65 to 3000 rows) and 143 (bf16, 33 to 3000 rows) shapes, each timed both ways; with them the slower way is taken in one of
-// either by more than 5 % (with whole tiles throughout 9 % are lost in the mean, with sharing throughout 6 and 5 %). us, whole tiles / shared: FP8,
+// constants are fits to 174 (FP8) and 97 (bf16) shapes of 65 to 3000 rows, each timed both ways; with them the slower way is taken in one of them
+// by more than 5 % (with whole tiles throughout 9 and 11 % are lost in the mean, with sharing throughout 6 %). us, whole tiles / shared: FP8,
 // two terms, 512 rows, K x 5120, K = 1536 17 / 24, 2176 20 / 26, 4096 45 / 43, 17408 108 / 88; 2048 rows of 12288 x 5120 208 / 231; 128 rows, K = 17408,
-// 123 / 59; bf16, 300 rows of 10304 x 4096 36 / 39, 1900 of 1088 x 1024 14 / 19, 33 of 20480 x 4096 38 / 44, 129 of it 60 / 50, 512 88 / 79.
+// 123 / 59; bf16, 300 rows of 10304 x 4096 36 / 39, 1900 of 1088 x 1024 14 / 19, 168 of 10304 x 4096 45 / 43.
 struct StreamKCost {
   int least;                      // blocks of a group
   double fixed, part, share;      // of the exchange, for each part of a tile, for each block of a group
-  double stream;                  // for each block of a group of few rows: the SMs that whole tiles leave idle would only divide the weights' bandwidth
 };
 inline bool streamk_pays(int tiles_m, int tiles_n, int num_kb, int sms, const StreamKCost& c) {
   const StreamKMode mode = streamk_mode();
@@ -46,7 +45,7 @@ inline bool streamk_pays(int tiles_m, int tiles_n, int num_kb, int sms, const St
   if (mode == StreamKMode::never || groups < 2 || tiles >= 0.88 * rounds * sms || (long long)tiles_n * num_kb < (long long)groups * c.least) return false;
   if (mode == StreamKMode::forced) return true;
   const double shared = (double)tiles_n * num_kb / groups, parts = groups > tiles_n ? (double)groups / tiles_n : 1.;
-  return (double)rounds * num_kb - shared > c.fixed + c.part * parts + (c.share + c.stream / (tiles_m * tiles_m)) * shared;
+  return (double)rounds * num_kb - shared > c.fixed + c.part * parts + c.share * shared;
 }
 
 // Work spaces by stream, since launches on several streams can run at the same time: at most `kStreamKStreams` per device (19 MB each with

@@ -648,7 +648,7 @@ static int gemm(const void* A, int lda, const void* W, bool w_held, int M, int N
   const int sms = sm_count > 0 ? sm_count : 148;
   int grid = tiles < sms ? tiles : sms;
   // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time) and that is more than the exchange.
-  constexpr pk::StreamKCost kCost{8, 6., 8., 0., 1.};
+  constexpr pk::StreamKCost kCost{8, 2., 8., 0.1};
   p.streamk = 0;
   if (pk::StreamK b; pk::streamk_pays(p.tiles_m, p.tiles_n, K / BK, sms, kCost) && pk::streamk_take(sms, stream, b)) {
     p.streamk = 1;

@@ -618,7 +618,7 @@ static int gemm(const void* Aq, int terms, int m_pad, const float* a_scale, int 
   int grid = tiles < sms ? tiles : sms;
   const int num_kb = K / BK;
   // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time) and that is more than the exchange.
-  constexpr pk::StreamKCost kCost{4, 4., 4., 0.1, 0.};
+  constexpr pk::StreamKCost kCost{4, 4., 4., 0.1};
   if (pk::StreamK b; pk::streamk_pays(p.tiles_m, p.tiles_n, num_kb, sms, kCost) && pk::streamk_take(sms, stream, b)) {
     p.streamk = 1;
     p.ws = b.ws;
