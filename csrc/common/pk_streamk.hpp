@@ -14,13 +14,11 @@ struct StreamK {
   uint32_t seq = 0;             // this launch's
 };
 
-// The schedule is taken where `streamk_pays` says so; POCKET_GEMM_NO_STREAMK or POCKET_GEMM_STREAMK=0 turn it off, POCKET_GEMM_STREAMK=1 takes it
-// wherever whole tiles would leave SMs idle and a group of CTAs gets some blocks.
-enum class StreamKMode { never, cost, forced };
-inline StreamKMode streamk_mode() {
-  if (getenv("POCKET_GEMM_NO_STREAMK") != nullptr) return StreamKMode::never;
+// The schedule is the default wherever whole tiles would leave SMs idle; POCKET_GEMM_NO_STREAMK or POCKET_GEMM_STREAMK=0 turn it off.
+inline bool streamk_allowed() {
+  if (getenv("POCKET_GEMM_NO_STREAMK") != nullptr) return false;
   const char* v = getenv("POCKET_GEMM_STREAMK");
-  return v == nullptr ? StreamKMode::cost : v[0] == '1' ? StreamKMode::forced : StreamKMode::never;
+  return v == nullptr || v[0] != '0';
 }
 
 // Allocations that another thread's capture does not mind.
@@ -29,24 +27,6 @@ struct RelaxedCapture {
   RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
-
-// Whether sharing pays: what whole tiles take against what the groups of CTAs take, in blocks of K, against the exchange of the parts. The
-// constants are fits to 174 (FP8) and 97 (bf16) shapes of 65 to 3000 rows, each timed both ways; with them the slower way is taken in one of them
-// by more than 5 % (with whole tiles throughout 9 and 11 % are lost in the mean, with sharing throughout 6 %). us, whole tiles / shared: FP8,
-// two terms, 512 rows, K x 5120, K = 1536 17 / 24, 2176 20 / 26, 4096 45 / 43, 17408 108 / 88; 2048 rows of 12288 x 5120 208 / 231; 128 rows, K = 17408,
-// 123 / 59; bf16, 300 rows of 10304 x 4096 36 / 39, 1900 of 1088 x 1024 14 / 19, 168 of 10304 x 4096 45 / 43.
-struct StreamKCost {
-  int least;                      // blocks of a group
-  double fixed, part, share;      // of the exchange, for each part of a tile, for each block of a group
-};
-inline bool streamk_pays(int tiles_m, int tiles_n, int num_kb, int sms, const StreamKCost& c) {
-  const StreamKMode mode = streamk_mode();
-  const int tiles = tiles_m * tiles_n, rounds = (tiles + sms - 1) / sms, groups = tiles_m <= sms ? sms / tiles_m : 0;
-  if (mode == StreamKMode::never || groups < 2 || tiles >= 0.88 * rounds * sms || (long long)tiles_n * num_kb < (long long)groups * c.least) return false;
-  if (mode == StreamKMode::forced) return true;
-  const double shared = (double)tiles_n * num_kb / groups, parts = groups > tiles_n ? (double)groups / tiles_n : 1.;
-  return (double)rounds * num_kb - shared > c.fixed + c.part * parts + c.share * shared;
-}
 
 // Work spaces by stream, since launches on several streams can run at the same time: at most `kStreamKStreams` per device (19 MB each with
 // 148 SMs), one for each of the first streams that ask. The streams after them work whole tiles, and so does every stream under capture (a

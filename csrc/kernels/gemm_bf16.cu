@@ -647,16 +647,21 @@ static int gemm(const void* A, int lda, const void* W, bool w_held, int M, int N
   const int tiles = p.tiles_m * p.tiles_n;
   const int sms = sm_count > 0 ? sm_count : 148;
   int grid = tiles < sms ? tiles : sms;
-  // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time) and that is more than the exchange.
-  constexpr pk::StreamKCost kCost{8, 2., 8., 0.1};
+  // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time).
+  const int num_kb = K / BK;
+  const double rounds = (double)tiles / sms;
+  const double eff = rounds / (double)((tiles + sms - 1) / sms);
   p.streamk = 0;
-  if (pk::StreamK b; pk::streamk_pays(p.tiles_m, p.tiles_n, K / BK, sms, kCost) && pk::streamk_take(sms, stream, b)) {
+  const int groups = p.tiles_m <= sms ? sms / p.tiles_m : 0;
+  // us without and with (eight k steps to a group of CTAs at least): 512 rows, N = 5120, K = 4096 43 / 42, 168 rows, N = 10304 45 / 43. (Before the
+  // parts were laid out by threads, the exchange took 20 us and paid only from 96 k steps on.)
+  if (pk::StreamK b; eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 8 && pk::streamk_allowed() && pk::streamk_take(sms, stream, b)) {
     p.streamk = 1;
     p.ws = b.ws;
     p.flags = b.flags;
     p.seq = b.seq;
     p.timeout_us = 2000000;
-    grid = sms / p.tiles_m * p.tiles_m;
+    grid = groups * p.tiles_m;
   }
   PK_LAUNCH_PDL(gemm_bf16_kernel, dim3(grid), dim3(kThreads), smem, stream, tmap_a, tmap_w, p);
   PK_CHECK_LAUNCH();

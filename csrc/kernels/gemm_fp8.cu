@@ -617,15 +617,19 @@ static int gemm(const void* Aq, int terms, int m_pad, const float* a_scale, int 
   const int sms = sm_count > 0 ? sm_count : 148;
   int grid = tiles < sms ? tiles : sms;
   const int num_kb = K / BK;
-  // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time) and that is more than the exchange.
-  constexpr pk::StreamKCost kCost{4, 4., 4., 0.1};
-  if (pk::StreamK b; pk::streamk_pays(p.tiles_m, p.tiles_n, num_kb, sms, kCost) && pk::streamk_take(sms, stream, b)) {
+  const double rounds = (double)tiles / sms;
+  const double eff = rounds / (double)((tiles + sms - 1) / sms);
+  const int groups = p.tiles_m <= sms ? sms / p.tiles_m : 0;
+  // Stream-K when whole tiles would leave many SMs idle in the last round (or the whole time), four k blocks to a group of CTAs at least.
+  // us without and with: 512 rows, N = 5120, K = 4096 45 / 43, K = 5120 51 / 48; 128 rows, N = 5120, K = 17408 123 / 59, N = 12288, K = 5120
+  // 47 / 41. (Before the parts were laid out by threads, the exchange took 15 us and paid only from 48 k blocks on.)
+  if (pk::StreamK b; eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 4 && pk::streamk_allowed() && pk::streamk_take(sms, stream, b)) {
     p.streamk = 1;
     p.ws = b.ws;
     p.flags = b.flags;
     p.seq = b.seq;
     p.timeout_us = 2000000;
-    grid = sms / p.tiles_m * p.tiles_m;
+    grid = groups * p.tiles_m;
   }
   return terms == 1 ? launch<1>(tmap_a, tmap_w, p, grid, stream) : launch<2>(tmap_a, tmap_w, p, grid, stream);
 }
@@ -650,7 +654,7 @@ PK_API int pk_gemm_fp8_held(const void* Aq, int terms, int m_pad, const float* a
 PK_API void pk_gemm_reserve(int sm_count, cudaStream_t stream) {
   pk::StreamKPool& pool = pk::streamk_pool();
   std::lock_guard<std::mutex> lock(pool.mu);
-  if (pk::streamk_mode() != pk::StreamKMode::never) pool.of(stream, sm_count > 0 ? sm_count : 148, true);
+  if (pk::streamk_allowed()) pool.of(stream, sm_count > 0 ? sm_count : 148, true);
 }
 PK_API void pk_gemm_release(cudaStream_t stream) {
   pk::StreamKPool& pool = pk::streamk_pool();

@@ -299,7 +299,6 @@ def test_stream_k_on_several_streams_and_under_capture(M, N, K, monkeypatch):
     """Tiles whose K is shared: launches on more streams than there are work spaces, and replays of a captured launch with new rows, which
     is the schedule of whole tiles to the bit."""
     from pocketllm_b200 import ops
-    monkeypatch.setenv("POCKET_GEMM_STREAMK", "1")
     w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
     xs = [torch.randn(M, K, device="cuda").to(torch.bfloat16) for _ in range(10)]
     want = [x.float() @ w.float().t() for x in xs]
@@ -346,7 +345,6 @@ want = x.float() @ w.float().t()
 os.environ["POCKET_GEMM_NO_STREAMK"] = "1"
 whole = ops.gemm_bf16(x, w, epi=ops.EPI_F32)
 del os.environ["POCKET_GEMM_NO_STREAMK"]
-os.environ["POCKET_GEMM_STREAMK"] = "1"
 streams, outs = [stream() for _ in range(12)], []
 def launches(which, rounds):
     for _ in range(rounds):
