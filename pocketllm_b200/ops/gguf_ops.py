@@ -315,7 +315,7 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
                              routes: "Routes", *, expert_offset: int = 0, local_experts: int | None = None,
                              out: torch.Tensor | None = None, peer=None, status: torch.Tensor | None = None) -> torch.Tensor:
     """Routed experts of this rank on the tensor cores, for steps with many routes (prefill). Types in `UMMA_TYPES` are decoded
-    inside the product up to `_umma_max_routes`; otherwise the rank's experts are decoded to bf16 once per call
+    inside the product up to `UMMA_MAX_ROUTES_PER_EXPERT`; otherwise the rank's experts are decoded to bf16 once per call
     into a scratch that is reused across layers, token rows are gathered in expert order, and two
     grouped tcgen05 GEMMs (gate|up with the SwiGLU epilogue, then down) run one persistent launch each over every
     (expert, row tile, column block) that has rows; the tile list comes from the route segments on the device. The
@@ -331,7 +331,7 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     if out is None:
         out = torch.zeros(T, H, device=dev, dtype=torch.float32)
     K = _lib.kernels()
-    if R <= _umma_max_routes(H, inter) * E and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
+    if R <= UMMA_MAX_ROUTES_PER_EXPERT * E and _umma_experts_take(w13_raw, w2_raw, type13, type2, H, inter, local):
         ybuf = _umma_experts(x, w13_raw, w2_raw, type13, type2, inter, routes, 0.0, E, expert_offset, local, 1, status)
     else:
         key = (dev.index, local, H, inter)
@@ -367,16 +367,10 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     return _reduce_routes(ybuf, routes, x.shape, expert_offset, local, out)
 
 
-def _umma_max_routes(H: int, inter: int) -> int:
-    """Routes per expert, in the mean, up to which blocks are decoded inside the product. Beyond, a decode per 64 routes costs more than one decode to a
-    bf16 scratch; the smaller the matrices, the earlier, since a tile with few blocks of K has little to set against filling and folding. Time inside
-    the product over that with the scratch, routes spread at random, IQ2_XXS / Q4_K / Q5_K, at 192, 256, 320, 384 routes: 512 x 1024
-    1.04 / .97 / .97, 1.21 / 1.14 / 1.14 ...; 768 x 2048 .81 / .78 / .79, .95 / .91 / .95, 1.07 / 1.04 / 1.06, 1.14 / 1.13 / 1.17; 1024 x 2048 .78 / .76 / .76,
-    .93 / .89 / .91, 1.03 / .99 / 1.03, 1.15 / 1.12 / 1.15; 1536 x 3072 .63 / .61 / .64, .76 / .73 / .76, .86 / .84 / .87, .94 / .91 / .96, even at 448;
-    1536 x 4096 .65 / .59 / .62, .77 / .70 / .75, .87 / .82 / .85, .94 / .89 / .94."""
-    return 384 if H * inter > 1 << 22 else 256 if H * inter >= 3 << 19 else 192
-
-
+UMMA_MAX_ROUTES_PER_EXPERT = 384      # far above this a decode per 64 routes costs more than one decode to a bf16 scratch, us: 256 experts of the
+#                                        MiniMax-M2 shape, IQ2_XXS, 192 routes 3081 against 6452, 384 6342 / 7867, 512 8399 / 8999; 64 experts of
+#                                        2 x 1536 x 3072, 384 routes, IQ2_XXS 1602 / 2029, Q4_K 1666 / 2151, Q5_K 1991 / 2357; of 2 x 1024 x 2048, 384
+#                                        routes, IQ2_XXS 910 / 999, Q5_K 1089 / 1145, 512 routes 1186 / 1127, 1419 / 1275
 GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local expert costs more than the route kernels' per-route decode
 
 
