@@ -1291,7 +1291,8 @@ void QwenEngine::run_chunk(int M, bool mtp, bool more) {
       gemm(xn_, hidden_, L.in_proj, 0, proj_, nullptr, ld_proj_);
       check(pk_linear_narrow(xn_, hidden_, L.in_proj_ab, M, 2 * vh_l_, hidden_, (char*)proj_ + (size_t)L.in_proj.N * 2, ld_proj_, stream_),
             "linear_narrow(ab)");
-      // token by token up to 48 rows: 32 / 48 / 64 rows of 32 heads 32 / 46 / 60 us against 48 / 49 / 47 in chunks of 64
+      // token by token up to 48 rows, us against chunks of 64 at 40 / 48 / 56 rows: 32 value heads 40 / 46 / 54 against 43, 16 and fewer (a rank's share)
+      // 32 / 38 / 44 against 42, 64 47 / 55 / 64 against 55
       if (M > 48) {
         check(pk_deltanet_chunked(proj_, ld_proj_, M, kh_l_, vh_l_, kHeadDim, kHeadDim, L.conv_w, L.conv_state, L.A_log,
                                   L.dt_bias, L.lin_norm, eps, L.lin_state, attn_out_, lin_ws_, stream_),

@@ -537,9 +537,6 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Per-device stream-K scratch: one fp32 tile and one flag per CTA. Allocated on first use.
-
-
 bool encode_bf16_2d(EncodeTiledFn encode, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
                     uint32_t box_inner, uint32_t box_outer) {
   const cuuint64_t gdim[2] = {inner, outer};
@@ -653,8 +650,10 @@ static int gemm(const void* A, int lda, const void* W, bool w_held, int M, int N
   const double eff = rounds / (double)((tiles + sms - 1) / sms);
   p.streamk = 0;
   const int groups = p.tiles_m <= sms ? sms / p.tiles_m : 0;
-  // us without and with (eight k steps to a group of CTAs at least): 512 rows, N = 5120, K = 4096 43 / 42, 168 rows, N = 10304 45 / 43. (Before the
-  // parts were laid out by threads, the exchange took 20 us and paid only from 96 k steps on.)
+  // us without and with (eight k steps to a group of CTAs at least): 512 rows, N = 5120, K = 4096 43 / 42, 168 rows, N = 10304 45 / 43, K =
+  // 17408 107 / 81. (Before the parts were laid out by threads, the exchange took 20 us and paid only from 96 k steps on.) Over 143 shapes of 33 to 3000 rows sharing
+  // is 5 % faster in the mean; it loses where K is short (1900 rows of 1088 x 1024 13 / 20, 129 of 16384 x 2048 19 / 29) or the weights' bandwidth bounds whole
+  // tiles too (33 rows of 20480 x 4096 38 / 44). Those share all the same: whole tiles would add in another order.
   if (pk::StreamK b; eff < 0.88 && groups >= 2 && (long long)p.tiles_n * num_kb >= (long long)groups * 8 && pk::streamk_allowed() && pk::streamk_take(sms, stream, b)) {
     p.streamk = 1;
     p.ws = b.ws;

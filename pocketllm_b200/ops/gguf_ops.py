@@ -59,7 +59,8 @@ UMMA_TYPES = frozenset({"iq2_xxs", "q4_k", "q5_k"})
 # Against decoding per eight rows or (from 32 rows) to a bf16 scratch, 4096 x 4096 / 8192 x 3072 / 24576 x 6144, us: IQ2_XXS, 256 rows
 # 28 / 36 / 187 against 47 / 58 / 244, 384 rows 45 / 54 / 242 against 47 / 60 / 288, 512 rows 48 / 72 / 310 against 50 / 66 / 285; Q4_K, 384 rows
 # 44 / 57 / 226 against 51 / 65 / 308; Q5_K, 256 rows 30 / 45 / 220 against 54 / 73 / 297, 384 rows 58 / 70 / 280 against 54 / 81 / 339, 512 rows
-# 63 / 90 / 365 against 61 / 78 / 337. Up to 2^24 weights their tiles fill the SMs a second time from 257 rows on.
+# 63 / 90 / 365 against 61 / 78 / 337. Up to 2^24 weights the line stays at 256 rows, from when the kernel was slower: with 257 to 384 rows it takes 0.32 to 0.93 of
+# the scratch's time at 4096 x 4096, 8192 x 2048, 2048 x 8192 and 1024 x 16384.
 UMMA_MAX_ROWS, UMMA_MAX_ROWS_LARGE = 257, 385
 UMMA_SPLIT_ROUTES = 64
 UMMA_MAX_GROUPS = 512
@@ -78,7 +79,8 @@ def _registers_faster(type_name: str, rows: int, weights: int) -> bool:
     a multiply-add per weight and row. Weights from memory, us: one row of 2048 x 2048 / 4096 x 4096 / 8192 x 3072, IQ2_XXS 6.5 against
     13.3, 14.2 / 15.9, 20.4 / 16.9; Q4_K 7.9 / 11.9, 17.4 / 15.0, 23.5 / 16.3; Q5_K 8.8 / 12.8, 21.2 / 16.6, 27.4 / 17.9. Four rows of
     2048 x 2048: 12.3 / 13.6, 13.2 / 12.1, 14.1 / 12.5; eight 19.9 / 13.5, 20.1 / 12.3, 21.1 / 12.9. Lines at half these
-    sizes would be up to 3 us faster; they stay, and with them the order in which single rows and pairs of rows have been added."""
+    sizes would be up to 3 us faster (one row of 8192 x 3072 in IQ2_XXS); they stay, since the two forms add in other orders, and a row's bits
+    would change with the line."""
     if rows > 8:
         return False
     width = 1 << (rows - 1).bit_length()        # the kernels have one, two, four or eight rows
@@ -367,10 +369,12 @@ def gguf_moe_forward_grouped(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: tor
     return _reduce_routes(ybuf, routes, x.shape, expert_offset, local, out)
 
 
-UMMA_MAX_ROUTES_PER_EXPERT = 384      # far above this a decode per 64 routes costs more than one decode to a bf16 scratch, us: 256 experts of the
-#                                        MiniMax-M2 shape, IQ2_XXS, 192 routes 3081 against 6452, 384 6342 / 7867, 512 8399 / 8999; 64 experts of
-#                                        2 x 1536 x 3072, 384 routes, IQ2_XXS 1602 / 2029, Q4_K 1666 / 2151, Q5_K 1991 / 2357; of 2 x 1024 x 2048, 384
-#                                        routes, IQ2_XXS 910 / 999, Q5_K 1089 / 1145, 512 routes 1186 / 1127, 1419 / 1275
+UMMA_MAX_ROUTES_PER_EXPERT = 384      # far above this a decode per 64 routes costs more than one decode to a bf16 scratch. Time inside the product over that
+#                                        with the scratch, routes spread at random, IQ2_XXS / Q4_K / Q5_K, at 192, 256, 320, 384 routes: 1536 x 3072 .63 / .61 / .64,
+#                                        .76 / .73 / .76, .86 / .84 / .87, .94 / .91 / .96, even at 448; 1024 x 2048 .78 / .76 / .76, .93 / .89 / .91, 1.03 / .99 / 1.03,
+#                                        1.15 / 1.12 / 1.15; 768 x 2048 .81 / .78 / .79, .95 / .91 / .95, 1.07 / 1.04 / 1.06, 1.14 / 1.13 / 1.17. The smaller matrices,
+#                                        whose tiles have few blocks of K to set against filling and folding, lose from 300 routes on; hidden values keep 11 bits
+#                                        here and 8 with the scratch, so the line is the same for all
 GROUPED_MIN_ROUTES_PER_EXPERT = 4     # below this the decode of every local expert costs more than the route kernels' per-route decode
 
 
