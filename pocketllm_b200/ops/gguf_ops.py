@@ -152,12 +152,17 @@ def _umma_cost(tiles: int, K: int, parts: int, slots: int, columns: int) -> floa
     IQ2_XXS, 192 tiles of K = 3072 22.5 / 26.6 / 29.4 (1 / 2 / 3), 24 tiles 20.5 / 18.4 / 16.4 / 16.4 (1 / 2 / 4 / 6); Q5_K, 24 tiles of K =
     6144, 16 columns 32.7 / 23.4 / 19.2 / 17.2 / 22.6 (1 / 2 / 4 / 6 / 8), 64 columns 36.9 / 27.6 / 24.6 / 25.4 / 36.8; 64 tiles of K = 3072
     22.5 / 18.5 / 22.5 (1 / 2 / 3); Q4_K, 256 tiles 28.7 / 38.9 / 43.0."""
-    return -(-tiles * parts // slots) * (K / 256 / parts + (3 + parts * columns / 32 if parts > 1 else 0))
+    return -(-tiles * parts // slots) * (K / 256 / parts + (3 + parts * columns / 32 if parts > 1 and columns else 0))
 
 
-def _umma_splits(tiles: int, K: int, slots: int, columns: int) -> int:
-    """Parts of K for `tiles` tiles of `columns` columns on `slots` CTAs, two 256-weight blocks in a part at least."""
+def _umma_splits(tiles: int, K: int, slots: int, columns: int = 0) -> int:
+    """Parts of K for `tiles` tiles of `columns` columns on `slots` CTAs (columns 0: as if the exchange cost nothing, which no product asks for), two
+    256-weight blocks in a part at least."""
     return min(range(1, max(1, min(K // 512, 4 * slots // tiles)) + 1), key=lambda s: _umma_cost(tiles, K, s, slots, columns))
+
+
+def _umma_slots(type_name: str, columns: int) -> int:
+    return _sm_count()      # resident CTAs of the kernel: one an SM for every type and tile
 
 
 def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, gamma, eps: float, epi: int,
@@ -165,7 +170,7 @@ def _umma_linear(x: torch.Tensor, w_raw: torch.Tensor, type_name: str, N: int, g
     M, K = x.shape
     columns = 16 if M <= 16 else 32 if M <= 32 else 64
     tiles = (-(-(N // 2) // 64) if epi == 1 else -(-N // 128)) * -(-M // columns)
-    splits = _umma_splits(tiles, K, _sm_count(), columns)      # a CTA per SM
+    splits = _umma_splits(tiles, K, _umma_slots(type_name, columns), columns)
     st = _Staged(x, type_name, M, 1, gamma=gamma, eps=eps, counters=tiles if splits > 1 else 0, ws_floats=tiles * splits * columns * 128 if splits > 1 else 0)
     y = torch.empty(M, N // 2 if epi == 1 else N, device=x.device, dtype=torch.float32 if epi == 2 else torch.bfloat16)
     _umma(st, w_raw, type_name, N, K, None, 1, epi, y, 0.0, columns, splits, splits, status)
@@ -178,7 +183,6 @@ def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, 
     seg, tok, _ = routes
     H, R, dev = x.shape[1], tok.numel(), x.device
     seg = seg[expert_offset:]
-    slots = _sm_count()      # a CTA per SM
 
     def columns(t: int) -> int:      # of an expert's tile: what most experts with routes need
         n = t * R / E      # a rank's experts see their share of the routes: the same tiles however the experts are split
@@ -188,6 +192,7 @@ def _umma_experts(x: torch.Tensor, w13_raw: torch.Tensor, w2_raw: torch.Tensor, 
         c, row_tiles = columns(t), -(-(N // 2) // 64) if epi == 3 else -(-N // 128)
         most = max(1, min(R, local)) * row_tiles        # tiles, if every route is an expert of its own
         parts = splits = 1
+        slots = _umma_slots(type_name, c)
         if c == 16:
             # K is cut as for one token's routes whatever the step holds and however the experts are split over ranks: a token's sum does
             # not depend on the tokens beside it. CTAs of their own take the parts where that fills the SMs better.

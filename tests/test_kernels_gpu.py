@@ -294,8 +294,34 @@ def test_gemm_fp8_stream_k_and_many_tiles(M, N, K, epi):
     assert _rel_err(c2, planes @ wd2.t()) < 6e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 5120, 1024), (200, 2304, 3072)])
+def test_stream_k_on_several_streams_and_under_capture(M, N, K):
+    """Tiles whose K is shared: launches on more streams than there are work spaces, and replays of a captured launch with new rows."""
+    from pocketllm_b200 import ops
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    xs = [torch.randn(M, K, device="cuda").to(torch.bfloat16) for _ in range(10)]
+    want = [x.float() @ w.float().t() for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = []
+    for x, st in zip(xs, streams):
+        with torch.cuda.stream(st):
+            got.append([ops.gemm_bf16(x, w) for _ in range(3)])
+    torch.cuda.synchronize()
+    for g, r in zip(got, want):
+        assert all(_rel_err(y, r) < 6e-3 for y in g) and torch.equal(g[0], g[1]) and torch.equal(g[1], g[2])
+    x = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ops.gemm_bf16(x, w)
+    for new, r in zip(xs, want):
+        x.copy_(new)
+        graph.replay()
+        assert _rel_err(y, r) < 6e-3
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 5120, 4096), (200, 2304, 4352)])
-def test_stream_k_on_several_streams_and_under_capture(M, N, K, monkeypatch):
+def test_stream_k_replays_are_whole_tiles(M, N, K, monkeypatch):
     """Tiles whose K is shared: launches on more streams than there are work spaces, and replays of a captured launch with new rows, which
     is the schedule of whole tiles to the bit."""
     from pocketllm_b200 import ops
@@ -498,11 +524,22 @@ def test_deltanet_chunked_matches_serial_recurrence(Hk, Hv, T):
     S3, cs3 = S.clone(), conv_state.clone()
     out3 = ops.deltanet_seq(proj, Hk, Hv, conv_w, cs3, A_log, dt_bias, norm_w, 1e-6, S3)
     assert _rel_err(out, out3) < 1e-2 and _rel_err(S2, S3) < 2e-3
-    # a state that begins on any float
-    for off in (1, 2, 3):
-        S4, cs4 = torch.cat((S.new_zeros(off), S.flatten(), S.new_zeros(1))), conv_state.clone()
-        out4 = ops.deltanet_chunked(proj, Hk, Hv, conv_w, cs4, A_log, dt_bias, norm_w, 1e-6, S4[off:-1].view_as(S))
-        assert torch.equal(out4, out) and torch.equal(S4[off:-1].view_as(S), S2) and S4[0] == 0 and S4[-1] == 0
+
+
+@pytest.mark.parametrize("off", [1, 2, 3])
+def test_deltanet_chunks_with_a_state_on_any_float(off):
+    from pocketllm_b200 import ops
+    torch.manual_seed(off)
+    Hk, Hv, T = 1, 2, 100
+    KD, VD = Hk * 128, Hv * 128
+    proj = torch.randn(T, (2 * KD + 2 * VD + 2 * Hv + 7) // 8 * 8, device="cuda").to(torch.bfloat16)
+    conv_w, conv_state = torch.randn(2 * KD + VD, 4, device="cuda") * 0.3, torch.randn(2 * KD + VD, 3, device="cuda")
+    A_log, dt_bias, norm_w = torch.randn(Hv, device="cuda") * 0.5, torch.randn(Hv, device="cuda") * 0.5, 1 + torch.randn(128, device="cuda") * 0.05
+    S = torch.randn(Hv, 128, 128, device="cuda") * 0.1
+    S2 = torch.cat((S.new_zeros(off), S.flatten(), S.new_zeros(1)))
+    got = ops.deltanet_chunked(proj, Hk, Hv, conv_w, conv_state.clone(), A_log, dt_bias, norm_w, 1e-6, S2[off:-1].view_as(S))
+    want = ops.deltanet_chunked(proj, Hk, Hv, conv_w, conv_state.clone(), A_log, dt_bias, norm_w, 1e-6, S)
+    assert torch.equal(got, want) and torch.equal(S2[off:-1].view_as(S), S) and S2[0] == 0 and S2[-1] == 0
 
 
 @pytest.mark.parametrize("M,ctx,Hq,Hkv,nsplit", [(1, 1, 4, 2, 4), (1, 700, 10, 2, 8), (5, 300, 5, 1, 3), (8, 64, 8, 8, 2)])

@@ -162,10 +162,40 @@ def test_experts(t13, t2, T, E, topk, limit):
         assert _rel(go.gguf_moe_forward_grouped(x, raw13, raw2, t13, t2, E, I, routes), want) < 5e-4
 
 
+@pytest.mark.parametrize("t13,t2,E,topk,H,I", [("iq2_xxs", "iq2_xxs", 64, 8, 1536, 768), ("q4_k", "q5_k", 16, 2, 2048, 1280), ("iq2_xxs", "q4_k", 40, 3, 3072, 512)])
+def test_a_token_gives_the_same_bits_in_any_company(t13, t2, E, topk, H, I):
+    """One token alone (K in parts over CTAs) and the same token among others (all parts in one CTA), up to the four routes per expert
+    from which prompts take the grouped form."""
+    from pocketllm_b200.ops import gguf_ops as go
+    def raw(name, rows, K, seed):        # any payload, scale fields 2^-11
+        n = {"iq2_xxs": 66, "q4_k": 144, "q5_k": 176}[name]
+        b = torch.randint(0, 256, (rows * K // 256, n), dtype=torch.uint8, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+        b[:, :2 if name == "iq2_xxs" else 4] = torch.tensor([0, 0x10] * (1 if name == "iq2_xxs" else 2), dtype=torch.uint8)
+        return b.view(-1)
+
+    raw13, raw2 = raw(t13, E * 2 * I, H, 1), raw(t2, E * H, I, 2)
+    g = torch.Generator().manual_seed(0)
+    T = 4 * E // topk
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(E, generator=g)[:topk] for _ in range(T)]).int().cuda()
+    weight = torch.rand(T, topk, generator=g).cuda()
+    assert go._umma_splits(topk * (2 * I // 128), H, go._umma_slots(t13, 16)) > 1
+
+    def run(n, **k):
+        routes = go.group_routes(ids[:n].contiguous(), weight[:n].contiguous(), E)
+        return go.gguf_moe_forward(x[:n].contiguous(), k.pop("a", raw13), k.pop("b", raw2), t13, t2, E, I, *routes, routes=routes, **k)
+
+    half, n13, n2 = E // 2, raw13.numel() // 2, raw2.numel() // 2
+    for kw in ({}, dict(a=raw13[n13:].clone(), b=raw2[n2:].clone(), expert_offset=half, local_experts=half)):
+        alone = run(1, **kw)
+        for n in (2, 3, 5, 8, 17, T):
+            assert torch.equal(run(n, **kw)[:1], alone), n
+
+
 @pytest.mark.parametrize("t13,t2,E,topk,H,I,cut", [("iq2_xxs", "iq2_xxs", 64, 8, 1536, 768, (False, False)), ("iq2_xxs", "iq2_xxs", 64, 2, 4096, 1024, (True, False)),
                                                    ("iq2_xxs", "iq2_xxs", 64, 2, 1024, 3072, (False, True)),
                                                    ("q4_k", "q5_k", 16, 2, 2048, 1280, (True, False)), ("iq2_xxs", "q4_k", 40, 3, 3072, 512, (True, False))])
-def test_a_token_gives_the_same_bits_in_any_company(t13, t2, E, topk, H, I, cut, monkeypatch):
+def test_a_token_in_any_company_and_the_parts_of_its_products(t13, t2, E, topk, H, I, cut, monkeypatch):
     """One token alone (K in parts over CTAs) and the same token among others (all parts in one CTA), up to the four routes per expert
     from which prompts take the grouped form."""
     from pocketllm_b200.ops import gguf_ops as go
