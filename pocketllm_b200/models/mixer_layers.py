@@ -100,7 +100,7 @@ class FusedLinear:
         out = ctx.ws.rows(name, x.shape[0], self.N, dtype)
         if self.split:
             return mo.linear2(beside, x, self.split, self.w, out, ctx.status)
-        return mo.linear(x, self.w, out, ctx.status)
+        return mo.linear(x, self.w, out, ctx.status, held=True)
 
 
 def _f32(t: torch.Tensor, device) -> torch.Tensor:
@@ -434,7 +434,7 @@ class LatentAttentionMixer:
             c = ws.rows("lat_rows", total, self.row, torch.bfloat16)
             mo.latent_gather(self.cache, ctx.table, ctx.long, gather, ctx.n_long, longest, c)
             kv = ws.rows("lat_kv", total, self.kv_w.shape[0], torch.bfloat16)
-            mo.linear(c, self.kv_w, kv, ctx.status)
+            mo.linear(c, self.kv_w, kv, ctx.status, held=True)
             mo.latent_prefill(qf, T, kv, total, ctx.tiles, ctx.n_tiles, ctx.long, gather, H, self.qk_panels, self.v_panels, V, self.window, self.scale,
                               self.sink, mix, ctx.status, gate)
         if nrows:
@@ -621,7 +621,7 @@ class SwiGLU:
 
     def forward(self, ctx: StepContext, h: torch.Tensor) -> dict:
         mid = ctx.ws.rows("mid" + self.name, ctx.T, self.ff, self.dtype)
-        mo.linear(h, self.gate_up, mid, ctx.status, swiglu=True)
+        mo.linear(h, self.gate_up, mid, ctx.status, swiglu=True, held=True)
         return {"y": self.down(ctx, mid, "y" + self.name, torch.float32)}
 
 

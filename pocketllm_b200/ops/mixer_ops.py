@@ -65,7 +65,7 @@ def sm_count() -> int:
 
 # argument kinds of the launchers, the stream excepted: p pointer, i int, f float
 _SIGNATURES = {
-    "pk_linear_f32": "pipiiiipi", "pk_linear_rows": "pipiiiipii", "pk_linear_rows2": "ppiipiiiipii", "pk_gemm_bf16_held": "pipiiiippippi",
+    "pk_linear_f32": "pipiiiipi", "pk_linear_rows": "pipiiiipii", "pk_linear_rows2": "ppiipiiiipii", "pk_gemm_bf16": "pipiiiippippi", "pk_gemm_bf16_held": "pipiiiippippi",
     "pk_sandwich_norm": "pppifipipifpiippp" "iipifpii", "pk_feed_tokens": "pipppp" "ip", "pk_post_norm": "p", "pk_argmax": "piiiiipppp",
     "pk_state_rows": "ppi", "pk_state_chunks": "ppippip", "pk_state_out": "ppifpipii", "pk_ssd_out": "ppifpppipiii", "pk_ssd_tiles": "ppippipp", "pk_ssd_rows": "ppii",
     "pk_scan_conv": "pi", "pk_scan_split": "piiiip", "pk_scan_rows": "ppi", "pk_scan_tiles": "ppi",
@@ -96,10 +96,11 @@ def _call(name: str, *args) -> None:
         _check(st, name)
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, *, swiglu: bool = False) -> torch.Tensor:
+def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, *, swiglu: bool = False, held: bool = False) -> torch.Tensor:
     """out[M, :] = x[M, K] w[N, K]^T. fp32 x: fp32 arithmetic. bf16 x: weight streaming up to eight rows, the tcgen05 GEMM
-    beyond (K a multiple of 64); `out` bf16 or fp32. `swiglu`: w holds gate rows, then as many up rows. bf16: `w` is a weight that the
-    program holds, not the result of a launch still under way; its first rows are read while the launch before this one ends."""
+    beyond (K a multiple of 64); `out` bf16 or fp32. `swiglu`: w holds gate rows, then as many up rows. `held`: `w` is a weight
+    that the program holds, not the result of a launch that may be under way, so that its first tiles are read while the launch before this one ends (up to
+    eight bf16 rows its first rows are in any case)."""
     M, K = x.shape
     N = w.shape[0]
     if x.dtype == torch.float32:
@@ -111,7 +112,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Te
         _call("pk_linear_rows", x, x.stride(0), w, M, N, K, epi, out, out.stride(0), sm_count())
     else:
         epi = EPI_SWIGLU if swiglu else EPI_F32 if f32 else EPI_BF16
-        _call("pk_gemm_bf16_held", x, x.stride(0), w, M, N, K, epi, out, None, out.stride(0), status, None, sm_count())
+        _call("pk_gemm_bf16_held" if held else "pk_gemm_bf16", x, x.stride(0), w, M, N, K, epi, out, None, out.stride(0), status, None, sm_count())
     return out
 
 

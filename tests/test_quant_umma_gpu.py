@@ -414,3 +414,22 @@ def test_product_behind_the_decode_of_its_weight(name, M, N, K):
         y = go.gguf_linear(x, raw, name, N, epi=2, status=status)
         assert _rel(y.view(want.shape), want) < 2 ** -8
     assert status.item() == 0
+
+
+def test_mixer_linear_behind_the_launch_that_makes_its_weight():
+    """More than eight rows times a weight that the launch directly before writes over NaN."""
+    from pocketllm_b200.ops import gguf_ops as go, mixer_ops as mo
+    M, N, K = 20, 32768, 3072
+    raw, w = _raw("q8_0", 32, K, 5)
+    raw = raw.repeat(N // 32)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    want = (x.double() @ w.T)[:, None].expand(-1, N // 32, -1)
+    y, status = torch.empty(M, N, device="cuda"), torch.zeros(1, device="cuda", dtype=torch.int32)
+    scratch = go._dequant_scratch(raw, "q8_0", N, K)
+    for _ in range(10):
+        scratch.fill_(float("nan"))
+        y.zero_()
+        assert go._dequant_scratch(raw, "q8_0", N, K).data_ptr() == scratch.data_ptr()
+        mo.linear(x, scratch, y, status)
+        assert _rel(y.view(want.shape), want) < 2 ** -8
+    assert status.item() == 0
